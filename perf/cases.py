@@ -262,7 +262,10 @@ def prepare(case, seed):
 
 
 def _field(s):
-    return s["g"].field_tensor()[:, :, :s["case"]["nt"]]
+    """The handle's own field: a view, which keeps the handle alive."""
+    f = s["g"].field_tensor()[:, :, :s["case"]["nt"]]
+    f.handle = s["g"]
+    return f
 
 
 def run(s):
