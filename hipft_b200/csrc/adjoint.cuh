@@ -12,7 +12,7 @@
 #pragma once
 
 #include "kernels.cuh"
-#include "sts_pair_ws.cuh"  // PairTables (coefficient tables of k_pair_tables)
+#include "sts_march.cuh"  // PairTables (coefficient tables of k_pair_tables)
 
 namespace hipft {
 

@@ -7,7 +7,7 @@
 // stage count follow (src/hipft.f90:4551-4695, 5361-5475).  Here those
 // decisions are made by one-block "schedule" kernels that leave their results
 // in device memory, and the loops whose trip counts they decide (subcycles,
-// stage pairs, advection substeps) are conditional WHILE nodes of the graph,
+// passes, advection substeps) are conditional WHILE nodes of the graph,
 // continued or ended by cudaGraphSetConditional from the kernel that closes
 // each iteration.  The arithmetic of every decision is the host path's (same
 // expressions, same order), so a graph-run step and a host-driven step give
@@ -18,7 +18,7 @@
 
 namespace hipft {
 
-constexpr int kGUnrollMax = 16;      // most stage pairs per iteration of the pair loop (an even number: buffer roles repeat)
+constexpr int kGUnrollMax = 8;       // most passes per iteration of the pass loop (an even number: buffer roles repeat)
 constexpr int kGMaxCycles = 60;      // max_sc of diffusion_step (src/hipft.f90:4565)
 constexpr int kGAdvLimit = 100000;   // advection substeps after which the loop stops and reports an error
 constexpr int kGSubLimit = 1000;     // subcycles likewise (PTL forces the last one at kGMaxCycles - 1)
@@ -29,8 +29,8 @@ struct GState {
   double dt;                // the split step
   int cyc;                  // diffusion subcycle (1-based)
   int nact;                 // realizations still subcycling
-  int npairs;               // stage pairs of the longest super-step of this subcycle
-  int pctr;                 // first stage pair of the current pair-loop iteration
+  int npasses;              // passes of the longest super-step of this subcycle
+  int pctr;                 // first pass of the current pass-loop iteration
   int nsub;                 // advection substeps of the slowest realization
   int qctr;                 // current advection substep
   int err;                  // 1: a table was too small, 2: a loop hit its iteration limit
@@ -42,7 +42,7 @@ struct GState {
   long long kernels;        // kernels the step ran
 };
 
-// Per-realization and per-pair arrays of the schedule, and the mode.
+// Per-realization and per-pass arrays of the schedule, and the mode.
 struct GArrays {
   GState *st;
   double *ts, *d;                 // [nr] time subcycled so far, current subcycle length
@@ -54,15 +54,14 @@ struct GArrays {
   int *rl_dif;                    // [nr] active realizations by stage count (descending), -1 after the last
   int *rl_adv, *rl_adv_all;       // [nr] realizations of the current advection substep (-1 padded), all by substeps
   int *nsub_i, *cycles_i;         // [nr] advection substeps, subcycles run
-  int *nactp;                     // [paircap] realizations taking part in stage pair p
+  int *nactp, *colsp;             // [passcap] realizations taking part in pass p, its columns per warp
   long long *s_i, *s_last;        // [nr] stage count of the current / last super-step
-  StageCoef *c1;                  // [nr] stage-1 coefficients
-  StageCoef *rc;                  // [paircap][nr][2] stage-pair coefficients
+  StageCoef *rc;                  // [passcap][nr][kMS] stage coefficients
   unsigned long long *bits;       // PTL reductions: [2 nr] ragged, [2] plain
-  double *ring0, *ring1;          // diffusion ring sums of stage inputs / outputs
-  int nr, paircap;
+  int nr, passcap;
   int method, auto_sc, subcycles, ragged, strang, nadv;  // nadv: advection stages per substep
-  int unroll;                     // stage pairs per pair-loop iteration (even)
+  int n2, strips, slots, poles;   // march_cols' arguments
+  int unroll;                     // passes per pass-loop iteration (even)
 };
 
 __device__ __forceinline__ double bits_to_double(unsigned long long b) { return __longlong_as_double((long long)b); }
@@ -189,10 +188,10 @@ __global__ void k_g_ptl_reset(GArrays g) {
 // One subcycle's schedule (one block): each active realization's subcycle
 // length from its PTL limit or the fixed count (the decisions of
 // hipft_gpu_diffusion_step / ragged_diffusion_step in their order), its stage
-// count and stage-1 coefficients, the realizations sorted by stage count, and
-// how many take part in each stage pair.  Plain mode reads one shared PTL
+// count, the realizations sorted by stage count, and how many take part in
+// each pass.  Plain mode reads one shared PTL
 // limit and one Euler limit, so every realization gets the same schedule.
-__global__ void __launch_bounds__(256) k_g_plan(GArrays g, cudaGraphConditionalHandle hpair) {
+__global__ void __launch_bounds__(256) k_g_plan(GArrays g, cudaGraphConditionalHandle hpass) {
   GState &st = *g.st;
   const int nr = g.nr, tid = threadIdx.x;
   const double dtl = st.dt;
@@ -238,11 +237,8 @@ __global__ void __launch_bounds__(256) k_g_plan(GArrays g, cudaGraphConditionalH
     g.s_i[i] = s;
     g.s_last[i] = s;
     g.cycles_i[i] = cyc;
-    double uj, vj, ubj, gj;
-    sts_stage(g.method, s, 1, uj, vj, ubj, gj);
-    g.c1[i] = StageCoef{d, ubj, 0.0, 0.0, 0.0};
     atomicAdd(&s_na, 1);
-    atomicMax(&s_pmax, (int)((s - 1) / 2));
+    atomicMax(&s_pmax, (int)sts_passes(s));
     atomicAdd((unsigned long long *)&s_ssum, (unsigned long long)s);
     atomicMax((unsigned long long *)&s_smax, (unsigned long long)s);
   }
@@ -253,15 +249,16 @@ __global__ void __launch_bounds__(256) k_g_plan(GArrays g, cudaGraphConditionalH
   const int na = s_na;
   for (int e = na + tid; e < nr; e += blockDim.x) g.rl_dif[e] = -1;
   int np = s_pmax;
-  const bool fits = np + g.unroll <= g.paircap;
+  const bool fits = np + g.unroll <= g.passcap;
   if (!fits) np = 0;
   for (int p = tid; p < np + g.unroll; p += blockDim.x) {
     int c = 0;
-    for (int e = 0; e < na; ++e) c += ((g.s_i[g.rl_dif[e]] - 1) / 2 > p) ? 1 : 0;
+    for (int e = 0; e < na; ++e) c += (sts_passes(g.s_i[g.rl_dif[e]]) > p) ? 1 : 0;
     g.nactp[p] = c;
+    g.colsp[p] = march_cols(g.n2, g.strips, c, g.slots, g.poles);
   }
   if (tid == 0) {
-    st.npairs = np;
+    st.npasses = np;
     st.pctr = 0;
     if (!fits) st.err = 1;
     st.stage_sum += s_ssum;
@@ -269,55 +266,51 @@ __global__ void __launch_bounds__(256) k_g_plan(GArrays g, cudaGraphConditionalH
     if (s_smax > st.smax) st.smax = s_smax;
     st.cycles = cyc;
     st.kernels += 1;
-    cudaGraphSetConditional(hpair, np > 0 ? 1u : 0u);
+    cudaGraphSetConditional(hpass, np > 0 ? 1u : 0u);
   }
 }
 
-// Stage-pair coefficients of the subcycle (src/hipft.f90:5224-5235): entry
-// (p, i) holds stages 2p+2 and 2p+3 of realization i.  Grid over paircap x nr.
+// Stage coefficients of the subcycle's passes (src/hipft.f90:5211-5235).
+// Grid over passcap x nr.
 __global__ void k_g_coefs(GArrays g) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx == 0) g.st->kernels += 1;
   const int nr = g.nr;
   const int p = (int)(idx / nr), i = (int)(idx % nr);
-  if (p >= g.st->npairs || !g.act[i]) return;
+  if (p >= g.st->npasses || !g.act[i]) return;
   const long long s = g.s_i[i];
-  if (p >= (s - 1) / 2) return;
-  const long long k = 2 + 2 * (long long)p;
-  g.rc[idx * 2] = sts_combine(g.method, s, k, g.d[i]);
-  g.rc[idx * 2 + 1] = sts_combine(g.method, s, k + 1, g.d[i]);
+  if (p >= sts_passes(s)) return;
+  for (int q = 0; q < kMS; ++q) g.rc[idx * kMS + q] = sts_slot(g.method, s, (int64_t)kMS * p + q, g.d[i]);
 }
 
-// End of a pair-loop iteration (one thread).
-__global__ void k_g_pair_tick(GArrays g, cudaGraphConditionalHandle hc) {
+// End of a pass-loop iteration (one thread; pass_kernels: kernels of a pass).
+__global__ void k_g_pass_tick(GArrays g, int pass_kernels, cudaGraphConditionalHandle hc) {
   GState &st = *g.st;
   const int p = st.pctr + g.unroll;
   st.pctr = p;
-  st.kernels += 2 * g.unroll + 1;
-  // npairs fits the tables (k_g_plan), so the loop ends within paircap / unroll iterations
-  cudaGraphSetConditional(hc, p < st.npairs ? 1u : 0u);
+  st.kernels += pass_kernels * g.unroll + 1;
+  // npasses fits the tables (k_g_plan), so the loop ends within passcap / unroll iterations
+  cudaGraphSetConditional(hc, p < st.npasses ? 1u : 0u);
 }
 
-// After the pair loop: each realization of the super-step has Y_s in y_even
-// (its last pair had an even index) or y_odd; the plane goes back into the
-// field buffer.  In plain mode the ring sums of Y_s move to ring0 as well
-// (the host path reuses the fused kernels' ring sums in the next subcycle;
-// ragged batches recompute them).  Grid (nr, chunks).
+// After the pass loop: each realization of the super-step has Y_s in y_even
+// (its last pass had an even index) or y_odd; the plane goes back into the
+// field buffer, with its seam columns (which the passes do not write).  Grid
+// (nr, chunks).
 __global__ void k_g_gather(GArrays g, Mesh m, double *f, const double *__restrict__ y_even,
                            const double *__restrict__ y_odd) {
   const int i = blockIdx.x;
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) g.st->kernels += 1;
   if (!g.act[i]) return;
-  const long long P = (g.s_i[i] - 1) / 2;
-  const bool odd = ((P - 1) & 1) != 0;
+  const bool odd = ((sts_passes(g.s_i[i]) - 1) & 1) != 0;
   const double *src = (odd ? y_odd : y_even) + (int64_t)i * m.plane;
   double *dst = f + (int64_t)i * m.plane;
-  const int64_t n2 = m.plane / 2;
-  const double2 *s2 = reinterpret_cast<const double2 *>(src);
-  double2 *d2 = reinterpret_cast<double2 *>(dst);
-  for (int64_t e = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; e < n2; e += (int64_t)gridDim.y * blockDim.x)
-    d2[e] = s2[e];
-  if (!g.ragged && odd && blockIdx.y == 0 && threadIdx.x < 2) g.ring0[2 * i + threadIdx.x] = g.ring1[2 * i + threadIdx.x];
+  for (int c = blockIdx.y; c < m.npm; c += gridDim.y) {
+    const int cs = c == 0 ? m.npm - 2 : c == m.npm - 1 ? 1 : c;
+    const double2 *s2 = reinterpret_cast<const double2 *>(src + (int64_t)cs * m.ldt);
+    double2 *d2 = reinterpret_cast<double2 *>(dst + (int64_t)c * m.ldt);
+    for (int e = threadIdx.x; e < m.ldt / 2; e += blockDim.x) d2[e] = s2[e];
+  }
 }
 
 // dst = src over whole fields (n doubles, n even; 16-byte aligned).

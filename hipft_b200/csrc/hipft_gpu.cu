@@ -3,7 +3,6 @@
 // sequences the kernels of kernels.cuh the way HipFT's Fortran routines
 // sequence their do-concurrent loops (src/hipft.f90).
 #include <cuda_runtime.h>
-#include <cudaTypedefs.h>  // PFN_cuTensorMapEncodeTiled
 
 #include <algorithm>
 #include <array>
@@ -20,8 +19,7 @@
 
 #include "../../include/hipft_gpu.h"
 #include "kernels.cuh"
-#include "sts_pair_ws.cuh"
-#include "sts_quad_ws.cuh"
+#include "sts_march.cuh"
 #include "adjoint.cuh"
 #include "graph_step.cuh"
 
@@ -46,18 +44,9 @@ constexpr double c_sixth = 0.16666666666666666;
 constexpr double c_two_third = 0.66666666666666666;
 constexpr double c_third = 0.33333333333333333;
 
-constexpr int kNBuf = 8;  // current field + scratch: u0, dty0, two inputs and up to four outputs of a pass
+constexpr int kNBuf = 6;  // current field + scratch: u0, dty0, two inputs and two outputs of a pass
 
 int round_up(int a, int b) { return (a + b - 1) / b * b; }
-
-// Two-stage kernel kinds (see the autotuner) and the plan a handle uses.
-enum { PK_SINGLE = 0, PK_WS_ROWS1 = 4, PK_WS_ROWS2 = 5, PK_WS_BULK = 6, PK_WS_QUAD = 7 };
-struct PairPlan {
-  int kind = -1;    // PK_*; -1: not chosen yet
-  int ctas_per_sm = 2;
-  double ms = 0.0;  // timed ms per launch pair (0: not timed)
-  int candidates = 0;
-};
 
 double pow3(double c) { return c * c * c; }
 double pow5(double c) { return c * c * c * c * c; }
@@ -69,10 +58,9 @@ namespace {
 // One RKG2 super-step of the replay.  With q == 0 the tape holds every stage:
 // slots t0 = u0, t0+1 = dty0, t0+1+k = Y_k (k = 1..s-1).  With stage
 // checkpoints (q > 0, even) it holds u0, dty0 and, for each block start
-// c = 1, 1+q, 1+2q, ... (odd, the output of a stage pair), the pair
-// (Y_{c-1}, Y_c) in slots t0+2+2b, t0+3+2b (b = block index; Y_0 = u0 is
-// not stored twice) and the pole-ring sums of Y_c; the reverse pass
-// recomputes the stages of one block at a time from its pair.
+// c = 1, 1+q, 1+2q, ..., the pair (Y_{c-1}, Y_c) (b = block index; Y_0 = u0 is
+// not stored twice); the reverse pass recomputes the stages of one block at a
+// time from its pair.
 struct AdjSub {
   double dtl;
   int64_t s;
@@ -81,14 +69,13 @@ struct AdjSub {
   int64_t q = 0;
   std::vector<int64_t> cstart;        // block starts c
   std::vector<size_t> ck_prev, ck_cur;  // tape slots of Y_{c-1} (SIZE_MAX: u0) and Y_c
-  size_t ring0 = 0;                   // first ring-checkpoint slot (2*nr doubles each)
 };
 
 // One taped (recorded) flux_transport_step: its tape slots sit on the tape's
-// stack from `first`, its ring checkpoints from `ring_first`.
+// stack from `first`.
 struct AdjRec {
   double dt = 0.0;
-  size_t first = 0, ring_first = 0;
+  size_t first = 0;
   size_t ta1[4] = {}, ta2[4] = {};  // SSPRK(4,3) stage inputs of the advection calls
   std::vector<AdjSub> subs;         // RKG2 super-steps
 };
@@ -115,7 +102,7 @@ struct hipft_gpu {
   double bc_flow_n = 0, bc_flow_s = 0, bc_diff_n = 0, bc_diff_s = 0;
   // fields
   double *buf[kNBuf] = {};
-  int nbuf = 6;             // allocated fields (8 once the four-stage path is in use)
+  int nbuf = kNBuf;         // allocated fields
   int cur = 0;
   bool field_set = false;
   // flows
@@ -141,17 +128,9 @@ struct hipft_gpu {
   double *d_rpart = nullptr;
   unsigned int *d_rcount = nullptr;
   int nkb = 0;
-  PairTables ptab{};        // coefficient tables of the warp-specialised two-stage kernel
-  PairPlan plan{};          // two-stage kernel chosen for this grid (autotuner)
-  std::unordered_map<uint64_t, CUtensorMap> ws_map_cache;  // tensor maps of field buffers, by (pointer, box)
-  CUtensorMap ws_rt_map{};               // tensor map of ptab.row
-  bool ws_rt_ok = false;
-  // four stages per pass on the interior theta blocks
-  int q_rb_lo = 0, q_rb_hi = -1;         // interior blocks (none when q_rb_hi < q_rb_lo)
-  double *d_qcol = nullptr;              // column table of the quad tiles
-  int q_LC = 0, q_nkt = 0;
-  CUtensorMap q_rt_map{};
-  bool q_rt_ok = false;
+  PairTables ptab{};        // coefficient tables of the RKG2/RKL2 passes
+  int m_strips = 0, m_slots = 0;         // theta strips, resident warps of k_sts_march
+  double *d_pscratch = nullptr;          // strips of k_sts_poles_any
   // adjoint: fields of one taped forward step, folded work fields (seam
   // columns stay zero), per-block partial sums and pole sums
   std::vector<double *> tape;             // tape slots (allocated in chunks, see adj_slot)
@@ -160,8 +139,6 @@ struct hipft_gpu {
   size_t adj_top_max = 0;                 // most tape slots in use at once since the last release
   std::vector<AdjRec> adj_recs;           // recorded steps, oldest first
   std::vector<double *> adj_block;        // stage fields of one recomputed block
-  double *d_adj_rings = nullptr;          // ring sums of the stage checkpoints
-  size_t adj_rings_cap = 0, adj_rings_n = 0;
   int64_t adj_tape_limit = 0;             // fields the tape may use (0: half the free memory)
   int64_t adj_force_q = 0;                // stage-checkpoint spacing forced by the caller (0: automatic)
   size_t adj_free_seen = 0;               // free device memory + 1 as seen at the run's first record (0: not yet)
@@ -176,9 +153,9 @@ struct hipft_gpu {
   std::vector<double> r_dt_euler, r_dtmax;
   bool r_dtmax_valid = false;
   int *d_rlist_dif = nullptr, *d_rlist_adv = nullptr;  // [nr] realization lists of the launches
-  StageCoef *d_rcoef = nullptr;                         // [pairs][nr][2] coefficients of a super-step
-  size_t rcoef_pairs = 0;
-  StageCoef *d_r1coef = nullptr;                        // [nr] stage-1 coefficients
+  StageCoef *d_rcoef = nullptr;                         // [passes][nr][4] coefficients of a super-step
+  size_t rcoef_passes = 0;
+  double *d_rlen = nullptr;                             // [nr] super-step lengths
   double *d_rdt = nullptr;                              // [nr] advection substeps
   unsigned long long *d_rbits = nullptr;                // [2*nr] per-realization reductions
   std::vector<int64_t> r_s, r_cycles, r_substeps;       // the last step's schedule
@@ -190,15 +167,12 @@ struct hipft_gpu {
   cudaStream_t g_side[3] = {};      // streams the step (and its loop bodies) are captured on
   GArrays GA{};                     // device schedule arrays
   int g_cur = -1;                   // buffer the capture used as the field
-  int g_paircap = 0;                // stage pairs the coefficient tables hold
-  bool g_pdl = true;                // programmatic launches inside the captured pair loop
+  bool g_pdl = true;                // programmatic launches inside the captured pass loop
   std::vector<unsigned char> g_key; // launch parameters the capture baked in
   GState g_last{};                  // statistics of the last graph-run step
   bool g_stats_valid = true;        // g_last read back since the last launch
   hipft_allreduce_cb red_cb = nullptr;  // scalar all-reduce over ranks (plain-mode sharding)
   void *red_user = nullptr;
-  PoleScratch pole{};       // chunk shares of the ring sums for k_pair_poles
-  int pole_nch = 0;
   int *d_err = nullptr;   // set by kernels whose bounded waits gave up
   int num_sms = 148;
   unsigned long long *d_bits = nullptr;
@@ -458,32 +432,28 @@ static int current_dring(hipft_gpu *h, const double **ring) {
   return HIPFT_OK;
 }
 
-constexpr int kKPT3 = 4;  // phi columns per thread of the fused single-stage kernel (two rows per thread)
+constexpr int kKPT3 = 4;  // phi columns per thread of the explicit Euler kernel (two rows per thread)
 
-// One fused RKG2/RKL2 (or Euler) stage, k_sts_stage_v3; leaves the ring sums
-// of its output for the next stage.
-template <int MODE>
-static int sts_stage_v2(hipft_gpu *h, const double *x, const double *ykm2, const double *u0, const double *dty0,
-                        double *out, double *out2, StageCoef sc) {
+// One explicit Euler step, k_euler_step; leaves the ring sums of its output
+// for the next.
+static int euler_step(hipft_gpu *h, const double *x, double *out, double dte) {
   const int nkb = (h->npm - 2 + kKPT3 - 1) / kKPT3;
   RingOut ro{h->d_ringbuf[1 - h->ring_cur], h->d_rpart, h->d_rcount, nkb};
   {
-    ProfScope ps(h, MODE == MODE_STSK ? HIPFT_K_STS : HIPFT_K_OTHER);
+    ProfScope ps(h, HIPFT_K_OTHER);
     // odd ntm: keep the thread owning row ntm off lane 0 (row ntm-1 is its left neighbour)
     const int jshift = (h->ntm % 2 == 1 && ((h->ntm - 1) / 2) % 32 == 0) ? 1 : 0;
     const int nthr = (h->ntm + 2 * jshift + 1) / 2;
     dim3 grd((unsigned)((nthr + 127) / 128), (unsigned)nkb, (unsigned)h->nr);
-    k_sts_stage_v3<MODE, kKPT3><<<grd, 128, 0, h->stream>>>(h->M, h->DC.dfac, x, ykm2, u0, dty0, out, out2,
-                                                           h->d_ringbuf[h->ring_cur], h->bc_diff_n, h->bc_diff_s, sc,
-                                                           ro, jshift);
+    k_euler_step<kKPT3><<<grd, 128, 0, h->stream>>>(h->M, h->DC.dfac, x, out, h->d_ringbuf[h->ring_cur],
+                                                    h->bc_diff_n, h->bc_diff_s, dte, ro, jshift);
     LAUNCHED(h);
   }
   h->ring_cur = 1 - h->ring_cur;  // the output's ring is now current
   return HIPFT_OK;
 }
 
-// HIPFT_PDL=0 turns off the programmatic (overlapping) launch of the
-// two-stage kernel after the previous pair's pole-row kernel.
+// HIPFT_PDL=0 turns off the programmatic (overlapping) launches.
 static bool ws_pdl() {
   static int v = -1;
   if (v < 0) {
@@ -493,420 +463,112 @@ static bool ws_pdl() {
   return v == 1;
 }
 
-// HIPFT_WS_TMAP=0 turns off the tensor-map tile loads of k_sts_pair_ws (one
-// bulk copy per column on every tile instead).
-static bool ws_tmap_enabled() {
-  static int v = -1;
-  if (v < 0) {
-    const char *e = std::getenv("HIPFT_WS_TMAP");
-    v = (e && std::atoi(e) == 0) ? 0 : 1;
-  }
-  return v == 1;
-}
-
-// cuTensorMapEncodeTiled from the driver, through the runtime (no libcuda link)
-static PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q{};
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-  }
-  return fn;
-}
-
-// 3-D f64 tensor map (dims d0 x d1 x d2, byte strides s1, s2 of dims 1, 2),
-// box b0 x b1 x 1, no swizzle, zero fill outside; false if the driver refuses
-// (e.g. a base address or stride that is not a multiple of 16 bytes)
-static bool encode_f64_3d(CUtensorMap *m, const void *base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1,
-                          uint64_t s2, uint32_t b0, uint32_t b1) {
-  PFN_cuTensorMapEncodeTiled_v12000 fn = tmap_encoder();
-  if (!fn) return false;
-  cuuint64_t dims[3] = {d0, d1, d2};
-  cuuint64_t strides[2] = {s1, s2};
-  cuuint32_t box[3] = {b0, b1, 1};
-  cuuint32_t es[3] = {1, 1, 1};
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<void *>(base), dims, strides, box, es,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// a field buffer's map with a box of rows x cols (cached)
-static bool field_map(hipft_gpu *h, const double *p, int cols, CUtensorMap *out, int rows = kWR) {
-  // key: the address (user-space pointers fit 48 bits) with the box shape above it
-  const uint64_t key = (uint64_t)(uintptr_t)p | ((uint64_t)(cols & 0xff) << 48) | ((uint64_t)(rows & 0xff) << 56);
-  const auto it = h->ws_map_cache.find(key);
-  if (it != h->ws_map_cache.end()) {
-    *out = it->second;
-    return true;
-  }
-  CUtensorMap mp;
-  if (!encode_f64_3d(&mp, p, (uint64_t)h->ldt, (uint64_t)h->npm, (uint64_t)h->nr, (uint64_t)h->ldt * 8,
-                     (uint64_t)h->plane * 8, (uint32_t)rows, (uint32_t)cols))
-    return false;
-  h->ws_map_cache.emplace(key, mp);
-  *out = mp;
-  return true;
-}
-
-// the tensor maps of one k_sts_pair_ws launch; on = 0 (bulk copies per
-// column) when they are turned off or cannot be made
-static WsMaps ws_maps(hipft_gpu *h, const double *ykm1, const double *ykm2, const double *u0, const double *dty0) {
-  WsMaps tm;
-  std::memset(&tm, 0, sizeof(tm));
-  if (!ws_tmap_enabled() || !h->ws_rt_ok) return tm;
-  if (!field_map(h, ykm1, kWK + 4, &tm.x1) || !field_map(h, ykm2, kWK + 2, &tm.y2) ||
-      !field_map(h, u0, kWK + 2, &tm.u) || !field_map(h, dty0, kWK + 2, &tm.d))
-    return tm;
-  tm.rt = h->ws_rt_map;
-  tm.on = 1;
-  return tm;
-}
-
-// ------------------------------------------------------------ autotuner
-// The two-stage launch has several implementations whose speed depends on
-// the grid and the batch.  The persistent warp-specialised family shares one
-// tile (128 theta rows x 8 phi columns), one ring-sum order and the pole
-// kernel, so its members give bitwise the same values: two theta rows per
-// consumer thread (PK_WS_ROWS2) at 2 or 1 CTAs per SM, the same with bulk
-// stores (PK_WS_BULK), one row per thread (PK_WS_ROWS1).  On the first
-// two-stage super-step of a grid size (ntm, npm, nr) on a device the library
-// times each of them over a few launches on the handle's own buffers and
-// keeps the fastest for the process.  HIPFT_STS_PAIR (0: one stage per
-// launch, 4/5/6: the warp-specialised kinds, 7: four stages per pass on the
-// interior theta blocks) fixes the choice, and HIPFT_TUNE=0 takes PK_WS_ROWS2
-// at 2 CTAs per SM without timing.  The four-stage path (PK_WS_QUAD,
-// sts_quad_ws.cuh) computes the same cell values and is a candidate whenever
-// the grid has interior blocks.
-
-static const char *pair_kind_name(int k) {
-  switch (k) {
-    case PK_SINGLE: return "single-stage";
-    case PK_WS_ROWS1: return "ws-rows1";
-    case PK_WS_ROWS2: return "ws-rows2";
-    case PK_WS_BULK: return "ws-bulk";
-    case PK_WS_QUAD: return "ws-quad (four stages per pass on interior blocks)";
-  }
-  return "?";
-}
-
-static std::mutex g_plan_mutex;
-static std::vector<std::pair<std::array<int, 4>, PairPlan>> g_plans;  // (ntm, npm, nr, device) -> plan
-
-static bool env_plan(PairPlan &p) {
-  const char *e = std::getenv("HIPFT_STS_PAIR");
-  if (e) {
-    const int v = std::atoi(e);
-    p.kind = (v == 0 || v == 4 || v == 6 || v == 7) ? v : PK_WS_ROWS2;
-    return true;
-  }
-  const char *t = std::getenv("HIPFT_TUNE");
-  if (t && std::atoi(t) == 0) {
-    p.kind = PK_WS_ROWS2;
-    return true;
-  }
-  return false;
-}
-
-static bool sts_pairs_enabled(const hipft_gpu *h) { return h->plan.kind != PK_SINGLE; }
-
 static int check_wait_flag(hipft_gpu *h, const char *what);
 
-// Two RKG2 stages per launch (stages k, k+1 of diffusion_step_sts_cd,
-// src/hipft.f90:5222-5237) with the handle's plan.  overlap_prev: the launch
-// before this one on the stream is the previous pair's k_pair_poles (so the
-// warp-specialised kernel may start while it runs; everything else it reads
-// was finished by the kernels before that one).
-static int sts_pair_plan(hipft_gpu *h, const PairPlan &pl, const double *ykm1, const double *ykm2, const double *u0,
-                         const double *dty0, double *out_k, double *out_k1, StageCoef ca, StageCoef cb,
-                         bool overlap_prev) {
-  static_assert(kWK == kPK && kWJ == kPJ, "the two-stage kernels share one tile shape");
-  {
-    ProfScope ps(h, HIPFT_K_STS);
-    const int nkt = (h->npm - 2 + kWK - 1) / kWK;
-    RingOut ro{h->d_ringbuf[1 - h->ring_cur], h->d_rpart, h->d_rcount, nkt};
-    const int grid = std::min(h->ptab.ntiles, pl.ctas_per_sm * h->num_sms);
-    const PairArgs pa{ca, cb, h->d_err};
-    const double *rin = h->d_ringbuf[h->ring_cur];
-    const WsMaps tmaps = ws_maps(h, ykm1, ykm2, u0, dty0);
-    // programmatic dependent launch: may overlap the previous pair's
-    // k_pair_poles (the kernel's pole tiles wait for it)
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kWThreads);
-    cfg.dynamicSmemBytes = kWSmem;
-    cfg.stream = h->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = (ws_pdl() && overlap_prev) ? 1 : 0;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaError_t le;
-    // bulk stores need 16-byte aligned output columns (ldt and the plane
-    // are multiples of 16 elements)
-    const bool aligned = ((reinterpret_cast<uintptr_t>(out_k) | reinterpret_cast<uintptr_t>(out_k1)) & 15) == 0;
-    if (pl.kind == PK_WS_BULK && aligned)
-      le = cudaLaunchKernelEx(&cfg, k_sts_pair_ws<true, true>, h->M, (const double *)h->DC.dfac, ykm1, ykm2, u0,
-                              dty0, out_k, out_k1, rin, h->bc_diff_n, h->bc_diff_s, pa, ro, h->ptab, tmaps);
-    else if (pl.kind == PK_WS_ROWS1)
-      le = cudaLaunchKernelEx(&cfg, k_sts_pair_ws<false>, h->M, (const double *)h->DC.dfac, ykm1, ykm2, u0, dty0,
-                              out_k, out_k1, rin, h->bc_diff_n, h->bc_diff_s, pa, ro, h->ptab, tmaps);
-    else
-      le = cudaLaunchKernelEx(&cfg, k_sts_pair_ws<true>, h->M, (const double *)h->DC.dfac, ykm1, ykm2, u0, dty0,
-                              out_k, out_k1, rin, h->bc_diff_n, h->bc_diff_s, pa, ro, h->ptab, tmaps);
-    if (le != cudaSuccess) return fail(h, HIPFT_ECUDA, "k_sts_pair_ws launch: %s", cudaGetErrorString(le));
-    LAUNCHED(h);
-    dim3 pg((unsigned)h->nr, (unsigned)h->pole_nch);
-    k_pair_poles<<<pg, kPoleThreads, 0, h->stream>>>(h->M, h->DC.dfac, ykm1, ykm2, u0, dty0, out_k1, rin,
-                                                     h->bc_diff_n, h->bc_diff_s, pa, ro, h->pole);
-    LAUNCHED(h);
-  }
-  h->ring_cur = 1 - h->ring_cur;
-  return HIPFT_OK;
-}
-
-static int sts_pair(hipft_gpu *h, const double *ykm1, const double *ykm2, const double *u0, const double *dty0,
-                    double *out_k, double *out_k1, StageCoef ca, StageCoef cb, bool overlap_prev) {
-  PairPlan pl = h->plan;
-  if (pl.kind == PK_WS_QUAD) pl.kind = PK_WS_ROWS2;  // lone pairs of a four-stage plan
-  return sts_pair_plan(h, pl, ykm1, ykm2, u0, dty0, out_k, out_k1, ca, cb, overlap_prev);
-}
-
 // ------------------------------------------------ four stages per pass
-// The interior theta blocks rb_lo..rb_hi (rows j0-3 .. j0+130 of a block
-// inside 2..ntm-1, see sts_quad_ws.cuh); false when there are none.
-static bool quad_eligible(const hipft_gpu *h) {
-  if (h->DC.grid || !h->ptab.row || h->ntm < kQJ + 132) return false;
-  const int rb_hi = (h->ntm - 132) / kQJ;  // largest rb with 128 rb + 132 <= ntm
-  return h->ptab.nb - rb_hi <= 6;           // pole blocks: 0 and rb_hi+1 .. nb-1
+// The fixed part of a pass's arguments.
+static MarchArgs march_args(const hipft_gpu *h, const double *u0, const double *dty0) {
+  MarchArgs a{};
+  a.u = u0;
+  a.d = dty0;
+  a.nreal = h->nr;
+  a.strips = h->m_strips;
+  a.dfac = h->DC.dfac;
+  a.bcn = h->bc_diff_n;
+  a.bcs = h->bc_diff_s;
+  return a;
 }
 
-// Tables, tensor map and the two extra fields of the four-stage path.
-static int quad_setup(hipft_gpu *h) {
-  if (h->d_qcol) return HIPFT_OK;
-  h->q_rb_lo = 1;
-  h->q_rb_hi = (h->ntm - 132) / kQJ;
-  while (h->nbuf < kNBuf) {
-    TRY(dalloc(h, &h->buf[h->nbuf], h->fieldn));
-    CK(h, cudaMemsetAsync(h->buf[h->nbuf], 0, h->fieldn * sizeof(double), h->stream));
-    ++h->nbuf;
-  }
-  h->q_nkt = (h->npm - 2 + kQK - 1) / kQK;
-  h->q_LC = h->q_nkt * kQK + 24;
-  TRY(dalloc(h, &h->d_qcol, (size_t)h->nr * h->q_LC * 2));
-  k_quad_coltab<<<2 * h->num_sms, 256, 0, h->stream>>>(h->M, h->DC.dfac, h->q_LC, h->d_qcol);
-  LAUNCHED(h);
-  h->q_rt_ok = encode_f64_3d(&h->q_rt_map, h->ptab.row, (uint64_t)h->ptab.LR, 3, (uint64_t)h->nr,
-                             (uint64_t)h->ptab.LR * 8, (uint64_t)h->ptab.LR * 24, kQR, 3);
-  CK(h, cudaFuncSetAttribute(k_sts_quad_ws<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kQSmem));
-  CK(h, cudaFuncSetAttribute(k_sts_quad_ws<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kQSmem));
-  return HIPFT_OK;
+// A column per thread in k_sts_poles, or k_sts_poles_any.
+static bool poles_by_column(const hipft_gpu *h) { return poles_threads(h->npm - 2) <= kPMaxThreads; }
+
+static int march_columns(const hipft_gpu *h, int nreal) {
+  const int n2 = h->npm - 2;
+  return march_cols(n2, h->m_strips, nreal, h->m_slots, 2 * poles_ranks(n2));
 }
 
-// The pole blocks (every block outside rb_lo..rb_hi) of `nreal` realizations
-// for the two-stage launches of the four-stage path.
-static PairTables quad_pole_tables(const hipft_gpu *h, int nreal) {
-  PairTables pt = h->ptab;
-  pt.nsel = 0;
-  for (int rb = 0; rb < pt.nb; ++rb)
-    if (rb < h->q_rb_lo || rb > h->q_rb_hi) pt.sel[pt.nsel++] = rb;
-  pt.ntiles = pt.nsel * pt.nkt * nreal;
-  return pt;
+static int64_t march_blocks(const hipft_gpu *h, int nreal) {
+  const int n2 = h->npm - 2, c = march_columns(h, nreal), nch = (n2 + c - 1) / c;
+  return (int64_t)h->m_strips * ((nch + kMWarps - 1) / kMWarps) * nreal;
 }
 
-// Two-stage launch (k_sts_pair_ws, two rows per consumer) plus k_pair_poles
-// over the tiles of `pt`; rlist/rc (may be null): the realizations of a
-// ragged batch and their coefficients.  flip: the launch's output ring sums
-// become current (a launch that shares its input ring with a following one
-// leaves that to the last of them).
-static int ws_pair_launch(hipft_gpu *h, const PairTables &pt, int cps, const double *ykm1, const double *ykm2,
-                          const double *u0, const double *dty0, double *out_k, double *out_k1, StageCoef ca,
-                          StageCoef cb, bool overlap_prev, const int *rlist = nullptr, int nreal = 0,
-                          const StageCoef *rc = nullptr, bool flip = true) {
-  const int nkt = (h->npm - 2 + kWK - 1) / kWK;
-  RingOut ro{h->d_ringbuf[1 - h->ring_cur], h->d_rpart, h->d_rcount, nkt};
-  const int grid = std::min(pt.ntiles, cps * h->num_sms);
-  PairArgs pa{ca, cb, h->d_err, rlist, rc};
-  const double *rin = h->d_ringbuf[h->ring_cur];
-  const WsMaps tmaps = ws_maps(h, ykm1, ykm2, u0, dty0);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(kWThreads);
-  cfg.dynamicSmemBytes = kWSmem;
-  cfg.stream = h->stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = (ws_pdl() && overlap_prev) ? 1 : 0;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t le = rlist ? cudaLaunchKernelEx(&cfg, k_sts_pair_ws<true, false, true>, h->M, (const double *)h->DC.dfac,
-                                              ykm1, ykm2, u0, dty0, out_k, out_k1, rin, h->bc_diff_n, h->bc_diff_s,
-                                              pa, ro, pt, tmaps)
-                         : cudaLaunchKernelEx(&cfg, k_sts_pair_ws<true>, h->M, (const double *)h->DC.dfac, ykm1, ykm2,
-                                              u0, dty0, out_k, out_k1, rin, h->bc_diff_n, h->bc_diff_s, pa, ro, pt,
-                                              tmaps);
-  if (le != cudaSuccess) return fail(h, HIPFT_ECUDA, "k_sts_pair_ws launch: %s", cudaGetErrorString(le));
-  LAUNCHED(h);
-  dim3 pg((unsigned)(rlist ? nreal : h->nr), (unsigned)h->pole_nch);
-  k_pair_poles<<<pg, kPoleThreads, 0, h->stream>>>(h->M, h->DC.dfac, ykm1, ykm2, u0, dty0, out_k1, rin, h->bc_diff_n,
-                                                   h->bc_diff_s, pa, ro, h->pole);
-  LAUNCHED(h);
-  if (flip) h->ring_cur = 1 - h->ring_cur;
-  return HIPFT_OK;
+// k_sts_march for these arguments; byte offsets in 32 bits while a plane has them.
+typedef void (*MarchKernel)(Mesh, MarchArgs, PairTables);
+static MarchKernel march_kernel(bool table, bool keep, bool wide) {
+  if (wide) return table ? k_sts_march<true, false, uint64_t> : keep ? k_sts_march<false, true, uint64_t> : k_sts_march<false, false, uint64_t>;
+  return table ? k_sts_march<true, false, uint32_t> : keep ? k_sts_march<false, true, uint32_t> : k_sts_march<false, false, uint32_t>;
 }
 
-// The four-stage launch over the interior blocks of all realizations, or of
-// the n realizations of rlist with coefficients rcA (stages k, k+1) and rcB
-// (k+2, k+3).  It reads nothing the pole blocks' first two-stage launch
-// writes, so it may start while that launch's pole kernel runs.
-static int quad_launch(hipft_gpu *h, const double *ykm1, const double *ykm2, const double *u0, const double *dty0,
-                       double *ok, double *ok1, double *ok2, double *ok3, const StageCoef c[4],
-                       const int *rlist = nullptr, int n = 0, const StageCoef *rcA = nullptr,
-                       const StageCoef *rcB = nullptr) {
-  QuadArgs qa{};
-  for (int q = 0; q < 4; ++q) qa.c[q] = c[q];
-  qa.err = h->d_err;
-  qa.rb_lo = h->q_rb_lo;
-  qa.nbi = h->q_rb_hi - h->q_rb_lo + 1;
-  qa.nkt = h->q_nkt;
-  qa.ntiles = qa.nbi * qa.nkt * (rlist ? n : h->nr);
-  qa.edge_lo = (h->q_rb_lo > 0) ? h->q_rb_lo : -1;
-  qa.edge_hi = (h->q_rb_hi < h->ptab.nb - 1) ? h->q_rb_hi : -1;
-  qa.col = h->d_qcol;
-  qa.LC = h->q_LC;
-  qa.rlist = rlist;
-  qa.rcA = rcA;
-  qa.rcB = rcB;
-  QuadMaps qm;
-  std::memset(&qm, 0, sizeof(qm));
-  if (ws_tmap_enabled() && h->q_rt_ok && field_map(h, ykm1, kQX, &qm.x1, kQR) && field_map(h, ykm2, kQI, &qm.y2, kQR) &&
-      field_map(h, u0, kQI, &qm.u, kQR) && field_map(h, dty0, kQI, &qm.d, kQR)) {
-    qm.rt = h->q_rt_map;
-    qm.on = 1;
+// One pass on stream s.  after_pass: the launch before it on the stream is
+// the previous pass, whose end it waits for on the device, so it may be
+// launched programmatically.  blocks: k_sts_march's grid (0: for a.nreal
+// realizations, and so its columns per warp).
+static cudaError_t launch_pass(const hipft_gpu *h, cudaStream_t s, MarchArgs a, bool pdl, bool after_pass,
+                               int64_t blocks = 0) {
+  if (!blocks) {
+    blocks = march_blocks(h, a.nreal);
+    a.cols = march_columns(h, a.nreal);
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)std::min(qa.ntiles, h->num_sms));  // one CTA (two tile buffers) per SM
-  cfg.blockDim = dim3(kQThreads);
-  cfg.dynamicSmemBytes = kQSmem;
-  cfg.stream = h->stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = ws_pdl() ? 1 : 0;
+  cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  PairTables pt = h->ptab;
-  cudaError_t le = rlist ? cudaLaunchKernelEx(&cfg, k_sts_quad_ws<true>, h->M, ykm1, ykm2, u0, dty0, ok, ok1, ok2,
-                                              ok3, qa, pt, qm)
-                         : cudaLaunchKernelEx(&cfg, k_sts_quad_ws<false>, h->M, ykm1, ykm2, u0, dty0, ok, ok1, ok2,
-                                              ok3, qa, pt, qm);
-  if (le != cudaSuccess) return fail(h, HIPFT_ECUDA, "k_sts_quad_ws launch: %s", cudaGetErrorString(le));
-  LAUNCHED(h);
-  return HIPFT_OK;
+  if (h->ntm < kMMinRows) {
+    attr[0].val.programmaticStreamSerializationAllowed = 0;
+    cfg.gridDim = dim3((unsigned)a.nreal);
+    cfg.blockDim = dim3(256);
+    return cudaLaunchKernelEx(&cfg, k_sts_whole, h->M, a, h->ptab);
+  }
+  const int n2 = h->npm - 2, nc = poles_ranks(n2);
+  const bool bycol = poles_by_column(h);
+  attr[0].val.programmaticStreamSerializationAllowed = (pdl && after_pass) ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)nc;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.numAttrs = 2;
+  cfg.gridDim = dim3((unsigned)(2 * a.nreal * nc));
+  cfg.blockDim = dim3((unsigned)(bycol ? poles_threads(n2) : kPAThreads));
+  cfg.dynamicSmemBytes = bycol ? poles_smem(poles_threads(n2)) : 0;
+  auto poles = poles_threads(n2) <= kPMidThreads ? k_sts_poles<kPMidThreads> : k_sts_poles<kPMaxThreads>;
+  cudaError_t e = bycol ? cudaLaunchKernelEx(&cfg, poles, h->M, a, h->ptab)
+                        : cudaLaunchKernelEx(&cfg, k_sts_poles_any, h->M, a, h->ptab, h->d_pscratch);
+  if (e != cudaSuccess) return e;
+  attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3(32 * kMWarps);
+  cfg.dynamicSmemBytes = kMSmem;
+  return cudaLaunchKernelEx(&cfg, march_kernel(a.rc != nullptr, a.o[0] || a.o[1], h->plane >= (int64_t)1 << 29),
+                            h->M, a, h->ptab);
 }
 
-// Stages k..k+3: the pole blocks by two two-stage launches, the interior
-// blocks by one four-stage launch between them.  Outputs ok..ok3 hold
-// Y_k..Y_{k+3}; Y_k and Y_{k+1} only on the pole blocks and the interior
-// blocks' edge rows.
-static int quad_pass(hipft_gpu *h, const double *ykm1, const double *ykm2, const double *u0, const double *dty0,
-                     double *ok, double *ok1, double *ok2, double *ok3, const StageCoef c[4], bool overlap_prev) {
-  const int cps = h->plan.ctas_per_sm;
-  const PairTables pp = quad_pole_tables(h, h->nr);
+static int sts_pass(hipft_gpu *h, const MarchArgs &a, bool after_pass) {
   ProfScope ps(h, HIPFT_K_STS);
-  TRY(ws_pair_launch(h, pp, cps, ykm1, ykm2, u0, dty0, ok, ok1, c[0], c[1], overlap_prev));
-  TRY(quad_launch(h, ykm1, ykm2, u0, dty0, ok, ok1, ok2, ok3, c));
-  TRY(ws_pair_launch(h, pp, cps, ok1, ok, u0, dty0, ok2, ok3, c[2], c[3], false));
+  const cudaError_t e = launch_pass(h, h->stream, a, ws_pdl(), after_pass);
+  if (e != cudaSuccess) return fail(h, HIPFT_ECUDA, "RKG2 pass launch: %s", cudaGetErrorString(e));
+  h->launches += h->ntm < kMMinRows ? 1 : 2;
   return HIPFT_OK;
 }
 
-// Chooses the handle's two-stage plan (see the autotuner above) before the
-// first super-step.  Timing runs on four buffers other than the current
-// field, with the current field as an input, and leaves the field untouched;
-// the ring sums it disturbs are recomputed afterwards.
-static int ensure_pair_plan(hipft_gpu *h) {
-  if (h->plan.kind >= 0) return HIPFT_OK;
-  PairPlan p;
-  if (env_plan(p)) {
-    if (p.kind == PK_WS_QUAD) {
-      if (quad_eligible(h)) TRY(quad_setup(h));
-      else p.kind = PK_WS_ROWS2;
-    }
-    h->plan = p;
-    return HIPFT_OK;
-  }
-  const std::array<int, 4> key{h->ntm, h->npm, h->nr, h->dev};
-  {
-    std::lock_guard<std::mutex> lk(g_plan_mutex);
-    for (const auto &e : g_plans)
-      if (e.first == key) {
-        h->plan = e.second;
-        return HIPFT_OK;
-      }
-  }
-  std::vector<PairPlan> cands;
-  for (int c : {2, 1}) {
-    PairPlan q;
-    q.kind = PK_WS_ROWS2;
-    q.ctas_per_sm = c;
-    cands.push_back(q);
-  }
-  for (int k : {PK_WS_BULK, PK_WS_ROWS1}) {
-    PairPlan q;
-    q.kind = k;
-    cands.push_back(q);
-  }
-  if (quad_eligible(h)) {
-    TRY(quad_setup(h));
-    PairPlan q;
-    q.kind = PK_WS_QUAD;
-    cands.push_back(q);
-  }
-  const bool prof = h->profiling;
-  h->profiling = false;
-  const double *x = h->buf[h->cur];
-  double *bufs[6] = {};
-  for (int q = 0; q < 6 && q < h->nbuf - 1; ++q) bufs[q] = h->buf[scratch(h, q)];
-  const StageCoef ca{0.5, -0.1, 0.6, 1e-3, 0.0}, cb{0.5, -0.1, 0.6, 1e-3, 0.0};
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-  CK(h, cudaEventCreate(&e0));
-  CK(h, cudaEventCreate(&e1));
-  int best = 0;
-  const int reps = 3;
-  const StageCoef cq[4] = {ca, cb, ca, cb};
-  for (size_t c = 0; c < cands.size(); ++c) {
-    // time per two stages: a four-stage pass counts as two launch pairs
-    const bool quad = cands[c].kind == PK_WS_QUAD;
-    const PairPlan saved = h->plan;
-    h->plan = cands[c];
-    auto once = [&](bool ov) -> int {
-      if (quad) return quad_pass(h, x, bufs[0], x, bufs[1], bufs[2], bufs[3], bufs[4], bufs[5], cq, ov);
-      return sts_pair_plan(h, cands[c], x, bufs[0], x, bufs[1], bufs[2], bufs[3], ca, cb, ov);
-    };
-    int rc = once(false);  // warm-up
-    CK(h, cudaEventRecord(e0, h->stream));
-    for (int r = 0; r < reps && rc == HIPFT_OK; ++r) rc = once(r > 0);
-    h->plan = saved;
-    TRY(rc);
-    CK(h, cudaEventRecord(e1, h->stream));
-    CK(h, cudaEventSynchronize(e1));
-    float ms = 0.f;
-    CK(h, cudaEventElapsedTime(&ms, e0, e1));
-    cands[c].ms = ms / reps / (quad ? 2.0 : 1.0);
-    if (cands[c].ms < cands[best].ms) best = (int)c;
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  h->profiling = prof;
-  TRY(check_wait_flag(h, "pair autotuner: a bounded wait for staged tiles gave up"));
-  h->plan = cands[best];
-  h->plan.candidates = (int)cands.size();
-  h->dring_valid = false;
-  std::lock_guard<std::mutex> lk(g_plan_mutex);
-  g_plans.push_back({key, h->plan});
+// The seam columns of a field whose core columns the passes wrote.
+static int seam(hipft_gpu *h, double *f) {
+  ProfScope ps(h, HIPFT_K_OTHER);
+  k_seam<<<dim3((unsigned)((h->ntm + 127) / 128), (unsigned)h->nr), 128, 0, h->stream>>>(h->M, h->ntm, h->ldt, f);
+  LAUNCHED(h);
+  return HIPFT_OK;
+}
+
+// dty0 = dtl * A u0 from A u0 (src/hipft.f90:5211), for all realizations or
+// for the n of a list with a length each.
+static int scale_dty0(hipft_gpu *h, const double *af, double *dty0, double dtl, const int *rlist = nullptr, int n = 0,
+                      const double *rlen = nullptr) {
+  ProfScope ps(h, HIPFT_K_OTHER);
+  const unsigned chunks = (unsigned)std::min<int64_t>((h->plane / 2 + 255) / 256, 4 * h->num_sms);
+  k_scale<<<dim3(chunks, (unsigned)(rlist ? n : h->nr)), 256, 0, h->stream>>>(h->plane, af, dty0, dtl, rlist, rlen);
+  LAUNCHED(h);
   return HIPFT_OK;
 }
 
@@ -1067,15 +729,16 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
   if ((rc = dalloc(h, &h->d_rcount, (size_t)nr))) return bail(rc);
   if ((rc = dalloc(h, &h->d_err, 1))) return bail(rc);
   if (cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream) != cudaSuccess) return bail(HIPFT_ECUDA);
-  if (cudaFuncSetAttribute(k_sts_pair_ws<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWSmem) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(k_sts_pair_ws<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWSmem) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(k_sts_pair_ws<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWSmem) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(k_sts_pair_ws<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)kWSmem) != cudaSuccess)
-    return bail(fail(h, HIPFT_ECUDA, "cannot reserve shared memory for the two-stage kernels"));
+  bool smem_ok = true;
+  for (int v = 0; v < 8; ++v)
+    smem_ok = smem_ok && cudaFuncSetAttribute(march_kernel(v & 1, v & 2, v & 4), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)kMSmem) == cudaSuccess;
+  if (!smem_ok ||
+      cudaFuncSetAttribute(k_sts_poles<kPMidThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)poles_smem(kPMidThreads)) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sts_poles<kPMaxThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)poles_smem(kPMaxThreads)) != cudaSuccess)
+    return bail(fail(h, HIPFT_ECUDA, "cannot reserve shared memory for the RKG2 passes"));
   if (cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess || h->num_sms < 1)
     h->num_sms = 148;
   if (cudaMemsetAsync(h->d_rcount, 0, sizeof(unsigned int) * nr, h->stream) != cudaSuccess) return bail(HIPFT_ECUDA);
@@ -1097,26 +760,21 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
   h->DC.grid = prm->diffusion_coef_grid;
   if (prm->advance_diffusion && !prm->diffusion_coef_grid) {
     PairTables &pt = h->ptab;
-    pt.nb = (ntm + kWJ - 1) / kWJ;
-    pt.nkt = (npm - 2 + kWK - 1) / kWK;
-    pt.ntiles = pt.nb * pt.nkt * nr;
-    pt.LR = pt.nb * kWJ + 4;
-    pt.LC = pt.nkt * kWK + 4;
+    pt.LR = round_up(ntm + 4, 2);  // even: the column table behind the rows stays 16-byte aligned
+    pt.LC = npm + 2 + 2 * kColPad;
+    h->m_strips = std::max(1, (ntm - 2 * kMS + kMOwn - 1) / kMOwn);
+    h->m_slots = kMBlocks * kMWarps * h->num_sms;
+    if (!poles_by_column(h) &&
+        (rc = dalloc(h, &h->d_pscratch, (size_t)2 * nr * poles_ranks(npm - 2) * kPADoubles * poles_any_width(npm - 2))))
+      return bail(rc);
     double *tab = nullptr;
     const size_t nrow = (size_t)nr * pt.LR * 3, ncol = (size_t)nr * pt.LC * 2;
     if ((rc = dalloc(h, &tab, nrow + ncol))) return bail(rc);
     pt.row = tab;
-    pt.col = tab + nrow;
-    h->ws_rt_ok = encode_f64_3d(&h->ws_rt_map, pt.row, (uint64_t)pt.LR, 3, (uint64_t)nr, (uint64_t)pt.LR * 8,
-                                (uint64_t)pt.LR * 24, kWR, 3);
+    pt.col = tab + nrow + 2 * kColPad;
     k_pair_tables<<<2 * h->num_sms, 256, 0, h->stream>>>(h->M, d_dfac, pt.LR, pt.LC, tab, tab + nrow);
     h->launches++;
     if (cudaPeekAtLastError() != cudaSuccess) return bail(fail(h, HIPFT_ECUDA, "k_pair_tables launch failed"));
-    h->pole_nch = (npm + kPoleThreads - 1) / kPoleThreads;
-    if ((rc = dalloc(h, &h->pole.part, (size_t)nr * h->pole_nch * 2))) return bail(rc);
-    if ((rc = dalloc(h, &h->pole.count, (size_t)nr))) return bail(rc);
-    if (cudaMemsetAsync(h->pole.count, 0, sizeof(unsigned int) * nr, h->stream) != cudaSuccess)
-      return bail(HIPFT_ECUDA);
   }
   h->bc_diff_n = c_pi_i * h->dth_i[2] * h->dth_i[2];
   h->bc_diff_s = c_pi_i * h->dth_i[nt - 1] * h->dth_i[nt - 1];
@@ -1614,13 +1272,6 @@ static void sts_coefs(int method, double dtl, double dt_euler, StsTable &T) {
   }
 }
 
-// The stage-k combine coefficients of a super-step of length dtl
-// (src/hipft.f90:5224-5235).
-static StageCoef sts_stage_coef(const StsTable &T, int64_t k, double dtl) {
-  double uj = T.uj[k], vj = T.vj[k];
-  return StageCoef{uj, vj, 1.0 - uj - vj, T.ubj[k] * dtl, T.gj[k]};
-}
-
 static void load_sts(hipft_gpu *h, double dtl) {
   StsTable T;
   sts_coefs(h->P.diffusion_num_method, dtl, h->dt_euler, T);
@@ -1632,81 +1283,61 @@ static void load_sts(hipft_gpu *h, double dtl) {
   h->sts_gj = std::move(T.gj);
 }
 
-// diffusion_step_sts_cd (src/hipft.f90:5163-5242): stage 1 then the
-// s-1 fused stages, rotating three scratch fields.
-static int sts_super_step(hipft_gpu *h, double dtl) {
-  if (!h->DC.grid) TRY(ensure_pair_plan(h));
+// A u0 of the current field into scratch buffer 0, unless the practical time
+// step limit left it there.
+static int current_lap(hipft_gpu *h) {
+  const double *ring;
+  TRY(current_dring(h, &ring));
+  return diffusion_stage<MODE_AX>(h, h->buf[h->cur], nullptr, nullptr, nullptr, h->buf[scratch(h, 0)], nullptr, ring,
+                                  StageCoef{}, nullptr);
+}
+
+// diffusion_step_sts_cd (src/hipft.f90:5163-5242).  have_lap: scratch buffer 0
+// holds A u0 (not with a grid-dependent D).
+static int sts_super_step(hipft_gpu *h, double dtl, bool have_lap) {
   load_sts(h, dtl);
-  int u0 = h->cur, idty = scratch(h, 0), ia = scratch(h, 1), ib = scratch(h, 2);
-  const bool fused = !h->DC.grid;
-  if (fused) {
-    const double *r0;
-    TRY(current_dring(h, &r0));
-    TRY(sts_stage_v2<MODE_STS1>(h, h->buf[u0], nullptr, nullptr, nullptr, h->buf[ia], h->buf[idty],
-                                StageCoef{dtl, h->sts_ubj[1], 0, 0, 0}));
-  } else {
-    TRY(ring_diffusion(h, h->buf[u0], h->d_ring));
-    TRY(diffusion_stage<MODE_STS1>(h, h->buf[u0], nullptr, nullptr, nullptr, h->buf[ia], h->buf[idty], h->d_ring,
-                                   StageCoef{dtl, h->sts_ubj[1], 0, 0, 0}, nullptr));
+  const int u0 = h->cur, idty = scratch(h, 0);
+  const int64_t cells = (int64_t)h->ntm * (h->npm - 2) * h->nr;
+  h->rkg2_stages += h->sts_s - 1;
+  h->rkg2_cell_stages += cells * (h->sts_s - 1);
+  h->cell_updates += cells * h->sts_s;
+  if (!h->DC.grid) {
+    if (!have_lap) TRY(current_lap(h));
+    TRY(scale_dty0(h, h->buf[idty], h->buf[idty], dtl));
+    const int R[4] = {scratch(h, 1), scratch(h, 2), scratch(h, 3), scratch(h, 4)};
+    MarchArgs a = march_args(h, h->buf[u0], h->buf[idty]);
+    const int64_t np = sts_passes(h->sts_s);
+    for (int64_t p = 0; p < np; ++p) {
+      const int in = (p & 1) ? 0 : 2, out = 2 - in;
+      a.x2 = h->buf[R[in]];
+      a.x1 = h->buf[R[in + 1]];
+      a.o[2] = h->buf[R[out]];
+      a.o[3] = h->buf[R[out + 1]];
+      a.first = p == 0;
+      for (int q = 0; q < kMS; ++q) a.c[q] = sts_slot(h->P.diffusion_num_method, h->sts_s, kMS * p + q, dtl);
+      TRY(sts_pass(h, a, p > 0));
+      h->cur = R[out + 1];
+    }
+    h->dring_valid = false;
+    return seam(h, h->buf[h->cur]);
   }
+  const int ia = scratch(h, 1), ib = scratch(h, 2);
+  TRY(ring_diffusion(h, h->buf[u0], h->d_ring));
+  TRY(diffusion_stage<MODE_STS1>(h, h->buf[u0], nullptr, nullptr, nullptr, h->buf[ia], h->buf[idty], h->d_ring,
+                                 StageCoef{dtl, h->sts_ubj[1], 0, 0, 0}, nullptr));
   int ykm1 = ia, ykm2 = u0;
-  auto coef = [&](int64_t k) {
-    double uj = h->sts_uj[k], vj = h->sts_vj[k];
-    return StageCoef{uj, vj, 1.0 - uj - vj, h->sts_ubj[k] * dtl, h->sts_gj[k]};
-  };
-  // a buffer not holding u0, dty0, Y_{k-1}, Y_{k-2} (or `avoid`)
-  auto free_buf = [&](int avoid) {
-    for (int b = 0; b < h->nbuf; ++b)
-      if (b != u0 && b != idty && b != ykm1 && b != ykm2 && b != avoid) return b;
-    return -1;
-  };
-  (void)ib;
-  int64_t k = 2;
-  while (k <= h->sts_s) {
-    if (fused && h->plan.kind == PK_WS_QUAD && k + 3 <= h->sts_s) {
-      int ob[4], no = 0;
-      for (int b = 0; b < h->nbuf && no < 4; ++b)
-        if (b != u0 && b != idty && b != ykm1 && b != ykm2) ob[no++] = b;
-      const StageCoef cq[4] = {coef(k), coef(k + 1), coef(k + 2), coef(k + 3)};
-      TRY(quad_pass(h, h->buf[ykm1], h->buf[ykm2], h->buf[u0], h->buf[idty], h->buf[ob[0]], h->buf[ob[1]],
-                    h->buf[ob[2]], h->buf[ob[3]], cq, k > 2));
-      ykm2 = ob[2];
-      ykm1 = ob[3];
-      k += 4;
-      h->rkg2_stages += 4;
-      h->rkg2_cell_stages += 4 * (int64_t)h->ntm * (h->npm - 2) * h->nr;
-      continue;
-    }
-    if (fused && sts_pairs_enabled(h) && k + 1 <= h->sts_s) {
-      int bk = free_buf(-1), bk1 = free_buf(bk);
-      TRY(sts_pair(h, h->buf[ykm1], h->buf[ykm2], h->buf[u0], h->buf[idty], h->buf[bk], h->buf[bk1], coef(k),
-                   coef(k + 1), k > 2));
-      ykm2 = bk;
-      ykm1 = bk1;
-      k += 2;
-      h->rkg2_stages += 2;
-      h->rkg2_cell_stages += 2 * (int64_t)h->ntm * (h->npm - 2) * h->nr;
-      continue;
-    }
-    int out = (ykm2 == u0) ? free_buf(-1) : ykm2;
-    StageCoef sc = coef(k);
-    if (fused) {
-      TRY(sts_stage_v2<MODE_STSK>(h, h->buf[ykm1], h->buf[ykm2], h->buf[u0], h->buf[idty], h->buf[out], nullptr,
-                                  sc));
-    } else {
-      TRY(ring_diffusion(h, h->buf[ykm1], h->d_ring));
-      TRY(diffusion_stage<MODE_STSK>(h, h->buf[ykm1], h->buf[ykm2], h->buf[u0], h->buf[idty], h->buf[out],
-                                     nullptr, h->d_ring, sc, nullptr));
-    }
+  for (int64_t k = 2; k <= h->sts_s; ++k) {
+    const int out = (ykm2 == u0) ? ib : ykm2;
+    const double uj = h->sts_uj[k], vj = h->sts_vj[k];
+    TRY(ring_diffusion(h, h->buf[ykm1], h->d_ring));
+    TRY(diffusion_stage<MODE_STSK>(h, h->buf[ykm1], h->buf[ykm2], h->buf[u0], h->buf[idty], h->buf[out], nullptr,
+                                   h->d_ring, StageCoef{uj, vj, 1.0 - uj - vj, h->sts_ubj[k] * dtl, h->sts_gj[k]},
+                                   nullptr));
     ykm2 = ykm1;
     ykm1 = out;
-    k += 1;
-    h->rkg2_stages += 1;
-    h->rkg2_cell_stages += (int64_t)h->ntm * (h->npm - 2) * h->nr;
   }
   h->cur = ykm1;
-  h->dring_valid = fused;  // the last fused stage left the ring of the new field
-  h->cell_updates += (int64_t)h->ntm * (h->npm - 2) * h->nr * h->sts_s;
+  h->dring_valid = false;
   return HIPFT_OK;
 }
 
@@ -1720,8 +1351,7 @@ static int euler_steps(hipft_gpu *h, double dtl) {
     if (!h->DC.grid) {
       const double *r0;
       TRY(current_dring(h, &r0));
-      TRY(sts_stage_v2<MODE_EULER>(h, h->buf[h->cur], nullptr, nullptr, nullptr, h->buf[o], nullptr,
-                                   StageCoef{dte, 0, 0, 0, 0}));
+      TRY(euler_step(h, h->buf[h->cur], h->buf[o], dte));
       h->cur = o;
       h->dring_valid = true;
     } else {
@@ -1891,180 +1521,80 @@ static int ragged_ptl(hipft_gpu *h, std::vector<int> act, std::vector<double> &d
   return HIPFT_OK;
 }
 
-// Two-stage launch of a ragged super-step: the first n realizations of the
-// list d_rlist_dif, coefficients rc ([nr][2]).
-static int sts_pair_ragged(hipft_gpu *h, const double *ykm1, const double *ykm2, const double *u0,
-                           const double *dty0, double *out_k, double *out_k1, int n, const StageCoef *rc,
-                           bool overlap_prev) {
-  const int nkt = (h->npm - 2 + kWK - 1) / kWK;
-  RingOut ro{h->d_ringbuf[1 - h->ring_cur], h->d_rpart, h->d_rcount, nkt};
-  PairTables pt = h->ptab;
-  pt.ntiles = pt.nb * pt.nkt * n;
-  const int cps = (h->plan.kind == PK_WS_ROWS2) ? h->plan.ctas_per_sm : 2;
-  const int grid = std::min(pt.ntiles, cps * h->num_sms);
-  PairArgs pa{StageCoef{}, StageCoef{}, h->d_err, h->d_rlist_dif, rc};
-  const double *rin = h->d_ringbuf[h->ring_cur];
-  const WsMaps tmaps = ws_maps(h, ykm1, ykm2, u0, dty0);
-  {
-    ProfScope ps(h, HIPFT_K_STS);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kWThreads);
-    cfg.dynamicSmemBytes = kWSmem;
-    cfg.stream = h->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = (ws_pdl() && overlap_prev) ? 1 : 0;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaError_t le = cudaLaunchKernelEx(&cfg, k_sts_pair_ws<true, false, true>, h->M,
-                                        (const double *)h->DC.dfac, ykm1, ykm2, u0, dty0, out_k, out_k1, rin,
-                                        h->bc_diff_n, h->bc_diff_s, pa, ro, pt, tmaps);
-    if (le != cudaSuccess) return fail(h, HIPFT_ECUDA, "k_sts_pair_ws (ragged) launch: %s", cudaGetErrorString(le));
-    LAUNCHED(h);
-    dim3 pg((unsigned)n, (unsigned)h->pole_nch);
-    k_pair_poles<<<pg, kPoleThreads, 0, h->stream>>>(h->M, h->DC.dfac, ykm1, ykm2, u0, dty0, out_k1, rin,
-                                                     h->bc_diff_n, h->bc_diff_s, pa, ro, h->pole);
-    LAUNCHED(h);
-  }
-  h->ring_cur = 1 - h->ring_cur;
-  return HIPFT_OK;
-}
-
 // One RKG2/RKL2 super-step of every realization in `act`, realization i over
 // dtl[i] with its own stage count s_i (src/hipft.f90:5163-5242 per
-// realization).  The launch of stage pair p covers the realizations with
-// s_i >= 2p + 3; afterwards every realization's field is gathered into one
-// buffer, which becomes the current field.
+// realization).  Pass p covers the realizations with more than p passes;
+// afterwards every realization's field is gathered into one buffer, which
+// becomes the current field.  Scratch buffer 0 holds A u0 of the realizations.
 static int ragged_super_step(hipft_gpu *h, std::vector<int> act, const std::vector<double> &dtl) {
   const int nr = h->nr, method = h->P.diffusion_num_method;
-  TRY(ensure_pair_plan(h));
-  std::vector<StsTable> T(nr);
   std::vector<int64_t> s(nr, 0);
   int64_t smax = 0;
   for (int i : act) {
-    sts_coefs(method, dtl[i], h->r_dt_euler[i], T[i]);
-    s[i] = T[i].s;
-    h->r_s[i] = T[i].s;
+    s[i] = sts_count(method, dtl[i], h->r_dt_euler[i]);
+    h->r_s[i] = s[i];
     smax = std::max(smax, s[i]);
   }
   TRY(upload_list(h, h->d_rlist_dif, act, s));
   const int na = (int)act.size();
-  const int64_t npairs = (smax - 1) / 2;  // s is odd: stages 2..s are (s-1)/2 pairs
-  // stage-1 and pair coefficients, per realization
-  std::vector<StageCoef> c1(nr, StageCoef{});
-  for (int i : act) c1[i] = StageCoef{dtl[i], T[i].ubj[1], 0, 0, 0};
-  CK(h, cudaMemcpyAsync(h->d_r1coef, c1.data(), sizeof(StageCoef) * nr, cudaMemcpyHostToDevice, h->stream));
-  if ((size_t)npairs > h->rcoef_pairs) {
+  const int64_t np = sts_passes(smax);
+  if ((size_t)np > h->rcoef_passes) {
     if (h->d_rcoef) {
       CK(h, cudaStreamSynchronize(h->stream));
       cudaFree(h->d_rcoef);
       h->allocs.erase(std::remove(h->allocs.begin(), h->allocs.end(), (void *)h->d_rcoef), h->allocs.end());
       h->d_rcoef = nullptr;
     }
-    const size_t cap = (size_t)npairs + 64;
-    TRY(dalloc(h, &h->d_rcoef, cap * nr * 2));
-    h->rcoef_pairs = cap;
+    const size_t cap = (size_t)np + 32;
+    TRY(dalloc(h, &h->d_rcoef, cap * nr * kMS));
+    h->rcoef_passes = cap;
   }
-  std::vector<StageCoef> pc((size_t)npairs * nr * 2, StageCoef{});
+  std::vector<StageCoef> pc((size_t)np * nr * kMS, StageCoef{});
   for (int i : act)
-    for (int64_t q = 0; q < (s[i] - 1) / 2; ++q) {
-      const int64_t k = 2 + 2 * q;
-      pc[((size_t)q * nr + i) * 2] = sts_stage_coef(T[i], k, dtl[i]);
-      pc[((size_t)q * nr + i) * 2 + 1] = sts_stage_coef(T[i], k + 1, dtl[i]);
-    }
+    for (int64_t q = 0; q < kMS * sts_passes(s[i]); ++q)
+      pc[((size_t)(q / kMS) * nr + i) * kMS + q % kMS] = sts_slot(method, s[i], q, dtl[i]);
   CK(h, cudaMemcpyAsync(h->d_rcoef, pc.data(), sizeof(StageCoef) * pc.size(), cudaMemcpyHostToDevice, h->stream));
+  CK(h, cudaMemcpyAsync(h->d_rlen, dtl.data(), sizeof(double) * nr, cudaMemcpyHostToDevice, h->stream));
 
-  const int u0 = h->cur, idty = scratch(h, 0), ia = scratch(h, 1);
-  const double *r0;
-  TRY(current_dring(h, &r0));
-  {
-    // stage 1 (src/hipft.f90:5211-5218) of every realization in the list
-    const int nkb = (h->npm - 2 + kKPT3 - 1) / kKPT3;
-    RingOut ro{h->d_ringbuf[1 - h->ring_cur], h->d_rpart, h->d_rcount, nkb};
-    const int jshift = (h->ntm % 2 == 1 && ((h->ntm - 1) / 2) % 32 == 0) ? 1 : 0;
-    const int nthr = (h->ntm + 2 * jshift + 1) / 2;
-    dim3 grd((unsigned)((nthr + 127) / 128), (unsigned)nkb, (unsigned)na);
-    ProfScope ps(h, HIPFT_K_OTHER);
-    k_sts_stage_v3<MODE_STS1, kKPT3><<<grd, 128, 0, h->stream>>>(
-        h->M, h->DC.dfac, h->buf[u0], nullptr, nullptr, nullptr, h->buf[ia], h->buf[idty], h->d_ringbuf[h->ring_cur],
-        h->bc_diff_n, h->bc_diff_s, StageCoef{}, ro, jshift, h->d_rlist_dif, h->d_r1coef);
-    LAUNCHED(h);
-    h->ring_cur = 1 - h->ring_cur;
-  }
-  int ykm1 = ia, ykm2 = u0;
-  auto free_buf = [&](int avoid) {
-    for (int b = 0; b < h->nbuf; ++b)
-      if (b != u0 && b != idty && b != ykm1 && b != ykm2 && b != avoid) return b;
-    return -1;
-  };
+  const int u0 = h->cur, idty = scratch(h, 0);
+  const int R[4] = {scratch(h, 1), scratch(h, 2), scratch(h, 3), scratch(h, 4)};
+  TRY(scale_dty0(h, h->buf[idty], h->buf[idty], 0.0, h->d_rlist_dif, na, h->d_rlen));
   std::vector<int> fin(nr, u0);  // buffer holding each realization's result
   const int64_t cells = (int64_t)h->ntm * (h->npm - 2);
-  const bool quad = h->plan.kind == PK_WS_QUAD && h->d_qcol;
-  for (int64_t q = 0; q < npairs;) {
-    int n = 0;   // realizations with pair q
-    while (n < na && (s[act[n]] - 1) / 2 > q) ++n;
-    int nq = 0;  // realizations with pairs q and q+1: four stages in one pass
-    while (quad && nq < na && (s[act[nq]] - 1) / 2 >= q + 2) ++nq;
-    if (nq > 0) {
-      int ob[4], no = 0;
-      for (int b = 0; b < h->nbuf && no < 4; ++b)
-        if (b != u0 && b != idty && b != ykm1 && b != ykm2) ob[no++] = b;
-      const StageCoef *rcA = h->d_rcoef + (size_t)q * nr * 2, *rcB = h->d_rcoef + (size_t)(q + 1) * nr * 2;
-      const StageCoef none[4] = {};
-      const PairTables pp = quad_pole_tables(h, nq);
-      const int cps = h->plan.ctas_per_sm;
-      ProfScope ps(h, HIPFT_K_STS);
-      // stages k, k+1: the pole blocks of the four-stage realizations and, for
-      // the realizations whose last pair this is, every block
-      TRY(ws_pair_launch(h, pp, cps, h->buf[ykm1], h->buf[ykm2], h->buf[u0], h->buf[idty], h->buf[ob[0]],
-                         h->buf[ob[1]], StageCoef{}, StageCoef{}, q > 0, h->d_rlist_dif, nq, rcA, n == nq));
-      if (n > nq) {
-        PairTables pt = h->ptab;
-        pt.ntiles = pt.nb * pt.nkt * (n - nq);
-        TRY(ws_pair_launch(h, pt, cps, h->buf[ykm1], h->buf[ykm2], h->buf[u0], h->buf[idty], h->buf[ob[0]],
-                           h->buf[ob[1]], StageCoef{}, StageCoef{}, true, h->d_rlist_dif + nq, n - nq, rcA, true));
-      }
-      TRY(quad_launch(h, h->buf[ykm1], h->buf[ykm2], h->buf[u0], h->buf[idty], h->buf[ob[0]], h->buf[ob[1]],
-                      h->buf[ob[2]], h->buf[ob[3]], none, h->d_rlist_dif, nq, rcA, rcB));
-      TRY(ws_pair_launch(h, pp, cps, h->buf[ob[1]], h->buf[ob[0]], h->buf[u0], h->buf[idty], h->buf[ob[2]],
-                         h->buf[ob[3]], StageCoef{}, StageCoef{}, false, h->d_rlist_dif, nq, rcB, true));
-      for (int e = 0; e < n; ++e) {
-        const int64_t P = (s[act[e]] - 1) / 2;
-        if (e >= nq && P == q + 1) fin[act[e]] = ob[1];
-        if (e < nq && P == q + 2) fin[act[e]] = ob[3];
-      }
-      ykm2 = ob[2];
-      ykm1 = ob[3];
-      h->rkg2_stages += 4;
-      h->rkg2_cell_stages += 4 * cells * nq + 2 * cells * (n - nq);
-      q += 2;
-      continue;
-    }
-    const int bk = free_buf(-1), bk1 = free_buf(bk);
-    TRY(sts_pair_ragged(h, h->buf[ykm1], h->buf[ykm2], h->buf[u0], h->buf[idty], h->buf[bk], h->buf[bk1], n,
-                        h->d_rcoef + (size_t)q * nr * 2, q > 0));
+  MarchArgs a = march_args(h, h->buf[u0], h->buf[idty]);
+  a.rlist = h->d_rlist_dif;
+  int dst = u0;
+  for (int64_t p = 0; p < np; ++p) {
+    int n = 0;  // realizations with pass p
+    while (n < na && sts_passes(s[act[n]]) > p) ++n;
+    const int in = (p & 1) ? 0 : 2, out = 2 - in;
+    a.x2 = h->buf[R[in]];
+    a.x1 = h->buf[R[in + 1]];
+    a.o[2] = h->buf[R[out]];
+    a.o[3] = h->buf[R[out + 1]];
+    a.first = p == 0;
+    a.nreal = n;
+    a.rc = h->d_rcoef + (size_t)p * nr * kMS;
+    TRY(sts_pass(h, a, p > 0));
+    h->rkg2_stages += kMS;
+    dst = R[out + 1];
     for (int e = 0; e < n; ++e)
-      if ((s[act[e]] - 1) / 2 == q + 1) fin[act[e]] = bk1;
-    ykm2 = bk;
-    ykm1 = bk1;
-    h->rkg2_stages += 2;
-    h->rkg2_cell_stages += 2 * cells * n;
-    q += 1;
+      if (sts_passes(s[act[e]]) == p + 1) fin[act[e]] = dst;
   }
   // gather: realizations that finished earlier, and those not in this
-  // super-step at all (still in u0), into the last pair's output
-  const int dst = ykm1;
+  // super-step at all (still in u0), into the last pass's output
   const size_t pbytes = (size_t)h->plane * sizeof(double);
   for (int i = 0; i < nr; ++i)
     if (fin[i] != dst)
       CK(h, cudaMemcpyAsync(h->buf[dst] + (size_t)i * h->plane, h->buf[fin[i]] + (size_t)i * h->plane, pbytes,
                             cudaMemcpyDeviceToDevice, h->stream));
+  TRY(seam(h, h->buf[dst]));
   h->cur = dst;
-  h->dring_valid = false;  // the ring sums of the finished realizations sit in either buffer
+  h->dring_valid = false;
   int64_t tot = 0;
   for (int i : act) tot += s[i];
   h->cell_updates += cells * tot;
+  h->rkg2_cell_stages += cells * (tot - na);
   return HIPFT_OK;
 }
 
@@ -2082,6 +1612,7 @@ static int ragged_diffusion_step(hipft_gpu *h, double dtl, hipft_diffusion_info 
   int64_t smax = 0;
   while (!act.empty()) {
     if (h->auto_sc) TRY(ragged_ptl(h, act, d));
+    else TRY(current_lap(h));
     std::vector<int> done;
     for (int i : act) {
       bool fin = false;
@@ -2198,7 +1729,7 @@ extern "C" int hipft_gpu_set_ragged(hipft_gpu *h, int on) {
     TRY(dalloc(h, &h->d_rbits, 2 * (size_t)nr));
     TRY(dalloc(h, &h->d_rlist_dif, (size_t)nr));
     TRY(dalloc(h, &h->d_rlist_adv, (size_t)nr));
-    TRY(dalloc(h, &h->d_r1coef, (size_t)nr));
+    TRY(dalloc(h, &h->d_rlen, (size_t)nr));
     TRY(dalloc(h, &h->d_rdt, (size_t)nr));
   }
   if (h->P.advance_diffusion) TRY(ragged_gershgorin(h));
@@ -2218,7 +1749,7 @@ extern "C" int hipft_gpu_flow_dtmax_each(hipft_gpu *h, double *dtmax) {
     TRY(dalloc(h, &h->d_rbits, 2 * (size_t)h->nr));
     TRY(dalloc(h, &h->d_rlist_dif, (size_t)h->nr));
     TRY(dalloc(h, &h->d_rlist_adv, (size_t)h->nr));
-    TRY(dalloc(h, &h->d_r1coef, (size_t)h->nr));
+    TRY(dalloc(h, &h->d_rlen, (size_t)h->nr));
     TRY(dalloc(h, &h->d_rdt, (size_t)h->nr));
   }
   h->r_dtmax_valid = false;
@@ -2284,7 +1815,7 @@ extern "C" int hipft_gpu_diffusion_step(hipft_gpu *h, double dtl, hipft_cycle_cb
     }
     if (h->auto_sc && h->P.verbose > 0) h->subcycles_state = (int64_t)std::ceil((dtl - time_stepped) / dtl2);
     if (h->P.diffusion_num_method == 1) TRY(euler_steps(h, dtl2));
-    else TRY(sts_super_step(h, dtl2));
+    else TRY(sts_super_step(h, dtl2, h->auto_sc));
     time_stepped = time_stepped + dtl2;
     if (cb) {
       CK(h, cudaStreamSynchronize(h->stream));
@@ -2313,9 +1844,9 @@ extern "C" int hipft_gpu_diffusion_step(hipft_gpu *h, double dtl, hipft_cycle_cb
 // are made on the device by the schedule kernels of graph_step.cuh, and the
 // loops they size are WHILE nodes.  The capture fixes the buffers: the field
 // stays in buffer g_cur; stage outputs rotate through four others with fixed
-// roles (an even stage pair reads (R0, R3) and writes (R1, R2), an odd one
-// reads (R2, R1) and writes (R3, R0)); each realization's result is gathered
-// back into the field buffer after its super-step.
+// roles (an even pass reads (R2, R3) and writes (R0, R1), an odd one the other
+// way round); each realization's result is gathered back into the field buffer
+// after its super-step.
 
 static void graph_release(hipft_gpu *h) {
   if (h->g_exec) cudaGraphExecDestroy(h->g_exec);
@@ -2333,8 +1864,8 @@ static void dfree(hipft_gpu *h, T *&p) {
   p = nullptr;
 }
 
-// Schedule arrays for the handle's realizations and `paircap` stage pairs.
-static int graph_alloc(hipft_gpu *h, int paircap) {
+// Schedule arrays for the handle's realizations and `passcap` passes.
+static int graph_alloc(hipft_gpu *h, int passcap) {
   GArrays &g = h->GA;
   const size_t nr = (size_t)h->nr;
   if (!g.st) {
@@ -2355,7 +1886,6 @@ static int graph_alloc(hipft_gpu *h, int paircap) {
     TRY(dalloc(h, &g.cycles_i, nr));
     TRY(dalloc(h, &g.s_i, nr));
     TRY(dalloc(h, &g.s_last, nr));
-    TRY(dalloc(h, &g.c1, nr));
     TRY(dalloc(h, &g.bits, 2 * nr));
     g.dt_euler = de;
     g.dtmax = dm;
@@ -2365,26 +1895,28 @@ static int graph_alloc(hipft_gpu *h, int paircap) {
     CK(h, cudaMemsetAsync(g.nsub_i, 0, nr * sizeof(int), h->stream));
     g.nr = h->nr;
   }
-  if (paircap > g.paircap) {
+  if (passcap > g.passcap) {
     dfree(h, g.nactp);
+    dfree(h, g.colsp);
     dfree(h, g.rc);
-    TRY(dalloc(h, &g.nactp, (size_t)paircap));
-    TRY(dalloc(h, &g.rc, (size_t)paircap * nr * 2));
-    g.paircap = paircap;
+    TRY(dalloc(h, &g.nactp, (size_t)passcap));
+    TRY(dalloc(h, &g.colsp, (size_t)passcap));
+    TRY(dalloc(h, &g.rc, (size_t)passcap * nr * kMS));
+    g.passcap = passcap;
   }
   return HIPFT_OK;
 }
 
-// Stage pairs (with the pair loop's slack) a step of length dt can need: one
+// Passes (with the pass loop's slack) a step of length dt can need: one
 // subcycle over the whole step at the smallest Euler limit bounds every
 // realization's stage count.
-static int graph_pairs_needed(const hipft_gpu *h, double dt) {
+static int graph_passes_needed(const hipft_gpu *h, double dt) {
   if (!h->P.advance_diffusion) return kGUnrollMax;
   double dte = h->dt_euler;
   if (h->ragged)
     for (double v : h->r_dt_euler) dte = std::min(dte, v);
   const int64_t s = sts_count(h->P.diffusion_num_method, dt, dte);
-  return (int)((s - 1) / 2) + kGUnrollMax;
+  return (int)sts_passes(s) + kGUnrollMax;
 }
 
 // Launch parameters a capture bakes in besides the buffers; any change (new
@@ -2400,7 +1932,7 @@ static std::vector<unsigned char> graph_key(const hipft_gpu *h) {
   add(&h->ptab, sizeof(h->ptab));
   const double bc[4] = {h->bc_flow_n, h->bc_flow_s, h->bc_diff_n, h->bc_diff_s};
   add(bc, sizeof(bc));
-  const int flags[6] = {h->ragged ? 1 : 0, h->cur, h->GA.paircap, h->g_pdl ? 1 : 0, h->auto_sc ? 1 : 0,
+  const int flags[6] = {h->ragged ? 1 : 0, h->cur, h->GA.passcap, h->g_pdl ? 1 : 0, h->auto_sc ? 1 : 0,
                         (int)h->P.diffusion_subcycles};
   add(flags, sizeof(flags));
   return k;
@@ -2451,22 +1983,25 @@ static int graph_capture(hipft_gpu *h) {
   G.subcycles = (int)h->P.diffusion_subcycles;
   G.ragged = h->ragged ? 1 : 0;
   G.strang = h->P.strang_splitting ? 1 : 0;
+  G.n2 = h->npm - 2;
+  G.strips = h->m_strips;
+  G.slots = h->m_slots;
+  G.poles = 2 * poles_ranks(h->npm - 2);
   G.nadv = (h->adv_time == 1) ? 1 : ((h->adv_time == 2) ? 3 : 4);
   {
     const char *e = std::getenv("HIPFT_GRAPH_UNROLL");
     const int u = e ? std::atoi(e) : kGUnrollMax;  // each iteration boundary costs ~11 us (tick, node relaunch)
     G.unroll = std::max(2, std::min(kGUnrollMax, u - u % 2));
   }
-  G.ring0 = h->d_ringbuf[0];
-  G.ring1 = h->d_ringbuf[1];
   const GArrays g = G;
   h->g_cur = h->cur;
   double *F = h->buf[h->cur];
-  double *Bd = h->buf[scratch(h, 0)];  // dty0
+  double *Bd = h->buf[scratch(h, 0)];  // A u0, then dty0
   double *R[4] = {h->buf[scratch(h, 1)], h->buf[scratch(h, 2)], h->buf[scratch(h, 3)], h->buf[scratch(h, 4)]};
   const Mesh M = h->M;
   const int64_t nfield = (int64_t)h->fieldn;
   const int cblocks = 4 * h->num_sms;
+  double *ring = h->d_ringbuf[0];
   cudaError_t first = cudaSuccess;
   auto ok = [&](cudaError_t e) {
     if (e != cudaSuccess && first == cudaSuccess) first = e;
@@ -2522,41 +2057,25 @@ static int graph_capture(hipft_gpu *h) {
     end_body(s1);
   };
 
-  // ---- one stage pair of the loop body: pair q of the iteration (q = 0..3)
-  const int nkt = (h->npm - 2 + kWK - 1) / kWK;
-  auto pair = [&](cudaStream_t s, int q, bool overlap) {
-    const bool even = (q % 2) == 0;
-    const double *ykm1 = even ? R[0] : R[2], *ykm2 = even ? R[3] : R[1];
-    double *ok_ = even ? R[1] : R[3], *ok1 = even ? R[2] : R[0];
-    const double *rin = even ? g.ring1 : g.ring0;
-    double *rout = even ? g.ring0 : g.ring1;
-    RingOut ro{rout, h->d_rpart, h->d_rcount, nkt};
-    PairArgs pa{StageCoef{}, StageCoef{}, h->d_err, g.rl_dif, g.rc};
-    pa.dctr = &g.st->pctr;
-    pa.doff = q;
-    pa.dnact = g.nactp;
-    pa.dstride = 2 * nr;
-    PairTables pt = h->ptab;
-    pt.ntiles = pt.nb * pt.nkt * nr;
-    const int grid = std::min(pt.ntiles, 2 * h->num_sms);
-    const WsMaps tmaps = ws_maps(h, ykm1, ykm2, F, Bd);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kWThreads);
-    cfg.dynamicSmemBytes = kWSmem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = (h->g_pdl && overlap) ? 1 : 0;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    ok(cudaLaunchKernelEx(&cfg, k_sts_pair_ws<true, false, true>, M, (const double *)h->DC.dfac, ykm1, ykm2,
-                          (const double *)F, (const double *)Bd, ok_, ok1, rin, h->bc_diff_n, h->bc_diff_s, pa, ro,
-                          pt, tmaps));
-    const dim3 pg((unsigned)nr, (unsigned)h->pole_nch);
-    k_pair_poles<<<pg, kPoleThreads, 0, s>>>(M, h->DC.dfac, ykm1, ykm2, F, Bd, ok1, rin, h->bc_diff_n,
-                                             h->bc_diff_s, pa, ro, h->pole);
-    peek();
+  // ---- one pass of the loop body: pass q of the iteration.  Its grid covers
+  // any number of realizations that may still take part.
+  int64_t pass_blocks = 1;
+  for (int n = 1; n <= nr && h->P.advance_diffusion; ++n) pass_blocks = std::max(pass_blocks, march_blocks(h, n));
+  auto pass = [&](cudaStream_t s, int q, bool after_pass) {
+    const int in = (q & 1) ? 0 : 2, out = 2 - in;
+    MarchArgs a = march_args(h, F, Bd);
+    a.x2 = R[in];
+    a.x1 = R[in + 1];
+    a.o[2] = R[out];
+    a.o[3] = R[out + 1];
+    a.rlist = g.rl_dif;
+    a.rc = g.rc;
+    a.dctr = &g.st->pctr;
+    a.doff = q;
+    a.dnact = g.nactp;
+    a.dstride = kMS * nr;
+    a.dcols = g.colsp;
+    ok(launch_pass(h, s, a, h->g_pdl, after_pass, pass_blocks));
   };
 
   // ---- diffusion_step over dt (src/hipft.f90:4551-4695)
@@ -2564,68 +2083,51 @@ static int graph_capture(hipft_gpu *h) {
     cudaGraphConditionalHandle hsub{};
     ok(g_handle(s0, &hsub));
     if (first != cudaSuccess) return;
-    k_g_dif_begin<<<1, 256, 0, s0>>>(g, h->ragged ? 0 : 1, hsub);
+    k_g_dif_begin<<<1, 256, 0, s0>>>(g, 0, hsub);
     peek();
-    // plain mode: the ring of the field once; later subcycles reuse the ring
-    // sums the last stage pair left (the gather moves them to ring0)
-    if (!h->ragged) {
-      k_ring_diffusion<<<nr, 256, 0, s0>>>(M, h->DC, F, g.ring0);
-      peek();
-    }
     begin_body(s0, hsub, s1);
     if (first != cudaSuccess) return;
-    int body_kernels = 1;  // the subcycle tick itself
-    if (h->ragged) {
-      k_ring_diffusion<<<nr, 256, 0, s1>>>(M, h->DC, F, g.ring0);
+    int body_kernels = 3;  // ring sums, A u0 and the subcycle tick
+    k_ring_diffusion<<<nr, 256, 0, s1>>>(M, h->DC, F, ring);
+    peek();
+    const dim3 blk(32, 8);
+    const dim3 grd((unsigned)((h->ntm + 31) / 32), (unsigned)((h->npm - 2 + 7) / 8), (unsigned)nr);
+    const int pr = h->ragged ? 1 : 0;
+    unsigned long long *bmax = g.bits, *bmin = g.bits + (h->ragged ? nr : 1);
+    if (h->auto_sc) {
+      k_g_ptl_reset<<<1, 256, 0, s1>>>(g);
+      peek();
+    }
+    k_diffusion_stage<MODE_AX><<<grd, blk, 0, s1>>>(M, h->DC, F, nullptr, nullptr, nullptr, Bd, nullptr, ring,
+                                                    h->bc_diff_n, h->bc_diff_s, StageCoef{},
+                                                    h->auto_sc ? bmax : nullptr, g.rl_ptl, pr);
+    peek();
+    if (h->auto_sc) {  // PTL (src/hipft.f90:5042-5161) of the active realizations
+      k_ptl<<<grd, blk, 0, s1>>>(M, F, Bd, bmax, bmin, g.rl_ptl, pr);
       peek();
       ++body_kernels;
     }
-    const dim3 blk(32, 8);
-    const dim3 grd((unsigned)((h->ntm + 31) / 32), (unsigned)((h->npm - 2 + 7) / 8), (unsigned)nr);
-    if (h->auto_sc) {  // PTL (src/hipft.f90:5042-5161) of the active realizations
-      k_g_ptl_reset<<<1, 256, 0, s1>>>(g);
-      peek();
-      const int pr = h->ragged ? 1 : 0;
-      unsigned long long *bmax = g.bits, *bmin = g.bits + (h->ragged ? nr : 1);
-      k_diffusion_stage<MODE_AX><<<grd, blk, 0, s1>>>(M, h->DC, F, nullptr, nullptr, nullptr, R[0], nullptr, g.ring0,
-                                                      h->bc_diff_n, h->bc_diff_s, StageCoef{}, bmax, g.rl_ptl, pr);
-      peek();
-      k_ptl<<<grd, blk, 0, s1>>>(M, F, R[0], bmax, bmin, g.rl_ptl, pr);
-      peek();
-      body_kernels += 2;
-    }
-    cudaGraphConditionalHandle hpair{};
-    ok(g_handle(s1, &hpair));
+    cudaGraphConditionalHandle hpass{};
+    ok(g_handle(s1, &hpass));
     if (first != cudaSuccess) return;
-    k_g_plan<<<1, 256, 0, s1>>>(g, hpair);
+    k_g_plan<<<1, 256, 0, s1>>>(g, hpass);
     peek();
-    const int64_t ncoef = (int64_t)g.paircap * nr;
+    const int64_t ncoef = (int64_t)g.passcap * nr;
     k_g_coefs<<<(unsigned)((ncoef + 255) / 256), 256, 0, s1>>>(g);
     peek();
-    // stage 1 (src/hipft.f90:5211-5218): Y_1 into R0, dty0; Y_0 = u0 into R3
-    {
-      const int nkb = (h->npm - 2 + kKPT3 - 1) / kKPT3;
-      RingOut ro{g.ring1, h->d_rpart, h->d_rcount, nkb};
-      const int jshift = (h->ntm % 2 == 1 && ((h->ntm - 1) / 2) % 32 == 0) ? 1 : 0;
-      const int nthr = (h->ntm + 2 * jshift + 1) / 2;
-      const dim3 g1((unsigned)((nthr + 127) / 128), (unsigned)nkb, (unsigned)nr);
-      k_sts_stage_v3<MODE_STS1, kKPT3><<<g1, 128, 0, s1>>>(M, h->DC.dfac, F, nullptr, nullptr, nullptr, R[0], Bd,
-                                                           g.ring0, h->bc_diff_n, h->bc_diff_s, StageCoef{}, ro,
-                                                           jshift, g.rl_dif, g.c1);
-      peek();
-      k_g_copy<<<cblocks, 256, 0, s1>>>(R[3], F, nfield);
-      peek();
-      body_kernels += 2;
-    }
-    begin_body(s1, hpair, s2);
+    k_scale<<<dim3((unsigned)std::min<int64_t>((h->plane / 2 + 255) / 256, cblocks), (unsigned)nr), 256, 0, s1>>>(
+        h->plane, Bd, Bd, 0.0, g.rl_dif, g.d);
+    peek();
+    ++body_kernels;
+    begin_body(s1, hpass, s2);
     if (first != cudaSuccess) return;
-    for (int q = 0; q < g.unroll; ++q) pair(s2, q, q > 0);
-    k_g_pair_tick<<<1, 1, 0, s2>>>(g, hpair);
+    for (int q = 0; q < g.unroll; ++q) pass(s2, q, q > 0);
+    k_g_pass_tick<<<1, 1, 0, s2>>>(g, h->ntm < kMMinRows ? 1 : 2, hpass);
     peek();
     end_body(s2);
-    // the result of each realization back into the field: Y_s is in R2 after
-    // an even last pair, in R0 after an odd one
-    k_g_gather<<<dim3((unsigned)nr, 64u), 256, 0, s1>>>(g, M, F, R[2], R[0]);
+    // the result of each realization back into the field: Y_s is in R1 after
+    // an even last pass, in R3 after an odd one
+    k_g_gather<<<dim3((unsigned)nr, 64u), 256, 0, s1>>>(g, M, F, R[1], R[3]);
     peek();
     k_g_sub_tick<<<1, 256, 0, s1>>>(g, body_kernels, hsub);
     peek();
@@ -2689,9 +2191,8 @@ static int graph_collect(hipft_gpu *h) {
 // One split step as one graph launch.
 static int graph_step(hipft_gpu *h, double dt, hipft_diffusion_info *info) {
   TRY(graph_collect(h));
-  if (h->P.advance_diffusion) TRY(ensure_pair_plan(h));
-  const int need = graph_pairs_needed(h, dt);
-  const bool grow = need > h->GA.paircap;
+  const int need = graph_passes_needed(h, dt);
+  const bool grow = need > h->GA.passcap;
   TRY(graph_alloc(h, grow ? need + need / 4 : need));
   if (h->cur != h->g_cur && h->g_cur >= 0) {
     // another entry point left the field elsewhere: back into the captured buffer
@@ -3161,19 +2662,7 @@ extern "C" int hipft_gpu_info(const hipft_gpu *h, hipft_info *info) {
 
 extern "C" int hipft_gpu_describe(hipft_gpu *h, char *buf, size_t len) {
   if (!h || !buf || !len) return HIPFT_EINVAL;
-  const PairPlan &p = h->plan;
-  char kind[128];
-  if (p.kind < 0)
-    std::snprintf(kind, sizeof kind, "not chosen yet");
-  else if (p.kind == PK_SINGLE)
-    std::snprintf(kind, sizeof kind, "%s", pair_kind_name(p.kind));
-  else
-    std::snprintf(kind, sizeof kind, "%s, %d CTAs per SM", pair_kind_name(p.kind), p.ctas_per_sm);
-  if (p.candidates > 0)
-    std::snprintf(buf, len, "schedule=%s; two-stage kernel: %s (tuned over %d candidates, %.4f ms per launch pair)",
-                  h->ragged ? "ragged" : "shared", kind, p.candidates, p.ms);
-  else
-    std::snprintf(buf, len, "schedule=%s; two-stage kernel: %s", h->ragged ? "ragged" : "shared", kind);
+  std::snprintf(buf, len, "schedule=%s; RKG2 kernel: ws-quad (four stages per pass)", h->ragged ? "ragged" : "shared");
   return HIPFT_OK;
 }
 
@@ -3492,7 +2981,6 @@ static int adj_adv_fwd(hipft_gpu *h, double dtl, size_t &nt, size_t t[4]) {
 // stage fields are kept; same subcycle logic as hipft_gpu_diffusion_step.
 static int adj_diff_fwd(hipft_gpu *h, double dtl, size_t &nt, std::vector<AdjSub> &subs) {
   const int max_sc = 60;
-  TRY(ensure_pair_plan(h));
   int i = 1;
   bool done = false;
   double time_stepped = 0.0;
@@ -3526,7 +3014,8 @@ static int adj_diff_fwd(hipft_gpu *h, double dtl, size_t &nt, std::vector<AdjSub
       for (int64_t k = 1; k <= S.s - 1; ++k) TRY(adj_slot(h, nt++, &Y[k]));
     } else {
       // block starts c = 1, 1+q, ... below s; their pairs (Y_{c-1}, Y_c) are
-      // tape slots, the other stages go through a rotating scratch set
+      // tape slots; of the other stages a pass keeps its last two, which the
+      // next pass reads, in a rotating scratch set
       for (int64_t c = 1; c <= S.s - 1; c += S.q) S.cstart.push_back(c);
       for (size_t b = 0; b < S.cstart.size(); ++b) {
         const int64_t c = S.cstart[b];
@@ -3538,69 +3027,33 @@ static int adj_diff_fwd(hipft_gpu *h, double dtl, size_t &nt, std::vector<AdjSub
         S.ck_cur.push_back(nt);
         TRY(adj_slot(h, nt++, &Y[c]));
       }
-      S.ring0 = h->adj_rings_n;
-      h->adj_rings_n += S.cstart.size();
-      if (h->adj_rings_n > h->adj_rings_cap) {
-        // grown before any ring checkpoint of this step is written
-        double *nr_ = nullptr;
-        const size_t cap = h->adj_rings_n + 64;
-        TRY(dalloc(h, &nr_, cap * 2 * (size_t)h->nr));
-        if (h->d_adj_rings) {
-          CK(h, cudaMemcpyAsync(nr_, h->d_adj_rings, h->adj_rings_cap * 2 * (size_t)h->nr * sizeof(double),
-                                cudaMemcpyDeviceToDevice, h->stream));
-          CK(h, cudaStreamSynchronize(h->stream));
-          cudaFree(h->d_adj_rings);
-          h->allocs.erase(std::remove(h->allocs.begin(), h->allocs.end(), (void *)h->d_adj_rings), h->allocs.end());
-        }
-        h->d_adj_rings = nr_;
-        h->adj_rings_cap = cap;
-      }
-      // stages that are not checkpoints rotate through four scratch fields
-      // of the block buffer: a stage pair reads Y_{k-1}, Y_{k-2} and writes
-      // Y_k, Y_{k+1}, four distinct fields
       while (h->adj_block.size() < 4) {
         double *q = nullptr;
         TRY(dalloc(h, &q, h->fieldn));
         h->adj_block.push_back(q);
       }
-      int rot = 0;
-      for (int64_t k = 1; k <= S.s - 1; ++k)
-        if (!Y[k]) Y[k] = h->adj_block[(rot++) % 4];
     }
     Y[S.s] = h->buf[h->cur];
     CK(h, cudaMemcpyAsync(u0, h->buf[h->cur], h->fieldn * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    // the same kernels, in the same order, as sts_super_step (with its pole
-    // sums of the current field), writing every stage into the tape
-    const double *r0;
-    TRY(current_dring(h, &r0));
-    TRY(sts_stage_v2<MODE_STS1>(h, u0, nullptr, nullptr, nullptr, Y[1], dty0, StageCoef{dtl2, S.ubj[1], 0, 0, 0}));
-    auto coef = [&](int64_t k) {
-      const double uj = S.uj[k], vj = S.vj[k];
-      return StageCoef{uj, vj, 1.0 - uj - vj, S.ubj[k] * dtl2, S.gj[k]};
-    };
-    // ring sums of a block start's Y_c (the ring of the launch's output)
-    auto keep_ring = [&](int64_t c) -> int {
-      if (S.q == 0) return HIPFT_OK;
-      for (size_t b = 0; b < S.cstart.size(); ++b)
-        if (S.cstart[b] == c)
-          CK(h, cudaMemcpyAsync(h->d_adj_rings + (S.ring0 + b) * 2 * (size_t)h->nr, h->d_ringbuf[h->ring_cur],
-                                2 * (size_t)h->nr * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-      return HIPFT_OK;
-    };
-    TRY(keep_ring(1));
-    int64_t k = 2;
-    while (k <= S.s) {
-      if (sts_pairs_enabled(h) && k + 1 <= S.s) {
-        TRY(sts_pair(h, Y[k - 1], Y[k - 2], u0, dty0, Y[k], Y[k + 1], coef(k), coef(k + 1), k > 2));
-        TRY(keep_ring(k + 1));
-        k += 2;
-        continue;
+    // the passes of sts_super_step, with the tape's stages kept
+    if (!h->auto_sc) TRY(current_lap(h));
+    TRY(scale_dty0(h, h->buf[scratch(h, 0)], dty0, dtl2));
+    MarchArgs a = march_args(h, u0, dty0);
+    const int64_t np = sts_passes(S.s), pad = kMS * np - S.s;
+    for (int64_t p = 0; p < np; ++p) {
+      for (int q = 0; q < kMS; ++q) {
+        const int64_t k = kMS * p + q + 1 - pad;
+        a.c[q] = sts_slot(h->P.diffusion_num_method, S.s, kMS * p + q, dtl2);
+        a.o[q] = (k >= 1) ? Y[k] : nullptr;
+        if (q >= 2 && !a.o[q]) a.o[q] = S.q ? h->adj_block[2 * (p & 1) + q - 2] : h->buf[scratch(h, q - 1)];
       }
-      TRY(sts_stage_v2<MODE_STSK>(h, Y[k - 1], Y[k - 2], u0, dty0, Y[k], nullptr, coef(k)));
-      TRY(keep_ring(k));
-      k += 1;
+      a.first = p == 0;
+      TRY(sts_pass(h, a, p > 0));
+      a.x2 = a.o[kMS - 2];
+      a.x1 = a.o[kMS - 1];
     }
-    h->dring_valid = true;  // the last fused stage left the ring of the output
+    TRY(seam(h, Y[S.s]));
+    h->dring_valid = false;
     h->cell_updates += (int64_t)h->ntm * (h->npm - 2) * h->nr * S.s;
     subs.push_back(std::move(S));
     time_stepped = time_stepped + dtl2;
@@ -3651,36 +3104,31 @@ static int adj_adv_rev(hipft_gpu *h, double dtl, const size_t t[4], double *&W, 
 // sum mu~_k dt <A^T Wbar_k, Y_{k-1}> (+ dt <A^T dbar, u0>).  One launch per
 // stage: each leaves the pole-row partials of its output for the next.
 // Recomputes the stages Y_{c+1}..Y_e of stage-checkpoint block b (e = the
-// block's last stage input, at most s-1) from its pair (Y_{c-1}, Y_c) and the
-// ring sums of Y_c, with the replay's kernels and launch grouping, so the
-// values are bitwise those of the replay.  Y receives the block's fields.
+// block's last stage input, at most s-1) from its pair (Y_{c-1}, Y_c); the
+// values do not depend on how the stages are grouped into passes, so they are
+// bitwise those of the replay.  Y receives the block's fields.
 static int adj_block_recompute(hipft_gpu *h, const AdjSub &S, size_t b, std::vector<const double *> &Y) {
   const int64_t c = S.cstart[b], e = std::min(c + S.q - 1, S.s - 1);
-  while ((int64_t)h->adj_block.size() < S.q + 1) {
+  while ((int64_t)h->adj_block.size() < S.q + kMS - 1) {
     double *q = nullptr;
     TRY(dalloc(h, &q, h->fieldn));
     h->adj_block.push_back(q);
   }
   const double *u0 = h->tape[S.t0], *dty0 = h->tape[S.t0 + 1];
-  std::vector<double *> Yw((size_t)S.s + 2, nullptr);
+  std::vector<double *> Yw((size_t)(e + kMS) + 1, nullptr);
   Yw[c - 1] = (S.ck_prev[b] == SIZE_MAX) ? const_cast<double *>(u0) : h->tape[S.ck_prev[b]];
   Yw[c] = h->tape[S.ck_cur[b]];
-  for (int64_t k = c + 1; k <= std::min(e + 1, S.s); ++k) Yw[k] = h->adj_block[k - c - 1];
-  CK(h, cudaMemcpyAsync(h->d_ringbuf[h->ring_cur], h->d_adj_rings + (S.ring0 + b) * 2 * (size_t)h->nr,
-                        2 * (size_t)h->nr * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-  auto coef = [&](int64_t k) {
-    const double uj = S.uj[k], vj = S.vj[k];
-    return StageCoef{uj, vj, 1.0 - uj - vj, S.ubj[k] * S.dtl, S.gj[k]};
-  };
-  int64_t k = c + 1;
-  while (k <= e) {
-    if (sts_pairs_enabled(h) && k + 1 <= S.s) {
-      TRY(sts_pair(h, Yw[k - 1], Yw[k - 2], u0, dty0, Yw[k], Yw[k + 1], coef(k), coef(k + 1), k > c + 1));
-      k += 2;
-      continue;
+  for (int64_t k = c + 1; k < e + kMS; ++k) Yw[k] = h->adj_block[k - c - 1];
+  MarchArgs a = march_args(h, u0, dty0);
+  const int64_t pad = kMS * sts_passes(S.s) - S.s;
+  for (int64_t k = c + 1; k <= e; k += kMS) {
+    a.x2 = Yw[k - 2];
+    a.x1 = Yw[k - 1];
+    for (int q = 0; q < kMS; ++q) {
+      a.c[q] = sts_slot(h->P.diffusion_num_method, S.s, k + q - 1 + pad, S.dtl);
+      a.o[q] = Yw[k + q];
     }
-    TRY(sts_stage_v2<MODE_STSK>(h, Yw[k - 1], Yw[k - 2], u0, dty0, Yw[k], nullptr, coef(k)));
-    k += 1;
+    TRY(sts_pass(h, a, k > c + 1));
   }
   for (int64_t q = c - 1; q <= e; ++q) Y[q] = Yw[q];
   h->dring_valid = false;
@@ -3837,7 +3285,6 @@ static int adj_record(hipft_gpu *h, double dt) {
   AdjRec R;
   R.dt = dt;
   R.first = h->adj_top;
-  R.ring_first = h->adj_rings_n;
   size_t nt = h->adj_top;
   const bool strang = h->P.strang_splitting != 0;
   const double da = strang ? 0.5 * dt : dt;
@@ -3864,7 +3311,6 @@ static int adj_reverse(hipft_gpu *h, double *fbar, double *dacc, double *gflow) 
   if (h->P.advance_flow) TRY(adj_adv_rev(h, da, R.ta1, W, gflow));
   CK(h, cudaMemcpyAsync(fbar, W, bytes, cudaMemcpyDeviceToDevice, h->stream));
   h->adj_top = R.first;
-  h->adj_rings_n = R.ring_first;
   h->adj_recs.pop_back();
   h->dring_valid = false;
   return HIPFT_OK;
@@ -3904,7 +3350,6 @@ extern "C" int hipft_adj_clear(hipft_gpu *h) {
   if (!h) return HIPFT_EINVAL;
   h->adj_recs.clear();
   h->adj_top = 0;
-  h->adj_rings_n = 0;
   h->adj_free_seen = 0;
   return HIPFT_OK;
 }
@@ -3957,7 +3402,6 @@ extern "C" int hipft_adj_release(hipft_gpu *h) {
   h->adj_top = 0;
   h->adj_top_max = 0;
   h->adj_free_seen = 0;
-  h->adj_rings_n = 0;
   return HIPFT_OK;
 }
 

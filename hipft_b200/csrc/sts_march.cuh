@@ -1,0 +1,761 @@
+// Four RKG2/RKL2 stages per pass over the field.
+//
+// Stages k..k+3 of diffusion_step_sts_cd (src/hipft.f90:5222-5237) with the
+// 5-point operator of diffusion_operator_cd (src/hipft.f90:7927-7984), in two
+// kernels that run side by side:
+//
+//  * k_sts_march, the rows whose four stages never reach a pole row: one warp
+//    marches along phi over a strip of theta rows and keeps the stages'
+//    windows in registers;
+//  * k_sts_poles, the four rows next to each pole: their stages need the pole
+//    ring sums of every stage over all phi columns (src/hipft.f90:7969-7979),
+//    so one thread-block cluster per realization and pole holds the strip in
+//    shared memory and reduces the sums through distributed shared memory.
+//
+// A super-step of s stages takes ceil(s / 4) passes.  Its stages are
+// numbered from the back: the last pass ends with stage s, and the slots of
+// the first pass before stage 1 leave Y = u0 (s is odd, so one or three of
+// them).  Stage 1 (src/hipft.f90:5211-5218) is the combine with only u0 and
+// dty0.  The first pass therefore reads u0 and dty0 alone.
+//
+// Every cell value is computed by the expressions of the single-stage
+// operator in their order, whatever strip, chunk or pass it falls in, so the
+// fields do not depend on how the stages are grouped.
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include "kernels.cuh"
+
+namespace hipft {
+
+// Coefficient tables, in load_diffusion_matrix's operation order
+// (src/hipft.f90:6880-6920) for a per-realization constant D:
+//   rows    [nr][3][LR]: entry jj of the three arrays holds theta row j = jj-1:
+//           st_i(j), Dh dth_i(j) dt_i(j) st_i(j) sth(j), Dh dth_i(j+1) dt_i(j) st_i(j) sth(j+1)
+//           for 2 <= j <= ntm-1, zeros elsewhere;
+//   columns [nr][LC][2]: entry kk >= -kColPad holds phi column kk mapped onto the interior
+//           column kw in 2..npm-1 it duplicates: {Dh dph_i(kw) dp_i(kw), Dh dph_i(kw+1) dp_i(kw)}.
+constexpr int kColPad = 8;  // entries before column 0 and after column npm
+struct PairTables {
+  const double *row, *col;  // k_pair_tables output; col points at entry 0 of the first realization
+  int LR, LC;               // entries per realization
+};
+
+__global__ void k_pair_tables(Mesh m, const double *__restrict__ dfac, int LR, int LC, double *rowtab,
+                              double *coltab) {
+  const int64_t nrow = (int64_t)m.nr * LR, ncol = (int64_t)m.nr * LC;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nrow + ncol;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    if (e < nrow) {
+      const int i = (int)(e / LR) + 1, j = (int)(e % LR) - 1;
+      const double Dr = dfac[i];
+      const double Dh = kHalf * (Dr + Dr);
+      double st = 0.0, c2 = 0.0, c4 = 0.0;
+      if (j >= 2 && j <= m.ntm - 1) {
+        st = m.st_i[j];
+        c2 = Dh * m.dth_i[j] * m.dt_i[j] * st * m.sth[j];
+        c4 = Dh * m.dth_i[j + 1] * m.dt_i[j] * st * m.sth[j + 1];
+      }
+      double *o = rowtab + (int64_t)(i - 1) * 3 * LR + (e % LR);
+      o[0] = st;
+      o[LR] = c2;
+      o[2 * LR] = c4;
+    } else {
+      const int64_t f = e - nrow;
+      const int i = (int)(f / LC) + 1, kk = (int)(f % LC) - kColPad;
+      const int n2 = m.npm - 2;
+      const int kw = ((kk - 2) % n2 + n2) % n2 + 2;
+      const double Dr = dfac[i];
+      const double Dh = kHalf * (Dr + Dr);
+      coltab[2 * f] = Dh * m.dph_i[kw] * m.dp_i[kw];
+      coltab[2 * f + 1] = Dh * m.dph_i[kw + 1] * m.dp_i[kw];
+    }
+  }
+}
+
+// Exercises the error path of the bounded waits: waits for phase 0 of an
+// mbarrier that expects one arrival nobody makes, gives up after `limit`
+// polls, sets the error flag and returns.
+__global__ void k_wait_selftest(uint32_t limit, int *err) {
+  __shared__ uint64_t bar;
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    fence_mbar_init();
+  }
+  __syncthreads();
+  if (!mbar_wait_bounded(&bar, 0, limit) && threadIdx.x == 0) atomicExch(err, 1);
+}
+
+// ------------------------------------------------------------ one pass
+constexpr int kMS = 4;                      // stages per pass
+constexpr int kMOwn = 64 - 2 * kMS;         // theta rows a strip owns of the 64 it holds
+constexpr int kMWarps = 4;                  // warps per block of k_sts_march
+constexpr int kMBlocks = 3;                 // its blocks per SM (at most 168 registers)
+constexpr int kMGroup = 4;                  // columns per turn of its loop
+constexpr int kMSlots = 2 * kMGroup;        // columns of its shared-memory ring
+constexpr int kMRing = kMSlots * 4 * 64;    // doubles per warp: Y_{k-1}, Y_{k-2}, u0, dty0
+constexpr int kMCoef = 5 * kMS;             // the pass's stage coefficients
+constexpr size_t kMSmem = ((size_t)kMWarps * kMRing + kMCoef) * sizeof(double);
+constexpr int kMMinRows = 2 * kMS;          // smallest ntm of the strip kernels (k_sts_whole below it)
+
+struct MarchArgs {
+  const double *x1, *x2;  // Y_{k-1}, Y_{k-2} (not read in a super-step's first pass)
+  const double *u, *d;    // u0, dty0
+  double *o[kMS];         // Y_k .. Y_{k+3}; null: not kept
+  int first;              // this is the first pass of the super-step
+  int nreal;              // realizations of the launch
+  StageCoef c[kMS];       // the stages' coefficients, one set for all realizations ...
+  // ... or per realization (then the launch advances the realizations in
+  // rlist): rc[(i-1) * kMS + stage]
+  const int *rlist;
+  const StageCoef *rc;
+  // steps run as a CUDA graph (with rlist and rc): the pass is *dctr + doff,
+  // read on the device; dnact[pass] realizations of rlist take part and rc
+  // holds dstride coefficients per pass
+  const int *dctr;
+  int doff;
+  const int *dnact;
+  int dstride;
+  const int *dcols;       // ... and dcols[pass] the columns per warp
+  int strips, cols;       // theta strips, columns per warp (march_cols)
+  const double *dfac;     // [nr+1]
+  double bcn, bcs;        // pole factors
+};
+
+// Stage slot q (0-based, over the whole super-step) of an s-stage super-step
+// of length dtl: stage k = q + 1 - pad, pad = the slots of the first pass
+// before stage 1.
+__host__ __device__ inline int64_t sts_passes(int64_t s) { return (s + kMS - 1) / kMS; }
+__host__ __device__ inline StageCoef sts_slot(int method, int64_t s, int64_t q, double dtl) {
+  const int64_t k = q + 1 - (kMS * sts_passes(s) - s);
+  if (k < 1 || k > s) return StageCoef{0.0, 0.0, 1.0, 0.0, 0.0};
+  if (k == 1) {
+    double uj, vj, ubj, gj;
+    sts_stage(method, s, 1, uj, vj, ubj, gj);
+    return StageCoef{0.0, 0.0, 1.0, 0.0, ubj};
+  }
+  return sts_combine(method, s, k, dtl);
+}
+
+// Phi columns per warp, a multiple of kMGroup: the fewest full waves of
+// resident warps that keep the chunk at kMColsMax columns or less (a chunk
+// loads 2 kMS columns more than it owns, so longer chunks waste less; whole
+// waves leave no nearly empty one).  A block of k_sts_poles takes the place of
+// the blocks of an SM; a single wave leaves those SMs out, which would
+// otherwise start a second one.
+constexpr int kMColsMax = 96;
+__host__ __device__ inline int march_cols(int n2, int strips, int nreal, int slots, int poles) {
+  const int64_t per = (int64_t)strips * (nreal > 0 ? nreal : 1) * kMWarps;
+  for (int64_t w = 1;; ++w) {
+    int64_t free = w * slots;
+    const int64_t taken = (int64_t)poles * nreal * kMBlocks * kMWarps;
+    if (w == 1 && taken <= slots / 2) free -= taken;
+    const int64_t nch = free / per * kMWarps;  // whole blocks of chunks
+    if (nch < 1) continue;
+    const int64_t c = ((n2 + nch - 1) / nch + kMGroup - 1) / kMGroup * kMGroup;
+    if (c <= kMColsMax) return (int)c;
+  }
+}
+
+// The launch's realizations and coefficients.
+__device__ __forceinline__ void march_launch(const MarchArgs &a, int &nreal, bool &first, const StageCoef *&rc,
+                                             int &cols) {
+  nreal = a.nreal;
+  first = a.first != 0;
+  rc = a.rc;
+  cols = a.cols;
+  if (a.dctr) {
+    const int p = *a.dctr + a.doff;
+    nreal = a.dnact[p];
+    first = p == 0;
+    rc = a.rc + (int64_t)p * a.dstride;
+    cols = a.dcols[p];
+  }
+}
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ double2 lds2(uint32_t a) {
+  double2 v;
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a));
+  return v;
+}
+
+template <int N>
+struct IntC {
+  static constexpr int value = N;
+};
+
+// phi-neighbour coefficients and the diagonal of a row pair in one column
+struct PhiCoef {
+  double2 c1, c3, c5;
+};
+__device__ __forceinline__ PhiCoef phi_coef(double2 st, double2 c2, double2 c4, double2 P) {
+  PhiCoef r;
+  r.c1 = make_double2(P.x * st.x * st.x, P.x * st.y * st.y);
+  r.c5 = make_double2(P.y * st.x * st.x, P.y * st.y * st.y);
+  r.c3 = make_double2(-(r.c1.x + c2.x + c4.x + r.c5.x), -(r.c1.y + c2.y + c4.y + r.c5.y));
+  return r;
+}
+
+// One stage of a row pair (a, a+1) in one column: xl, xc, xr the stage input
+// in columns c-1, c, c+1; up, dn the rows a-1 and a+2 of column c; o2 the
+// combine's second input.
+__device__ __forceinline__ double2 pair_stage(double2 xl, double2 xc, double2 xr, double up, double dn,
+                                              const PhiCoef &c, double2 c2, double2 c4, double2 o2, double2 u,
+                                              double2 d, const StageCoef &sc) {
+  const double ax = c.c1.x * xl.x + c2.x * up + c.c3.x * xc.x + c4.x * xc.y + c.c5.x * xr.x;
+  const double ay = c.c1.y * xl.y + c2.y * xc.x + c.c3.y * xc.y + c4.y * dn + c.c5.y * xr.y;
+  return make_double2(sc.a * xc.x + sc.b * o2.x + sc.c * u.x + sc.d * ax + sc.e * d.x,
+                      sc.a * xc.y + sc.b * o2.y + sc.c * u.y + sc.d * ay + sc.e * d.y);
+}
+
+// Four stages of the rows kMS+1 .. ntm-kMS.
+//
+// A warp holds 64 theta rows, two per lane, and marches along the phi columns
+// of its chunk.  At the step that brings in column e of Y_{k-1}, stage k is
+// computed in column e-1, stage k+1 in e-2, stage k+2 in e-3 and stage k+3 in
+// e-4: each stage's input is the window of three columns that the stage before
+// it left in registers, the second input is one of those as well, and the
+// rows above and below come from the neighbouring lanes by shuffles.  The
+// outermost rows of the strip lose one row per stage, so a strip owns the 56
+// rows in its middle; strips start 56 rows apart at row 1, which makes the
+// rows lost at the poles exactly those that k_sts_poles computes.  The
+// column's phi coefficients are formed once and move on with the stages.
+// Y_{k-1}, Y_{k-2}, u0 and dty0 arrive three columns ahead through a ring in
+// shared memory, by asynchronous copies in which every lane fetches its own
+// two rows: no barriers, and warps are independent.  The loop takes kMGroup
+// columns per turn, so that windows, coefficients and ring slots are renamed
+// and not moved.  The four warps of a block march four neighbouring chunks of
+// one strip.  Seam columns are not written (nothing reads them in a stage).
+//
+// Bound: the FP64 pipe.  A pair of rows costs 4 x 36 + 14 instructions per
+// column (no contraction: every product is rounded as in the reference), and
+// 64/56 of that for the strip's halo; HBM sees 4 reads and 2 writes of 8 bytes
+// per cell and four stages.
+//
+// TABLE: coefficients per realization; KEEP: Y_k and Y_{k+1} are kept too;
+// Off: a byte offset within a realization's plane.
+template <bool TABLE, bool KEEP, typename Off>
+__global__ void __launch_bounds__(32 * kMWarps, kMBlocks) k_sts_march(Mesh m, MarchArgs a, PairTables pt) {
+  extern __shared__ __align__(16) double msm[];
+  pdl_trigger();  // the next pass's k_sts_poles may take its place on the SMs; it waits for this grid's end
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int npm = m.npm, n2 = npm - 2, ntm = m.ntm;
+  int nreal;
+  bool first;
+  const StageCoef *rc;
+  int ncol;
+  march_launch(a, nreal, first, rc, ncol);
+  const int nch = (n2 + ncol - 1) / ncol, nblk = (nch + kMWarps - 1) / kMWarps;
+  const int strip = blockIdx.x % a.strips;
+  const int rest = blockIdx.x / a.strips;
+  const int c0 = 2 + ((rest % nblk) * kMWarps + warp) * ncol, c1 = min(c0 + ncol - 1, npm - 1);
+  if (rest / nblk >= nreal) {
+    pdl_wait();
+    return;
+  }
+  const int i = a.rlist ? a.rlist[rest / nblk] : rest / nblk;  // 0-based
+  double *coef = msm + kMWarps * kMRing;
+  if (TABLE) {
+    if (threadIdx.x < kMCoef) coef[threadIdx.x] = reinterpret_cast<const double *>(rc + (int64_t)i * kMS)[threadIdx.x];
+    __syncthreads();
+  }
+  if (c0 > npm - 1) {
+    pdl_wait();
+    return;
+  }
+  const int r = 1 + kMOwn * strip + 2 * lane;  // this lane's rows r, r+1
+  const double *R = pt.row + (int64_t)i * 3 * pt.LR;  // entry jj holds row jj-1
+  const int e0 = min(r + 1, pt.LR - 1), e1 = min(r + 2, pt.LR - 1);
+  const double2 st = make_double2(R[e0], R[e1]);
+  const double2 c2 = make_double2(R[pt.LR + e0], R[pt.LR + e1]);
+  const double2 c4 = make_double2(R[2 * pt.LR + e0], R[2 * pt.LR + e1]);
+  const bool own = lane >= kMS / 2 && lane < 32 - kMS / 2;
+  const bool va = own && r <= ntm - kMS, vb = own && r + 1 <= ntm - kMS;
+
+  // byte offsets within the realization's plane; rows past the end of the
+  // column repeat its last pair (no owned row reads them)
+  const int64_t pb = (int64_t)i * m.plane;
+  const Off ldb = (Off)m.ldt * 8;
+  const Off rowb = (Off)min(r - 1, m.ldt - 2) * 8;
+  const char *gx1 = reinterpret_cast<const char *>((first ? a.u : a.x1) + pb);
+  const char *gx2 = reinterpret_cast<const char *>((first ? a.u : a.x2) + pb);
+  const char *gu = reinterpret_cast<const char *>(a.u + pb), *gd = reinterpret_cast<const char *>(a.d + pb);
+  const double2 *pt_col = reinterpret_cast<const double2 *>(pt.col) + (int64_t)i * pt.LC;
+  char *o0 = reinterpret_cast<char *>(a.o[0] + pb), *o1 = reinterpret_cast<char *>(a.o[1] + pb);
+  char *o2 = reinterpret_cast<char *>(a.o[2] + pb), *o3 = reinterpret_cast<char *>(a.o[3] + pb);
+  const bool k0keep = KEEP && a.o[0], k1keep = KEEP && a.o[1];
+
+  constexpr uint32_t kF = 512, kSlot = 4 * kF;  // bytes of one field in a slot, of a slot
+  const uint32_t sring = smem_addr(msm) + (uint32_t)warp * (kMRing * 8) + 16u * lane;
+  // column to fetch next, its offset, and the columns left to fetch
+  int fc = c0 - kMS, left = c1 - c0 + 1 + 2 * kMS;
+  if (fc < 2) fc += n2;
+  Off fo = (Off)(fc - 1) * ldb + rowb;
+  auto fetch = [&](uint32_t s) {
+    if (left > 0) {
+      cp_async16(s, gx1 + fo);
+      cp_async16(s + kF, gx2 + fo);
+      cp_async16(s + 2 * kF, gu + fo);
+      cp_async16(s + 3 * kF, gd + fo);
+    }
+    cp_async_commit();
+    --left;
+    fo += ldb;
+    if (++fc > npm - 1) {
+      fc = 2;
+      fo -= (Off)n2 * ldb;
+    }
+  };
+  fetch(sring);
+  fetch(sring + kSlot);
+  fetch(sring + 2 * kSlot);
+
+  auto put = [&](char *o, Off off, double2 y) {
+    if (vb) *reinterpret_cast<double2 *>(o + off) = y;
+    else if (va) *reinterpret_cast<double *>(o + off) = y.x;
+  };
+  // Step of column e = the j-th of its group (compile-time j, n = step number
+  // while the windows fill): W[s] holds columns e-2, e-1 of stage s's input
+  // at W[s][j & 1], W[s][1 - (j & 1)], K[q & 3] the phi coefficients of the
+  // column at position q of the turn; sa, sb: this turn's and the other half
+  // of the ring.
+  double2 W[kMS][2] = {};
+  PhiCoef K[4] = {};
+  int oc = -2 * kMS;                               // column e-4, counted from c0
+  Off wo = (Off)(c0 - 1 - 2 * kMS) * ldb + rowb;   // its offset
+  const int nown = c1 - c0 + 1;
+  const double2 *pp = pt_col + (c0 - kMS);
+  double2 Pn = pp[-1];  // the column table's entry of column e-1
+  auto step = [&](auto jc, auto nc, uint32_t sa, uint32_t sb) {
+    constexpr int j = decltype(jc)::value, n = decltype(nc)::value;  // n: 2 kMS and more: all stages
+    constexpr int A = j & 1, B = 1 - A;
+    auto slot = [&](int back) { return j >= back ? sa + (uint32_t)(j - back) * kSlot : sb + (uint32_t)(j - back + kMGroup) * kSlot; };
+    cp_async_wait<2>();
+    const double2 x0 = lds2(slot(0));
+    if (n >= 2) {
+      K[(j + 3) & 3] = phi_coef(st, c2, c4, Pn);
+    }
+    Pn = *pp++;
+    const StageCoef *q = TABLE ? reinterpret_cast<const StageCoef *>(coef) : a.c;
+    double2 y0 = {}, y1 = {}, y2 = {};
+    if (n >= 2) {
+      const uint32_t s = slot(1);
+      const double2 xc = W[0][B];
+      const double up = __shfl_up_sync(0xffffffffu, xc.y, 1), dn = __shfl_down_sync(0xffffffffu, xc.x, 1);
+      y0 = pair_stage(W[0][A], xc, x0, up, dn, K[(j + 3) & 3], c2, c4, lds2(s + kF), lds2(s + 2 * kF), lds2(s + 3 * kF),
+                      q[0]);
+      if (KEEP && n >= 5 && k0keep && oc + 3 < nown) put(o0, wo + 3 * ldb, y0);
+    }
+    if (n >= 4) {
+      const uint32_t s = slot(2);
+      const double2 xc = W[1][B];
+      const double up = __shfl_up_sync(0xffffffffu, xc.y, 1), dn = __shfl_down_sync(0xffffffffu, xc.x, 1);
+      y1 = pair_stage(W[1][A], xc, y0, up, dn, K[(j + 2) & 3], c2, c4, W[0][A], lds2(s + 2 * kF), lds2(s + 3 * kF), q[1]);
+      if (KEEP && n >= 6 && k1keep && oc + 2 < nown) put(o1, wo + 2 * ldb, y1);
+    }
+    if (n >= 6) {
+      const uint32_t s = slot(3);
+      const double2 xc = W[2][B];
+      const double up = __shfl_up_sync(0xffffffffu, xc.y, 1), dn = __shfl_down_sync(0xffffffffu, xc.x, 1);
+      y2 = pair_stage(W[2][A], xc, y1, up, dn, K[(j + 1) & 3], c2, c4, W[1][A], lds2(s + 2 * kF), lds2(s + 3 * kF), q[2]);
+      if (n >= 7 && oc + 1 < nown) put(o2, wo + ldb, y2);
+    }
+    if (n >= 8) {
+      const uint32_t s = slot(4);
+      const double2 xc = W[3][B];
+      const double up = __shfl_up_sync(0xffffffffu, xc.y, 1), dn = __shfl_down_sync(0xffffffffu, xc.x, 1);
+      const double2 y3 =
+          pair_stage(W[3][A], xc, y2, up, dn, K[j & 3], c2, c4, W[2][A], lds2(s + 2 * kF), lds2(s + 3 * kF), q[3]);
+      if (oc < nown) put(o3, wo, y3);
+    }
+    W[0][A] = x0;
+    W[1][A] = y0;
+    W[2][A] = y1;
+    W[3][A] = y2;
+    ++oc;
+    wo += ldb;
+    fetch(j + 3 < kMGroup ? sa + (j + 3) * kSlot : sb + (j + 3 - kMGroup) * kSlot);
+  };
+  uint32_t sa = sring, sb = sring + kMGroup * kSlot;
+  step(IntC<0>{}, IntC<0>{}, sa, sb);
+  step(IntC<1>{}, IntC<1>{}, sa, sb);
+  step(IntC<2>{}, IntC<2>{}, sa, sb);
+  step(IntC<3>{}, IntC<3>{}, sa, sb);
+  step(IntC<0>{}, IntC<4>{}, sb, sa);
+  step(IntC<1>{}, IntC<5>{}, sb, sa);
+  step(IntC<2>{}, IntC<6>{}, sb, sa);
+  step(IntC<3>{}, IntC<7>{}, sb, sa);
+#pragma unroll 1
+  for (int t = 0; t < nown; t += kMGroup) {
+    step(IntC<0>{}, IntC<8>{}, sa, sb);
+    step(IntC<1>{}, IntC<8>{}, sa, sb);
+    step(IntC<2>{}, IntC<8>{}, sa, sb);
+    step(IntC<3>{}, IntC<8>{}, sa, sb);
+    const uint32_t x = sa;
+    sa = sb;
+    sb = x;
+  }
+  cp_async_wait<0>();
+  // this grid ends after the pole strips' grid, so that the next pass, which
+  // waits for this one, has both
+  pdl_wait();
+}
+
+// Four stages of the rows 1..kMS and ntm-kMS+1..ntm: one cluster per
+// realization and pole, whose blocks share the phi columns, each with a halo
+// of kMS columns.  Strip row q = 0..7 is theta row q+1 (north) or ntm-q
+// (south); the rows still right after stage s are 0 .. 6-s.  The ring sum of a
+// stage's input is summed over the columns of a warp by shuffles, and over the
+// warps of all blocks by another tree that every warp evaluates for itself (the
+// blocks and their columns depend on npm alone, so the sums do not depend on
+// the batch); the rows that do not need it are computed while the cluster
+// barrier completes.
+constexpr int kPRows = 2 * kMS;  // strip rows of Y_{k-1}
+
+// k_sts_poles: a thread owns one column and keeps its rows in registers; the
+// neighbour columns are read from shared memory, where each stage leaves its
+// output for the next.  Bound by latency: one round of loads and four ring sums.
+// NT: the most threads of a launch (up to 288 the registers suffice for
+// everything a column needs, up to 544 some of it is spilled).
+constexpr int kPMidThreads = 288, kPMaxThreads = 544;
+__host__ __device__ inline int poles_ranks(int n2) {
+  const int c = (n2 + 247) / 248;
+  return c > 8 ? 8 : c;
+}
+__host__ __device__ inline int poles_threads(int n2) {
+  const int nc = poles_ranks(n2);
+  return ((n2 + nc - 1) / nc + 2 * kMS + 31) / 32 * 32;
+}
+__host__ __device__ inline int poles_stride(int threads) { return threads + 2; }  // 2 mod 32: no bank conflicts
+__host__ __device__ inline size_t poles_smem(int threads) {
+  return (size_t)4 * kPRows * poles_stride(threads) * sizeof(double);
+}
+
+template <int NT>
+__global__ void __launch_bounds__(NT, 1) k_sts_poles(Mesh m, MarchArgs a, PairTables pt) {
+  const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  extern __shared__ __align__(16) double psm[];
+  __shared__ double s_sum[kMS][8 * (NT / 32)];
+  __shared__ double s_row[3][kPRows];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const int npm = m.npm, n2 = npm - 2, ntm = m.ntm;
+  const int nc = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int unit = blockIdx.x / nc;
+  const bool south = (unit & 1) != 0;
+  // Everything below reads what the pass before this one wrote; the next
+  // launch on the stream, this pass's k_sts_march, reads and writes other rows
+  // and may start now.
+  pdl_wait();
+  pdl_trigger();
+  int nreal;
+  bool first;
+  const StageCoef *rc;
+  int cols;
+  march_launch(a, nreal, first, rc, cols);
+  if ((unit >> 1) >= nreal) return;  // the whole cluster
+  cluster_arrive();                  // waited for below: the blocks' shared memory may be written remotely
+  const int i = a.rlist ? a.rlist[unit >> 1] : (unit >> 1);
+  const int own = (n2 + nc - 1) / nc;
+  const int kb = 2 + rank * own, nown = max(0, min(own, npm - kb));  // columns kb .. kb+nown-1
+  const int w = nown + 2 * kMS;                                      // with the halo
+  const int S = poles_stride(blockDim.x);
+  const int64_t ld = m.ldt, pb = (int64_t)i * m.plane;
+  auto wrap = [&](int c) {  // onto the core columns
+    while (c < 2) c += n2;
+    while (c > npm - 1) c -= n2;
+    return c;
+  };
+  // eight lanes per column fetch the strips, all requests first
+  {
+    const double *g1 = (first ? a.u : a.x1) + pb, *g2 = (first ? a.u : a.x2) + pb;
+    const double *gu = a.u + pb, *gd = a.d + pb;
+    const int t = tid & 7, q = south ? kPRows - 1 - t : t;
+    const int row = south ? ntm - kPRows + t : t;
+    double v[4][kPRows];
+#pragma unroll
+    for (int n = 0; n < kPRows; ++n) {
+      const int c = min((tid >> 3) + n * (int)(blockDim.x >> 3), w - 1);
+      const int64_t g = (int64_t)(wrap(kb - kMS + c) - 1) * ld + row;
+      v[0][n] = g1[g];
+      v[1][n] = g2[g];
+      v[2][n] = gu[g];
+      v[3][n] = gd[g];
+    }
+#pragma unroll
+    for (int n = 0; n < kPRows; ++n) {
+      const int c = (tid >> 3) + n * (int)(blockDim.x >> 3);
+#pragma unroll
+      for (int f = 0; f < 4; ++f) psm[(f * kPRows + q) * S + c] = v[f][n];
+    }
+  }
+  if (tid < 3 * kPRows) {
+    const int f = tid / kPRows, q = tid % kPRows, j = south ? ntm - q : q + 1;
+    s_row[f][q] = pt.row[((int64_t)i * 3 + f) * pt.LR + j + 1];
+  }
+  const int c = min(tid, w - 1), cm = max(c - 1, 0), cp = min(c + 1, w - 1);
+  const bool mine = tid >= kMS && tid < kMS + nown;
+  const int k = wrap(kb - kMS + c);
+  const double2 P = reinterpret_cast<const double2 *>(pt.col)[(int64_t)i * pt.LC + k];
+  const double dpk = m.dp[k], Dr = a.dfac[i + 1];
+  __syncthreads();
+  double x[kPRows], z[kPRows - 1], u[kPRows - 1], d[kPRows - 1];
+  double c1[kPRows - 2], c3[kPRows - 2], c5[kPRows - 2], c2[kPRows - 2], c4[kPRows - 2];
+#pragma unroll
+  for (int q = 0; q < kPRows; ++q) x[q] = psm[q * S + c];
+#pragma unroll
+  for (int q = 0; q < kPRows - 1; ++q) {
+    z[q] = psm[(kPRows + q) * S + c];
+    u[q] = psm[(2 * kPRows + q) * S + c];
+    d[q] = psm[(3 * kPRows + q) * S + c];
+  }
+#pragma unroll
+  for (int q = 1; q < kPRows - 1; ++q) {
+    const double st = s_row[0][q];
+    c2[q - 1] = s_row[1][q];
+    c4[q - 1] = s_row[2][q];
+    c1[q - 1] = P.x * st * st;
+    c5[q - 1] = P.y * st * st;
+    c3[q - 1] = -(c1[q - 1] + c2[q - 1] + c4[q - 1] + c5[q - 1]);
+  }
+  cluster_wait();
+#pragma unroll
+  for (int s = 0; s < kMS; ++s) {
+    const StageCoef sc = rc ? rc[(int64_t)i * kMS + s] : a.c[s];
+    // the warp's share of the input's ring sum, to every block
+    double v = mine ? (Dr + Dr) * (south ? x[0] - x[1] : x[1] - x[0]) * dpk : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane < nc) *cl.map_shared_rank(&s_sum[s][rank * nw + warp], lane) = v;
+    __syncwarp();
+    cluster_arrive();
+    const double *in = psm + s * kPRows * S;
+    double y[kPRows];
+#pragma unroll
+    for (int q = 1; q < kPRows - 1 - s; ++q) {
+      const double up = south ? x[q + 1] : x[q - 1], dn = south ? x[q - 1] : x[q + 1];  // theta rows j-1, j+1
+      const double ax = c1[q - 1] * in[q * S + cm] + c2[q - 1] * up + c3[q - 1] * x[q] + c4[q - 1] * dn +
+                        c5[q - 1] * in[q * S + cp];
+      y[q] = sc.a * x[q] + sc.b * z[q] + sc.c * u[q] + sc.d * ax + sc.e * d[q];
+    }
+    cluster_wait();
+    double ring = 0.0;
+    for (int q = lane; q < nc * nw; q += 32) ring = ring + s_sum[s][q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ring += __shfl_xor_sync(0xffffffffu, ring, o);
+    const double axp = south ? -ring * a.bcs : ring * a.bcn;
+    y[0] = sc.a * x[0] + sc.b * z[0] + sc.c * u[0] + sc.d * axp + sc.e * d[0];
+    if (s < kMS - 1) {
+      // the neighbours' input of the next stage, in the area whose columns
+      // every thread has read into registers
+      double *out = psm + (s + 1) * kPRows * S;
+#pragma unroll
+      for (int q = 1; q < kPRows - 1 - s; ++q)
+        if (tid < w) out[q * S + tid] = y[q];
+      __syncthreads();
+    }
+    if (mine && a.o[s]) {
+      double *g = a.o[s] + pb + (int64_t)(k - 1) * ld + (south ? ntm - 1 : 0);
+#pragma unroll
+      for (int q = 0; q < kMS; ++q)
+        if (q < kPRows - 1 - s) g[south ? -q : q] = y[q];
+    }
+#pragma unroll
+    for (int q = 0; q < kPRows - 1 - s; ++q) {
+      z[q] = x[q];
+      x[q] = y[q];
+    }
+  }
+}
+
+// The same strips when a column per thread does not suffice (more than about
+// 4200 phi columns): the blocks loop over their columns and keep the strip in
+// a scratch area in global memory, in place: stage k over Y_{k-2}, stage k+1
+// over Y_{k-1}, and so on.
+constexpr int kPAThreads = 256;
+constexpr int kPADoubles = kPRows + (kPRows - 1);  // doubles per column
+__host__ __device__ inline int poles_any_width(int n2) { return (n2 + 7) / 8 + 2 * kMS; }
+
+__global__ void __launch_bounds__(kPAThreads) k_sts_poles_any(Mesh m, MarchArgs a, PairTables pt, double *scratch) {
+  const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  __shared__ double s_sum[kMS][8 * (kPAThreads / 32)];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = kPAThreads / 32;
+  const int npm = m.npm, n2 = npm - 2, ntm = m.ntm;
+  const int nc = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int unit = blockIdx.x / nc;
+  const bool south = (unit & 1) != 0;
+  pdl_wait();
+  pdl_trigger();
+  int nreal;
+  bool first;
+  const StageCoef *rc;
+  int cols;
+  march_launch(a, nreal, first, rc, cols);
+  if ((unit >> 1) >= nreal) return;
+  cluster_arrive();
+  const int i = a.rlist ? a.rlist[unit >> 1] : (unit >> 1);
+  const int W = poles_any_width(n2), own = W - 2 * kMS;
+  const int kb = 2 + rank * own, nown = max(0, min(own, npm - kb));
+  const int w = nown + 2 * kMS;
+  double *X = scratch + (int64_t)blockIdx.x * kPADoubles * W, *Y = X + (int64_t)kPRows * W;
+  const int64_t ld = m.ldt, pb = (int64_t)i * m.plane;
+  auto wrap = [&](int c) {
+    while (c < 2) c += n2;
+    while (c > npm - 1) c -= n2;
+    return c;
+  };
+  auto at = [&](int c, int q) { return pb + (int64_t)(wrap(kb - kMS + c) - 1) * ld + (south ? ntm - 1 - q : q); };
+  const double *x1 = first ? a.u : a.x1, *x2 = first ? a.u : a.x2;
+  for (int c = tid; c < w; c += kPAThreads)
+    for (int q = 0; q < kPRows; ++q) {
+      X[(int64_t)q * W + c] = x1[at(c, q)];
+      if (q < kPRows - 1) Y[(int64_t)q * W + c] = x2[at(c, q)];
+    }
+  const double Dr = a.dfac[i + 1];
+  const double *R = pt.row + (int64_t)i * 3 * pt.LR;
+  __syncthreads();
+  cluster_wait();
+  double *In = X, *Out = Y;  // stage input, and second input = output
+#pragma unroll 1
+  for (int s = 0; s < kMS; ++s) {
+    const StageCoef sc = rc ? rc[(int64_t)i * kMS + s] : a.c[s];
+    double v = 0.0;
+    for (int c = kMS + tid; c < kMS + nown; c += kPAThreads) {
+      const double t = south ? In[c] - In[W + c] : In[W + c] - In[c];
+      v = v + (Dr + Dr) * t * m.dp[kb - kMS + c];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane < nc) *cl.map_shared_rank(&s_sum[s][rank * nw + warp], lane) = v;
+    __syncwarp();
+    cluster_arrive();
+    __syncwarp();
+    cluster_wait();
+    double ring = 0.0;
+    for (int q = lane; q < nc * nw; q += 32) ring = ring + s_sum[s][q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ring += __shfl_xor_sync(0xffffffffu, ring, o);
+    const double axp = south ? -ring * a.bcs : ring * a.bcn;
+    double *o = a.o[s];
+    for (int c = s + 1 + tid; c <= w - 2 - s; c += kPAThreads) {
+      const double2 P = reinterpret_cast<const double2 *>(pt.col)[(int64_t)i * pt.LC + wrap(kb - kMS + c)];
+      for (int q = 0; q < kPRows - 1 - s; ++q) {
+        const int64_t e = (int64_t)q * W + c;
+        const int j = south ? ntm - q : q + 1;
+        double ax = axp;
+        if (q > 0) {
+          const double st = R[j + 1], c2 = R[pt.LR + j + 1], c4 = R[2 * pt.LR + j + 1];
+          const double c1 = P.x * st * st;
+          const double c5 = P.y * st * st;
+          const double c3 = -(c1 + c2 + c4 + c5);
+          const double up = In[e + (south ? W : -W)], dn = In[e + (south ? -W : W)];
+          ax = c1 * In[e - 1] + c2 * up + c3 * In[e] + c4 * dn + c5 * In[e + 1];
+        }
+        const int64_t g = at(c, q);
+        const double y = sc.a * In[e] + sc.b * Out[e] + sc.c * a.u[g] + sc.d * ax + sc.e * a.d[g];
+        Out[e] = y;
+        if (o && q < kMS && c >= kMS && c < kMS + nown) o[g] = y;
+      }
+    }
+    __syncthreads();
+    double *t = In;
+    In = Out;
+    Out = t;
+  }
+}
+
+// The whole pass of a grid with fewer than kMMinRows theta rows: one block
+// per realization, stage by stage in global memory (a stage writes over the
+// output of the stage two before it where that one is not kept).
+__global__ void __launch_bounds__(256) k_sts_whole(Mesh m, MarchArgs a, PairTables pt) {
+  __shared__ double sh[64];
+  __shared__ double s_ring[2];
+  pdl_wait();
+  pdl_trigger();
+  int nreal;
+  bool first;
+  const StageCoef *rc;
+  int cols;
+  march_launch(a, nreal, first, rc, cols);
+  if ((int)blockIdx.x >= nreal) return;
+  const int i = a.rlist ? a.rlist[blockIdx.x] : (int)blockIdx.x;
+  const int npm = m.npm, n2 = npm - 2, ntm = m.ntm;
+  const int64_t ld = m.ldt, pb = (int64_t)i * m.plane;
+  const double Dr = a.dfac[i + 1];
+  const double *R = pt.row + (int64_t)i * 3 * pt.LR;
+  const double2 *P = reinterpret_cast<const double2 *>(pt.col) + (int64_t)i * pt.LC;
+  const double *in = (first ? a.u : a.x1) + pb, *in2 = (first ? a.u : a.x2) + pb;
+  const double *u = a.u + pb, *d = a.d + pb;
+  for (int s = 0; s < kMS; ++s) {
+    const StageCoef sc = rc ? rc[(int64_t)i * kMS + s] : a.c[s];
+    double *out = (a.o[s] ? a.o[s] : a.o[s | 2]) + pb;
+    double fn = 0.0, fs = 0.0;
+    for (int k = 2 + threadIdx.x; k <= npm - 1; k += blockDim.x) {
+      const double *x = in + (int64_t)(k - 1) * ld;
+      fn = fn + (Dr + Dr) * (x[1] - x[0]) * m.dp[k];
+      fs = fs + (Dr + Dr) * (x[ntm - 1] - x[ntm - 2]) * m.dp[k];
+    }
+    block_sum2(fn, fs, sh);
+    if (threadIdx.x == 0) {
+      s_ring[0] = fn * a.bcn;
+      s_ring[1] = -fs * a.bcs;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < n2 * ntm; e += blockDim.x) {
+      const int k = 2 + e / ntm, j = 1 + e % ntm;
+      const int64_t g = (int64_t)(k - 1) * ld + (j - 1);
+      double ax;
+      if (j == 1 || j == ntm) {
+        ax = s_ring[j == 1 ? 0 : 1];
+      } else {
+        const int kl = k == 2 ? npm - 1 : k - 1, kr = k == npm - 1 ? 2 : k + 1;
+        const double st = R[j + 1], c2 = R[pt.LR + j + 1], c4 = R[2 * pt.LR + j + 1];
+        const double c1 = P[k].x * st * st;
+        const double c5 = P[k].y * st * st;
+        const double c3 = -(c1 + c2 + c4 + c5);
+        ax = c1 * in[(int64_t)(kl - 1) * ld + j - 1] + c2 * in[g - 1] + c3 * in[g] + c4 * in[g + 1] +
+             c5 * in[(int64_t)(kr - 1) * ld + j - 1];
+      }
+      const double y = sc.a * in[g] + sc.b * in2[g] + sc.c * u[g] + sc.d * ax + sc.e * d[g];
+      out[g] = y;
+    }
+    __syncthreads();
+    in2 = in;
+    in = out;
+  }
+}
+
+// d = scale * af, the first stage's dty0 (src/hipft.f90:5211) from A u0: one
+// scale for the launch, or per realization (rscale[i-1], realizations of
+// rlist; a negative entry: the slot does nothing).  Grid (chunks, slots).
+__global__ void k_scale(int64_t plane, const double *__restrict__ af, double *d, double scale,
+                        const int *__restrict__ rlist, const double *__restrict__ rscale) {
+  int i = blockIdx.y;
+  if (rlist) {
+    i = rlist[i];
+    if (i < 0) return;
+    scale = rscale[i];
+  }
+  const double2 *s2 = reinterpret_cast<const double2 *>(af + (int64_t)i * plane);
+  double2 *d2 = reinterpret_cast<double2 *>(d + (int64_t)i * plane);
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < plane / 2; e += (int64_t)gridDim.x * blockDim.x) {
+    const double2 v = s2[e];
+    d2[e] = make_double2(scale * v.x, scale * v.y);
+  }
+}
+
+}  // namespace hipft
