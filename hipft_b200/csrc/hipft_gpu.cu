@@ -476,6 +476,7 @@ static MarchArgs march_args(const hipft_gpu *h, const double *u0, const double *
   a.dfac = h->DC.dfac;
   a.bcn = h->bc_diff_n;
   a.bcs = h->bc_diff_s;
+  a.err = h->d_err;
   return a;
 }
 
@@ -532,7 +533,11 @@ static cudaError_t launch_pass(const hipft_gpu *h, cudaStream_t s, MarchArgs a, 
   cfg.gridDim = dim3((unsigned)(2 * a.nreal * nc));
   cfg.blockDim = dim3((unsigned)(bycol ? poles_threads(n2) : kPAThreads));
   cfg.dynamicSmemBytes = bycol ? poles_smem(poles_threads(n2)) : 0;
-  auto poles = poles_threads(n2) <= kPMidThreads ? k_sts_poles<kPMidThreads> : k_sts_poles<kPMaxThreads>;
+  // a march that leaves places free does not compete with the pole strips' registers
+  const bool roomy = blocks + 3 * (int64_t)cfg.gridDim.x <= (int64_t)kMBlocks * h->num_sms;
+  auto poles = poles_threads(n2) > kPMidThreads ? k_sts_poles<kPMaxThreads, 1>
+               : roomy                          ? k_sts_poles<kPMidThreads, 1>
+                                                : k_sts_poles<kPMidThreads, 3>;
   cudaError_t e = bycol ? cudaLaunchKernelEx(&cfg, poles, h->M, a, h->ptab)
                         : cudaLaunchKernelEx(&cfg, k_sts_poles_any, h->M, a, h->ptab, h->d_pscratch);
   if (e != cudaSuccess) return e;
@@ -734,9 +739,11 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
     smem_ok = smem_ok && cudaFuncSetAttribute(march_kernel(v & 1, v & 2, v & 4), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)kMSmem) == cudaSuccess;
   if (!smem_ok ||
-      cudaFuncSetAttribute(k_sts_poles<kPMidThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaFuncSetAttribute(k_sts_poles<kPMidThreads, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)poles_smem(kPMidThreads)) != cudaSuccess ||
-      cudaFuncSetAttribute(k_sts_poles<kPMaxThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaFuncSetAttribute(k_sts_poles<kPMidThreads, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)poles_smem(kPMidThreads)) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sts_poles<kPMaxThreads, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)poles_smem(kPMaxThreads)) != cudaSuccess)
     return bail(fail(h, HIPFT_ECUDA, "cannot reserve shared memory for the RKG2 passes"));
   if (cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess || h->num_sms < 1)

@@ -96,7 +96,10 @@ constexpr int kMGroup = 4;                  // columns per turn of its loop
 constexpr int kMSlots = 2 * kMGroup;        // columns of its shared-memory ring
 constexpr int kMRing = kMSlots * 4 * 64;    // doubles per warp: Y_{k-1}, Y_{k-2}, u0, dty0
 constexpr int kMCoef = 5 * kMS;             // the pass's stage coefficients
-constexpr size_t kMSmem = ((size_t)kMWarps * kMRing + kMCoef) * sizeof(double);
+constexpr int kMColsMax = 96;               // most columns per warp
+constexpr int kMTab = 2 * (kMColsMax + 2 * kMS + kMGroup);  // doubles of the column table per warp
+constexpr size_t kMSmem = ((size_t)kMWarps * (kMRing + kMTab) + kMCoef) * sizeof(double);
+static_assert(kMTab % 2 == 0, "16-byte aligned");
 constexpr int kMMinRows = 2 * kMS;          // smallest ntm of the strip kernels (k_sts_whole below it)
 
 struct MarchArgs {
@@ -121,6 +124,7 @@ struct MarchArgs {
   int strips, cols;       // theta strips, columns per warp (march_cols)
   const double *dfac;     // [nr+1]
   double bcn, bcs;        // pole factors
+  int *err;               // set to 1 when a bounded wait gives up
 };
 
 // Stage slot q (0-based, over the whole super-step) of an s-stage super-step
@@ -141,15 +145,14 @@ __host__ __device__ inline StageCoef sts_slot(int method, int64_t s, int64_t q, 
 // Phi columns per warp, a multiple of kMGroup: the fewest full waves of
 // resident warps that keep the chunk at kMColsMax columns or less (a chunk
 // loads 2 kMS columns more than it owns, so longer chunks waste less; whole
-// waves leave no nearly empty one).  A block of k_sts_poles takes the place of
-// the blocks of an SM; a single wave leaves those SMs out, which would
-// otherwise start a second one.
-constexpr int kMColsMax = 96;
+// waves leave no nearly empty one).  Blocks of k_sts_poles take the place of
+// blocks; a single wave leaves those places out, which would otherwise start a
+// second one.
 __host__ __device__ inline int march_cols(int n2, int strips, int nreal, int slots, int poles) {
   const int64_t per = (int64_t)strips * (nreal > 0 ? nreal : 1) * kMWarps;
   for (int64_t w = 1;; ++w) {
     int64_t free = w * slots;
-    const int64_t taken = (int64_t)poles * nreal * kMBlocks * kMWarps;
+    const int64_t taken = (int64_t)poles * nreal * kMWarps;
     if (w == 1 && taken <= slots / 2) free -= taken;
     const int64_t nch = free / per * kMWarps;  // whole blocks of chunks
     if (nch < 1) continue;
@@ -178,10 +181,45 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// the shared address of this block's `a` in block `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t a, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+// stores v at a shared address of the cluster and counts its 8 bytes on the
+// barrier there
+__device__ __forceinline__ void st_async(uint32_t dst, double v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst),
+               "l"(__double_as_longlong(v)), "r"(bar)
+               : "memory");
+}
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+// the same where p, of one pair of rows of four fields, kF bytes apart
+template <uint32_t kF>
+__device__ __forceinline__ void cp_async16x4(bool p, uint32_t dst, const void *a, const void *b, const void *c,
+                                             const void *d) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n"
+      " @p cp.async.cg.shared.global [%1], [%2], 16;\n @p cp.async.cg.shared.global [%1 + %6], [%3], 16;\n"
+      " @p cp.async.cg.shared.global [%1 + %7], [%4], 16;\n @p cp.async.cg.shared.global [%1 + %8], [%5], 16;\n}" ::"r"(
+          (uint32_t)p),
+      "r"(dst), "l"(a), "l"(b), "l"(c), "l"(d), "n"(kF), "n"(2 * kF), "n"(3 * kF)
+      : "memory");
+}
+// stores y where p, without a branch
+__device__ __forceinline__ void st_if(bool p, void *g, double2 y) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n @p st.global.v2.f64 [%1], {%2, %3};\n}" ::"r"((uint32_t)p),
+               "l"(g), "d"(y.x), "d"(y.y)
+               : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -269,7 +307,7 @@ __global__ void __launch_bounds__(32 * kMWarps, kMBlocks) k_sts_march(Mesh m, Ma
     return;
   }
   const int i = a.rlist ? a.rlist[rest / nblk] : rest / nblk;  // 0-based
-  double *coef = msm + kMWarps * kMRing;
+  double *coef = msm + kMWarps * (kMRing + kMTab);
   if (TABLE) {
     if (threadIdx.x < kMCoef) coef[threadIdx.x] = reinterpret_cast<const double *>(rc + (int64_t)i * kMS)[threadIdx.x];
     __syncthreads();
@@ -307,12 +345,7 @@ __global__ void __launch_bounds__(32 * kMWarps, kMBlocks) k_sts_march(Mesh m, Ma
   if (fc < 2) fc += n2;
   Off fo = (Off)(fc - 1) * ldb + rowb;
   auto fetch = [&](uint32_t s) {
-    if (left > 0) {
-      cp_async16(s, gx1 + fo);
-      cp_async16(s + kF, gx2 + fo);
-      cp_async16(s + 2 * kF, gu + fo);
-      cp_async16(s + 3 * kF, gd + fo);
-    }
+    cp_async16x4<kF>(left > 0, s, gx1 + fo, gx2 + fo, gu + fo, gd + fo);
     cp_async_commit();
     --left;
     fo += ldb;
@@ -321,13 +354,18 @@ __global__ void __launch_bounds__(32 * kMWarps, kMBlocks) k_sts_march(Mesh m, Ma
       fo -= (Off)n2 * ldb;
     }
   };
+  // the column table's entries of the chunk, with the first columns' copies
+  double *tab = msm + kMWarps * kMRing + warp * kMTab;
+  for (int t = lane; t < left + kMGroup - 1; t += 32) cp_async16(smem_addr(tab) + 16u * t, pt_col + c0 - kMS + t);
   fetch(sring);
   fetch(sring + kSlot);
   fetch(sring + 2 * kSlot);
 
-  auto put = [&](char *o, Off off, double2 y) {
-    if (vb) *reinterpret_cast<double2 *>(o + off) = y;
-    else if (va) *reinterpret_cast<double *>(o + off) = y.x;
+  // an odd last row: its lane stores one value of the pair
+  const bool odd = strip == a.strips - 1 && ((ntm - kMS) & 1);
+  auto put = [&](bool p, char *o, Off off, double2 y) {
+    st_if(p && vb, o + off, y);
+    if (odd && p && va && !vb) *reinterpret_cast<double *>(o + off) = y.x;
   };
   // Step of column e = the j-th of its group (compile-time j, n = step number
   // while the windows fill): W[s] holds columns e-2, e-1 of stage s's input
@@ -339,57 +377,55 @@ __global__ void __launch_bounds__(32 * kMWarps, kMBlocks) k_sts_march(Mesh m, Ma
   int oc = -2 * kMS;                               // column e-4, counted from c0
   Off wo = (Off)(c0 - 1 - 2 * kMS) * ldb + rowb;   // its offset
   const int nown = c1 - c0 + 1;
-  const double2 *pp = pt_col + (c0 - kMS);
-  double2 Pn = pp[-1];  // the column table's entry of column e-1
+  uint32_t ptab = smem_addr(tab);                  // the entry of column e-1
   auto step = [&](auto jc, auto nc, uint32_t sa, uint32_t sb) {
     constexpr int j = decltype(jc)::value, n = decltype(nc)::value;  // n: 2 kMS and more: all stages
     constexpr int A = j & 1, B = 1 - A;
     auto slot = [&](int back) { return j >= back ? sa + (uint32_t)(j - back) * kSlot : sb + (uint32_t)(j - back + kMGroup) * kSlot; };
     cp_async_wait<2>();
+    fetch(j + 3 < kMGroup ? sa + (j + 3) * kSlot : sb + (j + 3 - kMGroup) * kSlot);  // column e-5's slot
     const double2 x0 = lds2(slot(0));
-    if (n >= 2) {
-      K[(j + 3) & 3] = phi_coef(st, c2, c4, Pn);
-    }
-    Pn = *pp++;
+    if (n == 0) __syncwarp();  // the table was fetched by all lanes
+    if (n >= 2) K[(j + 3) & 3] = phi_coef(st, c2, c4, lds2(ptab));
+    if (n >= 1) ptab += 16;
     const StageCoef *q = TABLE ? reinterpret_cast<const StageCoef *>(coef) : a.c;
-    double2 y0 = {}, y1 = {}, y2 = {};
+    double2 y0 = {}, y1 = {}, y2 = {}, y3 = {};
     if (n >= 2) {
       const uint32_t s = slot(1);
       const double2 xc = W[0][B];
       const double up = __shfl_up_sync(0xffffffffu, xc.y, 1), dn = __shfl_down_sync(0xffffffffu, xc.x, 1);
       y0 = pair_stage(W[0][A], xc, x0, up, dn, K[(j + 3) & 3], c2, c4, lds2(s + kF), lds2(s + 2 * kF), lds2(s + 3 * kF),
                       q[0]);
-      if (KEEP && n >= 5 && k0keep && oc + 3 < nown) put(o0, wo + 3 * ldb, y0);
     }
     if (n >= 4) {
       const uint32_t s = slot(2);
       const double2 xc = W[1][B];
       const double up = __shfl_up_sync(0xffffffffu, xc.y, 1), dn = __shfl_down_sync(0xffffffffu, xc.x, 1);
       y1 = pair_stage(W[1][A], xc, y0, up, dn, K[(j + 2) & 3], c2, c4, W[0][A], lds2(s + 2 * kF), lds2(s + 3 * kF), q[1]);
-      if (KEEP && n >= 6 && k1keep && oc + 2 < nown) put(o1, wo + 2 * ldb, y1);
     }
     if (n >= 6) {
       const uint32_t s = slot(3);
       const double2 xc = W[2][B];
       const double up = __shfl_up_sync(0xffffffffu, xc.y, 1), dn = __shfl_down_sync(0xffffffffu, xc.x, 1);
       y2 = pair_stage(W[2][A], xc, y1, up, dn, K[(j + 1) & 3], c2, c4, W[1][A], lds2(s + 2 * kF), lds2(s + 3 * kF), q[2]);
-      if (n >= 7 && oc + 1 < nown) put(o2, wo + ldb, y2);
     }
     if (n >= 8) {
       const uint32_t s = slot(4);
       const double2 xc = W[3][B];
       const double up = __shfl_up_sync(0xffffffffu, xc.y, 1), dn = __shfl_down_sync(0xffffffffu, xc.x, 1);
-      const double2 y3 =
-          pair_stage(W[3][A], xc, y2, up, dn, K[j & 3], c2, c4, W[2][A], lds2(s + 2 * kF), lds2(s + 3 * kF), q[3]);
-      if (oc < nown) put(o3, wo, y3);
+      y3 = pair_stage(W[3][A], xc, y2, up, dn, K[j & 3], c2, c4, W[2][A], lds2(s + 2 * kF), lds2(s + 3 * kF), q[3]);
     }
+    // all stores at the end: the four stages stay in one block of instructions
+    if (KEEP && n >= 5 && k0keep) put(oc + 3 < nown, o0, wo + 3 * ldb, y0);
+    if (KEEP && n >= 6 && k1keep) put(oc + 2 < nown, o1, wo + 2 * ldb, y1);
+    if (n >= 7) put(oc + 1 < nown, o2, wo + ldb, y2);
+    if (n >= 8) put(oc < nown, o3, wo, y3);
     W[0][A] = x0;
     W[1][A] = y0;
     W[2][A] = y1;
     W[3][A] = y2;
     ++oc;
     wo += ldb;
-    fetch(j + 3 < kMGroup ? sa + (j + 3) * kSlot : sb + (j + 3 - kMGroup) * kSlot);
   };
   uint32_t sa = sring, sb = sring + kMGroup * kSlot;
   step(IntC<0>{}, IntC<0>{}, sa, sb);
@@ -423,18 +459,26 @@ __global__ void __launch_bounds__(32 * kMWarps, kMBlocks) k_sts_march(Mesh m, Ma
 // stage's input is summed over the columns of a warp by shuffles, and over the
 // warps of all blocks by another tree that every warp evaluates for itself (the
 // blocks and their columns depend on npm alone, so the sums do not depend on
-// the batch); the rows that do not need it are computed while the cluster
-// barrier completes.
+// the batch).  The warps send their sums to every block as stores that count on
+// a barrier there (a cluster barrier with release semantics took 700 cycles
+// more per stage); the rows that do not need the sum are computed meanwhile.
 constexpr int kPRows = 2 * kMS;  // strip rows of Y_{k-1}
 
-// k_sts_poles: a thread owns one column and keeps its rows in registers; the
-// neighbour columns are read from shared memory, where each stage leaves its
-// output for the next.  Bound by latency: one round of loads and four ring sums.
-// NT: the most threads of a launch (up to 288 the registers suffice for
-// everything a column needs, up to 544 some of it is spilled).
+// k_sts_poles: a thread owns one column, keeps its windows in registers and
+// reads the neighbour columns from shared memory, where each stage leaves its
+// output for the next.  Bound by latency: what the pass before does not change
+// (u0, dty0, the tables) is fetched before the wait for it, and after it come
+// one round of loads and four ring sums.  The stage loop is not unrolled: the
+// kernel's code is cold in every pass, and fetching it once costs less.
+//
+// Columns per block: few on narrow grids, where the FP64 work of a block would
+// otherwise outlast its ring sums.  NB = 3 holds the block's registers to those
+// of one block of k_sts_march, so that it takes the place of one where the
+// march fills the GPU; NB = 1 is faster by itself.
 constexpr int kPMidThreads = 288, kPMaxThreads = 544;
 __host__ __device__ inline int poles_ranks(int n2) {
-  const int c = (n2 + 247) / 248;
+  const int per = n2 <= 8 * 120 ? 120 : 280;
+  const int c = (n2 + per - 1) / per;
   return c > 8 ? 8 : c;
 }
 __host__ __device__ inline int poles_threads(int n2) {
@@ -442,144 +486,150 @@ __host__ __device__ inline int poles_threads(int n2) {
   return ((n2 + nc - 1) / nc + 2 * kMS + 31) / 32 * 32;
 }
 __host__ __device__ inline int poles_stride(int threads) { return threads + 2; }  // 2 mod 32: no bank conflicts
+constexpr int kPSmemRows = kPRows + 3 * (kPRows - 1);  // Y_{k-1}, Y_{k-2}, u0, dty0
 __host__ __device__ inline size_t poles_smem(int threads) {
-  return (size_t)4 * kPRows * poles_stride(threads) * sizeof(double);
+  return (size_t)kPSmemRows * poles_stride(threads) * sizeof(double);
 }
 
-template <int NT>
-__global__ void __launch_bounds__(NT, 1) k_sts_poles(Mesh m, MarchArgs a, PairTables pt) {
+template <int NT, int NB>
+__global__ void __launch_bounds__(NT, NB) k_sts_poles(Mesh m, MarchArgs a, PairTables pt) {
   const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
   extern __shared__ __align__(16) double psm[];
   __shared__ double s_sum[kMS][8 * (NT / 32)];
   __shared__ double s_row[3][kPRows];
+  __shared__ double s_coef[5 * kMS];
+  __shared__ uint64_t s_bar[kMS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   const int npm = m.npm, n2 = npm - 2, ntm = m.ntm;
   const int nc = (int)cl.num_blocks(), rank = (int)cl.block_rank();
   const int unit = blockIdx.x / nc;
   const bool south = (unit & 1) != 0;
-  // Everything below reads what the pass before this one wrote; the next
-  // launch on the stream, this pass's k_sts_march, reads and writes other rows
-  // and may start now.
-  pdl_wait();
-  pdl_trigger();
   int nreal;
   bool first;
   const StageCoef *rc;
   int cols;
   march_launch(a, nreal, first, rc, cols);
-  if ((unit >> 1) >= nreal) return;  // the whole cluster
-  cluster_arrive();                  // waited for below: the blocks' shared memory may be written remotely
+  if ((unit >> 1) >= nreal) {  // the whole cluster
+    pdl_wait();
+    pdl_trigger();
+    return;
+  }
+  if (tid == 0) {
+    for (int s = 0; s < kMS; ++s) {
+      mbar_init(&s_bar[s], 1);
+      mbar_expect_tx(&s_bar[s], (uint32_t)(nc * nw * 8));
+    }
+    fence_mbar_init();
+  }
+  __syncwarp();
+  cluster_arrive();  // waited for below: the blocks' barriers are ready
   const int i = a.rlist ? a.rlist[unit >> 1] : (unit >> 1);
   const int own = (n2 + nc - 1) / nc;
   const int kb = 2 + rank * own, nown = max(0, min(own, npm - kb));  // columns kb .. kb+nown-1
   const int w = nown + 2 * kMS;                                      // with the halo
   const int S = poles_stride(blockDim.x);
+  double *sX = psm, *sY = psm + kPRows * S, *sU = sY + (kPRows - 1) * S, *sD = sU + (kPRows - 1) * S;
   const int64_t ld = m.ldt, pb = (int64_t)i * m.plane;
   auto wrap = [&](int c) {  // onto the core columns
     while (c < 2) c += n2;
     while (c > npm - 1) c -= n2;
     return c;
   };
-  // eight lanes per column fetch the strips, all requests first
-  {
-    const double *g1 = (first ? a.u : a.x1) + pb, *g2 = (first ? a.u : a.x2) + pb;
-    const double *gu = a.u + pb, *gd = a.d + pb;
-    const int t = tid & 7, q = south ? kPRows - 1 - t : t;
-    const int row = south ? ntm - kPRows + t : t;
-    double v[4][kPRows];
-#pragma unroll
-    for (int n = 0; n < kPRows; ++n) {
-      const int c = min((tid >> 3) + n * (int)(blockDim.x >> 3), w - 1);
-      const int64_t g = (int64_t)(wrap(kb - kMS + c) - 1) * ld + row;
-      v[0][n] = g1[g];
-      v[1][n] = g2[g];
-      v[2][n] = gu[g];
-      v[3][n] = gd[g];
-    }
-#pragma unroll
-    for (int n = 0; n < kPRows; ++n) {
-      const int c = (tid >> 3) + n * (int)(blockDim.x >> 3);
-#pragma unroll
-      for (int f = 0; f < 4; ++f) psm[(f * kPRows + q) * S + c] = v[f][n];
-    }
-  }
-  if (tid < 3 * kPRows) {
-    const int f = tid / kPRows, q = tid % kPRows, j = south ? ntm - q : q + 1;
-    s_row[f][q] = pt.row[((int64_t)i * 3 + f) * pt.LR + j + 1];
-  }
   const int c = min(tid, w - 1), cm = max(c - 1, 0), cp = min(c + 1, w - 1);
   const bool mine = tid >= kMS && tid < kMS + nown;
   const int k = wrap(kb - kMS + c);
   const double2 P = reinterpret_cast<const double2 *>(pt.col)[(int64_t)i * pt.LC + k];
   const double dpk = m.dp[k], Dr = a.dfac[i + 1];
+  // eight lanes per column fetch two fields' strips into shared memory
+  const int t8 = tid & 7, q8 = south ? kPRows - 1 - t8 : t8, row8 = south ? ntm - kPRows + t8 : t8;
+  auto strips = [&](const double *ga, const double *gb, double *sa, double *sb, int rows_a) {
+    double v[2][kPRows];
+#pragma unroll
+    for (int n = 0; n < kPRows; ++n) {
+      const int cc = min((tid >> 3) + n * (int)(blockDim.x >> 3), w - 1);
+      const int64_t g = pb + (int64_t)(wrap(kb - kMS + cc) - 1) * ld + row8;
+      v[0][n] = ga[g];
+      v[1][n] = gb[g];
+    }
+#pragma unroll
+    for (int n = 0; n < kPRows; ++n) {
+      const int cc = (tid >> 3) + n * (int)(blockDim.x >> 3);
+      if (q8 < rows_a) sa[q8 * S + cc] = v[0][n];
+      if (q8 < kPRows - 1) sb[q8 * S + cc] = v[1][n];
+    }
+  };
+  strips(a.u, a.d, sU, sD, kPRows - 1);
+  if (tid < 3 * kPRows) {
+    const int f = tid / kPRows, q = tid % kPRows, j = south ? ntm - q : q + 1;
+    s_row[f][q] = pt.row[((int64_t)i * 3 + f) * pt.LR + j + 1];
+  }
+  if (tid < 5 * kMS) {
+    const StageCoef *q = rc ? rc + (int64_t)i * kMS : a.c;
+    s_coef[tid] = reinterpret_cast<const double *>(q)[tid];
+  }
+  // Everything below reads what the pass before this one wrote; the next
+  // launch on the stream, this pass's k_sts_march, reads and writes other rows
+  // and may start now.
+  pdl_wait();
+  pdl_trigger();
+  strips(first ? a.u : a.x1, first ? a.u : a.x2, sX, sY, kPRows);
   __syncthreads();
-  double x[kPRows], z[kPRows - 1], u[kPRows - 1], d[kPRows - 1];
-  double c1[kPRows - 2], c3[kPRows - 2], c5[kPRows - 2], c2[kPRows - 2], c4[kPRows - 2];
+  double x[kPRows], z[kPRows - 1];
 #pragma unroll
-  for (int q = 0; q < kPRows; ++q) x[q] = psm[q * S + c];
+  for (int q = 0; q < kPRows; ++q) x[q] = sX[q * S + c];
 #pragma unroll
-  for (int q = 0; q < kPRows - 1; ++q) {
-    z[q] = psm[(kPRows + q) * S + c];
-    u[q] = psm[(2 * kPRows + q) * S + c];
-    d[q] = psm[(3 * kPRows + q) * S + c];
-  }
-#pragma unroll
-  for (int q = 1; q < kPRows - 1; ++q) {
-    const double st = s_row[0][q];
-    c2[q - 1] = s_row[1][q];
-    c4[q - 1] = s_row[2][q];
-    c1[q - 1] = P.x * st * st;
-    c5[q - 1] = P.y * st * st;
-    c3[q - 1] = -(c1[q - 1] + c2[q - 1] + c4[q - 1] + c5[q - 1]);
-  }
+  for (int q = 0; q < kPRows - 1; ++q) z[q] = sY[q * S + c];
   cluster_wait();
-#pragma unroll
+  double *in = sX, *out = sY;  // the neighbours' input, and where the next stage finds its own
+#pragma unroll 1
   for (int s = 0; s < kMS; ++s) {
-    const StageCoef sc = rc ? rc[(int64_t)i * kMS + s] : a.c[s];
+    const StageCoef sc = reinterpret_cast<const StageCoef *>(s_coef)[s];
     // the warp's share of the input's ring sum, to every block
     double v = mine ? (Dr + Dr) * (south ? x[0] - x[1] : x[1] - x[0]) * dpk : 0.0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane < nc) *cl.map_shared_rank(&s_sum[s][rank * nw + warp], lane) = v;
-    __syncwarp();
-    cluster_arrive();
-    const double *in = psm + s * kPRows * S;
-    double y[kPRows];
+    if (lane < nc)
+      st_async(cluster_addr(smem_addr(&s_sum[s][rank * nw + warp]), lane), v, cluster_addr(smem_addr(&s_bar[s]), lane));
+    double y[kPRows - 1];
 #pragma unroll
-    for (int q = 1; q < kPRows - 1 - s; ++q) {
+    for (int q = 1; q < kPRows - 1; ++q) {  // rows past 6-s are not used any more
+      const double st = s_row[0][q], c2 = s_row[1][q], c4 = s_row[2][q];
+      const double c1 = P.x * st * st;
+      const double c5 = P.y * st * st;
+      const double c3 = -(c1 + c2 + c4 + c5);
       const double up = south ? x[q + 1] : x[q - 1], dn = south ? x[q - 1] : x[q + 1];  // theta rows j-1, j+1
-      const double ax = c1[q - 1] * in[q * S + cm] + c2[q - 1] * up + c3[q - 1] * x[q] + c4[q - 1] * dn +
-                        c5[q - 1] * in[q * S + cp];
-      y[q] = sc.a * x[q] + sc.b * z[q] + sc.c * u[q] + sc.d * ax + sc.e * d[q];
+      const double ax = c1 * in[q * S + cm] + c2 * up + c3 * x[q] + c4 * dn + c5 * in[q * S + cp];
+      y[q] = sc.a * x[q] + sc.b * z[q] + sc.c * sU[q * S + c] + sc.d * ax + sc.e * sD[q * S + c];
     }
-    cluster_wait();
+    if (!mbar_wait_bounded(&s_bar[s], 0, 1u << 22)) atomicExch(a.err, 1);
     double ring = 0.0;
     for (int q = lane; q < nc * nw; q += 32) ring = ring + s_sum[s][q];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ring += __shfl_xor_sync(0xffffffffu, ring, o);
     const double axp = south ? -ring * a.bcs : ring * a.bcn;
-    y[0] = sc.a * x[0] + sc.b * z[0] + sc.c * u[0] + sc.d * axp + sc.e * d[0];
-    if (s < kMS - 1) {
-      // the neighbours' input of the next stage, in the area whose columns
-      // every thread has read into registers
-      double *out = psm + (s + 1) * kPRows * S;
+    y[0] = sc.a * x[0] + sc.b * z[0] + sc.c * sU[c] + sc.d * axp + sc.e * sD[c];
+    // the neighbours' input of the next stage, over the one before this
+    // stage's, which every thread has read
 #pragma unroll
-      for (int q = 1; q < kPRows - 1 - s; ++q)
-        if (tid < w) out[q * S + tid] = y[q];
-      __syncthreads();
-    }
-    if (mine && a.o[s]) {
-      double *g = a.o[s] + pb + (int64_t)(k - 1) * ld + (south ? ntm - 1 : 0);
+    for (int q = 1; q < kPRows - 1; ++q) out[q * S + tid] = y[q];
+    double *o = a.o[s];
+    if (mine && o) {
+      double *g = o + pb + (int64_t)(k - 1) * ld + (south ? ntm - 1 : 0);
 #pragma unroll
-      for (int q = 0; q < kMS; ++q)
-        if (q < kPRows - 1 - s) g[south ? -q : q] = y[q];
+      for (int q = 0; q < kMS; ++q) g[south ? -q : q] = y[q];
     }
 #pragma unroll
-    for (int q = 0; q < kPRows - 1 - s; ++q) {
+    for (int q = 0; q < kPRows - 1; ++q) {
       z[q] = x[q];
       x[q] = y[q];
     }
+    double *t = in;
+    in = out;
+    out = t;
+    __syncthreads();
   }
+  cluster_arrive_relaxed();  // no block leaves while another may still send to it
+  cluster_wait();
 }
 
 // The same strips when a column per thread does not suffice (more than about
