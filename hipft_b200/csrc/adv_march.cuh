@@ -1,0 +1,430 @@
+// One explicit advection stage with the WENO3 operator (src/hipft.f90:
+// 7711-7925) and the integrator's combine (src/hipft.f90:7440-7578).
+#pragma once
+
+#include <algorithm>
+
+#include "sts_march.cuh"
+
+namespace hipft {
+
+constexpr int kAOwn = 60;     // theta rows a strip owns of the 64 it holds
+constexpr int kAWarps = 4;    // warps per block of k_adv_march
+constexpr int kABlocks = 2;   // its blocks per SM: with 168 registers (3) the four chains of a step were not kept apart
+constexpr int kASlots = 4;    // columns of its shared-memory ring
+constexpr int kAWt = 12;      // weights of a theta face
+constexpr int kAColsMax = 64;
+// doubles of a ring slot: x and f0, for 2-D flows vt, at, vp, vp of the next
+// column and ap, the phi face's row of Weno::ptab, and for 2-D flows the two
+// vt above the strip
+__host__ __device__ constexpr int adv_slot(bool flow2d) { return (flow2d ? 7 : 2) * 64 + kPhiTab + (flow2d ? 2 : 0); }
+__host__ __device__ constexpr size_t adv_smem(bool flow2d) {
+  return ((size_t)kAWt * 64 + (size_t)kAWarps * kASlots * adv_slot(flow2d)) * sizeof(double);
+}
+
+// WENO3 face value (weno_face) with the divisions of quot_nr; the two
+// normalising divisions of each side share one reciprocal.  FaceW: 1 + D_C_MC
+// (j-1), D_C_MC(j-1), D_C_MC(j), D_C_CP(j-1), 1 + D_C_CP(j), D_C_CP(j),
+// then D_P_T(j-1), D_MC_T(j-1), D_M_T(j), D_CP_T(j), eps(j-1), eps(j).  The
+// smoothness denominators are e = eps + 4 t^2 (4 t^2 is exact, so the fused
+// form rounds as the reference's); big collects their high words: while those
+// are below kBigE (2^100), and eps and the linear weights lie in
+// weno_consts_ok's range, every operand, reciprocal and quotient is a normal
+// double and the face equals weno_face's bit for bit.
+constexpr unsigned kBigE = (1023u + 100u) << 20;
+struct FaceW {
+  double a0, mc1, mc0, cp1, a1, cp0, pt, mct, mt, cpt, e1, e0;
+};
+__device__ __forceinline__ unsigned hi_word(double v) { return (unsigned)__double2hiint(v); }
+// One side of N faces, operation by operation over the faces: the faces are
+// independent, and their chains (two reciprocals and some thirty dependent
+// operations each) hide each other's latency when they are interleaved.  The
+// side's candidates are p0 = a v1 - d v0, p1 = f v1 + g v2 with differences
+// d (v1 - v0), g (v2 - v1), linear weights l0, l1 and eps.
+template <int N>
+__device__ __forceinline__ void face_side(const double (&v0)[N], const double (&v1)[N], const double (&v2)[N],
+                                          const double (&a)[N], const double (&d)[N], const double (&f)[N],
+                                          const double (&g)[N], const double (&l0)[N], const double (&l1)[N],
+                                          const double (&eps)[N], double (&u)[N], unsigned &big) {
+  double w0[N], w1[N], y0[N], y1[N];
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const double t0 = d[n] * (v1[n] - v0[n]), t1 = g[n] * (v2[n] - v1[n]);
+    const double e0 = fma(kFour, t0 * t0, eps[n]), e1 = fma(kFour, t1 * t1, eps[n]);
+    big = max(big, max(hi_word(e0), hi_word(e1)));
+    w0[n] = e0 * e0;
+    w1[n] = e1 * e1;
+  }
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    y0[n] = recip_nr(w0[n]);
+    y1[n] = recip_nr(w1[n]);
+  }
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    w0[n] = quot_nr(l0[n], w0[n], y0[n]);
+    w1[n] = quot_nr(l1[n], w1[n], y1[n]);
+    y1[n] = w0[n] + w1[n];
+  }
+#pragma unroll
+  for (int n = 0; n < N; ++n) y0[n] = recip_nr(y1[n]);
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const double p0 = a[n] * v1[n] - d[n] * v0[n];
+    const double p1 = f[n] * v1[n] + g[n] * v2[n];
+    u[n] = quot_nr(w0[n], y1[n], y0[n]) * p0 + quot_nr(w1[n], y1[n], y0[n]) * p1;
+  }
+}
+// the same with the IEEE division, for the faces out of range, its weights read
+// from shared memory: w[q * stride], in FaceW's order from t (theta faces) or
+// in Weno::ptab's (phi faces)
+__device__ __noinline__ double face_ieee(double LNm2, double LNm1, double LN0, double LPm1, double LP0, double LPp1,
+                                         const double *w, int stride) {
+  auto W = [&](int q) { return w[q * stride]; };
+  if (stride == 1)
+    return weno_face(LNm2, LNm1, LN0, LPm1, LP0, LPp1, W(0), W(1), W(2), W(3), W(4), W(5), W(6), W(7), W(8), W(9));
+  return weno_face(LNm2, LNm1, LN0, LPm1, LP0, LPp1, W(1), W(2), W(3), W(5), W(6), W(7), W(8), W(9), W(10), W(11));
+}
+
+// Phi columns per warp: the fewest full waves of resident warps that keep the
+// chunk at kAColsMax columns or less, and kAColsMin at least.
+constexpr int kAColsMin = 2;
+inline int adv_cols(int n2, int strips, int nreal, int slots) {
+  const int64_t per = (int64_t)strips * nreal * kAWarps;
+  for (int64_t w = 1;; ++w) {
+    const int64_t nch = w * slots / per * kAWarps;
+    if (nch < 1) continue;
+    const int64_t c = (n2 + nch - 1) / nch;
+    if (c <= kAColsMax) return (int)std::max<int64_t>(c, kAColsMin);
+  }
+}
+
+struct AdvArgs {
+  const double *x, *f0;   // stage input; f0 in combine mode 1
+  double *out;
+  AdvCombine cb;
+  // ragged batches: realization (0-based) of grid slice y (null: y itself; a
+  // negative entry: none), and its substep, which multiplies cb.C (null: 1)
+  const int *rlist;
+  const double *rdt;
+  int strips, cols;       // theta strips, phi columns per warp
+  double bcn, bcs;        // pole factors
+};
+
+// The pole rows 1 and ntm of a realization's stage, whose value needs the ring
+// sum of the upwind fluxes next to them over all phi columns (src/hipft.f90:
+// 7902-7915): one block.  The sums are those of 256 threads (two per thread
+// here) and a tree over them.
+__device__ __forceinline__ void adv_pole_rows(const Mesh &m, const Flow &fl, const AdvArgs &a, int i0, double *sh) {
+  const int i = i0 + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t ld = m.ldt;
+  const double *x = a.x + (int64_t)i0 * m.plane, *f0 = a.f0 + (int64_t)i0 * m.plane;
+  double *out = a.out + (int64_t)i0 * m.plane;
+#pragma unroll
+  for (int v = 0; v < 2; ++v) {
+    double fn = 0.0, fs = 0.0;
+#pragma unroll 4
+    for (int k = 2 + (int)threadIdx.x + 128 * v; k <= m.npm - 1; k += 256) {
+      const double *c = x + (int64_t)(k - 1) * ld;
+      const double ftn = upwind_flux(vt_at(m, fl, 2, k, i), fl.upwind, c[1], c[0]);
+      const double fts = upwind_flux(vt_at(m, fl, m.nt - 1, k, i), fl.upwind, c[m.ntm - 1], c[m.ntm - 2]);
+      fn = fn + ftn * m.dp[k];
+      fs = fs + fts * m.dp[k];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      fn += __shfl_down_sync(0xffffffffu, fn, o);
+      fs += __shfl_down_sync(0xffffffffu, fs, o);
+    }
+    if (lane == 0) {
+      sh[2 * (4 * v + warp)] = fn;
+      sh[2 * (4 * v + warp) + 1] = fs;
+    }
+  }
+  __syncthreads();
+  double fn = lane < 8 ? sh[2 * lane] : 0.0, fs = lane < 8 ? sh[2 * lane + 1] : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    fn += __shfl_down_sync(0xffffffffu, fn, o);
+    fs += __shfl_down_sync(0xffffffffu, fs, o);
+  }
+  const double an = __shfl_sync(0xffffffffu, fn, 0) * a.bcn, as = -__shfl_sync(0xffffffffu, fs, 0) * a.bcs;
+  const double C = a.rdt ? a.cb.C * a.rdt[i0] : a.cb.C;
+#pragma unroll 4
+  for (int k = 2 + (int)threadIdx.x; k <= m.npm - 1; k += 128) {
+    const int64_t q = (int64_t)(k - 1) * ld, sm = k == 2 ? (m.npm - 2) * ld : k == m.npm - 1 ? -(m.npm - 2) * ld : 0;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int64_t p = q + (s ? m.ntm - 1 : 0);
+      const double ax = s ? as : an;
+      const double y = a.cb.mode == 0 ? x[p] - C * ax : a.cb.A * f0[p] + a.cb.B * x[p] - C * ax;
+      out[p] = y;
+      if (sm) out[p + sm] = y;
+    }
+  }
+}
+
+// One stage; block 0 of a realization takes the pole rows, the others the rows
+// 2..ntm-1.  A warp holds 64 theta rows, two per lane, and
+// marches along the phi columns of its chunk: at the step that brings in
+// column e it computes the phi faces e-1 of its rows and, for the cells of
+// column k = e-2, the theta faces between its rows and above them: every face
+// once, four per lane and step, as independent chains.  The phi faces' inputs
+// are windows of the row in registers, the theta faces' come from the
+// neighbouring lanes by shuffles, and the outermost rows of the strip only
+// supply those.  Inputs arrive three columns ahead through a ring in shared
+// memory, by asynchronous copies of the lane's own rows (the phi faces' table
+// row by lanes 0..7); the theta faces' weights sit in shared memory, shared by
+// the block's warps, which march four neighbouring chunks of one strip.  The
+// next stage may be launched when this one's blocks have started; it sets up its
+// tables and then waits for this one.
+//
+// Bound: the FP64 pipe, about 95 instructions per face and 210 per cell, most
+// of them the eight divisions per face (two reciprocals shared).
+//
+// FLOW2D: 2-D velocities; MODE: the combine; Off: a byte offset in a plane.
+template <bool FLOW2D, int MODE, typename Off>
+__global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Flow fl, Weno wn, AdvArgs a) {
+  extern __shared__ __align__(16) double asm_[];
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ntm = m.ntm, npm = m.npm, n2 = npm - 2, nt = m.nt;
+  const int i = a.rlist ? a.rlist[blockIdx.y] : (int)blockIdx.y;  // 0-based
+  if (i < 0) {
+    pdl_wait();
+    return;
+  }
+  if (blockIdx.x == 0) {
+    pdl_wait();
+    adv_pole_rows(m, fl, a, i, asm_);
+    return;
+  }
+  const int blk = (int)blockIdx.x - 1, strip = blk % a.strips;
+  const int R0 = kAOwn * strip - 1;  // rows R0 .. R0+63, owned: R0+2 .. R0+61
+  for (int p = threadIdx.x; p < 64; p += 32 * kAWarps) {
+    // weights of the face above row R0+p
+    const int jw = min(max(R0 + p + 1, 2), nt - 1);
+    const double v[kAWt] = {kOne + wn.mct[jw - 1], wn.mct[jw - 1], wn.mct[jw], wn.cpt[jw - 1], kOne + wn.cpt[jw],
+                            wn.cpt[jw],            wn.pt[jw - 1],  wn.mctt[jw - 1], wn.mt[jw], wn.cptt[jw],
+                            wn.epst[jw - 1],       wn.epst[jw]};
+#pragma unroll
+    for (int q = 0; q < kAWt; ++q) asm_[q * 64 + p] = v[q];
+  }
+  __syncthreads();
+  const int c0 = 2 + (blk / a.strips * kAWarps + warp) * a.cols, c1 = min(c0 + a.cols - 1, npm - 1);
+  if (c0 > npm - 1) {
+    pdl_wait();
+    return;
+  }
+  const double C = a.rdt ? a.cb.C * a.rdt[i] : a.cb.C;
+  const int r = R0 + 2 * lane;  // this lane's rows r, r+1
+  const bool own = lane >= 1 && lane <= 30;
+  const bool va = own && r >= 2 && r <= ntm - 1, vb = own && r + 1 <= ntm - 1;
+  const bool tupA = r + 1 == 2 || r + 1 == ntm, tupB = r + 2 == 2 || r + 2 == ntm;
+  const bool wup = __any_sync(0xffffffffu, tupA || tupB);
+  const bool edge = __any_sync(0xffffffffu, va != vb);  // a pair stored by halves
+  const uint32_t swt = smem_addr(asm_) + 16u * lane;
+  bool tok;  // the weights of this lane's WENO faces (3 .. nt-2) are in range
+  {
+    auto ok = [&](int q) {
+      const int jf = R0 + q + 1;
+      const double *w = asm_ + q;
+      return jf < 3 || jf > nt - 2 ||
+             weno_consts_ok(w[6 * 64], w[7 * 64], w[8 * 64], w[9 * 64], w[10 * 64], w[11 * 64]);
+    };
+    tok = ok(2 * lane) && ok(2 * lane + 1);
+  }
+  // divergence factors of rows r, r+1
+  const int ra = min(max(r, 1), ntm), rb = min(max(r + 1, 1), ntm);
+  const double sth0 = m.sth[ra], sth1 = m.sth[min(max(r + 1, 1), nt)], sth2 = m.sth[min(max(r + 2, 1), nt)];
+  const double2 sti = make_double2(m.st_i[ra], m.st_i[rb]), dti = make_double2(m.dt_i[ra], m.dt_i[rb]);
+  // LN(c) = half x(c) (vt(c)+at(c)) and LP(c) = half x(c) (vt(c+1)-at(c)) are
+  // formed as x(c) * (half (vt(c)+at(c))) etc.: halving is exact, so the
+  // products are the reference's (for |x| above 2^-1021, i.e. any map)
+  double2 tn = {}, tp = {}, pn = {}, pp = {};
+  double vuA = 0.0, vuB = 0.0;  // velocities of the upwind faces r+1, r+2
+  if (!FLOW2D) {
+    const double *vt = fl.vt1 + (int64_t)i * (nt + 1), *at = fl.at1 + (int64_t)i * (ntm + 1);
+    const double *vp = fl.vp1 + (int64_t)i * (ntm + 1), *ap = fl.ap1 + (int64_t)i * (ntm + 1);
+    const double va0 = vt[ra], va1 = vt[min(max(r + 1, 1), nt)], va2 = vt[min(max(r + 2, 1), nt)];
+    tn = make_double2(kHalf * (va0 + at[ra]), kHalf * (va1 + at[rb]));
+    tp = make_double2(kHalf * (va1 - at[ra]), kHalf * (va2 - at[rb]));
+    pn = make_double2(kHalf * (vp[ra] + ap[ra]), kHalf * (vp[rb] + ap[rb]));
+    pp = make_double2(kHalf * (vp[ra] - ap[ra]), kHalf * (vp[rb] - ap[rb]));
+    vuA = va1;
+    vuB = va2;
+  }
+
+  // ring of input columns
+  constexpr uint32_t kF = 512, kSlot = adv_slot(FLOW2D) * 8;
+  double *rbase = asm_ + kAWt * 64 + warp * kASlots * adv_slot(FLOW2D);
+  const uint32_t sring = smem_addr(rbase) + 16u * lane, stab = smem_addr(rbase) + (FLOW2D ? 7 : 2) * kF;
+  const int64_t pb = (int64_t)i * m.plane, vb0 = (int64_t)i * fl.vplane;
+  const Off ldb = (Off)m.ldt * 8, lvb = (Off)fl.ldv * 8;
+  const Off rowb = (Off)min(max(r - 1, 0), m.ldt - 2) * 8, rowv = (Off)min(max(r - 1, 0), fl.ldv - 2) * 8;
+  const char *gx = reinterpret_cast<const char *>(a.x + pb), *gf = reinterpret_cast<const char *>(a.f0 + pb);
+  const char *gvt = reinterpret_cast<const char *>(fl.vt + vb0), *gat = reinterpret_cast<const char *>(fl.at + vb0);
+  const char *gvp = reinterpret_cast<const char *>(fl.vp + vb0), *gap = reinterpret_cast<const char *>(fl.ap + vb0);
+  char *go = reinterpret_cast<char *>(a.out + pb);
+  const Off upv = r + 1 <= fl.ldv - 2 ? 16 : 0;  // to the pair of rows r+2, r+3 (not read past the faces)
+  int fe = c0 - 2, fs = 0;  // column to fetch next, its slot
+  auto fetch = [&]() {
+    if (fe <= c1 + 2) {
+      const uint32_t s = sring + fs * kSlot;
+      const int cw = fe < 1 ? fe + n2 : fe > npm - 1 ? fe - n2 : fe;  // the reference's periodic pad
+      cp_async16(s, gx + ((Off)(cw - 1) * ldb + rowb));
+      if (FLOW2D) {
+        const Off o = (Off)(cw - 1) * lvb + rowv;
+        cp_async16(s + 4 * kF, gvp + o);
+        cp_async16(s + 5 * kF, gvp + (o + lvb));
+        cp_async16(s + 6 * kF, gap + o);
+      }
+      if (fe >= c0 + 1 && lane < kPhiTab / 2)
+        cp_async16(stab + fs * kSlot + 16u * lane, wn.ptab + (int64_t)(fe - 3) * kPhiTab + 2 * lane);
+      if (fe >= c0 + 2) {
+        if (MODE != 0) cp_async16(s + kF, gf + ((Off)(fe - 3) * ldb + rowb));
+        if (FLOW2D) {
+          const Off o = (Off)(fe - 3) * lvb + rowv;
+          cp_async16(s + 2 * kF, gvt + o);
+          cp_async16(s + 3 * kF, gat + o);
+          if (lane == 31) cp_async16(stab + fs * kSlot + kPhiTab * 8, gvt + (o + upv));
+        }
+      }
+    }
+    cp_async_commit();
+    ++fe;
+    fs = (fs + 1) & (kASlots - 1);
+  };
+  pdl_wait();
+  fetch();
+  fetch();
+  fetch();
+
+  // windows at the step of column e: LN at e-3, e-2, e-1; LP and x at e-2, e-1
+  double2 LN0 = {}, LN1 = {}, LN2 = {}, LP0 = {}, LP1 = {}, x0 = {}, x1 = {}, Fplo = {};
+  double dpk = 0.0;
+  int slot = 0;
+  auto step = [&](int e, auto phc) {
+    constexpr int PH = decltype(phc)::value;  // 0: fill the windows, 1: and the first phi face, 2: everything
+    cp_async_wait<2>();
+    __syncwarp();  // the table row came by other lanes; and the slot fetched next is read out
+    fetch();
+    const uint32_t s = sring + slot * kSlot, st = stab + slot * kSlot;
+    slot = (slot + 1) & (kASlots - 1);
+    const double2 xe = lds2(s);
+    double2 cN = pn, cP = pp;
+    if (FLOW2D) {
+      const double2 v0 = lds2(s + 4 * kF), v1 = lds2(s + 5 * kF), al = lds2(s + 6 * kF);
+      cN = make_double2(kHalf * (v0.x + al.x), kHalf * (v0.y + al.y));
+      cP = make_double2(kHalf * (v1.x - al.x), kHalf * (v1.y - al.y));
+    }
+    const double2 LN3 = make_double2(xe.x * cN.x, xe.y * cN.y), LP2 = make_double2(xe.x * cP.x, xe.y * cP.y);
+    double2 Fp = {};
+    double dpn = 0.0;
+    if (PH >= 1) {
+      unsigned big = 0;
+      const double2 q0 = lds2(st), q1 = lds2(st + 16), q2 = lds2(st + 32), q3 = lds2(st + 48), q4 = lds2(st + 64),
+                    q5 = lds2(st + 80), q6 = lds2(st + 96);
+      const FaceW wp{q6.x, q0.x, q0.y, q1.x, q6.y, q1.y, q2.x, q2.y, q3.x, q3.y, q4.x, q4.y};
+      dpn = q5.y;
+      if (PH == 1) {
+        double um[2], up[2];
+        face_side<2>({LN0.x, LN0.y}, {LN1.x, LN1.y}, {LN2.x, LN2.y}, {wp.a0, wp.a0}, {wp.mc1, wp.mc1}, {wp.mc0, wp.mc0},
+                     {wp.cp1, wp.cp1}, {wp.pt, wp.pt}, {wp.mct, wp.mct}, {wp.e1, wp.e1}, um, big);
+        face_side<2>({LP2.x, LP2.y}, {LP1.x, LP1.y}, {LP0.x, LP0.y}, {wp.a1, wp.a1}, {wp.cp0, wp.cp0}, {wp.cp1, wp.cp1},
+                     {wp.mc0, wp.mc0}, {wp.mt, wp.mt}, {wp.cpt, wp.cpt}, {wp.e0, wp.e0}, up, big);
+        Fp = make_double2(up[0] + um[0], up[1] + um[1]);
+      }
+      double FA = 0.0, FB = 0.0;
+      double2 fc = {}, LNt = {}, LPt = {};
+      double LNm = 0.0, LNp = 0.0, LPp = 0.0, LPq = 0.0;
+      if (PH == 2) {
+        double2 ctn = tn, ctp = tp;
+        if (FLOW2D) {
+          const double2 v = lds2(s + 2 * kF), al = lds2(s + 3 * kF);
+          const double vn = __shfl_down_sync(0xffffffffu, v.x, 1);
+          const double v2 = lane == 31 ? lds2(st + kPhiTab * 8).x : vn;
+          ctn = make_double2(kHalf * (v.x + al.x), kHalf * (v.y + al.y));
+          ctp = make_double2(kHalf * (v.y - al.x), kHalf * (v2 - al.y));
+          vuA = v.y;
+          vuB = v2;
+        }
+        if (MODE != 0) fc = lds2(s + kF);
+        LNt = make_double2(x0.x * ctn.x, x0.y * ctn.y);
+        LPt = make_double2(x0.x * ctp.x, x0.y * ctp.y);
+        LNm = __shfl_up_sync(0xffffffffu, LNt.y, 1);
+        LNp = __shfl_down_sync(0xffffffffu, LNt.x, 1);
+        LPp = __shfl_down_sync(0xffffffffu, LPt.x, 1);
+        LPq = __shfl_down_sync(0xffffffffu, LPt.y, 1);
+        double2 t[kAWt];
+#pragma unroll
+        for (int q = 0; q < kAWt; ++q) t[q] = lds2(swt + q * 512u);
+        const FaceW wA{t[0].x, t[1].x, t[2].x, t[3].x, t[4].x, t[5].x, t[6].x, t[7].x, t[8].x, t[9].x, t[10].x, t[11].x};
+        const FaceW wB{t[0].y, t[1].y, t[2].y, t[3].y, t[4].y, t[5].y, t[6].y, t[7].y, t[8].y, t[9].y, t[10].y, t[11].y};
+        // the phi faces e-1 and the theta faces of column e-2
+        double um[4], up[4];
+        face_side<4>({LN0.x, LN0.y, LNm, LNt.x}, {LN1.x, LN1.y, LNt.x, LNt.y}, {LN2.x, LN2.y, LNt.y, LNp},
+                     {wp.a0, wp.a0, wA.a0, wB.a0}, {wp.mc1, wp.mc1, wA.mc1, wB.mc1}, {wp.mc0, wp.mc0, wA.mc0, wB.mc0},
+                     {wp.cp1, wp.cp1, wA.cp1, wB.cp1}, {wp.pt, wp.pt, wA.pt, wB.pt}, {wp.mct, wp.mct, wA.mct, wB.mct},
+                     {wp.e1, wp.e1, wA.e1, wB.e1}, um, big);
+        face_side<4>({LP2.x, LP2.y, LPp, LPq}, {LP1.x, LP1.y, LPt.y, LPp}, {LP0.x, LP0.y, LPt.x, LPt.y},
+                     {wp.a1, wp.a1, wA.a1, wB.a1}, {wp.cp0, wp.cp0, wA.cp0, wB.cp0}, {wp.cp1, wp.cp1, wA.cp1, wB.cp1},
+                     {wp.mc0, wp.mc0, wA.mc0, wB.mc0}, {wp.mt, wp.mt, wA.mt, wB.mt}, {wp.cpt, wp.cpt, wA.cpt, wB.cpt},
+                     {wp.e0, wp.e0, wA.e0, wB.e0}, up, big);
+        Fp = make_double2(up[0] + um[0], up[1] + um[1]);
+        FA = up[2] + um[2];
+        FB = up[3] + um[3];
+      }
+      if (!(big < kBigE && tok && q5.x != 0.0)) {
+        const double *w = rbase + ((slot + kASlots - 1) & (kASlots - 1)) * adv_slot(FLOW2D) + (FLOW2D ? 7 : 2) * 64;
+        Fp.x = face_ieee(LN0.x, LN1.x, LN2.x, LP0.x, LP1.x, LP2.x, w, 1);
+        Fp.y = face_ieee(LN0.y, LN1.y, LN2.y, LP0.y, LP1.y, LP2.y, w, 1);
+        if (PH == 2) {
+          FA = face_ieee(LNm, LNt.x, LNt.y, LPt.x, LPt.y, LPp, asm_ + 2 * lane, 64);
+          FB = face_ieee(LNt.x, LNt.y, LNp, LPt.y, LPp, LPq, asm_ + 2 * lane + 1, 64);
+        }
+      }
+      if (PH == 2) {
+        if (wup) {  // first-order upwind next to the poles
+          const double xn = __shfl_down_sync(0xffffffffu, x0.x, 1);
+          if (tupA) FA = upwind_flux(vuA, fl.upwind, x0.y, x0.x);
+          if (tupB) FB = upwind_flux(vuB, fl.upwind, xn, x0.y);
+        }
+        const double Flo = __shfl_up_sync(0xffffffffu, FB, 1);
+        const double aopx = (sth1 * FA - sth0 * Flo) * sti.x * dti.x + (Fp.x - Fplo.x) * sti.x * dpk;
+        const double aopy = (sth2 * FB - sth1 * FA) * sti.y * dti.y + (Fp.y - Fplo.y) * sti.y * dpk;
+        const double2 y = MODE == 0 ? make_double2(x0.x - C * aopx, x0.y - C * aopy)
+                                    : make_double2(a.cb.A * fc.x + a.cb.B * x0.x - C * aopx,
+                                                   a.cb.A * fc.y + a.cb.B * x0.y - C * aopy);
+        const int k = e - 2;
+        char *g = go + ((Off)(k - 1) * ldb + rowb);
+        st_if(va && vb, g, y);
+        if (edge || k == 2 || k == npm - 1) {
+          const int64_t sm = k == 2 ? (int64_t)n2 * m.ldt : k == npm - 1 ? -(int64_t)n2 * m.ldt : 0;
+          double *d = reinterpret_cast<double *>(g);
+          if (va) d[sm] = y.x;
+          if (vb) d[sm + 1] = y.y;
+          if (va && !vb) d[0] = y.x;
+          if (vb && !va) d[1] = y.y;
+        }
+      }
+    }
+    LN0 = LN1;
+    LN1 = LN2;
+    LN2 = LN3;
+    LP0 = LP1;
+    LP1 = LP2;
+    x0 = x1;
+    x1 = xe;
+    Fplo = Fp;
+    dpk = dpn;
+  };
+#pragma unroll 1
+  for (int e = c0 - 2; e <= c0; ++e) step(e, IntC<0>{});
+  step(c0 + 1, IntC<1>{});
+#pragma unroll 1
+  for (int e = c0 + 2; e <= c1 + 2; ++e) step(e, IntC<2>{});
+  cp_async_wait<0>();
+}
+
+}  // namespace hipft

@@ -20,6 +20,7 @@
 #include "../../include/hipft_gpu.h"
 #include "kernels.cuh"
 #include "sts_march.cuh"
+#include "adv_march.cuh"
 #include "adjoint.cuh"
 #include "graph_step.cuh"
 
@@ -590,68 +591,59 @@ static int diffusion_stage(hipft_gpu *h, const double *x, const double *ykm2, co
   return HIPFT_OK;
 }
 
-// HIPFT_ADV_KERNEL selects the WENO3 stage kernel: "tile" the tile kernel
-// (k_advection_stage<32, 8, true>), "march" the phi-marching kernel on any
-// grid; unset, the library decides by grid size.  Both give bitwise the same
-// fields; the tests compare the two.
-static int adv_kernel_env() {
-  static int v = -1;
-  if (v < 0) {
-    const char *e = std::getenv("HIPFT_ADV_KERNEL");
-    v = (e && std::strcmp(e, "tile") == 0) ? 1 : (e && std::strcmp(e, "march") == 0) ? 2 : 0;
-  }
-  return v;
-}
-
 // One explicit advection stage over nz realization slots (rlist maps slot z
-// to a realization when non-null; rdt scales each realization's step).
-// WENO3 stages march along phi (k_adv_weno_march) when the grid, in chunks of
-// 64 or 32 phi columns, holds 1.5 waves of warps (16 resident per SM): on one
-// 1024 x 2048 realization the tile kernel is faster (0.090 against 0.102 ms),
-// on 64 of them the marching kernel (3.97 against 5.57 ms).  Upwind stages
-// take the tile kernel.
-static void launch_adv_stage(const hipft_gpu *h, const Mesh &M, cudaStream_t s, unsigned nz, const double *x,
-                             const double *f0, double *out, AdvCombine cb, const int *rlist, const double *rdt) {
-  if (h->adv_space == 2 && adv_kernel_env() != 1) {
-    const int64_t groups = (h->ntm - 1) / 31 + 1, fill = 24LL * h->num_sms;
-    auto warps = [&](int ncol) { return groups * ((h->npm - 2 + ncol - 1) / ncol) * (int64_t)nz; };
-    int ncol = kAdvColsMax;
-    while (ncol > 8 && warps(ncol) < fill) ncol /= 2;
-    if (ncol >= 32 || adv_kernel_env() == 2) {
-      const dim3 blk(32, kAdvWarps);
-      const dim3 grd((unsigned)((groups + kAdvWarps - 1) / kAdvWarps), (unsigned)((h->npm - 2 + ncol - 1) / ncol),
-                     nz);
-      auto kern = h->FL.flow2d ? (cb.mode == 0 ? k_adv_weno_march<true, 0> : k_adv_weno_march<true, 1>)
-                               : (cb.mode == 0 ? k_adv_weno_march<false, 0> : k_adv_weno_march<false, 1>);
-      kern<<<grd, blk, 0, s>>>(M, h->FL, h->W, x, f0, out, h->d_ring, h->bc_flow_n, h->bc_flow_s, cb, rlist, rdt,
-                               ncol);
-      return;
-    }
-  }
-  const dim3 blk(33, 9);  // (TJ+1) x (TK+1) threads for a 32 x 8 tile
-  const dim3 grd((unsigned)((h->ntm + 31) / 32), (unsigned)((h->npm - 2 + 7) / 8), nz);
-  if (h->adv_space == 2)
-    k_advection_stage<32, 8, true><<<grd, blk, 0, s>>>(M, h->FL, h->W, x, f0, out, h->d_ring, h->bc_flow_n,
-                                                        h->bc_flow_s, cb, rlist, rdt);
-  else
-    k_advection_stage<32, 8, false><<<grd, blk, 0, s>>>(M, h->FL, h->W, x, f0, out, h->d_ring, h->bc_flow_n,
-                                                         h->bc_flow_s, cb, rlist, rdt);
+// to a realization when non-null; rdt scales each realization's step), on
+// stream s.  chained: the launch before it on the stream is the stage before.
+typedef void (*AdvKernel)(Mesh, Flow, Weno, AdvArgs);
+static AdvKernel adv_kernel(bool flow2d, bool mode, bool wide) {
+  if (wide)
+    return flow2d ? (mode ? k_adv_march<true, 1, uint64_t> : k_adv_march<true, 0, uint64_t>)
+                  : (mode ? k_adv_march<false, 1, uint64_t> : k_adv_march<false, 0, uint64_t>);
+  return flow2d ? (mode ? k_adv_march<true, 1, uint32_t> : k_adv_march<true, 0, uint32_t>)
+                : (mode ? k_adv_march<false, 1, uint32_t> : k_adv_march<false, 0, uint32_t>);
 }
 
-static int advection_stage(hipft_gpu *h, const double *x, const double *f0, double *out, AdvCombine cb) {
-  {
-    ProfScope ps(h, HIPFT_K_RING);
-    k_ring_advection<<<h->nr, 256, 0, h->stream>>>(h->M, h->FL, x, h->d_ring);
-    LAUNCHED(h);
+static cudaError_t launch_adv_stage(const hipft_gpu *h, cudaStream_t s, unsigned nz, const double *x, const double *f0,
+                                    double *out, AdvCombine cb, const int *rlist, const double *rdt, bool pdl,
+                                    bool chained) {
+  if (h->adv_space != 2) {
+    k_ring_advection<<<h->nr, 256, 0, s>>>(h->M, h->FL, x, h->d_ring);
+    const dim3 blk(33, 9);  // (TJ+1) x (TK+1) threads for a 32 x 8 tile
+    const dim3 grd((unsigned)((h->ntm + 31) / 32), (unsigned)((h->npm - 2 + 7) / 8), nz);
+    k_adv_upwind<32, 8><<<grd, blk, 0, s>>>(h->M, h->FL, x, f0, out, h->d_ring, h->bc_flow_n, h->bc_flow_s, cb, rlist,
+                                            rdt);
+    return cudaPeekAtLastError();
   }
+  AdvArgs a{x, f0, out, cb, rlist, rdt, 0, 0, h->bc_flow_n, h->bc_flow_s};
+  const int n2 = h->npm - 2;
+  a.strips = (h->ntm - 1 + kAOwn - 1) / kAOwn;  // rows up to ntm-1
+  a.cols = adv_cols(n2, a.strips, (int)nz, kABlocks * kAWarps * h->num_sms);
+  const int nch = (n2 + a.cols - 1) / a.cols;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = (pdl && chained) ? 1 : 0;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3((unsigned)(1 + a.strips * ((nch + kAWarps - 1) / kAWarps)), nz);
+  cfg.blockDim = dim3(32 * kAWarps);
+  cfg.dynamicSmemBytes = adv_smem(h->FL.flow2d);
+  const bool wide = std::max(h->plane, h->FL.vplane) >= (int64_t)1 << 29;
+  return cudaLaunchKernelEx(&cfg, adv_kernel(h->FL.flow2d, cb.mode != 0, wide), h->M, h->FL, h->W, a);
+}
+
+static int advection_stage(hipft_gpu *h, const double *x, const double *f0, double *out, AdvCombine cb,
+                           bool chained, int n = 0, const int *rlist = nullptr, const double *rdt = nullptr) {
   ProfScope ps(h, HIPFT_K_ADV);
-  launch_adv_stage(h, h->M, h->stream, (unsigned)h->nr, x, f0, out, cb, nullptr, nullptr);
-  LAUNCHED(h);
-  h->cell_updates += (int64_t)h->ntm * (h->npm - 2) * h->nr;
+  if (!n) n = h->nr;
+  const cudaError_t e = launch_adv_stage(h, h->stream, (unsigned)n, x, f0, out, cb, rlist, rdt, ws_pdl(), chained);
+  if (e != cudaSuccess) return fail(h, HIPFT_ECUDA, "advection stage launch: %s", cudaGetErrorString(e));
+  h->launches += h->adv_space == 2 ? 1 : 2;
+  h->cell_updates += (int64_t)h->ntm * (h->npm - 2) * n;
   return HIPFT_OK;
 }
 
-// ---------------------------------------------------------------- create
 extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hipft_gpu **out) {
   if (!g || !prm || !out || !g->t || !g->p) return HIPFT_EINVAL;
   *out = nullptr;
@@ -738,6 +730,9 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
   for (int v = 0; v < 8; ++v)
     smem_ok = smem_ok && cudaFuncSetAttribute(march_kernel(v & 1, v & 2, v & 4), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)kMSmem) == cudaSuccess;
+  for (int v = 0; v < 8; ++v)
+    smem_ok = smem_ok && cudaFuncSetAttribute(adv_kernel(v & 1, v & 2, v & 4), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)adv_smem(v & 1)) == cudaSuccess;
   if (!smem_ok ||
       cudaFuncSetAttribute(k_sts_poles<kPMidThreads, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)poles_smem(kPMidThreads)) != cudaSuccess ||
@@ -820,6 +815,8 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
       double *row = pk.data() + tab0 + (size_t)(kf - 2) * kPhiTab;
       const double v[10] = {wp[1][kw - 1], wp[1][kw], wp[0][kw - 1], wp[0][kw], wp[4][kw - 1],
                             wp[5][kw - 1], wp[2][kw], wp[3][kw],     wp[6][kw - 1], wp[6][kw]};
+      row[12] = 1.0 + v[0];
+      row[13] = 1.0 + v[3];
       for (int q = 0; q < 10; ++q) row[q] = v[q];
       row[10] = weno_consts_ok(v[4], v[5], v[6], v[7], v[8], v[9]) ? 1.0 : 0.0;
       row[11] = (kf <= npm - 1) ? h->dp_i[kf] : 0.0;
@@ -1238,17 +1235,17 @@ static int plain_advection_step(hipft_gpu *h, double dt) {
   int ia = scratch(h, 0), ib = scratch(h, 1);
   double *A = h->buf[ia], *B = h->buf[ib];
   if (h->adv_time == 1) {  // FE (src/hipft.f90:7440-7444)
-    TRY(advection_stage(h, f, nullptr, A, AdvCombine{0, 0.0, 0.0, dt}));
+    TRY(advection_stage(h, f, nullptr, A, AdvCombine{0, 0.0, 0.0, dt}, false));
     h->cur = ia;
   } else if (h->adv_time == 2) {  // SSPRK(3,3) (7486-7505)
-    TRY(advection_stage(h, f, nullptr, A, AdvCombine{0, 0.0, 0.0, dt}));
-    TRY(advection_stage(h, A, f, B, AdvCombine{1, c_three_quarter, c_quarter, c_quarter * dt}));
-    TRY(advection_stage(h, B, f, f, AdvCombine{1, c_third, c_two_third, c_two_third * dt}));
+    TRY(advection_stage(h, f, nullptr, A, AdvCombine{0, 0.0, 0.0, dt}, false));
+    TRY(advection_stage(h, A, f, B, AdvCombine{1, c_three_quarter, c_quarter, c_quarter * dt}, true));
+    TRY(advection_stage(h, B, f, f, AdvCombine{1, c_third, c_two_third, c_two_third * dt}, true));
   } else {  // SSPRK(4,3) (7552-7574)
-    TRY(advection_stage(h, f, nullptr, A, AdvCombine{0, 0.0, 0.0, 0.5 * dt}));
-    TRY(advection_stage(h, A, nullptr, B, AdvCombine{0, 0.0, 0.0, 0.5 * dt}));
-    TRY(advection_stage(h, B, f, A, AdvCombine{1, c_two_third, c_third, c_sixth * dt}));
-    TRY(advection_stage(h, A, nullptr, f, AdvCombine{0, 0.0, 0.0, 0.5 * dt}));
+    TRY(advection_stage(h, f, nullptr, A, AdvCombine{0, 0.0, 0.0, 0.5 * dt}, false));
+    TRY(advection_stage(h, A, nullptr, B, AdvCombine{0, 0.0, 0.0, 0.5 * dt}, true));
+    TRY(advection_stage(h, B, f, A, AdvCombine{1, c_two_third, c_third, c_sixth * dt}, true));
+    TRY(advection_stage(h, A, nullptr, f, AdvCombine{0, 0.0, 0.0, 0.5 * dt}, true));
   }
   return HIPFT_OK;
 }
@@ -1663,20 +1660,6 @@ static int ragged_diffusion_step(hipft_gpu *h, double dtl, hipft_diffusion_info 
 // substep count: realization i takes n_i = ceil(dt / its own CFL limit)
 // substeps of dt / n_i (one substep when dt is within its limit, which is
 // the plain step).
-static int advection_stage_ragged(hipft_gpu *h, const double *x, const double *f0, double *out, AdvCombine cb,
-                                  int n) {
-  {
-    ProfScope ps(h, HIPFT_K_RING);
-    k_ring_advection<<<h->nr, 256, 0, h->stream>>>(h->M, h->FL, x, h->d_ring);
-    LAUNCHED(h);
-  }
-  ProfScope ps(h, HIPFT_K_ADV);
-  launch_adv_stage(h, h->M, h->stream, (unsigned)n, x, f0, out, cb, h->d_rlist_adv, h->d_rdt);
-  LAUNCHED(h);
-  h->cell_updates += (int64_t)h->ntm * (h->npm - 2) * n;
-  return HIPFT_OK;
-}
-
 static int plain_advection_step(hipft_gpu *h, double dt);
 
 static int ragged_advection_step(hipft_gpu *h, double dt) {
@@ -1706,14 +1689,14 @@ static int ragged_advection_step(hipft_gpu *h, double dt) {
     int na = 0;
     while (na < nr && n[act[na]] > q) ++na;
     if (h->adv_time == 2) {  // SSPRK(3,3) (src/hipft.f90:7486-7505)
-      TRY(advection_stage_ragged(h, f, nullptr, A, AdvCombine{0, 0.0, 0.0, 1.0}, na));
-      TRY(advection_stage_ragged(h, A, f, B, AdvCombine{1, c_three_quarter, c_quarter, c_quarter}, na));
-      TRY(advection_stage_ragged(h, B, f, f, AdvCombine{1, c_third, c_two_third, c_two_third}, na));
+      TRY(advection_stage(h, f, nullptr, A, AdvCombine{0, 0.0, 0.0, 1.0}, false, na, h->d_rlist_adv, h->d_rdt));
+      TRY(advection_stage(h, A, f, B, AdvCombine{1, c_three_quarter, c_quarter, c_quarter}, true, na, h->d_rlist_adv, h->d_rdt));
+      TRY(advection_stage(h, B, f, f, AdvCombine{1, c_third, c_two_third, c_two_third}, true, na, h->d_rlist_adv, h->d_rdt));
     } else {  // SSPRK(4,3) (src/hipft.f90:7552-7574)
-      TRY(advection_stage_ragged(h, f, nullptr, A, AdvCombine{0, 0.0, 0.0, 0.5}, na));
-      TRY(advection_stage_ragged(h, A, nullptr, B, AdvCombine{0, 0.0, 0.0, 0.5}, na));
-      TRY(advection_stage_ragged(h, B, f, A, AdvCombine{1, c_two_third, c_third, c_sixth}, na));
-      TRY(advection_stage_ragged(h, A, nullptr, f, AdvCombine{0, 0.0, 0.0, 0.5}, na));
+      TRY(advection_stage(h, f, nullptr, A, AdvCombine{0, 0.0, 0.0, 0.5}, false, na, h->d_rlist_adv, h->d_rdt));
+      TRY(advection_stage(h, A, nullptr, B, AdvCombine{0, 0.0, 0.0, 0.5}, true, na, h->d_rlist_adv, h->d_rdt));
+      TRY(advection_stage(h, B, f, A, AdvCombine{1, c_two_third, c_third, c_sixth}, true, na, h->d_rlist_adv, h->d_rdt));
+      TRY(advection_stage(h, A, nullptr, f, AdvCombine{0, 0.0, 0.0, 0.5}, true, na, h->d_rlist_adv, h->d_rdt));
     }
   }
   return HIPFT_OK;
@@ -2031,10 +2014,8 @@ static int graph_capture(hipft_gpu *h) {
 
   // ---- advection_step over frac * dt (src/hipft.f90:4509-4549)
   auto adv_stage = [&](cudaStream_t s, const double *x, const double *f0, double *out, AdvCombine cb) {
-    k_ring_advection<<<nr, 256, 0, s>>>(M, h->FL, x, h->d_ring);
-    peek();
-    launch_adv_stage(h, M, s, (unsigned)nr, x, f0, out, cb, g.rl_adv, g.rdt);
-    peek();
+    // the first stage reads the field, after a kernel that is not a stage
+    ok(launch_adv_stage(h, s, (unsigned)nr, x, f0, out, cb, g.rl_adv, g.rdt, h->g_pdl, x != F));
   };
   auto advection = [&](double frac) {
     cudaGraphConditionalHandle hc{};
@@ -2976,10 +2957,10 @@ static int adj_adv_fwd(hipft_gpu *h, double dtl, size_t &nt, size_t t[4]) {
   }
   double *f = h->buf[h->cur];
   CK(h, cudaMemcpyAsync(T[0], f, h->fieldn * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-  TRY(advection_stage(h, T[0], nullptr, T[1], AdvCombine{0, 0.0, 0.0, 0.5 * dtl}));
-  TRY(advection_stage(h, T[1], nullptr, T[2], AdvCombine{0, 0.0, 0.0, 0.5 * dtl}));
-  TRY(advection_stage(h, T[2], T[0], T[3], AdvCombine{1, c_two_third, c_third, c_sixth * dtl}));
-  TRY(advection_stage(h, T[3], nullptr, f, AdvCombine{0, 0.0, 0.0, 0.5 * dtl}));
+  TRY(advection_stage(h, T[0], nullptr, T[1], AdvCombine{0, 0.0, 0.0, 0.5 * dtl}, false));
+  TRY(advection_stage(h, T[1], nullptr, T[2], AdvCombine{0, 0.0, 0.0, 0.5 * dtl}, true));
+  TRY(advection_stage(h, T[2], T[0], T[3], AdvCombine{1, c_two_third, c_third, c_sixth * dtl}, true));
+  TRY(advection_stage(h, T[3], nullptr, f, AdvCombine{0, 0.0, 0.0, 0.5 * dtl}, true));
   h->dring_valid = false;
   return HIPFT_OK;
 }
