@@ -580,13 +580,40 @@ static int scale_dty0(hipft_gpu *h, const double *af, double *dty0, double dtl, 
 
 template <int MODE>
 static int diffusion_stage(hipft_gpu *h, const double *x, const double *ykm2, const double *u0, const double *dty0,
-                           double *out, double *out2, const double *ring, StageCoef sc,
-                           unsigned long long *absmax) {
+                           double *out, double *out2, const double *ring, StageCoef sc) {
   dim3 blk(32, 8);
   ProfScope ps(h, MODE == MODE_STSK ? HIPFT_K_STS : HIPFT_K_OTHER);
   k_diffusion_stage<MODE><<<stage_grid(h, 32, 8), blk, 0, h->stream>>>(h->M, h->DC, x, ykm2, u0, dty0, out, out2,
-                                                                       ring, h->bc_diff_n, h->bc_diff_s, sc,
-                                                                       absmax);
+                                                                       ring, h->bc_diff_n, h->bc_diff_s, sc);
+  LAUNCHED(h);
+  return HIPFT_OK;
+}
+
+// Grid of k_ax and k_ptl over n realizations.
+static dim3 ax_grid(const hipft_gpu *h, int n) {
+  return dim3((unsigned)((h->ntm + 31) / 32), (unsigned)((h->npm - 2 + 8 * kAxCols - 1) / (8 * kAxCols)), (unsigned)n);
+}
+
+// Maxima of k_ax's blocks.
+static unsigned long long *ax_block_max(const hipft_gpu *h) { return h->d_bits + 4; }
+
+// A u0 of the current field into scratch buffer 0 and, with absmax, the largest
+// |A u0| of all realizations or of each of the n in rlist (per_real).
+static int apply_lap(hipft_gpu *h, unsigned long long *absmax, const int *rlist, int n, int per_real) {
+  const double *ring;
+  TRY(current_dring(h, &ring));
+  ProfScope ps(h, HIPFT_K_OTHER);
+  k_ax<<<ax_grid(h, n), dim3(32, 8), 0, h->stream>>>(h->M, h->DC, h->buf[h->cur], h->buf[scratch(h, 0)], ring,
+                                                     h->bc_diff_n, h->bc_diff_s, absmax, ax_block_max(h), rlist,
+                                                     per_real);
+  LAUNCHED(h);
+  return HIPFT_OK;
+}
+static int ptl_cells(hipft_gpu *h, const unsigned long long *absmax, unsigned long long *ptl, const int *rlist, int n,
+                     int per_real) {
+  ProfScope ps(h, HIPFT_K_OTHER);
+  k_ptl<<<ax_grid(h, n), dim3(32, 8), 0, h->stream>>>(h->M, h->buf[h->cur], h->buf[scratch(h, 0)], absmax,
+                                                      ax_block_max(h), ptl, rlist, per_real);
   LAUNCHED(h);
   return HIPFT_OK;
 }
@@ -726,25 +753,33 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
   if ((rc = dalloc(h, &h->d_rcount, (size_t)nr))) return bail(rc);
   if ((rc = dalloc(h, &h->d_err, 1))) return bail(rc);
   if (cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream) != cudaSuccess) return bail(HIPFT_ECUDA);
+  // the kernels this grid can reach (setting an attribute loads the kernel)
+  const bool wide = h->plane >= (int64_t)1 << 29;
+  const bool vwide = wide || (int64_t)h->ldv * h->npm >= (int64_t)1 << 29;
   bool smem_ok = true;
-  for (int v = 0; v < 8; ++v)
-    smem_ok = smem_ok && cudaFuncSetAttribute(march_kernel(v & 1, v & 2, v & 4), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)kMSmem) == cudaSuccess;
-  for (int v = 0; v < 8; ++v)
-    smem_ok = smem_ok && cudaFuncSetAttribute(adv_kernel(v & 1, v & 2, v & 4), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)adv_smem(v & 1)) == cudaSuccess;
-  if (!smem_ok ||
-      cudaFuncSetAttribute(k_sts_poles<kPMidThreads, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)poles_smem(kPMidThreads)) != cudaSuccess ||
-      cudaFuncSetAttribute(k_sts_poles<kPMidThreads, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)poles_smem(kPMidThreads)) != cudaSuccess ||
-      cudaFuncSetAttribute(k_sts_poles<kPMaxThreads, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)poles_smem(kPMaxThreads)) != cudaSuccess)
+  auto reserve = [&](const void *kernel, size_t bytes) {
+    smem_ok = smem_ok && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+  };
+  if (prm->advance_flow && h->adv_space == 2)
+    for (int v = 0; v < 4; ++v) reserve((const void *)adv_kernel(v & 1, v & 2, vwide), adv_smem(v & 1));
+  if (prm->advance_diffusion && prm->diffusion_num_method >= 2 && !prm->diffusion_coef_grid && h->ntm >= kMMinRows) {
+    for (int v = 0; v < 3; ++v) reserve((const void *)march_kernel(v == 1, v == 2, wide), kMSmem);
+    if (poles_threads(npm - 2) > kPMidThreads) {
+      reserve((const void *)k_sts_poles<kPMaxThreads, 1>, poles_smem(kPMaxThreads));
+    } else {
+      reserve((const void *)k_sts_poles<kPMidThreads, 1>, poles_smem(kPMidThreads));
+      reserve((const void *)k_sts_poles<kPMidThreads, 3>, poles_smem(kPMidThreads));
+    }
+  }
+  if (!smem_ok)
     return bail(fail(h, HIPFT_ECUDA, "cannot reserve shared memory for the RKG2 passes"));
   if (cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess || h->num_sms < 1)
     h->num_sms = 148;
   if (cudaMemsetAsync(h->d_rcount, 0, sizeof(unsigned int) * nr, h->stream) != cudaSuccess) return bail(HIPFT_ECUDA);
-  if ((rc = dalloc(h, &h->d_bits, 4))) return bail(rc);
+  {  // two reduction slots and the maxima of k_ax's blocks
+    const dim3 g = ax_grid(h, nr);
+    if ((rc = dalloc(h, &h->d_bits, 4 + (size_t)g.x * g.y * g.z))) return bail(rc);
+  }
   if (cudaMallocHost((void **)&h->h_pin, sizeof(double) * std::max<size_t>(64, (size_t)nr * kNPart)) !=
       cudaSuccess)
     return bail(fail(h, HIPFT_ENOMEM, "cudaMallocHost failed"));
@@ -1212,7 +1247,8 @@ extern "C" int hipft_gpu_flow_dtmax(hipft_gpu *h, double *dtmax) {
   CK(h, cudaSetDevice(h->dev));
   unsigned long long init = 0x7fefffffffffffffULL;  // DBL_MAX bits
   CK(h, cudaMemcpyAsync(h->d_bits + 1, &init, 8, cudaMemcpyHostToDevice, h->stream));
-  dim3 blk(32, 8), grd((unsigned)((h->ntm - 2 + 31) / 32), (unsigned)((h->npm - 2 + 7) / 8), (unsigned)h->nr);
+  dim3 blk(32, 8), grd((unsigned)((h->ntm - 2 + 31) / 32),
+                       (unsigned)((h->npm - 2 + 8 * kAxCols - 1) / (8 * kAxCols)), (unsigned)h->nr);
   k_flow_dtmax<<<grd, blk, 0, h->stream>>>(h->M, h->FL, h->d_bits + 1);
   LAUNCHED(h);
   TRY(sync_read(h, h->d_bits + 1, 8));
@@ -1287,15 +1323,6 @@ static void load_sts(hipft_gpu *h, double dtl) {
   h->sts_gj = std::move(T.gj);
 }
 
-// A u0 of the current field into scratch buffer 0, unless the practical time
-// step limit left it there.
-static int current_lap(hipft_gpu *h) {
-  const double *ring;
-  TRY(current_dring(h, &ring));
-  return diffusion_stage<MODE_AX>(h, h->buf[h->cur], nullptr, nullptr, nullptr, h->buf[scratch(h, 0)], nullptr, ring,
-                                  StageCoef{}, nullptr);
-}
-
 // diffusion_step_sts_cd (src/hipft.f90:5163-5242).  have_lap: scratch buffer 0
 // holds A u0 (not with a grid-dependent D).
 static int sts_super_step(hipft_gpu *h, double dtl, bool have_lap) {
@@ -1306,7 +1333,7 @@ static int sts_super_step(hipft_gpu *h, double dtl, bool have_lap) {
   h->rkg2_cell_stages += cells * (h->sts_s - 1);
   h->cell_updates += cells * h->sts_s;
   if (!h->DC.grid) {
-    if (!have_lap) TRY(current_lap(h));
+    if (!have_lap) TRY(apply_lap(h, nullptr, nullptr, h->nr, 0));
     TRY(scale_dty0(h, h->buf[idty], h->buf[idty], dtl));
     const int R[4] = {scratch(h, 1), scratch(h, 2), scratch(h, 3), scratch(h, 4)};
     MarchArgs a = march_args(h, h->buf[u0], h->buf[idty]);
@@ -1328,15 +1355,14 @@ static int sts_super_step(hipft_gpu *h, double dtl, bool have_lap) {
   const int ia = scratch(h, 1), ib = scratch(h, 2);
   TRY(ring_diffusion(h, h->buf[u0], h->d_ring));
   TRY(diffusion_stage<MODE_STS1>(h, h->buf[u0], nullptr, nullptr, nullptr, h->buf[ia], h->buf[idty], h->d_ring,
-                                 StageCoef{dtl, h->sts_ubj[1], 0, 0, 0}, nullptr));
+                                 StageCoef{dtl, h->sts_ubj[1], 0, 0, 0}));
   int ykm1 = ia, ykm2 = u0;
   for (int64_t k = 2; k <= h->sts_s; ++k) {
     const int out = (ykm2 == u0) ? ib : ykm2;
     const double uj = h->sts_uj[k], vj = h->sts_vj[k];
     TRY(ring_diffusion(h, h->buf[ykm1], h->d_ring));
     TRY(diffusion_stage<MODE_STSK>(h, h->buf[ykm1], h->buf[ykm2], h->buf[u0], h->buf[idty], h->buf[out], nullptr,
-                                   h->d_ring, StageCoef{uj, vj, 1.0 - uj - vj, h->sts_ubj[k] * dtl, h->sts_gj[k]},
-                                   nullptr));
+                                   h->d_ring, StageCoef{uj, vj, 1.0 - uj - vj, h->sts_ubj[k] * dtl, h->sts_gj[k]}));
     ykm2 = ykm1;
     ykm1 = out;
   }
@@ -1361,7 +1387,7 @@ static int euler_steps(hipft_gpu *h, double dtl) {
     } else {
       TRY(ring_diffusion(h, h->buf[h->cur], h->d_ring));
       TRY(diffusion_stage<MODE_EULER>(h, h->buf[h->cur], nullptr, nullptr, nullptr, h->buf[o], nullptr, h->d_ring,
-                                      StageCoef{dte, 0, 0, 0, 0}, nullptr));
+                                      StageCoef{dte, 0, 0, 0, 0}));
       h->cur = o;
       h->dring_valid = false;
     }
@@ -1383,30 +1409,31 @@ static int check_wait_flag(hipft_gpu *h, const char *what) {
   return fail(h, HIPFT_ETIMEOUT, "%s", what);
 }
 
+// Both results come back in one read, unless the maximum over the processes of
+// a job is needed in between.
 static int ptl_dt(hipft_gpu *h, double *dtl) {
   double dtime_in = *dtl;
-  double *f = h->buf[h->cur], *af = h->buf[scratch(h, 0)];
-  CK(h, cudaMemsetAsync(h->d_bits, 0, 2 * sizeof(unsigned long long), h->stream));
-  const double *ring;
-  TRY(current_dring(h, &ring));
-  TRY(diffusion_stage<MODE_AX>(h, f, nullptr, nullptr, nullptr, af, nullptr, ring, StageCoef{}, h->d_bits));
-  TRY(sync_read(h, h->d_bits, 8));
-  double axabsmax;
-  std::memcpy(&axabsmax, h->h_pin, 8);
+  const unsigned long long init[2] = {0ULL, 0x7fefffffffffffffULL};
+  CK(h, cudaMemcpyAsync(h->d_bits, init, 16, cudaMemcpyHostToDevice, h->stream));
+  TRY(apply_lap(h, h->d_bits, nullptr, h->nr, 0));
+  double axabsmax, d = DBL_MAX, ptl;
   if (h->red_cb) {  // src/hipft.f90:5103: the PTL cells are those at the global maximum
+    TRY(sync_read(h, h->d_bits, 8));
+    std::memcpy(&axabsmax, h->h_pin, 8);
     TRY(allreduce(h, HIPFT_RED_MAX, &axabsmax));
+    if (!(axabsmax > 0.0)) {
+      *dtl = d;
+      return HIPFT_OK;
+    }
     CK(h, cudaMemcpyAsync(h->d_bits, &axabsmax, 8, cudaMemcpyHostToDevice, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
   }
-  double d = DBL_MAX;
+  TRY(ptl_cells(h, h->d_bits, h->d_bits + 1, nullptr, h->nr, 0));
+  TRY(sync_read(h, h->d_bits, 16));
+  std::memcpy(&axabsmax, h->h_pin, 8);
+  std::memcpy(&ptl, h->h_pin + 1, 8);
   if (axabsmax > 0.0) {
-    unsigned long long init = 0x7fefffffffffffffULL;
-    CK(h, cudaMemcpyAsync(h->d_bits + 1, &init, 8, cudaMemcpyHostToDevice, h->stream));
-    dim3 blk(32, 8);
-    k_ptl<<<stage_grid(h, 32, 8), blk, 0, h->stream>>>(h->M, f, af, h->d_bits, h->d_bits + 1);
-    LAUNCHED(h);
-    TRY(sync_read(h, h->d_bits + 1, 8));
-    std::memcpy(&d, h->h_pin, 8);
+    d = ptl;
     TRY(allreduce(h, HIPFT_RED_MIN, &d));  // src/hipft.f90:5141
     d = 0.95 * d;
     if (d < dtime_in) d = dtime_in;
@@ -1456,7 +1483,8 @@ static int ragged_dtmax(hipft_gpu *h) {
   std::vector<unsigned long long> bits(nr, 0x7fefffffffffffffULL);
   CK(h, cudaMemcpyAsync(h->d_rbits, bits.data(), sizeof(unsigned long long) * nr, cudaMemcpyHostToDevice,
                         h->stream));
-  dim3 blk(32, 8), grd((unsigned)((h->ntm - 2 + 31) / 32), (unsigned)((h->npm - 2 + 7) / 8), (unsigned)nr);
+  dim3 blk(32, 8), grd((unsigned)((h->ntm - 2 + 31) / 32),
+                       (unsigned)((h->npm - 2 + 8 * kAxCols - 1) / (8 * kAxCols)), (unsigned)nr);
   k_flow_dtmax<<<grd, blk, 0, h->stream>>>(h->M, h->FL, h->d_rbits, 1);
   LAUNCHED(h);
   CK(h, cudaMemcpyAsync(bits.data(), h->d_rbits, sizeof(unsigned long long) * nr, cudaMemcpyDeviceToHost,
@@ -1493,20 +1521,8 @@ static int ragged_ptl(hipft_gpu *h, std::vector<int> act, std::vector<double> &d
   for (int i = 0; i < nr; ++i) init[nr + i] = 0x7fefffffffffffffULL;
   CK(h, cudaMemcpyAsync(h->d_rbits, init.data(), sizeof(unsigned long long) * 2 * nr, cudaMemcpyHostToDevice,
                         h->stream));
-  double *f = h->buf[h->cur], *af = h->buf[scratch(h, 0)];
-  const double *ring;
-  TRY(current_dring(h, &ring));
-  dim3 blk(32, 8);
-  dim3 grd((unsigned)((h->ntm + 31) / 32), (unsigned)((h->npm - 2 + 7) / 8), (unsigned)na);
-  {
-    ProfScope ps(h, HIPFT_K_OTHER);
-    k_diffusion_stage<MODE_AX><<<grd, blk, 0, h->stream>>>(h->M, h->DC, f, nullptr, nullptr, nullptr, af, nullptr,
-                                                          ring, h->bc_diff_n, h->bc_diff_s, StageCoef{}, h->d_rbits,
-                                                          h->d_rlist_dif, 1);
-    LAUNCHED(h);
-    k_ptl<<<grd, blk, 0, h->stream>>>(h->M, f, af, h->d_rbits, h->d_rbits + nr, h->d_rlist_dif, 1);
-    LAUNCHED(h);
-  }
+  TRY(apply_lap(h, h->d_rbits, h->d_rlist_dif, na, 1));
+  TRY(ptl_cells(h, h->d_rbits, h->d_rbits + nr, h->d_rlist_dif, na, 1));
   std::vector<unsigned long long> bits(2 * (size_t)nr);
   CK(h, cudaMemcpyAsync(bits.data(), h->d_rbits, sizeof(unsigned long long) * 2 * nr, cudaMemcpyDeviceToHost,
                         h->stream));
@@ -1616,7 +1632,7 @@ static int ragged_diffusion_step(hipft_gpu *h, double dtl, hipft_diffusion_info 
   int64_t smax = 0;
   while (!act.empty()) {
     if (h->auto_sc) TRY(ragged_ptl(h, act, d));
-    else TRY(current_lap(h));
+    else TRY(apply_lap(h, nullptr, nullptr, h->nr, 0));
     std::vector<int> done;
     for (int i : act) {
       bool fin = false;
@@ -2078,20 +2094,19 @@ static int graph_capture(hipft_gpu *h) {
     int body_kernels = 3;  // ring sums, A u0 and the subcycle tick
     k_ring_diffusion<<<nr, 256, 0, s1>>>(M, h->DC, F, ring);
     peek();
-    const dim3 blk(32, 8);
-    const dim3 grd((unsigned)((h->ntm + 31) / 32), (unsigned)((h->npm - 2 + 7) / 8), (unsigned)nr);
+    const dim3 blk(32, 8), grd = ax_grid(h, nr);
+    unsigned long long *bblk = ax_block_max(h);
     const int pr = h->ragged ? 1 : 0;
     unsigned long long *bmax = g.bits, *bmin = g.bits + (h->ragged ? nr : 1);
     if (h->auto_sc) {
       k_g_ptl_reset<<<1, 256, 0, s1>>>(g);
       peek();
     }
-    k_diffusion_stage<MODE_AX><<<grd, blk, 0, s1>>>(M, h->DC, F, nullptr, nullptr, nullptr, Bd, nullptr, ring,
-                                                    h->bc_diff_n, h->bc_diff_s, StageCoef{},
-                                                    h->auto_sc ? bmax : nullptr, g.rl_ptl, pr);
+    k_ax<<<grd, blk, 0, s1>>>(M, h->DC, F, Bd, ring, h->bc_diff_n, h->bc_diff_s, h->auto_sc ? bmax : nullptr, bblk,
+                              g.rl_ptl, pr);
     peek();
     if (h->auto_sc) {  // PTL (src/hipft.f90:5042-5161) of the active realizations
-      k_ptl<<<grd, blk, 0, s1>>>(M, F, Bd, bmax, bmin, g.rl_ptl, pr);
+      k_ptl<<<grd, blk, 0, s1>>>(M, F, Bd, bmax, bblk, bmin, g.rl_ptl, pr);
       peek();
       ++body_kernels;
     }
@@ -3024,7 +3039,7 @@ static int adj_diff_fwd(hipft_gpu *h, double dtl, size_t &nt, std::vector<AdjSub
     Y[S.s] = h->buf[h->cur];
     CK(h, cudaMemcpyAsync(u0, h->buf[h->cur], h->fieldn * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
     // the passes of sts_super_step, with the tape's stages kept
-    if (!h->auto_sc) TRY(current_lap(h));
+    if (!h->auto_sc) TRY(apply_lap(h, nullptr, nullptr, h->nr, 0));
     TRY(scale_dty0(h, h->buf[scratch(h, 0)], dty0, dtl2));
     MarchArgs a = march_args(h, u0, dty0);
     const int64_t np = sts_passes(S.s), pad = kMS * np - S.s;
