@@ -192,8 +192,8 @@ struct hipft_gpu {
   double *d_da = nullptr, *d_daopt = nullptr;
   double *d_daw = nullptr;                   // mu^power weight planes
   int *d_dawidx = nullptr;                   // [nr+1] plane of each realization
+  double *d_dawkey = nullptr;                // [nr][2] power and limit of each plane
   size_t daw_cap = 0;
-  std::vector<double> h_daw;
   // sources: file term (one plane), two RFE frames, the blended source
   double *d_src_file = nullptr, *d_rfe[2] = {}, *d_src = nullptr, *d_rnd = nullptr, *d_rfe_aux = nullptr;
   bool src_set = false;
@@ -2381,7 +2381,6 @@ static int da_args(hipft_gpu *h, const double *data3_pt, const hipft_da_opts *o,
     TRY(dalloc(h, &h->d_daopt, 3 * (size_t)(nr + 1)));
     TRY(dalloc(h, &h->d_tidx, 2 * (size_t)(nr + 1)));
   }
-  CK(h, cudaMemcpyAsync(h->d_da, data3_pt, nd * sizeof(double), cudaMemcpyHostToDevice, h->stream));
   std::vector<double> opt(3 * (size_t)(nr + 1), 0.0);
   std::vector<int> tidx(2 * (size_t)(nr + 1), -1);
   for (int i = 1; i <= nr; ++i) {
@@ -2400,44 +2399,49 @@ static int da_args(hipft_gpu *h, const double *data3_pt, const hipft_da_opts *o,
   CK(h, cudaMemcpyAsync(h->d_tidx, tidx.data(), tidx.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
   if (o->custom_from_mu && (!o->mu_power || !o->mu_limit))
     return fail(h, HIPFT_EINVAL, "assimilate: custom_from_mu needs mu_power and mu_limit");
+  const size_t slice = (size_t)npm1 * ntm;
   if (o->custom_from_mu) {
-    // mu^power weights (src/hipft.f90:4246-4252) on the host, with the C
-    // library's pow: the weights then carry the reference's bits, which the
-    // 1e-12 field bar needs (a 2-ulp change of every weight moves the
-    // assimilated 1024x2048 fields by 1.8e-12 after 2.5 hours).  One plane
-    // per distinct (power, limit).
-    const size_t slice = (size_t)npm1 * ntm;
-    std::vector<std::pair<double, double>> keys;
+    // mu^power weights (src/hipft.f90:4246-4252), one plane per distinct
+    // (power, limit), evaluated on the device while the data slice is still
+    // on its way; the map's own weight slice is not read and not copied.
+    std::vector<double> keys;  // power, limit of each plane
     std::vector<int> widx((size_t)nr + 1, 0);
     for (int i = 1; i <= nr; ++i) {
-      const std::pair<double, double> key(o->mu_power[i - 1], o->mu_limit[i - 1]);
       size_t u = 0;
-      while (u < keys.size() && keys[u] != key) ++u;
-      if (u == keys.size()) keys.push_back(key);
+      while (2 * u < keys.size() && !(keys[2 * u] == o->mu_power[i - 1] && keys[2 * u + 1] == o->mu_limit[i - 1])) ++u;
+      if (2 * u == keys.size()) {
+        keys.push_back(o->mu_power[i - 1]);
+        keys.push_back(o->mu_limit[i - 1]);
+      }
       widx[i] = (int)u;
     }
-    if (keys.size() * slice > h->daw_cap) {
+    const size_t np = keys.size() / 2;
+    if (np * slice > h->daw_cap) {
       if (h->d_daw) {
         CK(h, cudaStreamSynchronize(h->stream));
         cudaFree(h->d_daw);
         h->allocs.erase(std::remove(h->allocs.begin(), h->allocs.end(), (void *)h->d_daw), h->allocs.end());
         h->d_daw = nullptr;
+        h->daw_cap = 0;
       }
-      TRY(dalloc(h, &h->d_daw, keys.size() * slice));
+      TRY(dalloc(h, &h->d_daw, np * slice));
+      h->daw_cap = np * slice;
+    }
+    if (!h->d_dawidx) {
       TRY(dalloc(h, &h->d_dawidx, (size_t)nr + 1));
-      h->daw_cap = keys.size() * slice;
+      TRY(dalloc(h, &h->d_dawkey, 2 * (size_t)nr));
     }
-    h->h_daw.resize(keys.size() * slice);
-    const double *mu = data3_pt + 2 * slice;
-    for (size_t u = 0; u < keys.size(); ++u) {
-      double *w = h->h_daw.data() + u * slice;
-      const double pw = keys[u].first, lim = keys[u].second;
-      for (size_t q = 0; q < slice; ++q) w[q] = (mu[q] > lim) ? std::pow(mu[q], pw) : 0.0;
-    }
-    CK(h, cudaMemcpyAsync(h->d_daw, h->h_daw.data(), keys.size() * slice * sizeof(double), cudaMemcpyHostToDevice,
-                          h->stream));
+    TRY(upload(h, h->d_dawkey, keys));
     CK(h, cudaMemcpyAsync(h->d_dawidx, widx.data(), widx.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
-    CK(h, cudaStreamSynchronize(h->stream));  // h_daw and widx are reused by the next call
+    CK(h, cudaMemcpyAsync(h->d_da + 2 * slice, data3_pt + 2 * slice, slice * sizeof(double), cudaMemcpyHostToDevice,
+                          h->stream));
+    k_da_mu_weights<<<dim3((unsigned)((slice + 255) / 256), (unsigned)np), 256, 0, h->stream>>>(
+        (int64_t)slice, h->d_da + 2 * slice, h->d_dawkey, h->d_daw);
+    LAUNCHED(h);
+    CK(h, cudaMemcpyAsync(h->d_da, data3_pt, slice * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    CK(h, cudaStreamSynchronize(h->stream));  // the caller's map and the vectors above are free again
+  } else {
+    CK(h, cudaMemcpyAsync(h->d_da, data3_pt, 2 * slice * sizeof(double), cudaMemcpyHostToDevice, h->stream));
   }
   a = DAArgs{};
   a.data = h->d_da;
