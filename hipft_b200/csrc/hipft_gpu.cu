@@ -496,9 +496,13 @@ static int64_t march_blocks(const hipft_gpu *h, int nreal) {
 
 // k_sts_march for these arguments; byte offsets in 32 bits while a plane has them.
 typedef void (*MarchKernel)(Mesh, MarchArgs, PairTables);
+template <typename Off>
+static MarchKernel march_kernel(bool table, bool keep) {
+  if (keep) return table ? k_sts_march<true, true, Off> : k_sts_march<false, true, Off>;
+  return table ? k_sts_march<true, false, Off> : k_sts_march<false, false, Off>;
+}
 static MarchKernel march_kernel(bool table, bool keep, bool wide) {
-  if (wide) return table ? k_sts_march<true, false, uint64_t> : keep ? k_sts_march<false, true, uint64_t> : k_sts_march<false, false, uint64_t>;
-  return table ? k_sts_march<true, false, uint32_t> : keep ? k_sts_march<false, true, uint32_t> : k_sts_march<false, false, uint32_t>;
+  return wide ? march_kernel<uint64_t>(table, keep) : march_kernel<uint32_t>(table, keep);
 }
 
 // One pass on stream s.  after_pass: the launch before it on the stream is
@@ -547,8 +551,9 @@ static cudaError_t launch_pass(const hipft_gpu *h, cudaStream_t s, MarchArgs a, 
   cfg.gridDim = dim3((unsigned)blocks);
   cfg.blockDim = dim3(32 * kMWarps);
   cfg.dynamicSmemBytes = kMSmem;
-  return cudaLaunchKernelEx(&cfg, march_kernel(a.rc != nullptr, a.o[0] || a.o[1], h->plane >= (int64_t)1 << 29),
-                            h->M, a, h->ptab);
+  const bool table = a.rc || a.cols > kMGroup;
+  return cudaLaunchKernelEx(&cfg, march_kernel(table, a.o[0] || a.o[1], h->plane >= (int64_t)1 << 29), h->M, a,
+                            h->ptab);
 }
 
 static int sts_pass(hipft_gpu *h, const MarchArgs &a, bool after_pass) {
@@ -763,7 +768,7 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
   if (prm->advance_flow && h->adv_space == 2)
     for (int v = 0; v < 4; ++v) reserve((const void *)adv_kernel(v & 1, v & 2, vwide), adv_smem(v & 1));
   if (prm->advance_diffusion && prm->diffusion_num_method >= 2 && !prm->diffusion_coef_grid && h->ntm >= kMMinRows) {
-    for (int v = 0; v < 3; ++v) reserve((const void *)march_kernel(v == 1, v == 2, wide), kMSmem);
+    for (int v = 0; v < 4; ++v) reserve((const void *)march_kernel(v & 1, v & 2, wide), kMSmem);
     if (poles_threads(npm - 2) > kPMidThreads) {
       reserve((const void *)k_sts_poles<kPMaxThreads, 1>, poles_smem(kPMaxThreads));
     } else {

@@ -285,8 +285,14 @@ __device__ __forceinline__ double2 pair_stage(double2 xl, double2 xc, double2 xr
 // 64/56 of that for the strip's halo; HBM sees 4 reads and 2 writes of 8 bytes
 // per cell and four stages.
 //
-// TABLE: coefficients per realization; KEEP: Y_k and Y_{k+1} are kept too;
-// Off: a byte offset within a realization's plane.
+// TABLE: the stages' coefficients are read from shared memory.  Those of all
+// realizations come as arguments, but from a chunk of more than one turn on
+// they go through shared memory too: as operands from the constant bank they
+// made 64 x 1024x2048 4 % and 2048x4096 6 % slower (363 and 378 against 378 and
+// 399 Gcell-stages/s); a chunk of one turn does not repay the block's barrier
+// (180x360: 1 % of a step).
+// KEEP: Y_k and Y_{k+1} are kept too; Off: a byte offset within a
+// realization's plane.
 template <bool TABLE, bool KEEP, typename Off>
 __global__ void __launch_bounds__(32 * kMWarps, kMBlocks) k_sts_march(Mesh m, MarchArgs a, PairTables pt) {
   extern __shared__ __align__(16) double msm[];
@@ -309,7 +315,9 @@ __global__ void __launch_bounds__(32 * kMWarps, kMBlocks) k_sts_march(Mesh m, Ma
   const int i = a.rlist ? a.rlist[rest / nblk] : rest / nblk;  // 0-based
   double *coef = msm + kMWarps * (kMRing + kMTab);
   if (TABLE) {
-    if (threadIdx.x < kMCoef) coef[threadIdx.x] = reinterpret_cast<const double *>(rc + (int64_t)i * kMS)[threadIdx.x];
+    if (threadIdx.x < kMCoef)
+      coef[threadIdx.x] = a.rc ? reinterpret_cast<const double *>(rc + (int64_t)i * kMS)[threadIdx.x]
+                               : reinterpret_cast<const double *>(a.c)[threadIdx.x];
     __syncthreads();
   }
   if (c0 > npm - 1) {
