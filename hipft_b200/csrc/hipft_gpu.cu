@@ -122,7 +122,6 @@ struct hipft_gpu {
   int64_t sts_s = 0, n_euler = 0, subcycles_state = 0;
   std::vector<double> sts_uj, sts_vj, sts_ubj, sts_gj, sts_b;
   // scratch
-  double *d_ring = nullptr;            // ring sums for kernels that take them from a launch of their own
   double *d_ringbuf[2] = {};           // diffusion ring of a stage's input / output (fused path)
   int ring_cur = 0;
   bool dring_valid = false;            // d_ringbuf[ring_cur] holds the ring of the current field
@@ -583,13 +582,23 @@ static int scale_dty0(hipft_gpu *h, const double *af, double *dty0, double dtl, 
   return HIPFT_OK;
 }
 
+// chained: the launch before it on the stream is a diffusion stage too.
 template <int MODE>
 static int diffusion_stage(hipft_gpu *h, const double *x, const double *ykm2, const double *u0, const double *dty0,
-                           double *out, double *out2, const double *ring, StageCoef sc) {
-  dim3 blk(32, 8);
+                           double *out, double *out2, StageCoef sc, bool chained) {
   ProfScope ps(h, MODE == MODE_STSK ? HIPFT_K_STS : HIPFT_K_OTHER);
-  k_diffusion_stage<MODE><<<stage_grid(h, 32, 8), blk, 0, h->stream>>>(h->M, h->DC, x, ykm2, u0, dty0, out, out2,
-                                                                       ring, h->bc_diff_n, h->bc_diff_s, sc);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = (ws_pdl() && chained) ? 1 : 0;
+  cfg.stream = h->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cfg.gridDim = stage_grid(h, 32, 8 * kDCols);
+  cfg.gridDim.y += 2;  // the pole rows' blocks
+  cfg.blockDim = dim3(32, 8);
+  CK(h, cudaLaunchKernelEx(&cfg, k_diffusion_stage<MODE>, h->M, h->DC, x, ykm2, u0, dty0, out, out2, h->bc_diff_n,
+                           h->bc_diff_s, sc));
   LAUNCHED(h);
   return HIPFT_OK;
 }
@@ -639,12 +648,17 @@ static cudaError_t launch_adv_stage(const hipft_gpu *h, cudaStream_t s, unsigned
                                     double *out, AdvCombine cb, const int *rlist, const double *rdt, bool pdl,
                                     bool chained) {
   if (h->adv_space != 2) {
-    k_ring_advection<<<h->nr, 256, 0, s>>>(h->M, h->FL, x, h->d_ring);
-    const dim3 blk(33, 9);  // (TJ+1) x (TK+1) threads for a 32 x 8 tile
-    const dim3 grd((unsigned)((h->ntm + 31) / 32), (unsigned)((h->npm - 2 + 7) / 8), nz);
-    k_adv_upwind<32, 8><<<grd, blk, 0, s>>>(h->M, h->FL, x, f0, out, h->d_ring, h->bc_flow_n, h->bc_flow_s, cb, rlist,
-                                            rdt);
-    return cudaPeekAtLastError();
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = (pdl && chained) ? 1 : 0;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3((unsigned)((h->ntm + 31) / 32), 2 + (unsigned)((h->npm - 2 + 7) / 8), nz);
+    cfg.blockDim = dim3(33, 9);  // (TJ+1) x (TK+1) threads for a 32 x 8 tile
+    return cudaLaunchKernelEx(&cfg, k_adv_upwind<32, 8>, h->M, h->FL, x, f0, out, h->bc_flow_n, h->bc_flow_s, cb,
+                              rlist, rdt);
   }
   AdvArgs a{x, f0, out, cb, rlist, rdt, 0, 0, h->bc_flow_n, h->bc_flow_s};
   const int n2 = h->npm - 2;
@@ -671,7 +685,7 @@ static int advection_stage(hipft_gpu *h, const double *x, const double *f0, doub
   if (!n) n = h->nr;
   const cudaError_t e = launch_adv_stage(h, h->stream, (unsigned)n, x, f0, out, cb, rlist, rdt, ws_pdl(), chained);
   if (e != cudaSuccess) return fail(h, HIPFT_ECUDA, "advection stage launch: %s", cudaGetErrorString(e));
-  h->launches += h->adv_space == 2 ? 1 : 2;
+  h->launches += 1;
   h->cell_updates += (int64_t)h->ntm * (h->npm - 2) * n;
   return HIPFT_OK;
 }
@@ -750,7 +764,6 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
     if ((rc = dalloc(h, &h->buf[b], h->fieldn))) return bail(rc);
     if (cudaMemsetAsync(h->buf[b], 0, h->fieldn * sizeof(double), h->stream) != cudaSuccess) return bail(HIPFT_ECUDA);
   }
-  if ((rc = dalloc(h, &h->d_ring, 2 * (size_t)nr))) return bail(rc);
   h->nkb = (npm - 2 + kKPT3 - 1) / kKPT3;  // partial slots for the smaller phi block
   if ((rc = dalloc(h, &h->d_ringbuf[0], 2 * (size_t)nr))) return bail(rc);
   if ((rc = dalloc(h, &h->d_ringbuf[1], 2 * (size_t)nr))) return bail(rc);
@@ -1358,16 +1371,14 @@ static int sts_super_step(hipft_gpu *h, double dtl, bool have_lap) {
     return seam(h, h->buf[h->cur]);
   }
   const int ia = scratch(h, 1), ib = scratch(h, 2);
-  TRY(ring_diffusion(h, h->buf[u0], h->d_ring));
-  TRY(diffusion_stage<MODE_STS1>(h, h->buf[u0], nullptr, nullptr, nullptr, h->buf[ia], h->buf[idty], h->d_ring,
-                                 StageCoef{dtl, h->sts_ubj[1], 0, 0, 0}));
+  TRY(diffusion_stage<MODE_STS1>(h, h->buf[u0], nullptr, nullptr, nullptr, h->buf[ia], h->buf[idty],
+                                 StageCoef{dtl, h->sts_ubj[1], 0, 0, 0}, false));
   int ykm1 = ia, ykm2 = u0;
   for (int64_t k = 2; k <= h->sts_s; ++k) {
     const int out = (ykm2 == u0) ? ib : ykm2;
     const double uj = h->sts_uj[k], vj = h->sts_vj[k];
-    TRY(ring_diffusion(h, h->buf[ykm1], h->d_ring));
     TRY(diffusion_stage<MODE_STSK>(h, h->buf[ykm1], h->buf[ykm2], h->buf[u0], h->buf[idty], h->buf[out], nullptr,
-                                   h->d_ring, StageCoef{uj, vj, 1.0 - uj - vj, h->sts_ubj[k] * dtl, h->sts_gj[k]}));
+                                   StageCoef{uj, vj, 1.0 - uj - vj, h->sts_ubj[k] * dtl, h->sts_gj[k]}, true));
     ykm2 = ykm1;
     ykm1 = out;
   }
@@ -1390,9 +1401,8 @@ static int euler_steps(hipft_gpu *h, double dtl) {
       h->cur = o;
       h->dring_valid = true;
     } else {
-      TRY(ring_diffusion(h, h->buf[h->cur], h->d_ring));
-      TRY(diffusion_stage<MODE_EULER>(h, h->buf[h->cur], nullptr, nullptr, nullptr, h->buf[o], nullptr, h->d_ring,
-                                      StageCoef{dte, 0, 0, 0, 0}));
+      TRY(diffusion_stage<MODE_EULER>(h, h->buf[h->cur], nullptr, nullptr, nullptr, h->buf[o], nullptr,
+                                      StageCoef{dte, 0, 0, 0, 0}, c > 0));
       h->cur = o;
       h->dring_valid = false;
     }
@@ -2061,7 +2071,7 @@ static int graph_capture(hipft_gpu *h) {
       adv_stage(s1, B, F, A, AdvCombine{1, c_two_third, c_third, c_sixth});
       adv_stage(s1, A, nullptr, F, AdvCombine{0, 0.0, 0.0, 0.5});
     }
-    k_g_adv_tick<<<1, 256, 0, s1>>>(g, (h->adv_time == 1) ? 4 : 2 * g.nadv + 1, hc);
+    k_g_adv_tick<<<1, 256, 0, s1>>>(g, (h->adv_time == 1) ? 3 : g.nadv + 1, hc);
     peek();
     end_body(s1);
   };
