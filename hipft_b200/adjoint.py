@@ -103,8 +103,7 @@ def misfit_weights(mesh: dict) -> np.ndarray:
     da_p[1] = 0.5 * dph[1]
     da_p[npm - 1] = 0.5 * dph[npm - 1]
     w = np.zeros((npm, ntm))
-    for k in range(1, npm):
-        w[k - 1, :] = da_p[k] * da_t[1:]
+    w[:npm - 1] = da_p[1:npm, None] * da_t[None, 1:]
     return w
 
 
@@ -127,22 +126,10 @@ def flow_profiles(mesh: dict, coef: dict):
     vp = torch.cat([torch.zeros_like(vp[:, :1]), vp[:, 1:]], dim=1)
     avt = vt.abs()
 
-    def vmax(lo, hi):  # max |vt(lo..hi)| per realization
-        return avt[:, lo:hi + 1].max(dim=1).values
-
-    at_cols = [torch.zeros_like(vt[:, 0])]
-    for j in range(1, ntm + 1):
-        if j == 1:
-            at_cols.append(vmax(1, 4))
-        elif j == 2:
-            at_cols.append(vmax(1, 5))
-        elif j == nt - 2:
-            at_cols.append(vmax(j - 2, j + 2))
-        elif j == nt - 1:
-            at_cols.append(vmax(j - 2, j + 1))
-        else:
-            at_cols.append(vmax(j - 2, j + 3))
-    at = torch.stack(at_cols, dim=1)
+    # row j: the largest |vt(j-2 .. j+3)| within 1..nt (a window cut short repeats its last entry)
+    j = torch.arange(1, ntm + 1, device=vt.device)[:, None]
+    win = torch.minimum((j - 2).clamp(min=1) + torch.arange(6, device=vt.device)[None, :], (j + 3).clamp(max=nt))
+    at = torch.cat([torch.zeros_like(vt[:, :1]), avt[:, win].max(dim=2).values], dim=1)
     ap = vp.abs()  # the six phi neighbours of a 1-D profile are equal
     return vt, at, vp, ap
 
@@ -236,9 +223,9 @@ class MisfitAdjoint:
     def loss_and_cotangent(self, fN: np.ndarray, target: np.ndarray):
         """Misfit and its folded cotangent (nr, npm, ntm)."""
         r = fN - target
-        loss = 0.5 * float(np.sum(self.w[None] * r * r))
         g = self.w[None] * r
-        return loss, fold_cotangent(g)
+        loss = 0.5 * float(np.sum(g * r))
+        return loss, _fold(g)
 
     # -- taping: a recorded step is a forward step whose tape stays on the
     # library's stack until its reverse; a segment is recorded while the
@@ -391,7 +378,7 @@ class MisfitAdjoint:
         nrec, _ = self._recorded()
         if nrec:
             raise RuntimeError(f"adjoint: {nrec} recorded steps left after the reverse pass")
-        grads = {"f0": fbar[:, :, :self.ntm].cpu().numpy().copy()}
+        grads = {"f0": fbar[:, :, :self.ntm].cpu().numpy()}
         grads["f0"][:, 0] = 0.0
         grads["f0"][:, self.npm - 1] = 0.0
         grads["D"] = dacc.cpu().numpy() / self.D
@@ -443,7 +430,11 @@ def fold_cotangent(g):
     """Folds a cotangent (nr, npm, ntm) of a periodic field: the seam columns
     1 and npm are copies of columns npm-1 and 2, so their entries move there
     and the seam entries become zero (numpy or torch)."""
-    gb = g.clone() if hasattr(g, "clone") else np.array(g, dtype=np.float64, copy=True)
+    return _fold(g.clone() if hasattr(g, "clone") else np.array(g, dtype=np.float64, copy=True))
+
+
+def _fold(gb):
+    """fold_cotangent in place."""
     npm = gb.shape[1]
     gb[:, npm - 2] += gb[:, 0]
     gb[:, 1] += gb[:, npm - 1]

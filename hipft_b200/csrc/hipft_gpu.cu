@@ -96,6 +96,8 @@ struct hipft_gpu {
   std::vector<double> t, p, th, ph, dt, dth, dp, dph, dt_i, dth_i, dp_i, dph_i, st, sth, ct, cth, st_i, sth_i;
   std::vector<void *> allocs;
   size_t dev_bytes = 0;
+  unsigned char *slab = nullptr;  // unused rest of the chunk dsmall carves from
+  size_t slab_left = 0;
   Mesh M{};
   DiffCoef DC{};
   Weno W{};
@@ -294,6 +296,39 @@ static int upload(hipft_gpu *h, T *d, const std::vector<T> &v) {
     int rc_ = (x);             \
     if (rc_ != HIPFT_OK) return rc_; \
   } while (0)
+
+// A small array that lives as long as the handle, from a chunk shared with
+// others: an allocation and its release take 60 us or more each, and a handle
+// has some thirty of them.
+template <typename T>
+static int dsmall(hipft_gpu *h, T **p, size_t n) {
+  constexpr size_t kChunk = (size_t)1 << 18, kAlign = 256;
+  const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + kAlign - 1) / kAlign * kAlign;
+  if (bytes > kChunk / 4) return dalloc(h, p, n);
+  if (bytes > h->slab_left) {
+    TRY(dalloc(h, &h->slab, kChunk));
+    h->slab_left = kChunk;
+  }
+  *p = reinterpret_cast<T *>(h->slab);
+  h->slab += bytes;
+  h->slab_left -= bytes;
+  return HIPFT_OK;
+}
+
+// Fields that live as long as the handle, several per allocation while they
+// are small (at most 256 MB each, as the tape's chunks).
+static int dfields(hipft_gpu *h, double **f, int n) {
+  const size_t per = std::max<size_t>(1, ((size_t)256 << 20) / (h->fieldn * sizeof(double)));
+  for (int b = 0; b < n;) {
+    const int c = (int)std::min<size_t>(per, (size_t)(n - b));
+    double *q = nullptr;
+    TRY(dalloc(h, &q, h->fieldn * c));
+    for (int e = 0; e < c; ++e) f[b + e] = q + e * h->fieldn;
+    CK(h, cudaMemsetAsync(q, 0, h->fieldn * c * sizeof(double), h->stream));
+    b += c;
+  }
+  return HIPFT_OK;
+}
 
 // ------------------------------------------------------------- set_mesh
 // src/hipft.f90:6495-6653, restated on 1-based host vectors.
@@ -744,7 +779,7 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
   size_t tot = 0;
   for (auto *a : arrs) tot += a->size();
   double *dm = nullptr;
-  if ((rc = dalloc(h, &dm, tot))) return bail(rc);
+  if ((rc = dsmall(h, &dm, tot))) return bail(rc);
   std::vector<double> packed;
   packed.reserve(tot);
   std::vector<size_t> offs;
@@ -759,17 +794,14 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
   h->M.st_i = dm + offs[4]; h->M.sth = dm + offs[5]; h->M.dp = dm + offs[6]; h->M.dth = dm + offs[7];
   h->M.dph = dm + offs[8];
 
-  // fields (the four-stage path adds two more when it is first used)
-  for (int b = 0; b < h->nbuf; ++b) {
-    if ((rc = dalloc(h, &h->buf[b], h->fieldn))) return bail(rc);
-    if (cudaMemsetAsync(h->buf[b], 0, h->fieldn * sizeof(double), h->stream) != cudaSuccess) return bail(HIPFT_ECUDA);
-  }
+  // the field, A u0 and the four of the RKG2 passes
+  if ((rc = dfields(h, h->buf, h->nbuf))) return bail(rc);
   h->nkb = (npm - 2 + kKPT3 - 1) / kKPT3;  // partial slots for the smaller phi block
-  if ((rc = dalloc(h, &h->d_ringbuf[0], 2 * (size_t)nr))) return bail(rc);
-  if ((rc = dalloc(h, &h->d_ringbuf[1], 2 * (size_t)nr))) return bail(rc);
-  if ((rc = dalloc(h, &h->d_rpart, 2 * (size_t)nr * h->nkb))) return bail(rc);
-  if ((rc = dalloc(h, &h->d_rcount, (size_t)nr))) return bail(rc);
-  if ((rc = dalloc(h, &h->d_err, 1))) return bail(rc);
+  if ((rc = dsmall(h, &h->d_ringbuf[0], 2 * (size_t)nr))) return bail(rc);
+  if ((rc = dsmall(h, &h->d_ringbuf[1], 2 * (size_t)nr))) return bail(rc);
+  if ((rc = dsmall(h, &h->d_rpart, 2 * (size_t)nr * h->nkb))) return bail(rc);
+  if ((rc = dsmall(h, &h->d_rcount, (size_t)nr))) return bail(rc);
+  if ((rc = dsmall(h, &h->d_err, 1))) return bail(rc);
   if (cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream) != cudaSuccess) return bail(HIPFT_ECUDA);
   // the kernels this grid can reach (setting an attribute loads the kernel)
   const bool wide = h->plane >= (int64_t)1 << 29;
@@ -796,7 +828,7 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
   if (cudaMemsetAsync(h->d_rcount, 0, sizeof(unsigned int) * nr, h->stream) != cudaSuccess) return bail(HIPFT_ECUDA);
   {  // two reduction slots and the maxima of k_ax's blocks
     const dim3 g = ax_grid(h, nr);
-    if ((rc = dalloc(h, &h->d_bits, 4 + (size_t)g.x * g.y * g.z))) return bail(rc);
+    if ((rc = dsmall(h, &h->d_bits, 4 + (size_t)g.x * g.y * g.z))) return bail(rc);
   }
   if (cudaMallocHost((void **)&h->h_pin, sizeof(double) * std::max<size_t>(64, (size_t)nr * kNPart)) !=
       cudaSuccess)
@@ -808,7 +840,7 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
     for (int i = 1; i <= nr; ++i)
       dfac[i] = prm->diffusion_coef_grid ? h->Dc[i - 1] : prm->diffusion_coef_factor * h->Dc[i - 1];
   double *d_dfac = nullptr;
-  if ((rc = dalloc(h, &d_dfac, nr + 1))) return bail(rc);
+  if ((rc = dsmall(h, &d_dfac, nr + 1))) return bail(rc);
   if ((rc = upload(h, d_dfac, dfac))) return bail(rc);
   h->DC.dfac = d_dfac;
   h->DC.factor = prm->diffusion_coef_factor;
@@ -824,7 +856,7 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
       return bail(rc);
     double *tab = nullptr;
     const size_t nrow = (size_t)nr * pt.LR * 3, ncol = (size_t)nr * pt.LC * 2;
-    if ((rc = dalloc(h, &tab, nrow + ncol))) return bail(rc);
+    if ((rc = dsmall(h, &tab, nrow + ncol))) return bail(rc);
     pt.row = tab;
     pt.col = tab + nrow + 2 * kColPad;
     k_pair_tables<<<2 * h->num_sms, 256, 0, h->stream>>>(h->M, d_dfac, pt.LR, pt.LC, tab, tab + nrow);
@@ -875,17 +907,17 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
       row[11] = (kf <= npm - 1) ? h->dp_i[kf] : 0.0;
     }
     double *dw = nullptr;
-    if ((rc = dalloc(h, &dw, pk.size()))) return bail(rc);
+    if ((rc = dsmall(h, &dw, pk.size()))) return bail(rc);
     if ((rc = upload(h, dw, pk))) return bail(rc);
     h->W.cpt = dw + wo[0]; h->W.mct = dw + wo[1]; h->W.mt = dw + wo[2]; h->W.cptt = dw + wo[3];
     h->W.pt = dw + wo[4]; h->W.mctt = dw + wo[5]; h->W.epst = dw + wo[6];
     h->W.cpp = dw + wo[7]; h->W.mcp = dw + wo[8]; h->W.mp = dw + wo[9]; h->W.cptp = dw + wo[10];
     h->W.pp = dw + wo[11]; h->W.mctp = dw + wo[12]; h->W.epsp = dw + wo[13];
     h->W.ptab = dw + tab0;
-    if ((rc = dalloc(h, &h->d_vt1, (size_t)nr * (nt + 1)))) return bail(rc);
-    if ((rc = dalloc(h, &h->d_vp1, (size_t)nr * (ntm + 1)))) return bail(rc);
-    if ((rc = dalloc(h, &h->d_at1, (size_t)nr * (ntm + 1)))) return bail(rc);
-    if ((rc = dalloc(h, &h->d_ap1, (size_t)nr * (ntm + 1)))) return bail(rc);
+    if ((rc = dsmall(h, &h->d_vt1, (size_t)nr * (nt + 1)))) return bail(rc);
+    if ((rc = dsmall(h, &h->d_vp1, (size_t)nr * (ntm + 1)))) return bail(rc);
+    if ((rc = dsmall(h, &h->d_at1, (size_t)nr * (ntm + 1)))) return bail(rc);
+    if ((rc = dsmall(h, &h->d_ap1, (size_t)nr * (ntm + 1)))) return bail(rc);
     h->FL.vt1 = h->d_vt1; h->FL.vp1 = h->d_vp1; h->FL.at1 = h->d_at1; h->FL.ap1 = h->d_ap1;
     h->FL.ldv = h->ldv;
     h->FL.vplane = (int64_t)h->ldv * npm;
@@ -928,17 +960,17 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
     }
     h->da_t.assign(da_t, da_t + ntm + 1);
     h->da_p.assign(da_p, da_p + npm);
-    if ((rc = dalloc(h, &h->d_anw, w.size()))) return bail(rc);
+    if ((rc = dsmall(h, &h->d_anw, w.size()))) return bail(rc);
     if ((rc = upload(h, h->d_anw, w))) return bail(rc);
     std::vector<unsigned char> masks(2 * (size_t)(ntm + 1), 0);
     for (int j = 1; j <= ntm; ++j) {
       masks[j] = (h->t[j] <= prm->pole_flux_lat_limit * c_d2r) ? 1 : 0;
       masks[ntm + 1 + j] = (h->t[j] >= c_pi - prm->pole_flux_lat_limit * c_d2r) ? 1 : 0;
     }
-    if ((rc = dalloc(h, &h->d_masks, masks.size()))) return bail(rc);
+    if ((rc = dsmall(h, &h->d_masks, masks.size()))) return bail(rc);
     if (cudaMemcpyAsync(h->d_masks, masks.data(), masks.size(), cudaMemcpyHostToDevice, h->stream) != cudaSuccess)
       return bail(HIPFT_ECUDA);
-    if ((rc = dalloc(h, &h->d_vscale, nr + 1))) return bail(rc);
+    if ((rc = dsmall(h, &h->d_vscale, nr + 1))) return bail(rc);
   }
   if (cudaStreamSynchronize(h->stream) != cudaSuccess) return bail(fail(h, HIPFT_ECUDA, "create: sync failed"));
   *out = h;
@@ -1193,7 +1225,7 @@ extern "C" int hipft_gpu_update_flow(hipft_gpu *h, int *updated) {
       std::vector<double> att(nr + 1, 0.0);
       for (int i = 1; i <= nr; ++i)
         att[i] = (h->f_att[i - 1] > 0.0) ? 1.0 / h->f_att[i - 1] : DBL_MAX;
-      TRY(dalloc(h, &h->d_atten, nr + 1));
+      TRY(dsmall(h, &h->d_atten, nr + 1));
       TRY(upload(h, h->d_atten, att));
     }
     if (h->fdef.flow_attenuate && !h->field_set) return fail(h, HIPFT_ESTATE, "update_flow: attenuation needs the field");
@@ -1747,11 +1779,11 @@ extern "C" int hipft_gpu_set_ragged(hipft_gpu *h, int on) {
     return fail(h, HIPFT_EINVAL, "set_ragged: needs SSPRK(3,3) or SSPRK(4,3) advection");
   const int nr = h->nr;
   if (!h->d_rbits) {
-    TRY(dalloc(h, &h->d_rbits, 2 * (size_t)nr));
-    TRY(dalloc(h, &h->d_rlist_dif, (size_t)nr));
-    TRY(dalloc(h, &h->d_rlist_adv, (size_t)nr));
-    TRY(dalloc(h, &h->d_rlen, (size_t)nr));
-    TRY(dalloc(h, &h->d_rdt, (size_t)nr));
+    TRY(dsmall(h, &h->d_rbits, 2 * (size_t)nr));
+    TRY(dsmall(h, &h->d_rlist_dif, (size_t)nr));
+    TRY(dsmall(h, &h->d_rlist_adv, (size_t)nr));
+    TRY(dsmall(h, &h->d_rlen, (size_t)nr));
+    TRY(dsmall(h, &h->d_rdt, (size_t)nr));
   }
   if (h->P.advance_diffusion) TRY(ragged_gershgorin(h));
   h->r_dtmax_valid = false;
@@ -1767,11 +1799,11 @@ extern "C" int hipft_gpu_flow_dtmax_each(hipft_gpu *h, double *dtmax) {
   if (!h->P.advance_flow) return fail(h, HIPFT_ESTATE, "flow_dtmax_each: advance_flow is off");
   CK(h, cudaSetDevice(h->dev));
   if (!h->d_rbits) {
-    TRY(dalloc(h, &h->d_rbits, 2 * (size_t)h->nr));
-    TRY(dalloc(h, &h->d_rlist_dif, (size_t)h->nr));
-    TRY(dalloc(h, &h->d_rlist_adv, (size_t)h->nr));
-    TRY(dalloc(h, &h->d_rlen, (size_t)h->nr));
-    TRY(dalloc(h, &h->d_rdt, (size_t)h->nr));
+    TRY(dsmall(h, &h->d_rbits, 2 * (size_t)h->nr));
+    TRY(dsmall(h, &h->d_rlist_dif, (size_t)h->nr));
+    TRY(dsmall(h, &h->d_rlist_adv, (size_t)h->nr));
+    TRY(dsmall(h, &h->d_rlen, (size_t)h->nr));
+    TRY(dsmall(h, &h->d_rdt, (size_t)h->nr));
   }
   h->r_dtmax_valid = false;
   TRY(ragged_dtmax(h));
@@ -1891,23 +1923,23 @@ static int graph_alloc(hipft_gpu *h, int passcap) {
   const size_t nr = (size_t)h->nr;
   if (!g.st) {
     double *de = nullptr, *dm = nullptr;
-    TRY(dalloc(h, &g.st, 1));
-    TRY(dalloc(h, &g.ts, nr));
-    TRY(dalloc(h, &g.d, nr));
-    TRY(dalloc(h, &de, nr));
-    TRY(dalloc(h, &dm, nr));
-    TRY(dalloc(h, &g.rdt, nr));
-    TRY(dalloc(h, &g.act, nr));
-    TRY(dalloc(h, &g.fin, nr));
-    TRY(dalloc(h, &g.rl_ptl, nr));
-    TRY(dalloc(h, &g.rl_dif, nr));
-    TRY(dalloc(h, &g.rl_adv, nr));
-    TRY(dalloc(h, &g.rl_adv_all, nr));
-    TRY(dalloc(h, &g.nsub_i, nr));
-    TRY(dalloc(h, &g.cycles_i, nr));
-    TRY(dalloc(h, &g.s_i, nr));
-    TRY(dalloc(h, &g.s_last, nr));
-    TRY(dalloc(h, &g.bits, 2 * nr));
+    TRY(dsmall(h, &g.st, 1));
+    TRY(dsmall(h, &g.ts, nr));
+    TRY(dsmall(h, &g.d, nr));
+    TRY(dsmall(h, &de, nr));
+    TRY(dsmall(h, &dm, nr));
+    TRY(dsmall(h, &g.rdt, nr));
+    TRY(dsmall(h, &g.act, nr));
+    TRY(dsmall(h, &g.fin, nr));
+    TRY(dsmall(h, &g.rl_ptl, nr));
+    TRY(dsmall(h, &g.rl_dif, nr));
+    TRY(dsmall(h, &g.rl_adv, nr));
+    TRY(dsmall(h, &g.rl_adv_all, nr));
+    TRY(dsmall(h, &g.nsub_i, nr));
+    TRY(dsmall(h, &g.cycles_i, nr));
+    TRY(dsmall(h, &g.s_i, nr));
+    TRY(dsmall(h, &g.s_last, nr));
+    TRY(dsmall(h, &g.bits, 2 * nr));
     g.dt_euler = de;
     g.dtmax = dm;
     CK(h, cudaMemsetAsync(g.st, 0, sizeof(GState), h->stream));
@@ -2393,8 +2425,8 @@ static int da_args(hipft_gpu *h, const double *data3_pt, const hipft_da_opts *o,
   size_t nd = (size_t)npm1 * ntm * 3;
   if (!h->d_da) {
     TRY(dalloc(h, &h->d_da, nd));
-    TRY(dalloc(h, &h->d_daopt, 3 * (size_t)(nr + 1)));
-    TRY(dalloc(h, &h->d_tidx, 2 * (size_t)(nr + 1)));
+    TRY(dsmall(h, &h->d_daopt, 3 * (size_t)(nr + 1)));
+    TRY(dsmall(h, &h->d_tidx, 2 * (size_t)(nr + 1)));
   }
   std::vector<double> opt(3 * (size_t)(nr + 1), 0.0);
   std::vector<int> tidx(2 * (size_t)(nr + 1), -1);
@@ -2443,8 +2475,8 @@ static int da_args(hipft_gpu *h, const double *data3_pt, const hipft_da_opts *o,
       h->daw_cap = np * slice;
     }
     if (!h->d_dawidx) {
-      TRY(dalloc(h, &h->d_dawidx, (size_t)nr + 1));
-      TRY(dalloc(h, &h->d_dawkey, 2 * (size_t)nr));
+      TRY(dsmall(h, &h->d_dawidx, (size_t)nr + 1));
+      TRY(dsmall(h, &h->d_dawkey, 2 * (size_t)nr));
     }
     TRY(upload(h, h->d_dawkey, keys));
     CK(h, cudaMemcpyAsync(h->d_dawidx, widx.data(), widx.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
@@ -2967,17 +2999,14 @@ static int adj_slot(hipft_gpu *h, size_t n, double **p) {
 
 static int adj_ensure(hipft_gpu *h) {
   if (h->adjw[0]) return HIPFT_OK;
-  for (auto &w : h->adjw) {
-    TRY(dalloc(h, &w, h->fieldn));
-    CK(h, cudaMemsetAsync(w, 0, h->fieldn * sizeof(double), h->stream));
-  }
+  TRY(dfields(h, h->adjw, (int)(sizeof(h->adjw) / sizeof(h->adjw[0]))));
   dim3 g = stage_grid(h, 32, 8);
   h->dpart_per_r = (int)(g.x * g.y);
-  TRY(dalloc(h, &h->d_dpart, (size_t)h->dpart_per_r * h->nr));
+  TRY(dsmall(h, &h->d_dpart, (size_t)h->dpart_per_r * h->nr));
   h->adj_nch = (h->npm - 2 + 255) / 256;
-  TRY(dalloc(h, &h->d_gring, 2 * (size_t)h->nr * h->adj_nch));
-  TRY(dalloc(h, &h->d_dpole, (size_t)h->nr * h->adj_nch));
-  for (auto &gp : h->d_gpart) TRY(dalloc(h, &gp, 2 * (size_t)g.y * h->nr));
+  TRY(dsmall(h, &h->d_gring, 2 * (size_t)h->nr * h->adj_nch));
+  TRY(dsmall(h, &h->d_dpole, (size_t)h->nr * h->adj_nch));
+  for (auto &gp : h->d_gpart) TRY(dsmall(h, &gp, 2 * (size_t)g.y * h->nr));
   return HIPFT_OK;
 }
 
