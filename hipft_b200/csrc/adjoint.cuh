@@ -187,6 +187,8 @@ __global__ void __launch_bounds__(256) k_adj_diff(Mesh m, DiffCoef dc, const dou
 }
 
 // ---------------------------------------------- two reverse stages per launch
+// For grids that the passes of adj_march.cuh do not take: fewer than 12 theta
+// rows or more phi columns than a thread each in a pole's cluster.
 // Stages k and k-1 of the reverse RKG2 recurrence in one pass over the field:
 //   W_{k-1} = a1 W_k + b1 W_{k+1} + c1 A^T W_k,
 //   W_{k-2} = a2 W_{k-1} + b2 W_k + c2 A^T W_{k-1},

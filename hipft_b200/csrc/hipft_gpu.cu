@@ -22,6 +22,7 @@
 #include "sts_march.cuh"
 #include "adv_march.cuh"
 #include "adjoint.cuh"
+#include "adj_march.cuh"
 #include "graph_step.cuh"
 
 using namespace hipft;
@@ -149,6 +150,9 @@ struct hipft_gpu {
   double *d_dpole = nullptr;  // [nr][adj_nch] D partials of the pole-row chunks
   int adj_nch = 1;            // phi-column chunks of k_adj_pole2
   int dpart_per_r = 0;
+  double *d_jpart = nullptr;  // D partials of the marching passes, [nr][jpart_per_r]
+  int jpart_per_r = 0;        // 0: the grid is not theirs
+  int j_strips = 0, j_cols = 0;  // their theta strips and columns per warp
   // ragged batches: every realization keeps the schedule it would have if run
   // alone (Euler limit, CFL substeps, PTL subcycles, stage counts)
   bool ragged = false;
@@ -2997,6 +3001,55 @@ static int adj_slot(hipft_gpu *h, size_t n, double **p) {
   return HIPFT_OK;
 }
 
+typedef void (*AdjPassKernel)(Mesh, AdjPassArgs, PairTables);
+static AdjPassKernel adj_march_kernel(int ns, bool wide) {
+  if (wide) return ns == 4 ? k_adj_march<4, uint64_t> : k_adj_march<2, uint64_t>;
+  return ns == 4 ? k_adj_march<4, uint32_t> : k_adj_march<2, uint32_t>;
+}
+static AdjPassKernel adj_poles_kernel(int ns, int threads) {
+  if (threads > kPMidThreads) return ns == 4 ? k_adj_poles<4, kPMaxThreads> : k_adj_poles<2, kPMaxThreads>;
+  return ns == 4 ? k_adj_poles<4, kPMidThreads> : k_adj_poles<2, kPMidThreads>;
+}
+
+// ns reverse stages (four or two) as the strips' and the march's launches;
+// after_pass: the launch before them on the stream is such a pass too.
+static int adj_pass(hipft_gpu *h, AdjPassArgs a, int ns, bool after_pass) {
+  const int n2 = h->npm - 2, nc = poles_ranks(n2);
+  a.dpart = h->d_jpart;
+  a.dstride = h->jpart_per_r;
+  a.strips = h->j_strips;
+  a.cols = h->j_cols;
+  a.dfac = h->DC.dfac;
+  a.bcn = h->bc_diff_n;
+  a.bcs = h->bc_diff_s;
+  a.err = h->d_err;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = (ws_pdl() && after_pass) ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)nc;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.stream = h->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  cfg.gridDim = dim3((unsigned)(2 * h->nr * nc));
+  cfg.blockDim = dim3((unsigned)poles_threads(n2));
+  cfg.dynamicSmemBytes = adj_poles_smem(ns, poles_threads(n2));
+  CK(h, cudaLaunchKernelEx(&cfg, adj_poles_kernel(ns, poles_threads(n2)), h->M, a, h->ptab));
+  LAUNCHED(h);
+  const int nch = (n2 + a.cols - 1) / a.cols;
+  attr[0].val.programmaticStreamSerializationAllowed = ws_pdl() ? 1 : 0;
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3((unsigned)((int64_t)a.strips * ((nch + kJWarps - 1) / kJWarps) * h->nr));
+  cfg.blockDim = dim3(32 * kJWarps);
+  cfg.dynamicSmemBytes = adj_march_smem(ns);
+  CK(h, cudaLaunchKernelEx(&cfg, adj_march_kernel(ns, h->plane >= (int64_t)1 << 29), h->M, a, h->ptab));
+  LAUNCHED(h);
+  return HIPFT_OK;
+}
+
 static int adj_ensure(hipft_gpu *h) {
   if (h->adjw[0]) return HIPFT_OK;
   TRY(dfields(h, h->adjw, (int)(sizeof(h->adjw) / sizeof(h->adjw[0]))));
@@ -3007,6 +3060,22 @@ static int adj_ensure(hipft_gpu *h) {
   TRY(dsmall(h, &h->d_gring, 2 * (size_t)h->nr * h->adj_nch));
   TRY(dsmall(h, &h->d_dpole, (size_t)h->nr * h->adj_nch));
   for (auto &gp : h->d_gpart) TRY(dsmall(h, &gp, 2 * (size_t)g.y * h->nr));
+  const int n2 = h->npm - 2;
+  if (h->ntm >= kJMinRows && poles_by_column(h)) {
+    h->j_strips = adj_strips(h->ntm);
+    // a strip's block leaves no room for the march's on its SM; with those SMs counted in,
+    // 512x1024 took a second wave and 34 us per pass instead of 20
+    const int sms = std::max(h->num_sms - 2 * h->nr * poles_ranks(n2), h->num_sms / 2);
+    h->j_cols = adj_cols(n2, h->j_strips, h->nr, kJWarps * kJBlocks * sms);
+    h->jpart_per_r = h->j_strips * ((n2 + h->j_cols - 1) / h->j_cols) + 2 * poles_ranks(n2);
+    for (int ns = 2; ns <= kMS; ns += 2) {
+      CK(h, cudaFuncSetAttribute(adj_march_kernel(ns, h->plane >= (int64_t)1 << 29),
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adj_march_smem(ns)));
+      CK(h, cudaFuncSetAttribute(adj_poles_kernel(ns, poles_threads(n2)), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)adj_poles_smem(ns, poles_threads(n2))));
+    }
+    TRY(dsmall(h, &h->d_jpart, (size_t)h->jpart_per_r * h->nr));
+  }
   return HIPFT_OK;
 }
 
@@ -3232,9 +3301,43 @@ static int adj_diff_rev(hipft_gpu *h, const AdjSub &S, double *&W, double *dacc)
     pp ^= 1;
     return HIPFT_OK;
   };
-  TRY(pole_sums(W));
   double *Wk = W, *Wk1 = nullptr;
   int64_t k = S.s;
+  // four or two reverse stages per pass, whose stage inputs lie in one
+  // stage-checkpoint block
+  if (h->jpart_per_r) {
+    CK(h, cudaMemsetAsync(h->d_jpart, 0, (size_t)h->jpart_per_r * h->nr * sizeof(double), h->stream));
+    bool after = false;
+    while (k >= 3 && adj_pairs_enabled()) {
+      if (S.q > 0 && (k - 2) / S.q != curb) {
+        curb = (k - 2) / S.q;
+        TRY(adj_block_recompute(h, S, (size_t)curb, Yr));
+        after = false;
+      }
+      const int64_t room = S.q > 0 ? (k - 2) % S.q + 1 : k - 1;  // stages whose inputs are at hand
+      if (room < 2) break;
+      const int ns = room >= kMS ? kMS : 2;
+      AdjPassArgs a{};
+      a.w0 = Wk;
+      a.w1 = Wk1 ? Wk1 : Wk;
+      a.o0 = adj_free(h, {Wk, Wk1, ub, db});
+      a.o1 = adj_free(h, {Wk, Wk1, ub, db, a.o0});
+      a.ub = ub;
+      a.db = db;
+      for (int q = 0; q < ns; ++q) {
+        const int64_t K = k - q;
+        const double nu = (K < S.s) ? S.vj[K + 1] : 0.0;
+        a.c[q] = AdjStage{S.uj[K], nu, S.ubj[K] * dtl, 1.0 - S.uj[K] - S.vj[K], S.gj[K], S.ubj[K] * dtl};
+        a.y[q] = Yt(K - 1);
+      }
+      TRY(adj_pass(h, a, ns, after));
+      after = true;
+      Wk1 = a.o0;
+      Wk = a.o1;
+      k -= ns;
+    }
+  }
+  if (k >= 2) TRY(pole_sums(Wk));
   // two reverse stages per launch (k_adj_diff2 + k_adj_pole2) while both of
   // their stage inputs Y_{k-1}, Y_{k-2} lie in one stage-checkpoint block
   // A pair launch follows the previous pair's k_adj_pole2 programmatically
@@ -3308,6 +3411,10 @@ static int adj_diff_rev(hipft_gpu *h, const AdjSub &S, double *&W, double *dacc)
   TRY(stage(db, ub, Yt(0), ub, nullptr, nullptr, AdjDiffCoef{0.0, 1.0, dtl, 0.0, 0.0, dtl}));
   k_adj_dsum<<<h->nr, 256, 0, h->stream>>>(h->d_dpart, h->dpart_per_r, h->d_dpole, h->adj_nch, 1.0, dacc);
   LAUNCHED(h);
+  if (h->jpart_per_r) {
+    k_adj_dsum<<<h->nr, 256, 0, h->stream>>>(h->d_jpart, h->jpart_per_r, nullptr, 0, 1.0, dacc);
+    LAUNCHED(h);
+  }
   W = ub;
   return HIPFT_OK;
 }
@@ -3394,6 +3501,8 @@ extern "C" int hipft_adj_reverse(hipft_gpu *h, double *fbar, double *dacc, doubl
   CK(h, cudaSetDevice(h->dev));
   TRY(adj_reverse(h, fbar, dacc, gflow));  // asynchronous on the handle's stream
   CK(h, cudaGetLastError());
+  // the last recorded step: the caller reads the gradient next
+  if (h->adj_recs.empty()) TRY(check_wait_flag(h, "adj_reverse: a bounded wait for ring sums gave up"));
   return HIPFT_OK;
 }
 
