@@ -70,7 +70,7 @@ __device__ __forceinline__ double adj_diff_at(const Mesh &m, const DiffCoef &dc,
 // The same, from the coefficient tables of k_pair_tables (per-realization
 // constant D): row j's st_i, c2, c4 and column k's {P1, P5}, with
 // c1 = P1 st_i^2, c5 = P5 st_i^2 and c3 = -(c1+c2+c4+c5) as in the forward
-// two-stage kernel; five table rows and columns instead of five coef5().
+// passes; five table rows and columns instead of five coef5().
 __device__ __forceinline__ double adj_diff_at_tab(const Mesh &m, const DiffCoef &dc, const PairTables &pt,
                                                   const double *__restrict__ w, int j, int k, int i, double gn,
                                                   double gs, double bcn, double bcs) {

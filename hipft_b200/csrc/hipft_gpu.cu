@@ -152,6 +152,7 @@ struct hipft_gpu {
   int dpart_per_r = 0;
   double *d_jpart = nullptr;  // D partials of the marching passes, [nr][jpart_per_r]
   int jpart_per_r = 0;        // 0: the grid is not theirs
+  int pass_clusters = 0;         // clusters of a merged pass that the GPU holds; 0: not on this grid
   int j_strips = 0, j_cols = 0;  // their theta strips and columns per warp
   // ragged batches: every realization keeps the schedule it would have if run
   // alone (Euler limit, CFL substeps, PTL subcycles, stage counts)
@@ -522,25 +523,48 @@ static MarchArgs march_args(const hipft_gpu *h, const double *u0, const double *
 // A column per thread in k_sts_poles, or k_sts_poles_any.
 static bool poles_by_column(const hipft_gpu *h) { return poles_threads(h->npm - 2) <= kPMaxThreads; }
 
+// Places of k_sts_march's blocks that one realization's strips take: a block of
+// the widest takes an SM.
+static int pole_places(int n2) {
+  return 2 * poles_ranks(n2) * (poles_threads(n2) > kPMidThreads ? kMBlocks : 1);
+}
+
 static int march_columns(const hipft_gpu *h, int nreal) {
   const int n2 = h->npm - 2;
-  return march_cols(n2, h->m_strips, nreal, h->m_slots, 2 * poles_ranks(n2));
+  return march_cols(n2, h->m_strips, nreal, h->m_slots, pole_places(n2));
 }
 
 static int64_t march_blocks(const hipft_gpu *h, int nreal) {
-  const int n2 = h->npm - 2, c = march_columns(h, nreal), nch = (n2 + c - 1) / c;
-  return (int64_t)h->m_strips * ((nch + kMWarps - 1) / kMWarps) * nreal;
+  return march_units(h->npm - 2, h->m_strips, march_columns(h, nreal), kMWarps) * nreal;
 }
 
 // k_sts_march for these arguments; byte offsets in 32 bits while a plane has them.
 typedef void (*MarchKernel)(Mesh, MarchArgs, PairTables);
 template <typename Off>
 static MarchKernel march_kernel(bool table, bool keep) {
-  if (keep) return table ? k_sts_march<true, true, Off> : k_sts_march<false, true, Off>;
-  return table ? k_sts_march<true, false, Off> : k_sts_march<false, false, Off>;
+  if (keep) return table ? k_sts_march<true, true, Off, false> : k_sts_march<false, true, Off, false>;
+  return table ? k_sts_march<true, false, Off, false> : k_sts_march<false, false, Off, false>;
 }
 static MarchKernel march_kernel(bool table, bool keep, bool wide) {
   return wide ? march_kernel<uint64_t>(table, keep) : march_kernel<uint32_t>(table, keep);
+}
+
+// Both parts of a pass in one launch, where the host knows its realizations, and
+// the columns per warp with which the GPU holds all of it at once; 0 columns: two
+// launches.
+static MarchKernel pass_kernel(bool table, bool keep) {
+  return table ? (keep ? k_sts_march<true, true, uint32_t, true> : k_sts_march<true, false, uint32_t, true>)
+               : (keep ? k_sts_march<false, true, uint32_t, true> : k_sts_march<false, false, uint32_t, true>);
+}
+static int pass_columns(const hipft_gpu *h, const MarchArgs &a) {
+  if (!h->pass_clusters || a.dctr) return 0;
+  const int n2 = h->npm - 2, nc = poles_ranks(n2), nw = poles_threads(n2) / 32;
+  const int64_t free = ((int64_t)h->pass_clusters - 2 * a.nreal) * nc;
+  if (free < 1) return 0;
+  const int64_t nch = free / a.nreal * nw / h->m_strips;
+  if (nch < 1) return 0;
+  const int64_t c = ((n2 + nch - 1) / nch + kMGroup - 1) / kMGroup * kMGroup;
+  return c <= kPassColsMax ? (int)c : 0;
 }
 
 // One pass on stream s.  after_pass: the launch before it on the stream is
@@ -568,6 +592,19 @@ static cudaError_t launch_pass(const hipft_gpu *h, cudaStream_t s, MarchArgs a, 
   const int n2 = h->npm - 2, nc = poles_ranks(n2);
   const bool bycol = poles_by_column(h);
   attr[0].val.programmaticStreamSerializationAllowed = (pdl && after_pass) ? 1 : 0;
+  if (const int pc = pass_columns(h, a)) {
+    a.cols = pc;
+    const int64_t mb = march_units(n2, h->m_strips, pc, poles_threads(n2) / 32) * a.nreal;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)nc;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+    cfg.gridDim = dim3((unsigned)(2 * a.nreal * nc + (mb + nc - 1) / nc * nc));
+    cfg.blockDim = dim3((unsigned)poles_threads(n2));
+    cfg.dynamicSmemBytes = pass_smem(poles_threads(n2));
+    return cudaLaunchKernelEx(&cfg, pass_kernel(a.rc || pc > kMGroup, a.o[0] || a.o[1]), h->M, a, h->ptab);
+  }
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = (unsigned)nc;
   attr[1].val.clusterDim.y = 1;
@@ -578,9 +615,10 @@ static cudaError_t launch_pass(const hipft_gpu *h, cudaStream_t s, MarchArgs a, 
   cfg.dynamicSmemBytes = bycol ? poles_smem(poles_threads(n2)) : 0;
   // a march that leaves places free does not compete with the pole strips' registers
   const bool roomy = blocks + 3 * (int64_t)cfg.gridDim.x <= (int64_t)kMBlocks * h->num_sms;
-  auto poles = poles_threads(n2) > kPMidThreads ? k_sts_poles<kPMaxThreads, 1>
-               : roomy                          ? k_sts_poles<kPMidThreads, 1>
-                                                : k_sts_poles<kPMidThreads, 3>;
+  auto poles = poles_threads(n2) > kPMidThreads    ? k_sts_poles<kPMaxThreads, 1>
+               : poles_threads(n2) <= kPMinThreads ? k_sts_poles<kPMinThreads, 3>
+               : roomy                             ? k_sts_poles<kPMidThreads, 1>
+                                                   : k_sts_poles<kPMidThreads, 3>;
   cudaError_t e = bycol ? cudaLaunchKernelEx(&cfg, poles, h->M, a, h->ptab)
                         : cudaLaunchKernelEx(&cfg, k_sts_poles_any, h->M, a, h->ptab, h->d_pscratch);
   if (e != cudaSuccess) return e;
@@ -598,7 +636,7 @@ static int sts_pass(hipft_gpu *h, const MarchArgs &a, bool after_pass) {
   ProfScope ps(h, HIPFT_K_STS);
   const cudaError_t e = launch_pass(h, h->stream, a, ws_pdl(), after_pass);
   if (e != cudaSuccess) return fail(h, HIPFT_ECUDA, "RKG2 pass launch: %s", cudaGetErrorString(e));
-  h->launches += h->ntm < kMMinRows ? 1 : 2;
+  h->launches += h->ntm < kMMinRows || pass_columns(h, a) ? 1 : 2;
   return HIPFT_OK;
 }
 
@@ -818,8 +856,27 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
     for (int v = 0; v < 4; ++v) reserve((const void *)adv_kernel(v & 1, v & 2, vwide), adv_smem(v & 1));
   if (prm->advance_diffusion && prm->diffusion_num_method >= 2 && !prm->diffusion_coef_grid && h->ntm >= kMMinRows) {
     for (int v = 0; v < 4; ++v) reserve((const void *)march_kernel(v & 1, v & 2, wide), kMSmem);
+    if (npm - 2 >= kPassColumns && poles_threads(npm - 2) <= kPassThreads && !wide) {
+      const int pt = poles_threads(npm - 2);
+      for (int v = 0; v < 4; ++v) reserve((const void *)pass_kernel(v & 1, v & 2), pass_smem(pt));
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)poles_ranks(npm - 2);
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.gridDim = dim3((unsigned)poles_ranks(npm - 2));
+      cfg.blockDim = dim3((unsigned)pt);
+      cfg.dynamicSmemBytes = pass_smem(pt);
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (!smem_ok || cudaOccupancyMaxActiveClusters(&h->pass_clusters, pass_kernel(true, true), &cfg) != cudaSuccess)
+        h->pass_clusters = 0;
+    }
     if (poles_threads(npm - 2) > kPMidThreads) {
       reserve((const void *)k_sts_poles<kPMaxThreads, 1>, poles_smem(kPMaxThreads));
+    } else if (poles_threads(npm - 2) <= kPMinThreads) {
+      reserve((const void *)k_sts_poles<kPMinThreads, 3>, poles_smem(kPMinThreads));
     } else {
       reserve((const void *)k_sts_poles<kPMidThreads, 1>, poles_smem(kPMidThreads));
       reserve((const void *)k_sts_poles<kPMidThreads, 3>, poles_smem(kPMidThreads));
@@ -1710,7 +1767,7 @@ static int ragged_diffusion_step(hipft_gpu *h, double dtl, hipft_diffusion_info 
     act.swap(next);
     cyc = cyc + 1;
   }
-  TRY(check_wait_flag(h, "diffusion_step: a bounded wait for staged tiles gave up"));
+  TRY(check_wait_flag(h, "diffusion_step: a bounded wait for ring sums gave up"));
   h->sts_s = smax;
   h->subcycles_state = cyc - 1;
   if (info) {
@@ -1883,7 +1940,7 @@ extern "C" int hipft_gpu_diffusion_step(hipft_gpu *h, double dtl, hipft_cycle_cb
     i = i + 1;
   }
   if (h->auto_sc) h->subcycles_state = i;
-  TRY(check_wait_flag(h, "diffusion_step: a bounded wait for staged tiles gave up"));
+  TRY(check_wait_flag(h, "diffusion_step: a bounded wait for ring sums gave up"));
   if (info) {
     info->dtime_diffusion_euler = h->dt_euler;
     info->sts_s = (h->P.diffusion_num_method == 1) ? h->n_euler : h->sts_s;
@@ -2043,7 +2100,7 @@ static int graph_capture(hipft_gpu *h) {
   G.n2 = h->npm - 2;
   G.strips = h->m_strips;
   G.slots = h->m_slots;
-  G.poles = 2 * poles_ranks(h->npm - 2);
+  G.poles = pole_places(h->npm - 2);
   G.nadv = (h->adv_time == 1) ? 1 : ((h->adv_time == 2) ? 3 : 4);
   {
     const char *e = std::getenv("HIPFT_GRAPH_UNROLL");
@@ -2276,7 +2333,7 @@ static int graph_step(hipft_gpu *h, double dt, hipft_diffusion_info *info) {
   h->ring_cur = 0;
   if (info) {
     TRY(graph_collect(h));
-    TRY(check_wait_flag(h, "graph-run step: a bounded wait for staged tiles gave up"));
+    TRY(check_wait_flag(h, "graph-run step: a bounded wait for ring sums gave up"));
     info->dtime_diffusion_euler = h->dt_euler;
     if (h->ragged && !h->r_dt_euler.empty())
       info->dtime_diffusion_euler = *std::min_element(h->r_dt_euler.begin(), h->r_dt_euler.end());

@@ -147,14 +147,21 @@ __host__ __device__ inline StageCoef sts_slot(int method, int64_t s, int64_t q, 
 // loads 2 kMS columns more than it owns, so longer chunks waste less; whole
 // waves leave no nearly empty one).  Blocks of k_sts_poles take the place of
 // blocks; a single wave leaves those places out, which would otherwise start a
-// second one.
+// second one.  A realization's chunks are dealt to its blocks' warps strip by
+// strip: whole blocks per strip left up to a third of the warps without one
+// (359x722 2.58 -> 2.20 us per stage, 256x512 2.30 -> 2.05).
+// blocks of nw warps for the chunks of `cols` columns of one realization's strips
+__host__ __device__ inline int64_t march_units(int n2, int strips, int cols, int nw) {
+  const int64_t nch = (n2 + cols - 1) / cols;
+  return (strips * nch + nw - 1) / nw;
+}
 __host__ __device__ inline int march_cols(int n2, int strips, int nreal, int slots, int poles) {
-  const int64_t per = (int64_t)strips * (nreal > 0 ? nreal : 1) * kMWarps;
+  const int64_t n = nreal > 0 ? nreal : 1;
   for (int64_t w = 1;; ++w) {
     int64_t free = w * slots;
     const int64_t taken = (int64_t)poles * nreal * kMWarps;
     if (w == 1 && taken <= slots / 2) free -= taken;
-    const int64_t nch = free / per * kMWarps;  // whole blocks of chunks
+    const int64_t nch = free / kMWarps / n * kMWarps / strips;  // whole blocks per realization
     if (nch < 1) continue;
     const int64_t c = ((n2 + nch - 1) / nch + kMGroup - 1) / kMGroup * kMGroup;
     if (c <= kMColsMax) return (int)c;
@@ -275,13 +282,16 @@ __device__ __forceinline__ double2 pair_stage(double2 xl, double2 xc, double2 xr
 // shared memory, by asynchronous copies in which every lane fetches its own
 // two rows: no barriers, and warps are independent.  The loop takes kMGroup
 // columns per turn, so that windows, coefficients and ring slots are renamed
-// and not moved.  The four warps of a block march four neighbouring chunks of
-// one strip.  Seam columns are not written (nothing reads them in a stage).
+// and not moved.  The four warps of a block march the same columns of
+// neighbouring strips where they can.  Seam columns are not written (nothing reads them in a stage).
 //
 // Bound: the FP64 pipe.  A pair of rows costs 4 x 36 + 14 instructions per
 // column (no contraction: every product is rounded as in the reference), and
 // 64/56 of that for the strip's halo; HBM sees 4 reads and 2 writes of 8 bytes
-// per cell and four stages.
+// per cell and four stages.  Where it fills the GPU, DRAM (82 % of the copy
+// rate), shared memory and the FP64 pipe (69 %) are all near their ends.
+// Gcell-stages/s, two stages per pass before and now: 64 x 1024x2048 165 and 393,
+// 1024x2048 150 and 336; 512x1024 198, 256x512 64 (latency).
 //
 // TABLE: the stages' coefficients are read from shared memory.  Those of all
 // realizations come as arguments, but from a chunk of more than one turn on
@@ -291,10 +301,31 @@ __device__ __forceinline__ double2 pair_stage(double2 xl, double2 xc, double2 xr
 // (180x360: 1 % of a step).
 // KEEP: Y_k and Y_{k+1} are kept too; Off: a byte offset within a
 // realization's plane.
-template <bool TABLE, bool KEEP, typename Off>
-__global__ void __launch_bounds__(32 * kMWarps, kMBlocks) k_sts_march(Mesh m, MarchArgs a, PairTables pt) {
+// MERGED: a pass that the GPU holds at once, in one launch: the first 2 nreal
+// clusters are the pole strips, the warps of all others march.  It is then one
+// grid that waits for the one before it, where the march's end would wait for
+// the strips' and the next strips for the march's: 512x1024 3.16 -> 2.67 us per
+// stage, 359x722 2.80 -> 2.58.  Not on narrower grids (256x512 2.30 -> 2.43:
+// the strips share their SMs with the march from the start) nor where more than
+// 16 columns per warp make the march the longer part.
+constexpr int kPassThreads = 160;   // most threads per block then (kPMinThreads)
+constexpr int kPassColumns = 640;   // fewest phi columns
+constexpr int kPassColsMax = 16;    // most columns per warp
+template <int NT, bool MERGED>
+__device__ __forceinline__ void poles_body(const Mesh &m, const MarchArgs &a, const PairTables &pt);
+
+template <bool TABLE, bool KEEP, typename Off, bool MERGED>
+__global__ void __launch_bounds__(MERGED ? kPassThreads : 32 * kMWarps, MERGED ? 2 : kMBlocks)
+    k_sts_march(Mesh m, MarchArgs a, PairTables pt) {
   extern __shared__ __align__(16) double msm[];
-  pdl_trigger();  // the next pass's k_sts_poles may take its place on the SMs; it waits for this grid's end
+  pdl_trigger();  // the next pass's blocks may take their place on the SMs; they wait for this grid's end
+  const int np = MERGED ? 2 * a.nreal * (int)cooperative_groups::this_cluster().num_blocks() : 0;
+  if (MERGED && (int)blockIdx.x < np) {
+    poles_body<kPassThreads, true>(m, a, pt);
+    return;
+  }
+  const unsigned block = blockIdx.x - np;
+  const int nw = MERGED ? (int)blockDim.x >> 5 : kMWarps;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int npm = m.npm, n2 = npm - 2, ntm = m.ntm;
   int nreal;
@@ -302,16 +333,17 @@ __global__ void __launch_bounds__(32 * kMWarps, kMBlocks) k_sts_march(Mesh m, Ma
   const StageCoef *rc;
   int ncol;
   march_launch(a, nreal, first, rc, ncol);
-  const int nch = (n2 + ncol - 1) / ncol, nblk = (nch + kMWarps - 1) / kMWarps;
-  const int strip = blockIdx.x % a.strips;
-  const int rest = blockIdx.x / a.strips;
-  const int c0 = 2 + ((rest % nblk) * kMWarps + warp) * ncol, c1 = min(c0 + ncol - 1, npm - 1);
-  if (rest / nblk >= nreal) {
+  // the realization's chunks, strip by strip, over its blocks' warps
+  const unsigned nblk = (unsigned)march_units(n2, a.strips, ncol, nw), real = block / nblk;
+  const unsigned unit = (block % nblk) * nw + warp;
+  const int strip = unit % a.strips;
+  const int c0 = 2 + (int)(unit / a.strips) * ncol, c1 = min(c0 + ncol - 1, npm - 1);
+  if ((int)real >= nreal) {
     pdl_wait();
     return;
   }
-  const int i = a.rlist ? a.rlist[rest / nblk] : rest / nblk;  // 0-based
-  double *coef = msm + kMWarps * (kMRing + kMTab);
+  const int i = a.rlist ? a.rlist[real] : (int)real;  // 0-based
+  double *coef = msm + nw * (kMRing + kMTab);
   if (TABLE) {
     if (threadIdx.x < kMCoef)
       coef[threadIdx.x] = a.rc ? reinterpret_cast<const double *>(rc + (int64_t)i * kMS)[threadIdx.x]
@@ -361,8 +393,9 @@ __global__ void __launch_bounds__(32 * kMWarps, kMBlocks) k_sts_march(Mesh m, Ma
     }
   };
   // the column table's entries of the chunk, with the first columns' copies
-  double *tab = msm + kMWarps * kMRing + warp * kMTab;
+  double *tab = msm + nw * kMRing + warp * kMTab;
   for (int t = lane; t < left + kMGroup - 1; t += 32) cp_async16(smem_addr(tab) + 16u * t, pt_col + c0 - kMS + t);
+  if (MERGED) pdl_wait();  // the pass before
   fetch(sring);
   fetch(sring + kSlot);
   fetch(sring + 2 * kSlot);
@@ -455,7 +488,7 @@ __global__ void __launch_bounds__(32 * kMWarps, kMBlocks) k_sts_march(Mesh m, Ma
   cp_async_wait<0>();
   // this grid ends after the pole strips' grid, so that the next pass, which
   // waits for this one, has both
-  pdl_wait();
+  if (!MERGED) pdl_wait();
 }
 
 // Four stages of the rows 1..kMS and ntm-kMS+1..ntm: one cluster per
@@ -480,10 +513,11 @@ constexpr int kPRows = 2 * kMS;  // strip rows of Y_{k-1}
 // Columns per block: few on narrow grids, where the FP64 work of a block would
 // otherwise outlast its ring sums.  NB = 3 holds the block's registers to those
 // of one block of k_sts_march, so that it takes the place of one where the
-// march fills the GPU; NB = 1 is faster by itself.
-constexpr int kPMidThreads = 288, kPMaxThreads = 544;
+// march fills the GPU (160 threads keep all they need then); NB = 1 is faster by
+// itself.
+constexpr int kPMinThreads = 160, kPMidThreads = 288, kPMaxThreads = 544;
 __host__ __device__ inline int poles_ranks(int n2) {
-  const int per = n2 <= 8 * 120 ? 120 : 280;
+  const int per = n2 <= 8 * 152 ? 120 : 280;
   const int c = (n2 + per - 1) / per;
   return c > 8 ? 8 : c;
 }
@@ -497,10 +531,10 @@ __host__ __device__ inline size_t poles_smem(int threads) {
   return (size_t)kPSmemRows * poles_stride(threads) * sizeof(double);
 }
 
-template <int NT, int NB>
-__global__ void __launch_bounds__(NT, NB) k_sts_poles(Mesh m, MarchArgs a, PairTables pt) {
-  const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+template <int NT, bool MERGED>
+__device__ __forceinline__ void poles_body(const Mesh &m, const MarchArgs &a, const PairTables &pt) {
   extern __shared__ __align__(16) double psm[];
+  const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
   __shared__ double s_sum[kMS][8 * (NT / 32)];
   __shared__ double s_row[3][kPRows];
   __shared__ double s_coef[5 * kMS];
@@ -517,7 +551,7 @@ __global__ void __launch_bounds__(NT, NB) k_sts_poles(Mesh m, MarchArgs a, PairT
   march_launch(a, nreal, first, rc, cols);
   if ((unit >> 1) >= nreal) {  // the whole cluster
     pdl_wait();
-    pdl_trigger();
+    if (!MERGED) pdl_trigger();
     return;
   }
   if (tid == 0) {
@@ -577,7 +611,7 @@ __global__ void __launch_bounds__(NT, NB) k_sts_poles(Mesh m, MarchArgs a, PairT
   // launch on the stream, this pass's k_sts_march, reads and writes other rows
   // and may start now.
   pdl_wait();
-  pdl_trigger();
+  if (!MERGED) pdl_trigger();
   strips(first ? a.u : a.x1, first ? a.u : a.x2, sX, sY, kPRows);
   __syncthreads();
   double x[kPRows], z[kPRows - 1];
@@ -638,6 +672,15 @@ __global__ void __launch_bounds__(NT, NB) k_sts_poles(Mesh m, MarchArgs a, PairT
   cluster_wait();
 }
 
+template <int NT, int NB>
+__global__ void __launch_bounds__(NT, NB) k_sts_poles(Mesh m, MarchArgs a, PairTables pt) {
+  poles_body<NT, false>(m, a, pt);
+}
+
+__host__ __device__ inline size_t pass_smem(int threads) {
+  const size_t march = ((size_t)(threads / 32) * (kMRing + kMTab) + kMCoef) * sizeof(double);
+  return march > poles_smem(threads) ? march : poles_smem(threads);
+}
 // The same strips when a column per thread does not suffice (more than about
 // 4200 phi columns): the blocks loop over their columns and keep the strip in
 // a scratch area in global memory, in place: stage k over Y_{k-2}, stage k+1
