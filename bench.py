@@ -61,11 +61,11 @@ sys.path.insert(0, ROOT)
 
 METRIC = "FP64 Gcell-updates/s"
 UNIT = "Gcell-updates/s"
-STS_BYTES_PER_CELL = 40  # RKG2 stage k>=2: read Y_{k-1}, Y_{k-2}, u0, dty0; write Y_k
-# two-stage kernel per HIPFT_STS_PAIR value (the library's default is 5); the
-# timed region of a "launch" is the kernel plus its pole-row launch
-STS_KERNELS = {"4": "k_sts_pair_ws+k_pair_poles", "5": "k_sts_pair_ws<rows2>+k_pair_poles",
-               "6": "k_sts_pair_ws<rows2, bulk stores>+k_pair_poles"}
+# an RKG2 pass of four stages reads Y_{k-1}, Y_{k-2}, u0 and dty0 and writes the
+# last two stages: 48 bytes per cell, 12 per stage.  The timed region of a
+# "launch" is the march plus its pole strips.
+STS_BYTES_PER_CELL = 12
+STS_KERNEL = "k_sts_march+k_sts_poles"
 
 WORKLOADS = {
     "batched64_1024x2048": dict(ntm=1024, npm1=2049, nr=64, seed=1),
@@ -405,21 +405,19 @@ def run_gpu(args, wl, name):
         launches = int(launches)
 
     peak, peak_kind = measured_peak()
-    # Algorithmic bytes: 40 B per unique cell per RKG2 stage (read Y_{k-1},
-    # Y_{k-2}, u0, dty0; write Y_k), times the cell-stages one launch advances
-    # (in a ragged batch a launch covers the realizations with stages left).
+    # Algorithmic bytes: 12 B per unique cell and RKG2 stage, times the
+    # cell-stages one launch advances (in a ragged batch a launch covers the
+    # realizations with stages left).
     stages_per_launch = rkg2_stages / max(sts_n, 1)
     bytes_per_launch = STS_BYTES_PER_CELL * rkg2_cell_stages / max(sts_n, 1)
     sts_avg_ms = sts_ms / max(sts_n, 1)
     achieved = bytes_per_launch / (sts_avg_ms * 1e-3) / 1e9 if sts_n else None
     traffic, traffic_src = None, None
-    sts_kernel = STS_KERNELS.get(os.environ.get("HIPFT_STS_PAIR", "5"), STS_KERNELS["5"]) if stages_per_launch > 1.5 \
-        else "k_sts_stage_v3"
     tpath = os.path.join(ROOT, "profiles", "sts_stage_traffic.json")
     if os.path.exists(tpath):
         with open(tpath) as fh:
             tj = json.load(fh)
-        if abs(tj.get("stages_per_launch", 1) - stages_per_launch) < 1e-9 and tj.get("kernel") == sts_kernel:
+        if abs(tj.get("stages_per_launch", 1) - stages_per_launch) < 1e-9 and tj.get("kernel") == STS_KERNEL:
             traffic = tj["dram_bytes_per_cell"] * ntm * (npm - 2) * nrl
             traffic_src = tj["source"]
     out = {
@@ -436,8 +434,7 @@ def run_gpu(args, wl, name):
                             "decided on the device)" if args.step == "graph" else "host-driven launches"),
                    "l2": "inputs larger than L2 (%.2f GB per field), no flush" % (ntm * npm * nrl * 8 / 1e9)},
         "roofline": {"bound": "hbm",
-                     "kernel": sts_kernel, "kernel_role": ("two fused RKG2 stages per launch"
-                                                           if stages_per_launch > 1.5 else "one fused RKG2 stage"),
+                     "kernel": STS_KERNEL, "kernel_role": "four RKG2 stages per pass",
                      "stages_per_launch": stages_per_launch, "traffic_source": traffic_src,
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None, "traffic": traffic,
@@ -566,7 +563,7 @@ def measure_plain(args, local: int):
            "l2": "256 MB buffer written before every timed step, each step timed alone (fields fit in L2)",
            "e2e": {"value": float(i3.cell_stage_updates - i2.cell_stage_updates) / w / 1e9, "unit": UNIT,
                    "h2d_bytes_per_step": ntm * npm * 8, "d2h_bytes_per_step": ntm * npm * 8},
-           "roofline": {"kernel": STS_KERNELS.get(os.environ.get("HIPFT_STS_PAIR", "5"), STS_KERNELS["5"]),
+           "roofline": {"kernel": STS_KERNEL,
                         "achieved": achieved, "peak": peak, "unit": "GB/s",
                         "frac": (achieved / peak) if achieved else None, "peak_source": peak_kind,
                         "avg_launch_ms": avg, "launches": sts_n,
@@ -643,7 +640,7 @@ def measure_adjoint(args, local: int, days: float = 27.27, checkpoint_every: int
     fwd_runs = [forward(g, f0)[1] for _ in range(5)]
     gc.enable()
     A = MisfitAdjoint(g, D, flow, checkpoint_every=checkpoint_every)
-    A.run(f0, target, dts)  # warm-up: tuner, tape allocation (kept by the handle)
+    A.run(f0, target, dts)  # warm-up: tape allocation (kept by the handle)
     grad_runs, phases = [], []
     import gc
     for _ in range(5):
@@ -798,7 +795,7 @@ def measure_c5_adjoint(args, local: int, steps: int = 6, checkpoint_every: int =
     forward(g, f0)
     fwd_runs = [forward(g, f0)[1] for _ in range(runs)]
     A = MisfitAdjoint(g, D, flow, checkpoint_every=checkpoint_every)
-    A.run(f0, target, dts)  # warm-up: tuner, tape allocation
+    A.run(f0, target, dts)  # warm-up: tape allocation
     grad_runs = []
     for _ in range(runs):
         torch.cuda.synchronize()

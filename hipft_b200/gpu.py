@@ -370,7 +370,7 @@ class HipftGPU:
 
     def set_graph(self, on: bool = True):
         """Run every flux_transport_step as one launch of a captured CUDA graph
-        whose loops (subcycles, stage pairs, advection substeps) are sized on
+        whose loops (subcycles, RKG2 passes, advection substeps) are sized on
         the device; same field, bit for bit, as the host-driven step."""
         self._ck(self.L.hipft_gpu_set_graph(self.h, int(on)), "set_graph")
 
@@ -452,7 +452,7 @@ class HipftGPU:
         return n.value, ms.value
 
     def describe(self) -> str:
-        """Schedule and the two-stage kernel the autotuner picked."""
+        """Schedule and the RKG2 kernel."""
         buf = ctypes.create_string_buffer(256)
         self._ck(self.L.hipft_gpu_describe(self.h, buf, 256), "describe")
         return buf.value.decode()
