@@ -845,7 +845,8 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
   if ((rc = dsmall(h, &h->d_rcount, (size_t)nr))) return bail(rc);
   if ((rc = dsmall(h, &h->d_err, 1))) return bail(rc);
   if (cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream) != cudaSuccess) return bail(HIPFT_ECUDA);
-  // the kernels this grid can reach (setting an attribute loads the kernel)
+  // the kernels this grid can reach (setting an attribute loads the kernel); the
+  // limit is the kernel's, not the handle's, so it is the most that any grid takes
   const bool wide = h->plane >= (int64_t)1 << 29;
   const bool vwide = wide || (int64_t)h->ldv * h->npm >= (int64_t)1 << 29;
   bool smem_ok = true;
@@ -858,7 +859,7 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
     for (int v = 0; v < 4; ++v) reserve((const void *)march_kernel(v & 1, v & 2, wide), kMSmem);
     if (npm - 2 >= kPassColumns && poles_threads(npm - 2) <= kPassThreads && !wide) {
       const int pt = poles_threads(npm - 2);
-      for (int v = 0; v < 4; ++v) reserve((const void *)pass_kernel(v & 1, v & 2), pass_smem(pt));
+      for (int v = 0; v < 4; ++v) reserve((const void *)pass_kernel(v & 1, v & 2), pass_smem(kPassThreads));
       cudaLaunchConfig_t cfg = {};
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -3128,8 +3129,9 @@ static int adj_ensure(hipft_gpu *h) {
     for (int ns = 2; ns <= kMS; ns += 2) {
       CK(h, cudaFuncSetAttribute(adj_march_kernel(ns, h->plane >= (int64_t)1 << 29),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adj_march_smem(ns)));
-      CK(h, cudaFuncSetAttribute(adj_poles_kernel(ns, poles_threads(n2)), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)adj_poles_smem(ns, poles_threads(n2))));
+      const int pt = poles_threads(n2);
+      CK(h, cudaFuncSetAttribute(adj_poles_kernel(ns, pt), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)adj_poles_smem(ns, pt > kPMidThreads ? kPMaxThreads : kPMidThreads)));
     }
     TRY(dsmall(h, &h->d_jpart, (size_t)h->jpart_per_r * h->nr));
   }

@@ -39,3 +39,30 @@ def test_merged_pass_equals_two_launches():
             g.diffusion_step(2.0)
             out.append(g.get_field())
     assert all(np.array_equal(out[0][0], f) for f in out[1])
+
+
+def test_handles_of_different_widths_side_by_side():
+    """A kernel's shared-memory limit serves every handle: a narrower grid made
+    later leaves a wider one's passes and reverse passes as they were."""
+    import hipft_b200 as H
+    from hipft_b200.adjoint import MisfitAdjoint
+    nt, zero = 70, {k: np.zeros(1) for k in ("p0", "p2", "p4", "p1", "p3", "p5")}
+    kw = dict(advance_flow=True, flow_num_method=4, strang_splitting=True, advance_diffusion=True,
+              diffusion_num_method=3, diffusion_subcycles=1, diffusion_coef_constants=np.array([300.0]))
+    t = np.linspace(0.0, np.pi, nt)
+    x = np.random.default_rng(0).standard_normal((1, 1202, nt))
+    x[:, 0], x[:, -1] = x[:, -2], x[:, 1]
+
+    def gradient(g):
+        A = MisfitAdjoint(g, np.array([300.0]), zero)
+        F = A.forward(x, [0.02])
+        return F, A.backward(x)["f0"]
+
+    with H.HipftGPU(t, np.linspace(0.0, 2.0 * np.pi, 1201), 1, **kw) as wide:
+        wide.set_flow(dr_model=1, mf_model=1)
+        F0, g0 = gradient(wide)
+        with H.HipftGPU(t, np.linspace(0.0, 2.0 * np.pi, 641), 1, **kw) as g:
+            g.set_flow(dr_model=1, mf_model=1)
+            MisfitAdjoint(g, np.array([300.0]), zero).forward(x[:, :642], [0.02])
+            F1, g1 = gradient(wide)
+        assert np.array_equal(F0, F1) and np.array_equal(g0, g1)
