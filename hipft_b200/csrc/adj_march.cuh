@@ -189,10 +189,11 @@ __global__ void __launch_bounds__(32 * kJWarps, kJBlocks) k_adj_march(Mesh m, Ad
         const double2 d0 = s ? D[s > 0 ? s - 1 : 0] : lds2(sl + 3 * kF);
         un[s] = make_double2(u0.x + c.c0 * xc.x, u0.y + c.c0 * xc.y);
         dn_[s] = make_double2(d0.x + c.g * xc.x, d0.y + c.g * xc.y);
+        // selected, not multiplied by zero: past the chunk the ring may hold anything, a NaN too
         const int col = oc + NS - 1 - s;
-        const double ds = (col >= 0 && col < nown) ? c.ds : 0.0;
-        dsx[s / 2] += ds * (ax * yv.x);
-        dsy[s / 2] += ds * (ay * yv.y);
+        const bool in = col >= 0 && col < nown;
+        dsx[s / 2] += in ? c.ds * (ax * yv.x) : 0.0;
+        dsy[s / 2] += in ? c.ds * (ay * yv.y) : 0.0;
       }
     }
     if (n >= 2 * NS - 1) put(oc + 1 < nown, o0, wo + ldb, y[NS - 1]);
