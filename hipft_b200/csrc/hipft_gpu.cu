@@ -2796,11 +2796,18 @@ extern "C" int hipft_gpu_set_stream(hipft_gpu *h, void *s) {
   return HIPFT_OK;
 }
 
-extern "C" int hipft_gpu_check_bounded_wait(hipft_gpu *h, unsigned int limit) {
+extern "C" int hipft_gpu_expire_wait(hipft_gpu *h, unsigned int limit) {
   if (!h || limit == 0 || limit > (1u << 22)) return HIPFT_EINVAL;
   CK(h, cudaSetDevice(h->dev));
   k_wait_selftest<<<1, 32, 0, h->stream>>>(limit, h->d_err);
   LAUNCHED(h);
+  return HIPFT_OK;
+}
+
+extern "C" int hipft_gpu_check_bounded_wait(hipft_gpu *h, unsigned int limit) {
+  if (!h || limit == 0 || limit > (1u << 22)) return HIPFT_EINVAL;
+  CK(h, cudaSetDevice(h->dev));
+  TRY(hipft_gpu_expire_wait(h, limit));
   return check_wait_flag(h, "check_bounded_wait: the wait gave up as intended");
 }
 
@@ -3543,7 +3550,7 @@ extern "C" int hipft_adj_step(hipft_gpu *h, double dt, const double *f_in, doubl
   TRY(adj_reverse(h, fbar, dacc, gflow));
   CK(h, cudaStreamSynchronize(h->stream));
   CK(h, cudaGetLastError());
-  return HIPFT_OK;
+  return check_wait_flag(h, "adj_step: a bounded wait for ring sums gave up");
 }
 
 extern "C" int hipft_adj_record(hipft_gpu *h, double dt) {
@@ -3552,17 +3559,20 @@ extern "C" int hipft_adj_record(hipft_gpu *h, double dt) {
   CK(h, cudaSetDevice(h->dev));
   TRY(adj_record(h, dt));
   CK(h, cudaGetLastError());
-  return HIPFT_OK;
+  const int rc = check_wait_flag(h, "adj_record: a bounded wait for ring sums gave up");
+  if (rc != HIPFT_OK) {  // a step that is not right is not kept
+    h->adj_top = h->adj_recs.back().first;
+    h->adj_recs.pop_back();
+  }
+  return rc;
 }
 
 extern "C" int hipft_adj_reverse(hipft_gpu *h, double *fbar, double *dacc, double *gflow) {
   if (!h || !fbar || !dacc || !gflow) return HIPFT_EINVAL;
   CK(h, cudaSetDevice(h->dev));
-  TRY(adj_reverse(h, fbar, dacc, gflow));  // asynchronous on the handle's stream
+  TRY(adj_reverse(h, fbar, dacc, gflow));
   CK(h, cudaGetLastError());
-  // the last recorded step: the caller reads the gradient next
-  if (h->adj_recs.empty()) TRY(check_wait_flag(h, "adj_reverse: a bounded wait for ring sums gave up"));
-  return HIPFT_OK;
+  return check_wait_flag(h, "adj_reverse: a bounded wait for ring sums gave up");
 }
 
 extern "C" int hipft_adj_clear(hipft_gpu *h) {

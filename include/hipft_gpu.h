@@ -280,6 +280,9 @@ int hipft_gpu_field_device_ptr(hipft_gpu *h, double **ptr, int *ldt);
  * handle's error flag; the call then returns HIPFT_ETIMEOUT, as a stalled
  * copy would, and the handle stays usable. */
 int hipft_gpu_check_bounded_wait(hipft_gpu *h, unsigned int limit);
+/* The same wait without the report: the flag stays set for the next call that
+ * reads it, as after a kernel whose wait gave up. */
+int hipft_gpu_expire_wait(hipft_gpu *h, unsigned int limit);
 
 /* ---- ragged batches (no counterpart in the reference) ---------------------- */
 
@@ -405,7 +408,10 @@ int hipft_adj_step(hipft_gpu *h, double dt, const double *f_in, double *fbar, do
  * arguments as hipft_adj_step) and pops its tape.  A segment of n steps is
  * recorded in order and reversed in the opposite order; hipft_adj_recorded
  * gives the number of steps on the stack and (slots_used may be NULL) the
- * tape fields they hold. */
+ * tape fields they hold.
+ * All three return when their kernels have finished; HIPFT_ETIMEOUT means that
+ * a bounded wait of theirs gave up, so the field or the gradient is not right
+ * (hipft_adj_record then leaves the step off the stack). */
 int hipft_adj_record(hipft_gpu *h, double dt);
 int hipft_adj_reverse(hipft_gpu *h, double *fbar, double *dacc, double *gflow);
 int hipft_adj_recorded(hipft_gpu *h, int64_t *n, int64_t *slots_used);
