@@ -154,6 +154,7 @@ struct hipft_gpu {
   int jpart_per_r = 0;        // 0: the grid is not theirs
   int pass_clusters = 0;         // clusters of a merged pass that the GPU holds; 0: not on this grid
   int j_strips = 0, j_cols = 0;  // their theta strips and columns per warp
+  bool adj_ready = false;        // adj_ensure has succeeded
   // ragged batches: every realization keeps the schedule it would have if run
   // alone (Euler limit, CFL substeps, PTL subcycles, stage counts)
   bool ragged = false;
@@ -284,7 +285,10 @@ template <typename T>
 static int dalloc(hipft_gpu *h, T **p, size_t n) {
   size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
   cudaError_t e = cudaMalloc((void **)p, bytes);
-  if (e != cudaSuccess) return fail(h, HIPFT_ENOMEM, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // reported here: a later launch does not take it for its own
+    return fail(h, HIPFT_ENOMEM, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
+  }
   h->allocs.push_back((void *)*p);
   h->dev_bytes += bytes;
   return HIPFT_OK;
@@ -321,10 +325,13 @@ static int dsmall(hipft_gpu *h, T **p, size_t n) {
 }
 
 // Fields that live as long as the handle, several per allocation while they
-// are small (at most 256 MB each, as the tape's chunks).
+// are small (at most 256 MB each, as the tape's chunks); those that an earlier
+// call got before it ran out of memory are kept.
 static int dfields(hipft_gpu *h, double **f, int n) {
   const size_t per = std::max<size_t>(1, ((size_t)256 << 20) / (h->fieldn * sizeof(double)));
-  for (int b = 0; b < n;) {
+  int b = 0;
+  while (b < n && f[b]) ++b;
+  while (b < n) {
     const int c = (int)std::min<size_t>(per, (size_t)(n - b));
     double *q = nullptr;
     TRY(dalloc(h, &q, h->fieldn * c));
@@ -3115,16 +3122,19 @@ static int adj_pass(hipft_gpu *h, AdjPassArgs a, int ns, bool after_pass) {
   return HIPFT_OK;
 }
 
+// Work arrays of the reverse pass.  A call that failed may be repeated: it goes
+// on with what is missing, and nothing is ready before everything is there.
 static int adj_ensure(hipft_gpu *h) {
-  if (h->adjw[0]) return HIPFT_OK;
+  if (h->adj_ready) return HIPFT_OK;
+  auto small = [&](double **p, size_t n) { return *p ? HIPFT_OK : dsmall(h, p, n); };
   TRY(dfields(h, h->adjw, (int)(sizeof(h->adjw) / sizeof(h->adjw[0]))));
   dim3 g = stage_grid(h, 32, 8);
   h->dpart_per_r = (int)(g.x * g.y);
-  TRY(dsmall(h, &h->d_dpart, (size_t)h->dpart_per_r * h->nr));
+  TRY(small(&h->d_dpart, (size_t)h->dpart_per_r * h->nr));
   h->adj_nch = (h->npm - 2 + 255) / 256;
-  TRY(dsmall(h, &h->d_gring, 2 * (size_t)h->nr * h->adj_nch));
-  TRY(dsmall(h, &h->d_dpole, (size_t)h->nr * h->adj_nch));
-  for (auto &gp : h->d_gpart) TRY(dsmall(h, &gp, 2 * (size_t)g.y * h->nr));
+  TRY(small(&h->d_gring, 2 * (size_t)h->nr * h->adj_nch));
+  TRY(small(&h->d_dpole, (size_t)h->nr * h->adj_nch));
+  for (auto &gp : h->d_gpart) TRY(small(&gp, 2 * (size_t)g.y * h->nr));
   const int n2 = h->npm - 2;
   if (h->ntm >= kJMinRows && poles_by_column(h)) {
     h->j_strips = adj_strips(h->ntm);
@@ -3132,7 +3142,7 @@ static int adj_ensure(hipft_gpu *h) {
     // 512x1024 took a second wave and 34 us per pass instead of 20
     const int sms = std::max(h->num_sms - 2 * h->nr * poles_ranks(n2), h->num_sms / 2);
     h->j_cols = adj_cols(n2, h->j_strips, h->nr, kJWarps * kJBlocks * sms);
-    h->jpart_per_r = h->j_strips * ((n2 + h->j_cols - 1) / h->j_cols) + 2 * poles_ranks(n2);
+    const int per_r = h->j_strips * ((n2 + h->j_cols - 1) / h->j_cols) + 2 * poles_ranks(n2);
     for (int ns = 2; ns <= kMS; ns += 2) {
       CK(h, cudaFuncSetAttribute(adj_march_kernel(ns, h->plane >= (int64_t)1 << 29),
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adj_march_smem(ns)));
@@ -3140,8 +3150,10 @@ static int adj_ensure(hipft_gpu *h) {
       CK(h, cudaFuncSetAttribute(adj_poles_kernel(ns, pt), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)adj_poles_smem(ns, pt > kPMidThreads ? kPMaxThreads : kPMidThreads)));
     }
-    TRY(dsmall(h, &h->d_jpart, (size_t)h->jpart_per_r * h->nr));
+    TRY(small(&h->d_jpart, (size_t)per_r * h->nr));
+    h->jpart_per_r = per_r;
   }
+  h->adj_ready = true;
   return HIPFT_OK;
 }
 
@@ -3523,7 +3535,7 @@ static int adj_record(hipft_gpu *h, double dt) {
 
 // Reverse of the most recently recorded step (popped from the stack).
 static int adj_reverse(hipft_gpu *h, double *fbar, double *dacc, double *gflow) {
-  if (h->adj_recs.empty()) return fail(h, HIPFT_ESTATE, "adjoint reverse: no recorded step");
+  if (h->adj_recs.empty() || !h->adj_ready) return fail(h, HIPFT_ESTATE, "adjoint reverse: no recorded step");
   const AdjRec &R = h->adj_recs.back();
   const size_t bytes = h->fieldn * sizeof(double);
   const bool strang = h->P.strang_splitting != 0;
