@@ -283,12 +283,12 @@ __global__ void k_g_coefs(GArrays g) {
   for (int q = 0; q < kMS; ++q) g.rc[idx * kMS + q] = sts_slot(g.method, s, (int64_t)kMS * p + q, g.d[i]);
 }
 
-// End of a pass-loop iteration (one thread; pass_kernels: kernels of a pass).
+// End of a pass-loop iteration (one thread; pass_kernels: kernels of its passes).
 __global__ void k_g_pass_tick(GArrays g, int pass_kernels, cudaGraphConditionalHandle hc) {
   GState &st = *g.st;
   const int p = st.pctr + g.unroll;
   st.pctr = p;
-  st.kernels += pass_kernels * g.unroll + 1;
+  st.kernels += pass_kernels + 1;
   // npasses fits the tables (k_g_plan), so the loop ends within passcap / unroll iterations
   cudaGraphSetConditional(hc, p < st.npasses ? 1u : 0u);
 }

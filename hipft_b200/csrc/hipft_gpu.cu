@@ -527,12 +527,16 @@ static MarchArgs march_args(const hipft_gpu *h, const double *u0, const double *
   return a;
 }
 
-// A column per thread in k_sts_poles, or k_sts_poles_any.
-static bool poles_by_column(const hipft_gpu *h) { return poles_threads(h->npm - 2) <= kPMaxThreads; }
+// The pole strips in one launch, a column per thread (k_sts_poles), or stage by
+// stage (k_sts_poles_any, and k_sts_whole on a low grid).
+static bool poles_by_column(const hipft_gpu *h) {
+  return h->ntm >= kMMinRows && poles_threads(h->npm - 2) <= kPMaxThreads;
+}
 
 // Places of k_sts_march's blocks that one realization's strips take: a block of
-// the widest takes an SM.
+// the widest takes an SM; none where the strips' launches are over by then.
 static int pole_places(int n2) {
+  if (poles_threads(n2) > kPMaxThreads) return 0;
   return 2 * poles_ranks(n2) * (poles_threads(n2) > kPMidThreads ? kMBlocks : 1);
 }
 
@@ -574,6 +578,19 @@ static int pass_columns(const hipft_gpu *h, const MarchArgs &a) {
   return c <= kPassColsMax ? (int)c : 0;
 }
 
+// k_sts_march of a pass, on the stream of cfg behind the strips' launches.
+static cudaError_t launch_march(const hipft_gpu *h, cudaLaunchConfig_t cfg, cudaLaunchAttribute *attr,
+                                const MarchArgs &a, int64_t blocks, bool pdl) {
+  attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3(32 * kMWarps);
+  cfg.dynamicSmemBytes = kMSmem;
+  const bool table = a.rc || a.cols > kMGroup;
+  return cudaLaunchKernelEx(&cfg, march_kernel(table, a.o[0] || a.o[1], h->plane >= (int64_t)1 << 29), h->M, a,
+                            h->ptab);
+}
+
 // One pass on stream s.  after_pass: the launch before it on the stream is
 // the previous pass, whose end it waits for on the device, so it may be
 // launched programmatically.  blocks: k_sts_march's grid (0: for a.nreal
@@ -590,14 +607,29 @@ static cudaError_t launch_pass(const hipft_gpu *h, cudaStream_t s, MarchArgs a, 
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (h->ntm < kMMinRows) {
-    attr[0].val.programmaticStreamSerializationAllowed = 0;
-    cfg.gridDim = dim3((unsigned)a.nreal);
-    cfg.blockDim = dim3(256);
-    return cudaLaunchKernelEx(&cfg, k_sts_whole, h->M, a, h->ptab);
-  }
   const int n2 = h->npm - 2, nc = poles_ranks(n2);
-  const bool bycol = poles_by_column(h);
+  if (!poles_by_column(h)) {
+    const bool low = h->ntm < kMMinRows;
+    cfg.gridDim = dim3((unsigned)poles_any_blocks(n2), low ? 1 : 2, (unsigned)a.nreal);
+    cfg.blockDim = dim3(kPAThreads);
+    const int s0 = after_pass ? 0 : -1;
+    int step = 1;
+    if (cfg.gridDim.x <= kPACluster) {
+      step = kMS - s0;
+      attr[1].id = cudaLaunchAttributeClusterDimension;
+      attr[1].val.clusterDim.x = cfg.gridDim.x;
+      attr[1].val.clusterDim.y = 1;
+      attr[1].val.clusterDim.z = 1;
+      cfg.numAttrs = cfg.gridDim.x > 1 ? 2 : 1;
+    }
+    for (int st = s0; st < kMS; st += step) {
+      attr[0].val.programmaticStreamSerializationAllowed = (pdl && (after_pass || st > s0)) ? 1 : 0;
+      const cudaError_t e = cudaLaunchKernelEx(&cfg, low ? k_sts_whole : k_sts_poles_any, h->M, a, h->ptab,
+                                               h->d_pscratch, st, st + step);
+      if (e != cudaSuccess) return e;
+    }
+    return low ? cudaSuccess : launch_march(h, cfg, attr, a, blocks, pdl);
+  }
   attr[0].val.programmaticStreamSerializationAllowed = (pdl && after_pass) ? 1 : 0;
   if (const int pc = pass_columns(h, a)) {
     a.cols = pc;
@@ -618,32 +650,29 @@ static cudaError_t launch_pass(const hipft_gpu *h, cudaStream_t s, MarchArgs a, 
   attr[1].val.clusterDim.z = 1;
   cfg.numAttrs = 2;
   cfg.gridDim = dim3((unsigned)(2 * a.nreal * nc));
-  cfg.blockDim = dim3((unsigned)(bycol ? poles_threads(n2) : kPAThreads));
-  cfg.dynamicSmemBytes = bycol ? poles_smem(poles_threads(n2)) : 0;
+  cfg.blockDim = dim3((unsigned)poles_threads(n2));
+  cfg.dynamicSmemBytes = poles_smem(poles_threads(n2));
   // a march that leaves places free does not compete with the pole strips' registers
   const bool roomy = blocks + 3 * (int64_t)cfg.gridDim.x <= (int64_t)kMBlocks * h->num_sms;
   auto poles = poles_threads(n2) > kPMidThreads    ? k_sts_poles<kPMaxThreads, 1>
                : poles_threads(n2) <= kPMinThreads ? k_sts_poles<kPMinThreads, 3>
                : roomy                             ? k_sts_poles<kPMidThreads, 1>
                                                    : k_sts_poles<kPMidThreads, 3>;
-  cudaError_t e = bycol ? cudaLaunchKernelEx(&cfg, poles, h->M, a, h->ptab)
-                        : cudaLaunchKernelEx(&cfg, k_sts_poles_any, h->M, a, h->ptab, h->d_pscratch);
-  if (e != cudaSuccess) return e;
-  attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
-  cfg.numAttrs = 1;
-  cfg.gridDim = dim3((unsigned)blocks);
-  cfg.blockDim = dim3(32 * kMWarps);
-  cfg.dynamicSmemBytes = kMSmem;
-  const bool table = a.rc || a.cols > kMGroup;
-  return cudaLaunchKernelEx(&cfg, march_kernel(table, a.o[0] || a.o[1], h->plane >= (int64_t)1 << 29), h->M, a,
-                            h->ptab);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, poles, h->M, a, h->ptab);
+  return e == cudaSuccess ? launch_march(h, cfg, attr, a, blocks, pdl) : e;
+}
+
+static int pass_launches(const hipft_gpu *h, const MarchArgs &a, bool after_pass) {
+  if (poles_by_column(h)) return pass_columns(h, a) ? 1 : 2;
+  const int strips = poles_any_blocks(h->npm - 2) <= kPACluster ? 1 : kMS + (after_pass ? 0 : 1);
+  return strips + (h->ntm < kMMinRows ? 0 : 1);
 }
 
 static int sts_pass(hipft_gpu *h, const MarchArgs &a, bool after_pass) {
   ProfScope ps(h, HIPFT_K_STS);
   const cudaError_t e = launch_pass(h, h->stream, a, ws_pdl(), after_pass);
   if (e != cudaSuccess) return fail(h, HIPFT_ECUDA, "RKG2 pass launch: %s", cudaGetErrorString(e));
-  h->launches += h->ntm < kMMinRows || pass_columns(h, a) ? 1 : 2;
+  h->launches += pass_launches(h, a, after_pass);
   return HIPFT_OK;
 }
 
@@ -881,7 +910,9 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
       if (!smem_ok || cudaOccupancyMaxActiveClusters(&h->pass_clusters, pass_kernel(true, true), &cfg) != cudaSuccess)
         h->pass_clusters = 0;
     }
-    if (poles_threads(npm - 2) > kPMidThreads) {
+    if (!poles_by_column(h)) {
+      // no dynamic shared memory
+    } else if (poles_threads(npm - 2) > kPMidThreads) {
       reserve((const void *)k_sts_poles<kPMaxThreads, 1>, poles_smem(kPMaxThreads));
     } else if (poles_threads(npm - 2) <= kPMinThreads) {
       reserve((const void *)k_sts_poles<kPMinThreads, 3>, poles_smem(kPMinThreads));
@@ -921,7 +952,7 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
     h->m_strips = std::max(1, (ntm - 2 * kMS + kMOwn - 1) / kMOwn);
     h->m_slots = kMBlocks * kMWarps * h->num_sms;
     if (!poles_by_column(h) &&
-        (rc = dalloc(h, &h->d_pscratch, (size_t)2 * nr * poles_ranks(npm - 2) * kPADoubles * poles_any_width(npm - 2))))
+        (rc = dalloc(h, &h->d_pscratch, (size_t)nr * poles_any_doubles(npm - 2))))
       return bail(rc);
     double *tab = nullptr;
     const size_t nrow = (size_t)nr * pt.LR * 3, ncol = (size_t)nr * pt.LC * 2;
@@ -2240,8 +2271,14 @@ static int graph_capture(hipft_gpu *h) {
     ++body_kernels;
     begin_body(s1, hpass, s2);
     if (first != cudaSuccess) return;
-    for (int q = 0; q < g.unroll; ++q) pass(s2, q, q > 0);
-    k_g_pass_tick<<<1, 1, 0, s2>>>(g, h->ntm < kMMinRows ? 1 : 2, hpass);
+    int pass_kernels = 0;
+    for (int q = 0; q < g.unroll; ++q) {
+      pass(s2, q, q > 0);
+      MarchArgs a{};
+      a.dctr = &g.st->pctr;
+      pass_kernels += pass_launches(h, a, q > 0);
+    }
+    k_g_pass_tick<<<1, 1, 0, s2>>>(g, pass_kernels, hpass);
     peek();
     end_body(s2);
     // the result of each realization back into the field: Y_s is in R1 after

@@ -681,161 +681,161 @@ __host__ __device__ inline size_t pass_smem(int threads) {
   const size_t march = ((size_t)(threads / 32) * (kMRing + kMTab) + kMCoef) * sizeof(double);
   return march > poles_smem(threads) ? march : poles_smem(threads);
 }
-// The same strips when a column per thread does not suffice (more than about
-// 4200 phi columns): the blocks loop over their columns and keep the strip in
-// a scratch area in global memory, in place: stage k over Y_{k-2}, stage k+1
-// over Y_{k-1}, and so on.
-constexpr int kPAThreads = 256;
-constexpr int kPADoubles = kPRows + (kPRows - 1);  // doubles per column
-__host__ __device__ inline int poles_any_width(int n2) { return (n2 + 7) / 8 + 2 * kMS; }
+// The same strips where a column per thread does not suffice (more than about
+// 4200 phi columns: k_sts_poles_any), and all rows of a grid with fewer than
+// kMMinRows (k_sts_whole): one launch per stage, a cell per thread, eight lanes
+// per column.  Every block adds up the ring sums that the launch before it left
+// as a partial per block; s = -1 leaves those of the pass's input, which is not
+// needed after a pass (its last stage left them).  A launch runs the stages s0
+// to s1-1, more than one where a cluster has all columns.  Stage outputs stay in a
+// scratch area, [column][8] twice: the third and fourth stage work in place.
+// Bound by launches and latency, some 4 us per stage whatever the width.  (One
+// cluster per pole took 112 us per pass at 64x8192, 65 with its strip in shared
+// memory, and one block for a whole low grid 345 at 7x4096; now 31 and 20.)
+constexpr int kPACols = 64;                          // columns per block
+constexpr int kPACluster = 8;                        // most blocks of a cluster
+constexpr int kPAThreads = kPRows * kPACols;
+__host__ __device__ inline int poles_any_blocks(int n2) { return (n2 + kPACols - 1) / kPACols; }
+// doubles per realization: two poles' strips, twice, and two sets of partials
+__host__ __device__ inline int64_t poles_any_strips(int n2) { return (int64_t)4 * kPRows * n2; }
+__host__ __device__ inline int64_t poles_any_doubles(int n2) { return poles_any_strips(n2) + 4 * poles_any_blocks(n2); }
 
-__global__ void __launch_bounds__(kPAThreads) k_sts_poles_any(Mesh m, MarchArgs a, PairTables pt, double *scratch) {
-  const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-  __shared__ double s_sum[kMS][8 * (kPAThreads / 32)];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = kPAThreads / 32;
-  const int npm = m.npm, n2 = npm - 2, ntm = m.ntm;
-  const int nc = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-  const int unit = blockIdx.x / nc;
-  const bool south = (unit & 1) != 0;
-  pdl_wait();
-  pdl_trigger();
+// Sum of v over the block, in a fixed order, for all its threads.
+__device__ __forceinline__ double strip_sum(double v, double *sh) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) sh[warp] = v;
+  __syncthreads();
+  v = lane < kPAThreads / 32 ? sh[lane] : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+template <bool WHOLE>
+__device__ __forceinline__ void poles_any_body(const Mesh &m, const MarchArgs &a, const PairTables &pt,
+                                               double *scratch, int s0, int s1) {
+  constexpr int NS = WHOLE ? 2 : 1;
+  __shared__ double sh[2 * NS][kPAThreads / 32];
+  const int tid = threadIdx.x, npm = m.npm, n2 = npm - 2, ntm = m.ntm, nb = gridDim.x;
+  const bool south = !WHOLE && blockIdx.y == 1;
   int nreal;
   bool first;
   const StageCoef *rc;
   int cols;
   march_launch(a, nreal, first, rc, cols);
-  if ((unit >> 1) >= nreal) return;
-  cluster_arrive();
-  const int i = a.rlist ? a.rlist[unit >> 1] : (unit >> 1);
-  const int W = poles_any_width(n2), own = W - 2 * kMS;
-  const int kb = 2 + rank * own, nown = max(0, min(own, npm - kb));
-  const int w = nown + 2 * kMS;
-  double *X = scratch + (int64_t)blockIdx.x * kPADoubles * W, *Y = X + (int64_t)kPRows * W;
-  const int64_t ld = m.ldt, pb = (int64_t)i * m.plane;
-  auto wrap = [&](int c) {
-    while (c < 2) c += n2;
-    while (c > npm - 1) c -= n2;
-    return c;
-  };
-  auto at = [&](int c, int q) { return pb + (int64_t)(wrap(kb - kMS + c) - 1) * ld + (south ? ntm - 1 - q : q); };
-  const double *x1 = first ? a.u : a.x1, *x2 = first ? a.u : a.x2;
-  for (int c = tid; c < w; c += kPAThreads)
-    for (int q = 0; q < kPRows; ++q) {
-      X[(int64_t)q * W + c] = x1[at(c, q)];
-      if (q < kPRows - 1) Y[(int64_t)q * W + c] = x2[at(c, q)];
-    }
+  if ((int)blockIdx.z >= nreal) {
+    pdl_wait();
+    pdl_trigger();
+    return;
+  }
+  const int i = a.rlist ? a.rlist[blockIdx.z] : (int)blockIdx.z;
+  // this thread's cell: strip row q = 0..7 is theta row q+1, or ntm-q at the south pole
+  const int q = tid & (kPRows - 1), k = 2 + (int)blockIdx.x * kPACols + (tid >> 3);
+  const bool live = k <= npm - 1 && q < (WHOLE ? ntm : kPRows);
+  const int row = south ? ntm - 1 - q : q, dir = south ? -1 : 1;
+  const int kl = k == 2 ? npm - 1 : k - 1, kr = k == npm - 1 ? 2 : k + 1;
+  const int64_t pb = (int64_t)i * m.plane + row;
+  auto at = [&](int c) { return pb + (int64_t)(c - 1) * m.ldt; };
+  double st = 0.0, c2 = 0.0, c4 = 0.0, u = 0.0, d = 0.0, dp = 0.0;
+  double2 P = {};
   const double Dr = a.dfac[i + 1];
-  const double *R = pt.row + (int64_t)i * 3 * pt.LR;
-  __syncthreads();
-  cluster_wait();
-  double *In = X, *Out = Y;  // stage input, and second input = output
+  if (k <= npm - 1) dp = m.dp[k];
+  if (live) {
+    const double *R = pt.row + (int64_t)i * 3 * pt.LR + row + 2;
+    st = R[0];
+    c2 = R[pt.LR];
+    c4 = R[2 * pt.LR];
+    P = reinterpret_cast<const double2 *>(pt.col)[(int64_t)i * pt.LC + k];
+    u = a.u[at(k)];
+    d = a.d[at(k)];
+  }
+  const int pole = south ? 1 : 0;
+  double *A = scratch + (int64_t)i * poles_any_doubles(n2) + (int64_t)pole * 2 * kPRows * n2, *B = A + (int64_t)kPRows * n2;
+  double *part = scratch + (int64_t)i * poles_any_doubles(n2) + poles_any_strips(n2);
+  auto parts = [&](int p, int stage) { return part + (int64_t)(2 * p + (stage & 1)) * nb; };
+  const double *x1 = first ? a.u : a.x1, *x2 = first ? a.u : a.x2;
+  // everything below reads what the launch before this one wrote; the march,
+  // which is launched after the last stage, reads and writes other rows
+  pdl_wait();
+  pdl_trigger();
 #pragma unroll 1
-  for (int s = 0; s < kMS; ++s) {
-    const StageCoef sc = rc ? rc[(int64_t)i * kMS + s] : a.c[s];
-    double v = 0.0;
-    for (int c = kMS + tid; c < kMS + nown; c += kPAThreads) {
-      const double t = south ? In[c] - In[W + c] : In[W + c] - In[c];
-      v = v + (Dr + Dr) * t * m.dp[kb - kMS + c];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane < nc) *cl.map_shared_rank(&s_sum[s][rank * nw + warp], lane) = v;
-    __syncwarp();
-    cluster_arrive();
-    __syncwarp();
-    cluster_wait();
-    double ring = 0.0;
-    for (int q = lane; q < nc * nw; q += 32) ring = ring + s_sum[s][q];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ring += __shfl_xor_sync(0xffffffffu, ring, o);
-    const double axp = south ? -ring * a.bcs : ring * a.bcn;
-    double *o = a.o[s];
-    for (int c = s + 1 + tid; c <= w - 2 - s; c += kPAThreads) {
-      const double2 P = reinterpret_cast<const double2 *>(pt.col)[(int64_t)i * pt.LC + wrap(kb - kMS + c)];
-      for (int q = 0; q < kPRows - 1 - s; ++q) {
-        const int64_t e = (int64_t)q * W + c;
-        const int j = south ? ntm - q : q + 1;
-        double ax = axp;
-        if (q > 0) {
-          const double st = R[j + 1], c2 = R[pt.LR + j + 1], c4 = R[2 * pt.LR + j + 1];
-          const double c1 = P.x * st * st;
-          const double c5 = P.y * st * st;
-          const double c3 = -(c1 + c2 + c4 + c5);
-          const double up = In[e + (south ? W : -W)], dn = In[e + (south ? -W : W)];
-          ax = c1 * In[e - 1] + c2 * up + c3 * In[e] + c4 * dn + c5 * In[e + 1];
-        }
-        const int64_t g = at(c, q);
-        const double y = sc.a * In[e] + sc.b * Out[e] + sc.c * a.u[g] + sc.d * ax + sc.e * a.d[g];
-        Out[e] = y;
-        if (o && q < kMS && c >= kMS && c < kMS + nown) o[g] = y;
+  for (int s = s0; s < s1; ++s) {
+    if (s > s0) {
+      if (nb == 1) {
+        __syncthreads();
+      } else {
+        cluster_arrive();
+        cluster_wait();
       }
     }
-    __syncthreads();
-    double *t = In;
-    In = Out;
-    Out = t;
+    const bool inner = live && q >= 1 && q <= (WHOLE ? ntm - 2 : kPRows - 2 - s);
+    const bool act = inner || (live && (q == 0 || (WHOLE && q == ntm - 1)));
+    double y = 0.0;
+    if (s < 0) {
+      if (live) y = x1[at(k)];
+    } else {
+      const StageCoef sc = rc ? rc[(int64_t)i * kMS + s] : a.c[s];
+      const int64_t e = (int64_t)(k - 2) * kPRows + q;
+      double xc = 0.0, xl = 0.0, xr = 0.0, up = 0.0, dn = 0.0, z = 0.0;
+      if (act) {
+        const double *in = s == 0 ? x1 + at(k) : (s == 2 ? B : A) + e;
+        const int64_t cs = s == 0 ? m.ldt : kPRows;
+        const int rs = s == 0 ? dir : 1;  // to the next strip row
+        xc = in[0];
+        z = s == 0 ? x2[at(k)] : s == 1 ? x1[at(k)] : (s == 2 ? A : B)[e];
+        if (inner) {
+          xl = in[(kl - k) * cs];
+          xr = in[(kr - k) * cs];
+          up = in[south ? rs : -rs];
+          dn = in[south ? -rs : rs];
+        }
+      }
+      double rn = 0.0, rsum = 0.0;
+#pragma unroll 4
+      for (int b = tid; b < nb; b += kPAThreads) {
+        rn = rn + parts(pole, s)[b];
+        if (WHOLE) rsum = rsum + parts(1, s)[b];
+      }
+      rn = strip_sum(rn, sh[0]);
+      if (WHOLE) rsum = strip_sum(rsum, sh[1]);
+      double ax;
+      if (inner) {
+        const double c1 = P.x * st * st;
+        const double c5 = P.y * st * st;
+        const double c3 = -(c1 + c2 + c4 + c5);
+        ax = c1 * xl + c2 * up + c3 * xc + c4 * dn + c5 * xr;
+      } else if (WHOLE) {
+        ax = q == 0 ? rn * a.bcn : -rsum * a.bcs;
+      } else {
+        ax = south ? -rn * a.bcs : rn * a.bcn;
+      }
+      y = sc.a * xc + sc.b * z + sc.c * u + sc.d * ax + sc.e * d;
+      if (act) {
+        if (s < kMS - 1) (s == 1 ? B : A)[e] = y;
+        double *o = a.o[s];
+        if (o && (WHOLE || q < kMS)) o[at(k)] = y;
+      }
+    }
+    // this block's share of the next stage's ring sums
+    const double dn = __shfl_down_sync(0xffffffffu, y, 1), up = __shfl_up_sync(0xffffffffu, y, 1);
+    const double vn = strip_sum(live && q == 0 ? (Dr + Dr) * (south ? y - dn : dn - y) * dp : 0.0, sh[NS]);
+    if (tid == 0) parts(pole, s + 1)[blockIdx.x] = vn;
+    if (WHOLE) {
+      const double vs = strip_sum(live && q == ntm - 1 ? (Dr + Dr) * (y - up) * dp : 0.0, sh[2 * NS - 1]);
+      if (tid == 0) parts(1, s + 1)[blockIdx.x] = vs;
+    }
   }
 }
 
-// The whole pass of a grid with fewer than kMMinRows theta rows: one block
-// per realization, stage by stage in global memory (a stage writes over the
-// output of the stage two before it where that one is not kept).
-__global__ void __launch_bounds__(256) k_sts_whole(Mesh m, MarchArgs a, PairTables pt) {
-  __shared__ double sh[64];
-  __shared__ double s_ring[2];
-  pdl_wait();
-  pdl_trigger();
-  int nreal;
-  bool first;
-  const StageCoef *rc;
-  int cols;
-  march_launch(a, nreal, first, rc, cols);
-  if ((int)blockIdx.x >= nreal) return;
-  const int i = a.rlist ? a.rlist[blockIdx.x] : (int)blockIdx.x;
-  const int npm = m.npm, n2 = npm - 2, ntm = m.ntm;
-  const int64_t ld = m.ldt, pb = (int64_t)i * m.plane;
-  const double Dr = a.dfac[i + 1];
-  const double *R = pt.row + (int64_t)i * 3 * pt.LR;
-  const double2 *P = reinterpret_cast<const double2 *>(pt.col) + (int64_t)i * pt.LC;
-  const double *in = (first ? a.u : a.x1) + pb, *in2 = (first ? a.u : a.x2) + pb;
-  const double *u = a.u + pb, *d = a.d + pb;
-  for (int s = 0; s < kMS; ++s) {
-    const StageCoef sc = rc ? rc[(int64_t)i * kMS + s] : a.c[s];
-    double *out = (a.o[s] ? a.o[s] : a.o[s | 2]) + pb;
-    double fn = 0.0, fs = 0.0;
-    for (int k = 2 + threadIdx.x; k <= npm - 1; k += blockDim.x) {
-      const double *x = in + (int64_t)(k - 1) * ld;
-      fn = fn + (Dr + Dr) * (x[1] - x[0]) * m.dp[k];
-      fs = fs + (Dr + Dr) * (x[ntm - 1] - x[ntm - 2]) * m.dp[k];
-    }
-    block_sum2(fn, fs, sh);
-    if (threadIdx.x == 0) {
-      s_ring[0] = fn * a.bcn;
-      s_ring[1] = -fs * a.bcs;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < n2 * ntm; e += blockDim.x) {
-      const int k = 2 + e / ntm, j = 1 + e % ntm;
-      const int64_t g = (int64_t)(k - 1) * ld + (j - 1);
-      double ax;
-      if (j == 1 || j == ntm) {
-        ax = s_ring[j == 1 ? 0 : 1];
-      } else {
-        const int kl = k == 2 ? npm - 1 : k - 1, kr = k == npm - 1 ? 2 : k + 1;
-        const double st = R[j + 1], c2 = R[pt.LR + j + 1], c4 = R[2 * pt.LR + j + 1];
-        const double c1 = P[k].x * st * st;
-        const double c5 = P[k].y * st * st;
-        const double c3 = -(c1 + c2 + c4 + c5);
-        ax = c1 * in[(int64_t)(kl - 1) * ld + j - 1] + c2 * in[g - 1] + c3 * in[g] + c4 * in[g + 1] +
-             c5 * in[(int64_t)(kr - 1) * ld + j - 1];
-      }
-      const double y = sc.a * in[g] + sc.b * in2[g] + sc.c * u[g] + sc.d * ax + sc.e * d[g];
-      out[g] = y;
-    }
-    __syncthreads();
-    in2 = in;
-    in = out;
-  }
+__global__ void __launch_bounds__(kPAThreads)
+    k_sts_poles_any(Mesh m, MarchArgs a, PairTables pt, double *scratch, int s0, int s1) {
+  poles_any_body<false>(m, a, pt, scratch, s0, s1);
+}
+__global__ void __launch_bounds__(kPAThreads)
+    k_sts_whole(Mesh m, MarchArgs a, PairTables pt, double *scratch, int s0, int s1) {
+  poles_any_body<true>(m, a, pt, scratch, s0, s1);
 }
 
 // d = scale * af, the first stage's dty0 (src/hipft.f90:5211) from A u0: one
