@@ -109,63 +109,75 @@ struct AdvArgs {
   const double *rdt;
   int strips, cols;       // theta strips, phi columns per warp
   double bcn, bcs;        // pole factors
+  int poles;              // blocks per pole row (adv_pole_blocks)
 };
 
 // The pole rows 1 and ntm of a realization's stage, whose value needs the ring
 // sum of the upwind fluxes next to them over all phi columns (src/hipft.f90:
-// 7902-7915): one block.  The sums are those of 256 threads (two per thread
-// here) and a tree over them.
-__device__ __forceinline__ void adv_pole_rows(const Mesh &m, const Flow &fl, const AdvArgs &a, int i0, double *sh) {
+// 7902-7915): `nb` blocks per pole, each of which adds up the whole ring, as 256
+// threads (two per thread here) and a tree over them do, and writes its share of
+// the row.  Bound by latency and, on wide grids, by the sectors one SM can take
+// in: one block for both poles, a column's loads behind the store of the one
+// before, held a stage of 64x8192 up for 63 us (now 36) and of 16x2048 for 19 (now
+// 10).  A block per kAPole columns is where the share's time and the
+// sum's meet.  Large batches, whose marches fill the GPU, have one block per pole
+// (16x2048 x 32: 395 us with two, 380 with one).
+constexpr int kAPole = 1024;
+inline int adv_pole_blocks(int n2, int nreal) {  // per pole
+  return std::min((n2 + kAPole - 1) / kAPole, std::max(1, kDPoleMax / nreal));
+}
+__device__ __forceinline__ void adv_pole_row(const Mesh &m, const Flow &fl, const AdvArgs &a, int i0, bool south,
+                                             int block, int nb, double *sh) {
   const int i = i0 + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t ld = m.ldt;
-  const double *x = a.x + (int64_t)i0 * m.plane, *f0 = a.f0 + (int64_t)i0 * m.plane;
-  double *out = a.out + (int64_t)i0 * m.plane;
+  const int64_t ld = m.ldt, p0 = (int64_t)i0 * m.plane + (south ? m.ntm - 1 : 0);
+  const int jv = south ? m.nt - 1 : 2;
 #pragma unroll
   for (int v = 0; v < 2; ++v) {
-    double fn = 0.0, fs = 0.0;
-#pragma unroll 4
+    double f = 0.0;
+    const double *c = a.x + p0;
+#pragma unroll 8
     for (int k = 2 + (int)threadIdx.x + 128 * v; k <= m.npm - 1; k += 256) {
-      const double *c = x + (int64_t)(k - 1) * ld;
-      const double ftn = upwind_flux(vt_at(m, fl, 2, k, i), fl.upwind, c[1], c[0]);
-      const double fts = upwind_flux(vt_at(m, fl, m.nt - 1, k, i), fl.upwind, c[m.ntm - 1], c[m.ntm - 2]);
-      fn = fn + ftn * m.dp[k];
-      fs = fs + fts * m.dp[k];
+      const double xp = c[(int64_t)(k - 1) * ld], xn = c[(int64_t)(k - 1) * ld + (south ? -1 : 1)];
+      const double ft = upwind_flux(vt_at(m, fl, jv, k, i), fl.upwind, south ? xp : xn, south ? xn : xp);
+      f = f + ft * m.dp[k];
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      fn += __shfl_down_sync(0xffffffffu, fn, o);
-      fs += __shfl_down_sync(0xffffffffu, fs, o);
-    }
-    if (lane == 0) {
-      sh[2 * (4 * v + warp)] = fn;
-      sh[2 * (4 * v + warp) + 1] = fs;
-    }
+    for (int o = 16; o > 0; o >>= 1) f += __shfl_down_sync(0xffffffffu, f, o);
+    if (lane == 0) sh[4 * v + warp] = f;
   }
   __syncthreads();
-  double fn = lane < 8 ? sh[2 * lane] : 0.0, fs = lane < 8 ? sh[2 * lane + 1] : 0.0;
+  double f = lane < 8 ? sh[lane] : 0.0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    fn += __shfl_down_sync(0xffffffffu, fn, o);
-    fs += __shfl_down_sync(0xffffffffu, fs, o);
-  }
-  const double an = __shfl_sync(0xffffffffu, fn, 0) * a.bcn, as = -__shfl_sync(0xffffffffu, fs, 0) * a.bcs;
+  for (int o = 16; o > 0; o >>= 1) f += __shfl_down_sync(0xffffffffu, f, o);
+  f = __shfl_sync(0xffffffffu, f, 0);
+  const double ax = south ? -f * a.bcs : f * a.bcn;
   const double C = a.rdt ? a.cb.C * a.rdt[i0] : a.cb.C;
-#pragma unroll 4
-  for (int k = 2 + (int)threadIdx.x; k <= m.npm - 1; k += 128) {
-    const int64_t q = (int64_t)(k - 1) * ld, sm = k == 2 ? (m.npm - 2) * ld : k == m.npm - 1 ? -(m.npm - 2) * ld : 0;
+  const int per = (m.npm - 2 + nb - 1) / nb, k1 = min(1 + per * (block + 1), m.npm - 1);
+  constexpr int G = 8;  // columns per turn, their loads all under way at once
+  for (int k0 = 2 + per * block + (int)threadIdx.x; k0 <= k1; k0 += 128 * G) {
+    double xv[G], fv[G];
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int64_t p = q + (s ? m.ntm - 1 : 0);
-      const double ax = s ? as : an;
-      const double y = a.cb.mode == 0 ? x[p] - C * ax : a.cb.A * f0[p] + a.cb.B * x[p] - C * ax;
-      out[p] = y;
-      if (sm) out[p + sm] = y;
+    for (int g = 0; g < G; ++g) {
+      if (k0 + 128 * g > k1) break;
+      const int64_t p = p0 + (int64_t)(k0 + 128 * g - 1) * ld;
+      xv[g] = a.x[p];
+      fv[g] = a.cb.mode == 0 ? 0.0 : a.f0[p];
+    }
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const int k = k0 + 128 * g;
+      if (k > k1) break;
+      const int64_t p = p0 + (int64_t)(k - 1) * ld;
+      const int64_t sm = k == 2 ? (m.npm - 2) * ld : k == m.npm - 1 ? -(m.npm - 2) * ld : 0;
+      const double y = a.cb.mode == 0 ? xv[g] - C * ax : a.cb.A * fv[g] + a.cb.B * xv[g] - C * ax;
+      a.out[p] = y;
+      if (sm) a.out[p + sm] = y;
     }
   }
 }
 
-// One stage; block 0 of a realization takes the pole rows, the others the rows
-// 2..ntm-1.  A warp holds 64 theta rows, two per lane, and
+// One stage; the first blocks of a realization take the pole rows, the others the
+// rows 2..ntm-1.  A warp holds 64 theta rows, two per lane, and
 // marches along the phi columns of its chunk: at the step that brings in
 // column e it computes the phi faces e-1 of its rows and, for the cells of
 // column k = e-2, the theta faces between its rows and above them: every face
@@ -194,12 +206,12 @@ __global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Fl
     pdl_wait();
     return;
   }
-  if (blockIdx.x == 0) {
+  if ((int)blockIdx.x < 2 * a.poles) {
     pdl_wait();
-    adv_pole_rows(m, fl, a, i, asm_);
+    adv_pole_row(m, fl, a, i, blockIdx.x & 1, (int)blockIdx.x >> 1, a.poles, asm_);
     return;
   }
-  const int blk = (int)blockIdx.x - 1, strip = blk % a.strips;
+  const int blk = (int)blockIdx.x - 2 * a.poles, strip = blk % a.strips;
   const int R0 = kAOwn * strip - 1;  // rows R0 .. R0+63, owned: R0+2 .. R0+61
   for (int p = threadIdx.x; p < 64; p += 32 * kAWarps) {
     // weights of the face above row R0+p

@@ -708,10 +708,11 @@ static int diffusion_stage(hipft_gpu *h, const double *x, const double *ykm2, co
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cfg.gridDim = stage_grid(h, 32, 8 * kDCols);
-  cfg.gridDim.y += 2;  // the pole rows' blocks
+  const int prows = pole_grid_rows(h->npm - 2, cfg.gridDim.x);
+  cfg.gridDim.y += prows;
   cfg.blockDim = dim3(32, 8);
   CK(h, cudaLaunchKernelEx(&cfg, k_diffusion_stage<MODE>, h->M, h->DC, x, ykm2, u0, dty0, out, out2, h->bc_diff_n,
-                           h->bc_diff_s, sc));
+                           h->bc_diff_s, sc, prows));
   LAUNCHED(h);
   return HIPFT_OK;
 }
@@ -768,12 +769,14 @@ static cudaError_t launch_adv_stage(const hipft_gpu *h, cudaStream_t s, unsigned
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cfg.gridDim = dim3((unsigned)((h->ntm + 31) / 32), 2 + (unsigned)((h->npm - 2 + 7) / 8), nz);
+    cfg.gridDim = dim3((unsigned)((h->ntm + 31) / 32), (unsigned)((h->npm - 2 + 7) / 8), nz);
+    const int prows = pole_grid_rows(h->npm - 2, cfg.gridDim.x);
+    cfg.gridDim.y += prows;
     cfg.blockDim = dim3(33, 9);  // (TJ+1) x (TK+1) threads for a 32 x 8 tile
     return cudaLaunchKernelEx(&cfg, k_adv_upwind<32, 8>, h->M, h->FL, x, f0, out, h->bc_flow_n, h->bc_flow_s, cb,
-                              rlist, rdt);
+                              rlist, rdt, prows);
   }
-  AdvArgs a{x, f0, out, cb, rlist, rdt, 0, 0, h->bc_flow_n, h->bc_flow_s};
+  AdvArgs a{x, f0, out, cb, rlist, rdt, 0, 0, h->bc_flow_n, h->bc_flow_s, adv_pole_blocks(h->npm - 2, (int)nz)};
   const int n2 = h->npm - 2;
   a.strips = (h->ntm - 1 + kAOwn - 1) / kAOwn;  // rows up to ntm-1
   a.cols = adv_cols(n2, a.strips, (int)nz, kABlocks * kAWarps * h->num_sms);
@@ -785,7 +788,7 @@ static cudaError_t launch_adv_stage(const hipft_gpu *h, cudaStream_t s, unsigned
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cfg.gridDim = dim3((unsigned)(1 + a.strips * ((nch + kAWarps - 1) / kAWarps)), nz);
+  cfg.gridDim = dim3((unsigned)(2 * a.poles + a.strips * ((nch + kAWarps - 1) / kAWarps)), nz);
   cfg.blockDim = dim3(32 * kAWarps);
   cfg.dynamicSmemBytes = adv_smem(h->FL.flow2d);
   const bool wide = std::max(h->plane, h->FL.vplane) >= (int64_t)1 << 29;
