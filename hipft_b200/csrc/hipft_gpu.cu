@@ -181,6 +181,7 @@ struct hipft_gpu {
   bool g_stats_valid = true;        // g_last read back since the last launch
   hipft_allreduce_cb red_cb = nullptr;  // scalar all-reduce over ranks (plain-mode sharding)
   void *red_user = nullptr;
+  mutable std::vector<const void *> smem_set;  // kernels whose shared-memory limit this handle has set
   int *d_err = nullptr;   // set by kernels whose bounded waits gave up
   int num_sms = 148;
   unsigned long long *d_bits = nullptr;
@@ -549,6 +550,17 @@ static int64_t march_blocks(const hipft_gpu *h, int nreal) {
   return march_units(h->npm - 2, h->m_strips, march_columns(h, nreal), kMWarps) * nreal;
 }
 
+// Before a kernel's first launch by this handle: the most dynamic shared memory
+// that it takes.  The limit is the kernel's, not the handle's, so `bytes` is the
+// most that any grid takes; setting it loads the kernel, which is why a handle
+// does it for the kernels it runs and not for all it might (0.5 ms in a process).
+static cudaError_t smem_limit(const hipft_gpu *h, const void *kernel, size_t bytes) {
+  if (std::find(h->smem_set.begin(), h->smem_set.end(), kernel) != h->smem_set.end()) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) h->smem_set.push_back(kernel);
+  return e;
+}
+
 // k_sts_march for these arguments; byte offsets in 32 bits while a plane has them.
 typedef void (*MarchKernel)(Mesh, MarchArgs, PairTables);
 template <typename Off>
@@ -586,9 +598,9 @@ static cudaError_t launch_march(const hipft_gpu *h, cudaLaunchConfig_t cfg, cuda
   cfg.gridDim = dim3((unsigned)blocks);
   cfg.blockDim = dim3(32 * kMWarps);
   cfg.dynamicSmemBytes = kMSmem;
-  const bool table = a.rc || a.cols > kMGroup;
-  return cudaLaunchKernelEx(&cfg, march_kernel(table, a.o[0] || a.o[1], h->plane >= (int64_t)1 << 29), h->M, a,
-                            h->ptab);
+  const MarchKernel kernel = march_kernel(a.rc || a.cols > kMGroup, a.o[0] || a.o[1], h->plane >= (int64_t)1 << 29);
+  const cudaError_t e = smem_limit(h, (const void *)kernel, kMSmem);
+  return e == cudaSuccess ? cudaLaunchKernelEx(&cfg, kernel, h->M, a, h->ptab) : e;
 }
 
 // One pass on stream s.  after_pass: the launch before it on the stream is
@@ -642,7 +654,9 @@ static cudaError_t launch_pass(const hipft_gpu *h, cudaStream_t s, MarchArgs a, 
     cfg.gridDim = dim3((unsigned)(2 * a.nreal * nc + (mb + nc - 1) / nc * nc));
     cfg.blockDim = dim3((unsigned)poles_threads(n2));
     cfg.dynamicSmemBytes = pass_smem(poles_threads(n2));
-    return cudaLaunchKernelEx(&cfg, pass_kernel(a.rc || pc > kMGroup, a.o[0] || a.o[1]), h->M, a, h->ptab);
+    const MarchKernel kernel = pass_kernel(a.rc || pc > kMGroup, a.o[0] || a.o[1]);
+    const cudaError_t e = smem_limit(h, (const void *)kernel, pass_smem(kPassThreads));
+    return e == cudaSuccess ? cudaLaunchKernelEx(&cfg, kernel, h->M, a, h->ptab) : e;
   }
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = (unsigned)nc;
@@ -654,11 +668,13 @@ static cudaError_t launch_pass(const hipft_gpu *h, cudaStream_t s, MarchArgs a, 
   cfg.dynamicSmemBytes = poles_smem(poles_threads(n2));
   // a march that leaves places free does not compete with the pole strips' registers
   const bool roomy = blocks + 3 * (int64_t)cfg.gridDim.x <= (int64_t)kMBlocks * h->num_sms;
-  auto poles = poles_threads(n2) > kPMidThreads    ? k_sts_poles<kPMaxThreads, 1>
-               : poles_threads(n2) <= kPMinThreads ? k_sts_poles<kPMinThreads, 3>
-               : roomy                             ? k_sts_poles<kPMidThreads, 1>
-                                                   : k_sts_poles<kPMidThreads, 3>;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, poles, h->M, a, h->ptab);
+  const MarchKernel poles = poles_threads(n2) > kPMidThreads    ? k_sts_poles<kPMaxThreads, 1>
+                            : poles_threads(n2) <= kPMinThreads ? k_sts_poles<kPMinThreads, 3>
+                            : roomy                             ? k_sts_poles<kPMidThreads, 1>
+                                                                : k_sts_poles<kPMidThreads, 3>;
+  cudaError_t e = smem_limit(h, (const void *)poles, poles_smem(poles_most_threads(n2)));
+  if (e != cudaSuccess) return e;
+  e = cudaLaunchKernelEx(&cfg, poles, h->M, a, h->ptab);
   return e == cudaSuccess ? launch_march(h, cfg, attr, a, blocks, pdl) : e;
 }
 
@@ -792,7 +808,9 @@ static cudaError_t launch_adv_stage(const hipft_gpu *h, cudaStream_t s, unsigned
   cfg.blockDim = dim3(32 * kAWarps);
   cfg.dynamicSmemBytes = adv_smem(h->FL.flow2d);
   const bool wide = std::max(h->plane, h->FL.vplane) >= (int64_t)1 << 29;
-  return cudaLaunchKernelEx(&cfg, adv_kernel(h->FL.flow2d, cb.mode != 0, wide), h->M, h->FL, h->W, a);
+  const AdvKernel kernel = adv_kernel(h->FL.flow2d, cb.mode != 0, wide);
+  const cudaError_t e = smem_limit(h, (const void *)kernel, adv_smem(h->FL.flow2d));
+  return e == cudaSuccess ? cudaLaunchKernelEx(&cfg, kernel, h->M, h->FL, h->W, a) : e;
 }
 
 static int advection_stage(hipft_gpu *h, const double *x, const double *f0, double *out, AdvCombine cb,
@@ -884,48 +902,27 @@ extern "C" int hipft_gpu_create(const hipft_grid *g, const hipft_params *prm, hi
   if ((rc = dsmall(h, &h->d_rcount, (size_t)nr))) return bail(rc);
   if ((rc = dsmall(h, &h->d_err, 1))) return bail(rc);
   if (cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream) != cudaSuccess) return bail(HIPFT_ECUDA);
-  // the kernels this grid can reach (setting an attribute loads the kernel); the
-  // limit is the kernel's, not the handle's, so it is the most that any grid takes
-  const bool wide = h->plane >= (int64_t)1 << 29;
-  const bool vwide = wide || (int64_t)h->ldv * h->npm >= (int64_t)1 << 29;
-  bool smem_ok = true;
-  auto reserve = [&](const void *kernel, size_t bytes) {
-    smem_ok = smem_ok && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
-  };
-  if (prm->advance_flow && h->adv_space == 2)
-    for (int v = 0; v < 4; ++v) reserve((const void *)adv_kernel(v & 1, v & 2, vwide), adv_smem(v & 1));
-  if (prm->advance_diffusion && prm->diffusion_num_method >= 2 && !prm->diffusion_coef_grid && h->ntm >= kMMinRows) {
-    for (int v = 0; v < 4; ++v) reserve((const void *)march_kernel(v & 1, v & 2, wide), kMSmem);
-    if (npm - 2 >= kPassColumns && poles_threads(npm - 2) <= kPassThreads && !wide) {
-      const int pt = poles_threads(npm - 2);
-      for (int v = 0; v < 4; ++v) reserve((const void *)pass_kernel(v & 1, v & 2), pass_smem(kPassThreads));
-      cudaLaunchConfig_t cfg = {};
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = (unsigned)poles_ranks(npm - 2);
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.gridDim = dim3((unsigned)poles_ranks(npm - 2));
-      cfg.blockDim = dim3((unsigned)pt);
-      cfg.dynamicSmemBytes = pass_smem(pt);
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      if (!smem_ok || cudaOccupancyMaxActiveClusters(&h->pass_clusters, pass_kernel(true, true), &cfg) != cudaSuccess)
-        h->pass_clusters = 0;
-    }
-    if (!poles_by_column(h)) {
-      // no dynamic shared memory
-    } else if (poles_threads(npm - 2) > kPMidThreads) {
-      reserve((const void *)k_sts_poles<kPMaxThreads, 1>, poles_smem(kPMaxThreads));
-    } else if (poles_threads(npm - 2) <= kPMinThreads) {
-      reserve((const void *)k_sts_poles<kPMinThreads, 3>, poles_smem(kPMinThreads));
-    } else {
-      reserve((const void *)k_sts_poles<kPMidThreads, 1>, poles_smem(kPMidThreads));
-      reserve((const void *)k_sts_poles<kPMidThreads, 3>, poles_smem(kPMidThreads));
+  if (prm->advance_diffusion && prm->diffusion_num_method >= 2 && !prm->diffusion_coef_grid && poles_by_column(h) &&
+      npm - 2 >= kPassColumns && poles_threads(npm - 2) <= kPassThreads && h->plane < (int64_t)1 << 29) {
+    const int pt = poles_threads(npm - 2);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)poles_ranks(npm - 2);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)poles_ranks(npm - 2));
+    cfg.blockDim = dim3((unsigned)pt);
+    cfg.dynamicSmemBytes = pass_smem(pt);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const MarchKernel kernel = pass_kernel(true, false);  // all four take two blocks per SM
+    if (smem_limit(h, (const void *)kernel, pass_smem(kPassThreads)) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&h->pass_clusters, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      h->pass_clusters = 0;
     }
   }
-  if (!smem_ok)
-    return bail(fail(h, HIPFT_ECUDA, "cannot reserve shared memory for the RKG2 passes"));
   if (cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess || h->num_sms < 1)
     h->num_sms = 148;
   if (cudaMemsetAsync(h->d_rcount, 0, sizeof(unsigned int) * nr, h->stream) != cudaSuccess) return bail(HIPFT_ECUDA);
@@ -3149,7 +3146,10 @@ static int adj_pass(hipft_gpu *h, AdjPassArgs a, int ns, bool after_pass) {
   cfg.gridDim = dim3((unsigned)(2 * h->nr * nc));
   cfg.blockDim = dim3((unsigned)poles_threads(n2));
   cfg.dynamicSmemBytes = adj_poles_smem(ns, poles_threads(n2));
-  CK(h, cudaLaunchKernelEx(&cfg, adj_poles_kernel(ns, poles_threads(n2)), h->M, a, h->ptab));
+  const AdjPassKernel poles = adj_poles_kernel(ns, poles_threads(n2));
+  const int most = std::max(kPMidThreads, poles_most_threads(n2));
+  CK(h, smem_limit(h, (const void *)poles, adj_poles_smem(ns, most)));
+  CK(h, cudaLaunchKernelEx(&cfg, poles, h->M, a, h->ptab));
   LAUNCHED(h);
   const int nch = (n2 + a.cols - 1) / a.cols;
   attr[0].val.programmaticStreamSerializationAllowed = ws_pdl() ? 1 : 0;
@@ -3157,7 +3157,9 @@ static int adj_pass(hipft_gpu *h, AdjPassArgs a, int ns, bool after_pass) {
   cfg.gridDim = dim3((unsigned)((int64_t)a.strips * ((nch + kJWarps - 1) / kJWarps) * h->nr));
   cfg.blockDim = dim3(32 * kJWarps);
   cfg.dynamicSmemBytes = adj_march_smem(ns);
-  CK(h, cudaLaunchKernelEx(&cfg, adj_march_kernel(ns, h->plane >= (int64_t)1 << 29), h->M, a, h->ptab));
+  const AdjPassKernel march = adj_march_kernel(ns, h->plane >= (int64_t)1 << 29);
+  CK(h, smem_limit(h, (const void *)march, adj_march_smem(ns)));
+  CK(h, cudaLaunchKernelEx(&cfg, march, h->M, a, h->ptab));
   LAUNCHED(h);
   return HIPFT_OK;
 }
@@ -3183,13 +3185,6 @@ static int adj_ensure(hipft_gpu *h) {
     const int sms = std::max(h->num_sms - 2 * h->nr * poles_ranks(n2), h->num_sms / 2);
     h->j_cols = adj_cols(n2, h->j_strips, h->nr, kJWarps * kJBlocks * sms);
     const int per_r = h->j_strips * ((n2 + h->j_cols - 1) / h->j_cols) + 2 * poles_ranks(n2);
-    for (int ns = 2; ns <= kMS; ns += 2) {
-      CK(h, cudaFuncSetAttribute(adj_march_kernel(ns, h->plane >= (int64_t)1 << 29),
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adj_march_smem(ns)));
-      const int pt = poles_threads(n2);
-      CK(h, cudaFuncSetAttribute(adj_poles_kernel(ns, pt), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)adj_poles_smem(ns, pt > kPMidThreads ? kPMaxThreads : kPMidThreads)));
-    }
     TRY(small(&h->d_jpart, (size_t)per_r * h->nr));
     h->jpart_per_r = per_r;
   }

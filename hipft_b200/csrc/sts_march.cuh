@@ -525,6 +525,10 @@ __host__ __device__ inline int poles_threads(int n2) {
   const int nc = poles_ranks(n2);
   return ((n2 + nc - 1) / nc + 2 * kMS + 31) / 32 * 32;
 }
+inline int poles_most_threads(int n2) {  // of the k_sts_poles that the grid takes
+  const int t = poles_threads(n2);
+  return t > kPMidThreads ? kPMaxThreads : t <= kPMinThreads ? kPMinThreads : kPMidThreads;
+}
 __host__ __device__ inline int poles_stride(int threads) { return threads + 2; }  // 2 mod 32: no bank conflicts
 constexpr int kPSmemRows = kPRows + 3 * (kPRows - 1);  // Y_{k-1}, Y_{k-2}, u0, dty0
 __host__ __device__ inline size_t poles_smem(int threads) {
