@@ -2820,9 +2820,21 @@ extern "C" int hipft_gpu_info(const hipft_gpu *h, hipft_info *info) {
   return HIPFT_OK;
 }
 
+// "ws-quad" stands for passes of four stages by independent warps (k_sts_march).
 extern "C" int hipft_gpu_describe(hipft_gpu *h, char *buf, size_t len) {
   if (!h || !buf || !len) return HIPFT_EINVAL;
-  std::snprintf(buf, len, "schedule=%s; RKG2 kernel: ws-quad (four stages per pass)", h->ragged ? "ragged" : "shared");
+  const char *k = "none";
+  if (h->P.advance_diffusion) {
+    MarchArgs a{};
+    a.nreal = h->nr;
+    if (h->P.diffusion_num_method == 1) k = "explicit Euler steps";
+    else if (h->DC.grid) k = "one stage per launch (k_diffusion_stage)";
+    else if (h->ntm < kMMinRows) k = "four stages per pass, all rows as pole rows (k_sts_whole)";
+    else if (!poles_by_column(h)) k = "ws-quad (four stages per pass): k_sts_march, pole strips stage by stage (k_sts_poles_any)";
+    else if (pass_columns(h, a) && !h->graph_on) k = "ws-quad (four stages per pass): k_sts_march and pole strips in one launch";
+    else k = "ws-quad (four stages per pass): k_sts_march, pole strips beside it (k_sts_poles)";
+  }
+  std::snprintf(buf, len, "schedule=%s; diffusion kernels: %s", h->ragged ? "ragged" : "shared", k);
   return HIPFT_OK;
 }
 

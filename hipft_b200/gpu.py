@@ -453,7 +453,7 @@ class HipftGPU:
         return n.value, ms.value
 
     def describe(self) -> str:
-        """Schedule and the RKG2 kernel."""
+        """Schedule and the kernels of the diffusion step."""
         buf = ctypes.create_string_buffer(256)
         self._ck(self.L.hipft_gpu_describe(self.h, buf, 256), "describe")
         return buf.value.decode()
