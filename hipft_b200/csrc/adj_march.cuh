@@ -129,6 +129,8 @@ __global__ void __launch_bounds__(32 * kJWarps, kJBlocks) k_adj_march(Mesh m, Ad
     }
   };
   for (int t = lane; t < left + kMGroup - 1; t += 32) cp_async16(smem_addr(tab) + 16u * t, pt_col + c0 - NS + t);
+  // what the pass before wrote: it has ended, since k_adj_poles, launched directly
+  // before this grid, triggers it only behind its own wait for that pass
   fetch(sring);
   fetch(sring + kSlot);
   fetch(sring + 2 * kSlot);

@@ -30,7 +30,7 @@ __host__ __device__ constexpr size_t adv_smem(bool flow2d) {
 // form rounds as the reference's); big collects their high words: while those
 // are below kBigE (2^100), and eps and the linear weights lie in
 // weno_consts_ok's range, every operand, reciprocal and quotient is a normal
-// double and the face equals weno_face's bit for bit.
+// double and the face equals weno_face's bit for bit (but for quot_nr's exception).
 constexpr unsigned kBigE = (1023u + 100u) << 20;
 struct FaceW {
   double a0, mc1, mc0, cp1, a1, cp0, pt, mct, mt, cpt, e1, e0;

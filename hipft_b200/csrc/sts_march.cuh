@@ -395,7 +395,11 @@ __global__ void __launch_bounds__(MERGED ? kPassThreads : 32 * kMWarps, MERGED ?
   // the column table's entries of the chunk, with the first columns' copies
   double *tab = msm + nw * kMRing + warp * kMTab;
   for (int t = lane; t < left + kMGroup - 1; t += 32) cp_async16(smem_addr(tab) + 16u * t, pt_col + c0 - kMS + t);
-  if (MERGED) pdl_wait();  // the pass before
+  // What the pass before wrote.  A merged pass waits for that pass here.  Two
+  // launches: the strips' blocks trigger this grid only behind their own wait for
+  // the pass before, so it has ended; that holds while the strips' launch comes
+  // directly before this one and their trigger behind their wait.
+  if (MERGED) pdl_wait();
   fetch(sring);
   fetch(sring + kSlot);
   fetch(sring + 2 * kSlot);
