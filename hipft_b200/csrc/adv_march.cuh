@@ -109,16 +109,16 @@ struct AdvArgs {
   const double *rdt;
   int strips, cols;       // theta strips, phi columns per warp
   double bcn, bcs;        // pole factors
-  int poles;              // blocks per pole row (adv_pole_blocks)
+  int poles, share;       // blocks per pole row (adv_pole_blocks) and their columns
 };
 
 // The pole rows 1 and ntm of a realization's stage, whose value needs the ring
 // sum of the upwind fluxes next to them over all phi columns (src/hipft.f90:
-// 7902-7915): `nb` blocks per pole, each of which adds up the whole ring, as 256
+// 7902-7915): a.poles blocks per pole, each of which adds up the whole ring, as 256
 // threads (two per thread here) and a tree over them do, and writes its share of
 // the row.  Bound by latency and, on wide grids, by the sectors one SM can take
 // in: one block for both poles, a column's loads behind the store of the one
-// before, held a stage of 64x8192 up for 63 us (now 36) and of 16x2048 for 19 (now
+// before, held a stage of 64x8192 up for 63 us (now 38) and of 16x2048 for 19 (now
 // 10).  A block per kAPole columns is where the share's time and the
 // sum's meet.  Large batches, whose marches fill the GPU, have one block per pole
 // (16x2048 x 32: 395 us with two, 380 with one).
@@ -127,7 +127,7 @@ inline int adv_pole_blocks(int n2, int nreal) {  // per pole
   return std::min((n2 + kAPole - 1) / kAPole, std::max(1, kDPoleMax / nreal));
 }
 __device__ __forceinline__ void adv_pole_row(const Mesh &m, const Flow &fl, const AdvArgs &a, int i0, bool south,
-                                             int block, int nb, double *sh) {
+                                             int block, double *sh) {
   const int i = i0 + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t ld = m.ldt, p0 = (int64_t)i0 * m.plane + (south ? m.ntm - 1 : 0);
   const int jv = south ? m.nt - 1 : 2;
@@ -135,7 +135,7 @@ __device__ __forceinline__ void adv_pole_row(const Mesh &m, const Flow &fl, cons
   for (int v = 0; v < 2; ++v) {
     double f = 0.0;
     const double *c = a.x + p0;
-#pragma unroll 8
+#pragma unroll 4
     for (int k = 2 + (int)threadIdx.x + 128 * v; k <= m.npm - 1; k += 256) {
       const double xp = c[(int64_t)(k - 1) * ld], xn = c[(int64_t)(k - 1) * ld + (south ? -1 : 1)];
       const double ft = upwind_flux(vt_at(m, fl, jv, k, i), fl.upwind, south ? xp : xn, south ? xn : xp);
@@ -152,9 +152,9 @@ __device__ __forceinline__ void adv_pole_row(const Mesh &m, const Flow &fl, cons
   f = __shfl_sync(0xffffffffu, f, 0);
   const double ax = south ? -f * a.bcs : f * a.bcn;
   const double C = a.rdt ? a.cb.C * a.rdt[i0] : a.cb.C;
-  const int per = (m.npm - 2 + nb - 1) / nb, k1 = min(1 + per * (block + 1), m.npm - 1);
-  constexpr int G = 8;  // columns per turn, their loads all under way at once
-  for (int k0 = 2 + per * block + (int)threadIdx.x; k0 <= k1; k0 += 128 * G) {
+  const int k1 = min(1 + a.share * (block + 1), m.npm - 1);
+  constexpr int G = 4;  // columns per turn, their loads all under way at once
+  for (int k0 = 2 + a.share * block + (int)threadIdx.x; k0 <= k1; k0 += 128 * G) {
     double xv[G], fv[G];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Fl
   }
   if ((int)blockIdx.x < 2 * a.poles) {
     pdl_wait();
-    adv_pole_row(m, fl, a, i, blockIdx.x & 1, (int)blockIdx.x >> 1, a.poles, asm_);
+    adv_pole_row(m, fl, a, i, blockIdx.x & 1, (int)blockIdx.x >> 1, asm_);
     return;
   }
   const int blk = (int)blockIdx.x - 2 * a.poles, strip = blk % a.strips;

@@ -792,8 +792,9 @@ static cudaError_t launch_adv_stage(const hipft_gpu *h, cudaStream_t s, unsigned
     return cudaLaunchKernelEx(&cfg, k_adv_upwind<32, 8>, h->M, h->FL, x, f0, out, h->bc_flow_n, h->bc_flow_s, cb,
                               rlist, rdt, prows);
   }
-  AdvArgs a{x, f0, out, cb, rlist, rdt, 0, 0, h->bc_flow_n, h->bc_flow_s, adv_pole_blocks(h->npm - 2, (int)nz)};
+  AdvArgs a{x, f0, out, cb, rlist, rdt, 0, 0, h->bc_flow_n, h->bc_flow_s, adv_pole_blocks(h->npm - 2, (int)nz), 0};
   const int n2 = h->npm - 2;
+  a.share = (n2 + a.poles - 1) / a.poles;
   a.strips = (h->ntm - 1 + kAOwn - 1) / kAOwn;  // rows up to ntm-1
   a.cols = adv_cols(n2, a.strips, (int)nz, kABlocks * kAWarps * h->num_sms);
   const int nch = (n2 + a.cols - 1) / a.cols;
