@@ -325,6 +325,13 @@ static int dsmall(hipft_gpu *h, T **p, size_t n) {
   return HIPFT_OK;
 }
 
+// An array made on first use; one that an earlier call got before it ran out of
+// memory is kept.
+template <typename T>
+static int once(hipft_gpu *h, T **p, size_t n) {
+  return *p ? HIPFT_OK : dsmall(h, p, n);
+}
+
 // Fields that live as long as the handle, several per allocation while they
 // are small (at most 256 MB each, as the tape's chunks); those that an earlier
 // call got before it ran out of memory are kept.
@@ -450,6 +457,7 @@ static int ensure_part(hipft_gpu *h, size_t n) {
     h->allocs.erase(std::remove(h->allocs.begin(), h->allocs.end(), (void *)h->d_part), h->allocs.end());
   }
   h->d_part = nullptr;
+  h->part_cap = 0;
   TRY(dalloc(h, &h->d_part, n));
   h->part_cap = n;
   return HIPFT_OK;
@@ -1258,10 +1266,8 @@ extern "C" int hipft_gpu_set_flow_from_files(hipft_gpu *h, const double *vt_pt, 
     for (int j = 1; j <= nt; ++j) { T(j, 1) = T(j, npm - 1); T(j, npm) = T(j, 2); }
     for (int j = 1; j <= ntm; ++j) { P(j, 1) = P(j, np - 1); P(j, np) = P(j, 2); }
   }
-  if (!h->d_vtf) {
-    TRY(dalloc(h, &h->d_vtf, vt.size()));
-    TRY(dalloc(h, &h->d_vpf, vp.size()));
-  }
+  TRY(once(h, &h->d_vtf, vt.size()));
+  TRY(once(h, &h->d_vpf, vp.size()));
   TRY(upload(h, h->d_vtf, vt));
   TRY(upload(h, h->d_vpf, vp));
   CK(h, cudaStreamSynchronize(h->stream));  // the host staging vectors go out of scope
@@ -1276,8 +1282,8 @@ extern "C" int hipft_gpu_update_flow(hipft_gpu *h, int *updated) {
   if (updated) *updated = 0;
   if (!(h->have_flow || h->have_file_flow) || !h->flow_needs_updating) return HIPFT_OK;
   CK(h, cudaSetDevice(h->dev));
-  h->flow_needs_updating = false;
   int nt = h->nt, ntm = h->ntm, nr = h->nr, npm = h->npm;
+  bool again = false;  // the flow changes before every step
   std::vector<double> vt1, vp1;
   analytic_profiles(h, vt1, vp1);
   TRY(upload(h, h->d_vt1, vt1));
@@ -1303,12 +1309,12 @@ extern "C" int hipft_gpu_update_flow(hipft_gpu *h, int *updated) {
     TRY(upload(h, h->d_ap1, ap1));
     h->FL.flow2d = 0;
   } else {
-    if (!h->d_vt) {
+    if (!h->d_atten) {  // the last of them
       size_t n2 = (size_t)h->ldv * npm * nr;
-      TRY(dalloc(h, &h->d_vt, n2));
-      TRY(dalloc(h, &h->d_vp, n2));
-      TRY(dalloc(h, &h->d_at, n2));
-      TRY(dalloc(h, &h->d_ap, n2));
+      TRY(once(h, &h->d_vt, n2));
+      TRY(once(h, &h->d_vp, n2));
+      TRY(once(h, &h->d_at, n2));
+      TRY(once(h, &h->d_ap, n2));
       CK(h, cudaMemsetAsync(h->d_at, 0, n2 * sizeof(double), h->stream));
       CK(h, cudaMemsetAsync(h->d_ap, 0, n2 * sizeof(double), h->stream));
       // cos(p), sin(p), cos(ph), theta metrics (1-based), attenuation factors
@@ -1321,7 +1327,7 @@ extern "C" int hipft_gpu_update_flow(hipft_gpu *h, int *updated) {
       }
       for (int j = 1; j <= nt; ++j) { trig[3 * L + j] = h->cth[j]; trig[4 * L + j] = h->sth[j]; }
       for (int j = 1; j <= ntm; ++j) { trig[5 * L + j] = h->ct[j]; trig[6 * L + j] = h->st[j]; }
-      TRY(dalloc(h, &h->d_trig, trig.size()));
+      TRY(once(h, &h->d_trig, trig.size()));
       TRY(upload(h, h->d_trig, trig));
       std::vector<double> att(nr + 1, 0.0);
       for (int i = 1; i <= nr; ++i)
@@ -1371,14 +1377,14 @@ extern "C" int hipft_gpu_update_flow(hipft_gpu *h, int *updated) {
     dim3 blk(32, 8), grd((unsigned)((nt + 31) / 32), (unsigned)((npm + 7) / 8), (unsigned)nr);
     k_flow_build<<<grd, blk, 0, h->stream>>>(h->M, b, h->ldv, h->buf[h->cur], h->d_vt, h->d_vp);
     LAUNCHED(h);
+    again = h->have_file_flow;  // src/hipft.f90:3423
     if (h->fdef.flow_attenuate) {
       k_seam<<<dim3((unsigned)((nt + 127) / 128), (unsigned)nr), 128, 0, h->stream>>>(h->M, nt, h->ldv, h->d_vt);
       LAUNCHED(h);
       k_seam<<<dim3((unsigned)((ntm + 127) / 128), (unsigned)nr), 128, 0, h->stream>>>(h->M, ntm, h->ldv, h->d_vp);
       LAUNCHED(h);
-      h->flow_needs_updating = true;  // Br changes every step (src/hipft.f90:3514)
+      again = true;  // Br changes every step (src/hipft.f90:3514)
     }
-    if (h->have_file_flow) h->flow_needs_updating = true;  // src/hipft.f90:3423
     if (h->adv_space == 2) {
       dim3 g2((unsigned)((ntm + 31) / 32), (unsigned)((npm + 7) / 8), (unsigned)nr);
       k_lf_alpha<<<g2, blk, 0, h->stream>>>(h->M, h->ldv, h->d_vt, h->d_vp, h->d_at, h->d_ap);
@@ -1387,6 +1393,8 @@ extern "C" int hipft_gpu_update_flow(hipft_gpu *h, int *updated) {
     h->FL.vt = h->d_vt; h->FL.vp = h->d_vp; h->FL.at = h->d_at; h->FL.ap = h->d_ap;
     h->FL.flow2d = 1;
   }
+  // only now: a call that failed leaves the flow to be built
+  h->flow_needs_updating = again;
   h->r_dtmax_valid = false;
   if (updated) *updated = 1;
   return HIPFT_OK;
@@ -1712,6 +1720,7 @@ static int ragged_super_step(hipft_gpu *h, std::vector<int> act, const std::vect
       cudaFree(h->d_rcoef);
       h->allocs.erase(std::remove(h->allocs.begin(), h->allocs.end(), (void *)h->d_rcoef), h->allocs.end());
       h->d_rcoef = nullptr;
+      h->rcoef_passes = 0;
     }
     const size_t cap = (size_t)np + 32;
     TRY(dalloc(h, &h->d_rcoef, cap * nr * kMS));
@@ -1866,6 +1875,16 @@ static int ragged_advection_step(hipft_gpu *h, double dt) {
   return HIPFT_OK;
 }
 
+static int ragged_arrays(hipft_gpu *h) {
+  const size_t nr = (size_t)h->nr;
+  TRY(once(h, &h->d_rbits, 2 * nr));
+  TRY(once(h, &h->d_rlist_dif, nr));
+  TRY(once(h, &h->d_rlist_adv, nr));
+  TRY(once(h, &h->d_rlen, nr));
+  TRY(once(h, &h->d_rdt, nr));
+  return HIPFT_OK;
+}
+
 extern "C" int hipft_gpu_set_ragged(hipft_gpu *h, int on) {
   if (!h) return HIPFT_EINVAL;
   CK(h, cudaSetDevice(h->dev));
@@ -1879,13 +1898,7 @@ extern "C" int hipft_gpu_set_ragged(hipft_gpu *h, int on) {
   if (h->P.advance_flow && h->adv_time == 1)
     return fail(h, HIPFT_EINVAL, "set_ragged: needs SSPRK(3,3) or SSPRK(4,3) advection");
   const int nr = h->nr;
-  if (!h->d_rbits) {
-    TRY(dsmall(h, &h->d_rbits, 2 * (size_t)nr));
-    TRY(dsmall(h, &h->d_rlist_dif, (size_t)nr));
-    TRY(dsmall(h, &h->d_rlist_adv, (size_t)nr));
-    TRY(dsmall(h, &h->d_rlen, (size_t)nr));
-    TRY(dsmall(h, &h->d_rdt, (size_t)nr));
-  }
+  TRY(ragged_arrays(h));
   if (h->P.advance_diffusion) TRY(ragged_gershgorin(h));
   h->r_dtmax_valid = false;
   h->r_s.assign(nr, 0);
@@ -1899,13 +1912,7 @@ extern "C" int hipft_gpu_flow_dtmax_each(hipft_gpu *h, double *dtmax) {
   if (!h || !dtmax) return HIPFT_EINVAL;
   if (!h->P.advance_flow) return fail(h, HIPFT_ESTATE, "flow_dtmax_each: advance_flow is off");
   CK(h, cudaSetDevice(h->dev));
-  if (!h->d_rbits) {
-    TRY(dsmall(h, &h->d_rbits, 2 * (size_t)h->nr));
-    TRY(dsmall(h, &h->d_rlist_dif, (size_t)h->nr));
-    TRY(dsmall(h, &h->d_rlist_adv, (size_t)h->nr));
-    TRY(dsmall(h, &h->d_rlen, (size_t)h->nr));
-    TRY(dsmall(h, &h->d_rdt, (size_t)h->nr));
-  }
+  TRY(ragged_arrays(h));
   h->r_dtmax_valid = false;
   TRY(ragged_dtmax(h));
   std::copy(h->r_dtmax.begin(), h->r_dtmax.end(), dtmax);
@@ -1916,7 +1923,7 @@ extern "C" int hipft_gpu_ragged_schedule(hipft_gpu *h, int64_t *sts_s, int64_t *
                                          double *dt_euler) {
   if (!h) return HIPFT_EINVAL;
   if (!h->ragged) return fail(h, HIPFT_ESTATE, "ragged_schedule: the handle is not in ragged mode");
-  if (h->graph_on && h->GA.st) {
+  if (h->graph_on && h->GA.nr) {
     // the device's record of the last graph-run step
     const int nr = h->nr;
     std::vector<long long> s(nr);
@@ -2022,25 +2029,25 @@ static void dfree(hipft_gpu *h, T *&p) {
 static int graph_alloc(hipft_gpu *h, int passcap) {
   GArrays &g = h->GA;
   const size_t nr = (size_t)h->nr;
-  if (!g.st) {
+  if (!g.nr) {  // set last
     double *de = nullptr, *dm = nullptr;
-    TRY(dsmall(h, &g.st, 1));
-    TRY(dsmall(h, &g.ts, nr));
-    TRY(dsmall(h, &g.d, nr));
+    TRY(once(h, &g.st, 1));
+    TRY(once(h, &g.ts, nr));
+    TRY(once(h, &g.d, nr));
     TRY(dsmall(h, &de, nr));
     TRY(dsmall(h, &dm, nr));
-    TRY(dsmall(h, &g.rdt, nr));
-    TRY(dsmall(h, &g.act, nr));
-    TRY(dsmall(h, &g.fin, nr));
-    TRY(dsmall(h, &g.rl_ptl, nr));
-    TRY(dsmall(h, &g.rl_dif, nr));
-    TRY(dsmall(h, &g.rl_adv, nr));
-    TRY(dsmall(h, &g.rl_adv_all, nr));
-    TRY(dsmall(h, &g.nsub_i, nr));
-    TRY(dsmall(h, &g.cycles_i, nr));
-    TRY(dsmall(h, &g.s_i, nr));
-    TRY(dsmall(h, &g.s_last, nr));
-    TRY(dsmall(h, &g.bits, 2 * nr));
+    TRY(once(h, &g.rdt, nr));
+    TRY(once(h, &g.act, nr));
+    TRY(once(h, &g.fin, nr));
+    TRY(once(h, &g.rl_ptl, nr));
+    TRY(once(h, &g.rl_dif, nr));
+    TRY(once(h, &g.rl_adv, nr));
+    TRY(once(h, &g.rl_adv_all, nr));
+    TRY(once(h, &g.nsub_i, nr));
+    TRY(once(h, &g.cycles_i, nr));
+    TRY(once(h, &g.s_i, nr));
+    TRY(once(h, &g.s_last, nr));
+    TRY(once(h, &g.bits, 2 * nr));
     g.dt_euler = de;
     g.dtmax = dm;
     CK(h, cudaMemsetAsync(g.st, 0, sizeof(GState), h->stream));
@@ -2053,6 +2060,7 @@ static int graph_alloc(hipft_gpu *h, int passcap) {
     dfree(h, g.nactp);
     dfree(h, g.colsp);
     dfree(h, g.rc);
+    g.passcap = 0;
     TRY(dalloc(h, &g.nactp, (size_t)passcap));
     TRY(dalloc(h, &g.colsp, (size_t)passcap));
     TRY(dalloc(h, &g.rc, (size_t)passcap * nr * kMS));
@@ -2464,10 +2472,8 @@ extern "C" int hipft_gpu_set_rfe_frame(hipft_gpu *h, int slot, int model, const 
     TRY(dalloc(h, &h->d_rfe[slot], h->fieldn));
     CK(h, cudaMemsetAsync(h->d_rfe[slot], 0, h->fieldn * sizeof(double), h->stream));
   }
-  if (!h->d_rnd) {
-    TRY(dalloc(h, &h->d_rnd, (size_t)ntm * npm));
-    TRY(dalloc(h, &h->d_rfe_aux, (size_t)(nr + 1) + (ntm + 1)));
-  }
+  TRY(once(h, &h->d_rnd, (size_t)ntm * npm));
+  TRY(once(h, &h->d_rfe_aux, (size_t)(nr + 1) + (ntm + 1)));
   // da_ti per theta row, model 1 (src/hipft.f90:8840-8853)
   std::vector<double> aux((size_t)(nr + 1) + (ntm + 1), 0.0);
   for (int i = 1; i <= nr; ++i) aux[i] = uf[i - 1];
@@ -2530,11 +2536,9 @@ extern "C" int hipft_gpu_source_step(hipft_gpu *h, double dt) {
 static int da_args(hipft_gpu *h, const double *data3_pt, const hipft_da_opts *o, DAArgs &a) {
   int ntm = h->ntm, npm1 = h->npm1, nr = h->nr;
   size_t nd = (size_t)npm1 * ntm * 3;
-  if (!h->d_da) {
-    TRY(dalloc(h, &h->d_da, nd));
-    TRY(dsmall(h, &h->d_daopt, 3 * (size_t)(nr + 1)));
-    TRY(dsmall(h, &h->d_tidx, 2 * (size_t)(nr + 1)));
-  }
+  TRY(once(h, &h->d_da, nd));
+  TRY(once(h, &h->d_daopt, 3 * (size_t)(nr + 1)));
+  TRY(once(h, &h->d_tidx, 2 * (size_t)(nr + 1)));
   std::vector<double> opt(3 * (size_t)(nr + 1), 0.0);
   std::vector<int> tidx(2 * (size_t)(nr + 1), -1);
   for (int i = 1; i <= nr; ++i) {
@@ -2581,10 +2585,8 @@ static int da_args(hipft_gpu *h, const double *data3_pt, const hipft_da_opts *o,
       TRY(dalloc(h, &h->d_daw, np * slice));
       h->daw_cap = np * slice;
     }
-    if (!h->d_dawidx) {
-      TRY(dsmall(h, &h->d_dawidx, (size_t)nr + 1));
-      TRY(dsmall(h, &h->d_dawkey, 2 * (size_t)nr));
-    }
+    TRY(once(h, &h->d_dawidx, (size_t)nr + 1));
+    TRY(once(h, &h->d_dawkey, 2 * (size_t)nr));
     TRY(upload(h, h->d_dawkey, keys));
     CK(h, cudaMemcpyAsync(h->d_dawidx, widx.data(), widx.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
     CK(h, cudaMemcpyAsync(h->d_da + 2 * slice, data3_pt + 2 * slice, slice * sizeof(double), cudaMemcpyHostToDevice,
@@ -3181,15 +3183,14 @@ static int adj_pass(hipft_gpu *h, AdjPassArgs a, int ns, bool after_pass) {
 // on with what is missing, and nothing is ready before everything is there.
 static int adj_ensure(hipft_gpu *h) {
   if (h->adj_ready) return HIPFT_OK;
-  auto small = [&](double **p, size_t n) { return *p ? HIPFT_OK : dsmall(h, p, n); };
   TRY(dfields(h, h->adjw, (int)(sizeof(h->adjw) / sizeof(h->adjw[0]))));
   dim3 g = stage_grid(h, 32, 8);
   h->dpart_per_r = (int)(g.x * g.y);
-  TRY(small(&h->d_dpart, (size_t)h->dpart_per_r * h->nr));
+  TRY(once(h, &h->d_dpart, (size_t)h->dpart_per_r * h->nr));
   h->adj_nch = (h->npm - 2 + 255) / 256;
-  TRY(small(&h->d_gring, 2 * (size_t)h->nr * h->adj_nch));
-  TRY(small(&h->d_dpole, (size_t)h->nr * h->adj_nch));
-  for (auto &gp : h->d_gpart) TRY(small(&gp, 2 * (size_t)g.y * h->nr));
+  TRY(once(h, &h->d_gring, 2 * (size_t)h->nr * h->adj_nch));
+  TRY(once(h, &h->d_dpole, (size_t)h->nr * h->adj_nch));
+  for (auto &gp : h->d_gpart) TRY(once(h, &gp, 2 * (size_t)g.y * h->nr));
   const int n2 = h->npm - 2;
   if (h->ntm >= kJMinRows && poles_by_column(h)) {
     h->j_strips = adj_strips(h->ntm);
@@ -3198,7 +3199,7 @@ static int adj_ensure(hipft_gpu *h) {
     const int sms = std::max(h->num_sms - 2 * h->nr * poles_ranks(n2), h->num_sms / 2);
     h->j_cols = adj_cols(n2, h->j_strips, h->nr, kJWarps * kJBlocks * sms);
     const int per_r = h->j_strips * ((n2 + h->j_cols - 1) / h->j_cols) + 2 * poles_ranks(n2);
-    TRY(small(&h->d_jpart, (size_t)per_r * h->nr));
+    TRY(once(h, &h->d_jpart, (size_t)per_r * h->nr));
     h->jpart_per_r = per_r;
   }
   h->adj_ready = true;
