@@ -110,7 +110,7 @@ struct hipft_gpu {
   int cur = 0;
   bool field_set = false;
   // flows
-  bool have_flow = false, flow_needs_updating = false, flow2d = false;
+  bool have_flow = false, flow_needs_updating = false, flow2d = false, atten_set = false;
   bool have_file_flow = false;               // flows from files are the base of vt, vp
   double *d_vtf = nullptr, *d_vpf = nullptr;  // [npm][nt+1], [np][ntm+1]
   double *d_fterms = nullptr;                 // analytic terms applied over the file flow
@@ -1202,6 +1202,7 @@ extern "C" int hipft_gpu_set_flow(hipft_gpu *h, const hipft_flow_def *def) {
   take(h->f_p0, def->dr_p0, 0); take(h->f_p2, def->dr_p2, 0); take(h->f_p4, def->dr_p4, 0);
   take(h->f_p1, def->mf_p1, 0); take(h->f_p3, def->mf_p3, 0); take(h->f_p5, def->mf_p5, 0);
   take(h->f_att, def->flow_attenuate_values, 0);
+  h->atten_set = false;
   h->fdef = *def;
   h->have_flow = true;
   h->flow_needs_updating = true;
@@ -1329,11 +1330,14 @@ extern "C" int hipft_gpu_update_flow(hipft_gpu *h, int *updated) {
       for (int j = 1; j <= ntm; ++j) { trig[5 * L + j] = h->ct[j]; trig[6 * L + j] = h->st[j]; }
       TRY(once(h, &h->d_trig, trig.size()));
       TRY(upload(h, h->d_trig, trig));
+      TRY(dsmall(h, &h->d_atten, nr + 1));
+    }
+    if (h->have_flow && !h->atten_set) {
       std::vector<double> att(nr + 1, 0.0);
       for (int i = 1; i <= nr; ++i)
         att[i] = (h->f_att[i - 1] > 0.0) ? 1.0 / h->f_att[i - 1] : DBL_MAX;
-      TRY(dsmall(h, &h->d_atten, nr + 1));
       TRY(upload(h, h->d_atten, att));
+      h->atten_set = true;
     }
     if (h->fdef.flow_attenuate && !h->field_set) return fail(h, HIPFT_ESTATE, "update_flow: attenuation needs the field");
     size_t L = (size_t)std::max(npm, nt) + 2;
