@@ -100,6 +100,7 @@ constexpr int kMColsMax = 96;               // most columns per warp
 constexpr int kMTab = 2 * (kMColsMax + 2 * kMS + kMGroup);  // doubles of the column table per warp
 constexpr size_t kMSmem = ((size_t)kMWarps * (kMRing + kMTab) + kMCoef) * sizeof(double);
 static_assert(kMTab % 2 == 0, "16-byte aligned");
+constexpr int kMBrief = 20;                 // longest chunk beside which a narrow strip's place counts (march_cols)
 constexpr int kMMinRows = 2 * kMS;          // smallest ntm of the strip kernels (k_sts_whole below it)
 
 struct MarchArgs {
@@ -142,20 +143,44 @@ __host__ __device__ inline StageCoef sts_slot(int method, int64_t s, int64_t q, 
   return sts_combine(method, s, k, dtl);
 }
 
+// Blocks and threads per block of a pole strip's cluster (k_sts_poles).
+constexpr int kPMinThreads = 160, kPMidThreads = 288, kPMaxThreads = 544;
+__host__ __device__ inline int poles_ranks(int n2) {
+  const int per = n2 <= 8 * 152 ? 120 : 280;
+  const int c = (n2 + per - 1) / per;
+  return c > 8 ? 8 : c;
+}
+__host__ __device__ inline int poles_threads(int n2) {
+  const int nc = poles_ranks(n2);
+  return ((n2 + nc - 1) / nc + 2 * kMS + 31) / 32 * 32;
+}
+inline int poles_most_threads(int n2) {  // of the k_sts_poles that the grid takes
+  const int t = poles_threads(n2);
+  return t > kPMidThreads ? kPMaxThreads : t <= kPMinThreads ? kPMinThreads : kPMidThreads;
+}
+__host__ __device__ inline bool poles_brief(int n2) { return poles_threads(n2) <= kPMinThreads; }
+
 // Phi columns per warp, a multiple of kMGroup: the fewest full waves of
 // resident warps that keep the chunk at kMColsMax columns or less (a chunk
 // loads 2 kMS columns more than it owns, so longer chunks waste less; whole
 // waves leave no nearly empty one).  Blocks of k_sts_poles take the place of
 // blocks; a single wave leaves those places out, which would otherwise start a
-// second one.  A realization's chunks are dealt to its blocks' warps strip by
-// strip: whole blocks per strip left up to a third of the warps without one
-// (359x722 2.58 -> 2.20 us per stage, 256x512 2.30 -> 2.05).
+// second one.  Not where the strips' blocks are narrow (kPMinThreads) and the
+// chunks would be longer than kMBrief columns: such strips end well before the
+// march, and shorter chunks on all places save more than the blocks that wait for
+// a strip's place lose (a super-step, places left out and not: 512x1024 x 8 2841
+// and 2445 us, 359x722 x 9 939 and 840, 256x512 x 16 510 and 459; but 512x1024 x 3,
+// 20 columns or 16, 1053 and 1086, and 640x1280 x 4, strips of 288 threads, 3021
+// and 3609).
+// A realization's chunks are dealt to its blocks' warps strip by strip: whole
+// blocks per strip left up to a third of the warps without one (359x722 2.58 ->
+// 2.20 us per stage, 256x512 2.30 -> 2.05).
 // blocks of nw warps for the chunks of `cols` columns of one realization's strips
 __host__ __device__ inline int64_t march_units(int n2, int strips, int cols, int nw) {
   const int64_t nch = (n2 + cols - 1) / cols;
   return (strips * nch + nw - 1) / nw;
 }
-__host__ __device__ inline int march_cols(int n2, int strips, int nreal, int slots, int poles) {
+__host__ __device__ inline int march_cols_beside(int n2, int strips, int nreal, int slots, int poles) {
   const int64_t n = nreal > 0 ? nreal : 1;
   for (int64_t w = 1;; ++w) {
     int64_t free = w * slots;
@@ -166,6 +191,10 @@ __host__ __device__ inline int march_cols(int n2, int strips, int nreal, int slo
     const int64_t c = ((n2 + nch - 1) / nch + kMGroup - 1) / kMGroup * kMGroup;
     if (c <= kMColsMax) return (int)c;
   }
+}
+__host__ __device__ inline int march_cols(int n2, int strips, int nreal, int slots, int poles) {
+  const int c = march_cols_beside(n2, strips, nreal, slots, poles);
+  return poles_brief(n2) && c > kMBrief ? march_cols_beside(n2, strips, nreal, slots, 0) : c;
 }
 
 // The launch's realizations and coefficients.
@@ -307,7 +336,11 @@ __device__ __forceinline__ double2 pair_stage(double2 xl, double2 xc, double2 xr
 // the strips' and the next strips for the march's: 512x1024 3.16 -> 2.67 us per
 // stage, 359x722 2.80 -> 2.58.  Not on narrower grids (256x512 2.30 -> 2.43:
 // the strips share their SMs with the march from the start) nor where more than
-// 16 columns per warp make the march the longer part.
+// 16 columns per warp make the march the longer part.  One launch against two, a
+// super-step: 361x722 x 1 to 4 0.82 to 0.86, 512x1024 0.79 and x 2 0.98, 880x880
+// 0.86, 304x1216 0.98, 344x1150 x 2 0.84.  Where the march fills little more than
+// half of the places two launches would take a few percent less (440x880 and
+// 640x640 1.04, 210x900 1.06; 500x760 0.97, 140x700 x 3 0.90).
 constexpr int kPassThreads = 160;   // most threads per block then (kPMinThreads)
 constexpr int kPassColumns = 640;   // fewest phi columns
 constexpr int kPassColsMax = 16;    // most columns per warp
@@ -519,20 +552,6 @@ constexpr int kPRows = 2 * kMS;  // strip rows of Y_{k-1}
 // of one block of k_sts_march, so that it takes the place of one where the
 // march fills the GPU (160 threads keep all they need then); NB = 1 is faster by
 // itself.
-constexpr int kPMinThreads = 160, kPMidThreads = 288, kPMaxThreads = 544;
-__host__ __device__ inline int poles_ranks(int n2) {
-  const int per = n2 <= 8 * 152 ? 120 : 280;
-  const int c = (n2 + per - 1) / per;
-  return c > 8 ? 8 : c;
-}
-__host__ __device__ inline int poles_threads(int n2) {
-  const int nc = poles_ranks(n2);
-  return ((n2 + nc - 1) / nc + 2 * kMS + 31) / 32 * 32;
-}
-inline int poles_most_threads(int n2) {  // of the k_sts_poles that the grid takes
-  const int t = poles_threads(n2);
-  return t > kPMidThreads ? kPMaxThreads : t <= kPMinThreads ? kPMinThreads : kPMidThreads;
-}
 __host__ __device__ inline int poles_stride(int threads) { return threads + 2; }  // 2 mod 32: no bank conflicts
 constexpr int kPSmemRows = kPRows + 3 * (kPRows - 1);  // Y_{k-1}, Y_{k-2}, u0, dty0
 __host__ __device__ inline size_t poles_smem(int threads) {
