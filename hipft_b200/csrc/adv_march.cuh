@@ -109,69 +109,96 @@ struct AdvArgs {
   const double *rdt;
   int strips, cols;       // theta strips, phi columns per warp
   double bcn, bcs;        // pole factors
-  int poles, share;       // blocks per pole row (adv_pole_blocks) and their columns
+  int poles, pgrid;       // blocks per pole row (adv_pole_blocks), and for both rows
+  int share;              // columns of a block's share
 };
 
 // The pole rows 1 and ntm of a realization's stage, whose value needs the ring
 // sum of the upwind fluxes next to them over all phi columns (src/hipft.f90:
-// 7902-7915): a.poles blocks per pole, each of which adds up the whole ring, as 256
-// threads (two per thread here) and a tree over them do, and writes its share of
-// the row.  Bound by latency and, on wide grids, by the sectors one SM can take
-// in: one block for both poles, a column's loads behind the store of the one
-// before, held a stage of 64x8192 up for 63 us (now 38) and of 16x2048 for 19 (now
-// 10).  A block per kAPole columns is where the share's time and the
-// sum's meet.  Large batches, whose marches fill the GPU, have one block per pole
-// (16x2048 x 32: 395 us with two, 380 with one).
+// 7902-7915): NP rows of the block, from `south0` (0: row 1) on, each added up whole,
+// as 256 threads (two per thread here) and a tree over them do, and this block's
+// share of the columns written.  Bound by latency and, on wide grids, by the
+// sectors one SM can take in.  a.poles blocks per pole, a block per kAPole columns:
+// one block for both poles, a column's loads behind the store of the one before,
+// held a stage of 64x8192 up for 63 us (now 38) and of 16x2048 for 19 (now 10).
+// From kAPoleBoth realizations on, one block takes both rows where one per pole
+// would do: their number is what counts then (four stages, a block per row and one:
+// 20x40 x 100 48.8 and 44.6 us, 12x12 x 100 30.9 and 27.4, 16x1000 x 8 67.7 and 53.9,
+// 64x128 x 30 61.6 and 57.5; 33x600 x 8 39.6 and 41.1); with fewer its latency does
+// (180x360 20.6 and 22.7, 90x181 18.6 and 20.6).
+constexpr int kAPoleBoth = 8;
 constexpr int kAPole = 1024;
 inline int adv_pole_blocks(int n2, int nreal) {  // per pole
   return std::min((n2 + kAPole - 1) / kAPole, std::max(1, kDPoleMax / nreal));
 }
-__device__ __forceinline__ void adv_pole_row(const Mesh &m, const Flow &fl, const AdvArgs &a, int i0, bool south,
-                                             int block, double *sh) {
+inline int adv_pole_grid(int n2, int nreal) {  // for both rows
+  const int b = adv_pole_blocks(n2, nreal);
+  return b > 1 || nreal < kAPoleBoth ? 2 * b : 1;
+}
+template <int NP>
+__device__ __forceinline__ void adv_pole_rows(const Mesh &m, const Flow &fl, const AdvArgs &a, int i0, int south0,
+                                              int block, double *sh) {
   const int i = i0 + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t ld = m.ldt, p0 = (int64_t)i0 * m.plane + (south ? m.ntm - 1 : 0);
-  const int jv = south ? m.nt - 1 : 2;
+  const int64_t ld = m.ldt, p0 = (int64_t)i0 * m.plane;
 #pragma unroll
   for (int v = 0; v < 2; ++v) {
-    double f = 0.0;
-    const double *c = a.x + p0;
+    double f[NP] = {};
 #pragma unroll 4
     for (int k = 2 + (int)threadIdx.x + 128 * v; k <= m.npm - 1; k += 256) {
-      const double xp = c[(int64_t)(k - 1) * ld], xn = c[(int64_t)(k - 1) * ld + (south ? -1 : 1)];
-      const double ft = upwind_flux(vt_at(m, fl, jv, k, i), fl.upwind, south ? xp : xn, south ? xn : xp);
-      f = f + ft * m.dp[k];
+#pragma unroll
+      for (int s = 0; s < NP; ++s) {
+        const bool south = south0 + s != 0;
+        const double *c = a.x + p0 + (int64_t)(k - 1) * ld + (south ? m.ntm - 1 : 0);
+        const double xp = c[0], xn = c[south ? -1 : 1];
+        const double ft = upwind_flux(vt_at(m, fl, south ? m.nt - 1 : 2, k, i), fl.upwind, south ? xp : xn, south ? xn : xp);
+        f[s] = f[s] + ft * m.dp[k];
+      }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) f += __shfl_down_sync(0xffffffffu, f, o);
-    if (lane == 0) sh[4 * v + warp] = f;
+    for (int s = 0; s < NP; ++s) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) f[s] += __shfl_down_sync(0xffffffffu, f[s], o);
+      if (lane == 0) sh[8 * s + 4 * v + warp] = f[s];
+    }
   }
   __syncthreads();
-  double f = lane < 8 ? sh[lane] : 0.0;
+  double ax[NP];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) f += __shfl_down_sync(0xffffffffu, f, o);
-  f = __shfl_sync(0xffffffffu, f, 0);
-  const double ax = south ? -f * a.bcs : f * a.bcn;
+  for (int s = 0; s < NP; ++s) {
+    double f = lane < 8 ? sh[8 * s + lane] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) f += __shfl_down_sync(0xffffffffu, f, o);
+    f = __shfl_sync(0xffffffffu, f, 0);
+    ax[s] = south0 + s ? -f * a.bcs : f * a.bcn;
+  }
   const double C = a.rdt ? a.cb.C * a.rdt[i0] : a.cb.C;
   const int k1 = min(1 + a.share * (block + 1), m.npm - 1);
-  constexpr int G = 4;  // columns per turn, their loads all under way at once
+  constexpr int G = 4 / NP;  // columns per turn, their loads all under way at once
   for (int k0 = 2 + a.share * block + (int)threadIdx.x; k0 <= k1; k0 += 128 * G) {
-    double xv[G], fv[G];
+    double xv[G][NP], fv[G][NP];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       if (k0 + 128 * g > k1) break;
-      const int64_t p = p0 + (int64_t)(k0 + 128 * g - 1) * ld;
-      xv[g] = a.x[p];
-      fv[g] = a.cb.mode == 0 ? 0.0 : a.f0[p];
+#pragma unroll
+      for (int s = 0; s < NP; ++s) {
+        const int64_t p = p0 + (int64_t)(k0 + 128 * g - 1) * ld + (south0 + s ? m.ntm - 1 : 0);
+        xv[g][s] = a.x[p];
+        fv[g][s] = a.cb.mode == 0 ? 0.0 : a.f0[p];
+      }
     }
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       const int k = k0 + 128 * g;
       if (k > k1) break;
-      const int64_t p = p0 + (int64_t)(k - 1) * ld;
       const int64_t sm = k == 2 ? (m.npm - 2) * ld : k == m.npm - 1 ? -(m.npm - 2) * ld : 0;
-      const double y = a.cb.mode == 0 ? xv[g] - C * ax : a.cb.A * fv[g] + a.cb.B * xv[g] - C * ax;
-      a.out[p] = y;
-      if (sm) a.out[p + sm] = y;
+#pragma unroll
+      for (int s = 0; s < NP; ++s) {
+        const int64_t p = p0 + (int64_t)(k - 1) * ld + (south0 + s ? m.ntm - 1 : 0);
+        const double y =
+            a.cb.mode == 0 ? xv[g][s] - C * ax[s] : a.cb.A * fv[g][s] + a.cb.B * xv[g][s] - C * ax[s];
+        a.out[p] = y;
+        if (sm) a.out[p + sm] = y;
+      }
     }
   }
 }
@@ -194,8 +221,10 @@ __device__ __forceinline__ void adv_pole_row(const Mesh &m, const Flow &fl, cons
 // Bound: the FP64 pipe, about 95 instructions per face and 210 per cell, most
 // of them the eight divisions per face (two reciprocals shared).
 //
-// FLOW2D: 2-D velocities; MODE: the combine; Off: a byte offset in a plane.
-template <bool FLOW2D, int MODE, typename Off>
+// FLOW2D: 2-D velocities; MODE: the combine; Off: a byte offset in a plane; BOTH:
+// one block for both pole rows (adv_pole_grid; code for either in one kernel made
+// a stage of 512x1024 0.4 us longer).
+template <bool FLOW2D, int MODE, typename Off, bool BOTH>
 __global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Flow fl, Weno wn, AdvArgs a) {
   extern __shared__ __align__(16) double asm_[];
   pdl_trigger();
@@ -206,12 +235,12 @@ __global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Fl
     pdl_wait();
     return;
   }
-  if ((int)blockIdx.x < 2 * a.poles) {
+  if ((int)blockIdx.x < a.pgrid) {
     pdl_wait();
-    adv_pole_row(m, fl, a, i, blockIdx.x & 1, (int)blockIdx.x >> 1, asm_);
+    adv_pole_rows<BOTH ? 2 : 1>(m, fl, a, i, BOTH ? 0 : (int)blockIdx.x & 1, BOTH ? 0 : (int)blockIdx.x >> 1, asm_);
     return;
   }
-  const int blk = (int)blockIdx.x - 2 * a.poles, strip = blk % a.strips;
+  const int blk = (int)blockIdx.x - a.pgrid, strip = blk % a.strips;
   const int R0 = kAOwn * strip - 1;  // rows R0 .. R0+63, owned: R0+2 .. R0+61
   for (int p = threadIdx.x; p < 64; p += 32 * kAWarps) {
     // weights of the face above row R0+p

@@ -774,12 +774,14 @@ static int ptl_cells(hipft_gpu *h, const unsigned long long *absmax, unsigned lo
 // to a realization when non-null; rdt scales each realization's step), on
 // stream s.  chained: the launch before it on the stream is the stage before.
 typedef void (*AdvKernel)(Mesh, Flow, Weno, AdvArgs);
-static AdvKernel adv_kernel(bool flow2d, bool mode, bool wide) {
-  if (wide)
-    return flow2d ? (mode ? k_adv_march<true, 1, uint64_t> : k_adv_march<true, 0, uint64_t>)
-                  : (mode ? k_adv_march<false, 1, uint64_t> : k_adv_march<false, 0, uint64_t>);
-  return flow2d ? (mode ? k_adv_march<true, 1, uint32_t> : k_adv_march<true, 0, uint32_t>)
-                : (mode ? k_adv_march<false, 1, uint32_t> : k_adv_march<false, 0, uint32_t>);
+template <typename Off, bool BOTH>
+static AdvKernel adv_kernel(bool flow2d, bool mode) {
+  return flow2d ? (mode ? k_adv_march<true, 1, Off, BOTH> : k_adv_march<true, 0, Off, BOTH>)
+                : (mode ? k_adv_march<false, 1, Off, BOTH> : k_adv_march<false, 0, Off, BOTH>);
+}
+static AdvKernel adv_kernel(bool flow2d, bool mode, bool wide, bool both) {
+  if (wide) return adv_kernel<uint64_t, false>(flow2d, mode);
+  return both ? adv_kernel<uint32_t, true>(flow2d, mode) : adv_kernel<uint32_t, false>(flow2d, mode);
 }
 
 static cudaError_t launch_adv_stage(const hipft_gpu *h, cudaStream_t s, unsigned nz, const double *x, const double *f0,
@@ -800,8 +802,10 @@ static cudaError_t launch_adv_stage(const hipft_gpu *h, cudaStream_t s, unsigned
     return cudaLaunchKernelEx(&cfg, k_adv_upwind<32, 8>, h->M, h->FL, x, f0, out, h->bc_flow_n, h->bc_flow_s, cb,
                               rlist, rdt, prows);
   }
-  AdvArgs a{x, f0, out, cb, rlist, rdt, 0, 0, h->bc_flow_n, h->bc_flow_s, adv_pole_blocks(h->npm - 2, (int)nz), 0};
+  AdvArgs a{x, f0, out, cb, rlist, rdt, 0, 0, h->bc_flow_n, h->bc_flow_s, adv_pole_blocks(h->npm - 2, (int)nz), 0, 0};
   const int n2 = h->npm - 2;
+  const bool wide = std::max(h->plane, h->FL.vplane) >= (int64_t)1 << 29;
+  a.pgrid = wide ? 2 * a.poles : adv_pole_grid(n2, (int)nz);  // eight such planes do not fit the GPU
   a.share = (n2 + a.poles - 1) / a.poles;
   a.strips = (h->ntm - 1 + kAOwn - 1) / kAOwn;  // rows up to ntm-1
   a.cols = adv_cols(n2, a.strips, (int)nz, kABlocks * kAWarps * h->num_sms);
@@ -813,11 +817,10 @@ static cudaError_t launch_adv_stage(const hipft_gpu *h, cudaStream_t s, unsigned
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cfg.gridDim = dim3((unsigned)(2 * a.poles + a.strips * ((nch + kAWarps - 1) / kAWarps)), nz);
+  cfg.gridDim = dim3((unsigned)(a.pgrid + a.strips * ((nch + kAWarps - 1) / kAWarps)), nz);
   cfg.blockDim = dim3(32 * kAWarps);
   cfg.dynamicSmemBytes = adv_smem(h->FL.flow2d);
-  const bool wide = std::max(h->plane, h->FL.vplane) >= (int64_t)1 << 29;
-  const AdvKernel kernel = adv_kernel(h->FL.flow2d, cb.mode != 0, wide);
+  const AdvKernel kernel = adv_kernel(h->FL.flow2d, cb.mode != 0, wide, a.pgrid == 1);
   const cudaError_t e = smem_limit(h, (const void *)kernel, adv_smem(h->FL.flow2d));
   return e == cudaSuccess ? cudaLaunchKernelEx(&cfg, kernel, h->M, h->FL, h->W, a) : e;
 }
