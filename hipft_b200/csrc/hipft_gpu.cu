@@ -799,8 +799,9 @@ static cudaError_t launch_adv_stage(const hipft_gpu *h, cudaStream_t s, unsigned
     const int prows = pole_grid_rows(h->npm - 2, cfg.gridDim.x);
     cfg.gridDim.y += prows;
     cfg.blockDim = dim3(33, 9);  // (TJ+1) x (TK+1) threads for a 32 x 8 tile
-    return cudaLaunchKernelEx(&cfg, k_adv_upwind<32, 8>, h->M, h->FL, x, f0, out, h->bc_flow_n, h->bc_flow_s, cb,
-                              rlist, rdt, prows);
+    const bool many = (int64_t)cfg.gridDim.x * cfg.gridDim.y * nz > (int64_t)16 * h->num_sms;
+    return cudaLaunchKernelEx(&cfg, many ? k_adv_upwind<32, 8, 6> : k_adv_upwind<32, 8, 4>, h->M, h->FL, x, f0, out,
+                              h->bc_flow_n, h->bc_flow_s, cb, rlist, rdt, prows);
   }
   AdvArgs a{x, f0, out, cb, rlist, rdt, 0, 0, h->bc_flow_n, h->bc_flow_s, adv_pole_blocks(h->npm - 2, (int)nz), 0, 0};
   const int n2 = h->npm - 2;

@@ -1,15 +1,17 @@
-"""Advection stages whose pole rows' blocks follow from the number of realizations:
-a block per pole row (fewer than 8 realizations) or one for both, and two per row
-beyond 1024 columns.  The realizations of a batch bit for bit as one alone."""
+"""Advection stages whose pole rows' blocks, or whose blocks per SM, follow from the
+number of realizations: the realizations of a batch bit for bit as one alone.
+WENO3: a block per pole row (fewer than 8 realizations) or one for both, and two
+per row beyond 1024 columns; upwind: grids of up to 16 blocks per SM and larger."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 WENO = [(20, 40, 8), (12, 130, 9), (33, 257, 8), (16, 1000, 8), (12, 1030, 8), (12, 1030, 17), (70, 66, 30)]
+UPWIND = [(300, 500, 9), (64, 514, 40), (200, 1030, 5)]
 
 
-@pytest.mark.parametrize("nt,npp,nr,method", [g + (4,) for g in WENO])
+@pytest.mark.parametrize("nt,npp,nr,method", [g + (4,) for g in WENO] + [g + (2,) for g in UPWIND])
 def test_batch_equals_one_alone(nt, npp, nr, method):
     import hipft_b200 as H
     t, p = np.linspace(0.0, np.pi, nt), np.linspace(0.0, 2.0 * np.pi, npp + 1)
