@@ -8,18 +8,21 @@
 
 namespace hipft {
 
-constexpr int kAOwn = 60;     // theta rows a strip owns of the 64 it holds
+// theta rows a strip owns: a warp holds 64 rows of one strip, or 32 each of two chunks of it (hb = 2)
+__host__ __device__ constexpr int adv_own(int hb) { return 64 / hb - 4; }
 constexpr int kAWarps = 4;    // warps per block of k_adv_march
 constexpr int kABlocks = 2;   // its blocks per SM: with 168 registers (3) the four chains of a step were not kept apart
 constexpr int kASlots = 4;    // columns of its shared-memory ring
 constexpr int kAWt = 12;      // weights of a theta face
 constexpr int kAColsMax = 64;
 // doubles of a ring slot: x and f0, for 2-D flows vt, at, vp, vp of the next
-// column and ap, the phi face's row of Weno::ptab, and for 2-D flows the two
-// vt above the strip
-__host__ __device__ constexpr int adv_slot(bool flow2d) { return (flow2d ? 7 : 2) * 64 + kPhiTab + (flow2d ? 2 : 0); }
-__host__ __device__ constexpr size_t adv_smem(bool flow2d) {
-  return ((size_t)kAWt * 64 + (size_t)kAWarps * kASlots * adv_slot(flow2d)) * sizeof(double);
+// column and ap; then, per chunk of the warp, the phi face's row of Weno::ptab and
+// for 2-D flows the two vt above the strip
+__host__ __device__ constexpr int adv_fields(bool flow2d) { return (flow2d ? 7 : 2) * 64; }
+__host__ __device__ constexpr int adv_tab(bool flow2d) { return kPhiTab + (flow2d ? 2 : 0); }
+__host__ __device__ constexpr int adv_slot(bool flow2d, int hb) { return adv_fields(flow2d) + hb * adv_tab(flow2d); }
+__host__ __device__ constexpr size_t adv_smem(bool flow2d, int hb) {
+  return ((size_t)kAWt * 64 + (size_t)kAWarps * kASlots * adv_slot(flow2d, hb)) * sizeof(double);
 }
 
 // WENO3 face value (weno_face) with the divisions of quot_nr; the two
@@ -86,13 +89,21 @@ __device__ __noinline__ double face_ieee(double LNm2, double LNm1, double LN0, d
   return weno_face(LNm2, LNm1, LN0, LPm1, LP0, LPp1, W(1), W(2), W(3), W(5), W(6), W(7), W(8), W(9), W(10), W(11));
 }
 
-// Phi columns per warp: the fewest full waves of resident warps that keep the
+inline int adv_strips(int ntm, int hb) { return (ntm - 1 + adv_own(hb) - 1) / adv_own(hb); }  // rows up to ntm-1
+// Chunks per warp in batches whose pole rows take one block: two of 32 rows where
+// that is three quarters of the work of one of 64, or less, which holds for up to 29
+// rows and for 62 to 85.  Four stages with one and two: 12x200 x 200 295 and 160 us
+// (tiles of 32 rows before the marches 232), 29x60 x 300 157 and 98 (138), 20x40 x 500
+// 143 and 92 (133), 64x128 x 100 191 and 168 (172), 80x160 x 16 41 and 35; 130x260 x 20,
+// five sixths of the work, 105 and 107.
+inline int adv_halves(int ntm) { return 2 * adv_strips(ntm, 2) <= 3 * adv_strips(ntm, 1) ? 2 : 1; }
+// Phi columns per chunk: the fewest full waves of resident warps that keep the
 // chunk at kAColsMax columns or less, and kAColsMin at least.
 constexpr int kAColsMin = 2;
-inline int adv_cols(int n2, int strips, int nreal, int slots) {
+inline int adv_cols(int n2, int strips, int nreal, int slots, int hb) {
   const int64_t per = (int64_t)strips * nreal * kAWarps;
   for (int64_t w = 1;; ++w) {
-    const int64_t nch = w * slots / per * kAWarps;
+    const int64_t nch = w * slots / per * kAWarps * hb;
     if (nch < 1) continue;
     const int64_t c = (n2 + nch - 1) / nch;
     if (c <= kAColsMax) return (int)std::max<int64_t>(c, kAColsMin);
@@ -224,7 +235,8 @@ __device__ __forceinline__ void adv_pole_rows(const Mesh &m, const Flow &fl, con
 // FLOW2D: 2-D velocities; MODE: the combine; Off: a byte offset in a plane; BOTH:
 // one block for both pole rows (adv_pole_grid; code for either in one kernel made
 // a stage of 512x1024 0.4 us longer).
-template <bool FLOW2D, int MODE, typename Off, bool BOTH>
+// HB: chunks per warp (adv_halves), the second one by the upper half of its lanes.
+template <bool FLOW2D, int MODE, typename Off, bool BOTH, int HB>
 __global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Flow fl, Weno wn, AdvArgs a) {
   extern __shared__ __align__(16) double asm_[];
   pdl_trigger();
@@ -241,8 +253,10 @@ __global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Fl
     return;
   }
   const int blk = (int)blockIdx.x - a.pgrid, strip = blk % a.strips;
-  const int R0 = kAOwn * strip - 1;  // rows R0 .. R0+63, owned: R0+2 .. R0+61
-  for (int p = threadIdx.x; p < 64; p += 32 * kAWarps) {
+  constexpr int LH = 32 / HB, ROWS = 64 / HB;
+  const int hl = lane & (LH - 1), half = lane / LH;
+  const int R0 = adv_own(HB) * strip - 1;  // rows R0 .. R0+ROWS-1, owned: R0+2 .. R0+ROWS-3
+  for (int p = threadIdx.x; p < ROWS; p += 32 * kAWarps) {
     // weights of the face above row R0+p
     const int jw = min(max(R0 + p + 1, 2), nt - 1);
     const double v[kAWt] = {kOne + wn.mct[jw - 1], wn.mct[jw - 1], wn.mct[jw], wn.cpt[jw - 1], kOne + wn.cpt[jw],
@@ -252,19 +266,23 @@ __global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Fl
     for (int q = 0; q < kAWt; ++q) asm_[q * 64 + p] = v[q];
   }
   __syncthreads();
-  const int c0 = 2 + (blk / a.strips * kAWarps + warp) * a.cols, c1 = min(c0 + a.cols - 1, npm - 1);
-  if (c0 > npm - 1) {
+  const int cw = 2 + (blk / a.strips * kAWarps + warp) * HB * a.cols, n0 = min(a.cols, npm - cw);
+  if (cw > npm - 1) {
     pdl_wait();
     return;
   }
+  // this lane's chunk; a second one past the end has no columns: nothing is fetched or
+  // stored for it, and what its lanes compute is not looked at
+  const int ch = cw + half * a.cols;
+  const int c0 = ch > npm - 1 ? 2 : ch, c1 = ch > npm - 1 ? -4 : min(c0 + a.cols - 1, npm - 1);
   const double C = a.rdt ? a.cb.C * a.rdt[i] : a.cb.C;
-  const int r = R0 + 2 * lane;  // this lane's rows r, r+1
-  const bool own = lane >= 1 && lane <= 30;
+  const int r = R0 + 2 * hl;  // this lane's rows r, r+1
+  const bool own = hl >= 1 && hl <= LH - 2;
   const bool va = own && r >= 2 && r <= ntm - 1, vb = own && r + 1 <= ntm - 1;
   const bool tupA = r + 1 == 2 || r + 1 == ntm, tupB = r + 2 == 2 || r + 2 == ntm;
   const bool wup = __any_sync(0xffffffffu, tupA || tupB);
   const bool edge = __any_sync(0xffffffffu, va != vb);  // a pair stored by halves
-  const uint32_t swt = smem_addr(asm_) + 16u * lane;
+  const uint32_t swt = smem_addr(asm_) + 16u * hl;
   bool tok;  // the weights of this lane's WENO faces (3 .. nt-2) are in range
   {
     auto ok = [&](int q) {
@@ -273,7 +291,7 @@ __global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Fl
       return jf < 3 || jf > nt - 2 ||
              weno_consts_ok(w[6 * 64], w[7 * 64], w[8 * 64], w[9 * 64], w[10 * 64], w[11 * 64]);
     };
-    tok = ok(2 * lane) && ok(2 * lane + 1);
+    tok = ok(2 * hl) && ok(2 * hl + 1);
   }
   // divergence factors of rows r, r+1
   const int ra = min(max(r, 1), ntm), rb = min(max(r + 1, 1), ntm);
@@ -297,9 +315,10 @@ __global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Fl
   }
 
   // ring of input columns
-  constexpr uint32_t kF = 512, kSlot = adv_slot(FLOW2D) * 8;
-  double *rbase = asm_ + kAWt * 64 + warp * kASlots * adv_slot(FLOW2D);
-  const uint32_t sring = smem_addr(rbase) + 16u * lane, stab = smem_addr(rbase) + (FLOW2D ? 7 : 2) * kF;
+  constexpr uint32_t kF = 512, kSlot = adv_slot(FLOW2D, HB) * 8;
+  double *rbase = asm_ + kAWt * 64 + warp * kASlots * adv_slot(FLOW2D, HB);
+  double *rtab = rbase + adv_fields(FLOW2D) + half * adv_tab(FLOW2D);
+  const uint32_t sring = smem_addr(rbase) + 16u * lane, stab = smem_addr(rtab);
   const int64_t pb = (int64_t)i * m.plane, vb0 = (int64_t)i * fl.vplane;
   const Off ldb = (Off)m.ldt * 8, lvb = (Off)fl.ldv * 8;
   const Off rowb = (Off)min(max(r - 1, 0), m.ldt - 2) * 8, rowv = (Off)min(max(r - 1, 0), fl.ldv - 2) * 8;
@@ -312,23 +331,23 @@ __global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Fl
   auto fetch = [&]() {
     if (fe <= c1 + 2) {
       const uint32_t s = sring + fs * kSlot;
-      const int cw = fe < 1 ? fe + n2 : fe > npm - 1 ? fe - n2 : fe;  // the reference's periodic pad
-      cp_async16(s, gx + ((Off)(cw - 1) * ldb + rowb));
+      const int cp = fe < 1 ? fe + n2 : fe > npm - 1 ? fe - n2 : fe;  // the reference's periodic pad
+      cp_async16(s, gx + ((Off)(cp - 1) * ldb + rowb));
       if (FLOW2D) {
-        const Off o = (Off)(cw - 1) * lvb + rowv;
+        const Off o = (Off)(cp - 1) * lvb + rowv;
         cp_async16(s + 4 * kF, gvp + o);
         cp_async16(s + 5 * kF, gvp + (o + lvb));
         cp_async16(s + 6 * kF, gap + o);
       }
-      if (fe >= c0 + 1 && lane < kPhiTab / 2)
-        cp_async16(stab + fs * kSlot + 16u * lane, wn.ptab + (int64_t)(fe - 3) * kPhiTab + 2 * lane);
+      if (fe >= c0 + 1 && hl < kPhiTab / 2)
+        cp_async16(stab + fs * kSlot + 16u * hl, wn.ptab + (int64_t)(fe - 3) * kPhiTab + 2 * hl);
       if (fe >= c0 + 2) {
         if (MODE != 0) cp_async16(s + kF, gf + ((Off)(fe - 3) * ldb + rowb));
         if (FLOW2D) {
           const Off o = (Off)(fe - 3) * lvb + rowv;
           cp_async16(s + 2 * kF, gvt + o);
           cp_async16(s + 3 * kF, gat + o);
-          if (lane == 31) cp_async16(stab + fs * kSlot + kPhiTab * 8, gvt + (o + upv));
+          if (hl == LH - 1) cp_async16(stab + fs * kSlot + kPhiTab * 8, gvt + (o + upv));
         }
       }
     }
@@ -384,7 +403,7 @@ __global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Fl
         if (FLOW2D) {
           const double2 v = lds2(s + 2 * kF), al = lds2(s + 3 * kF);
           const double vn = __shfl_down_sync(0xffffffffu, v.x, 1);
-          const double v2 = lane == 31 ? lds2(st + kPhiTab * 8).x : vn;
+          const double v2 = hl == LH - 1 ? lds2(st + kPhiTab * 8).x : vn;
           ctn = make_double2(kHalf * (v.x + al.x), kHalf * (v.y + al.y));
           ctp = make_double2(kHalf * (v.y - al.x), kHalf * (v2 - al.y));
           vuA = v.y;
@@ -416,13 +435,13 @@ __global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Fl
         FA = up[2] + um[2];
         FB = up[3] + um[3];
       }
-      if (!(big < kBigE && tok && q5.x != 0.0)) {
-        const double *w = rbase + ((slot + kASlots - 1) & (kASlots - 1)) * adv_slot(FLOW2D) + (FLOW2D ? 7 : 2) * 64;
+      if (!(big < kBigE && tok && q5.x != 0.0) && (HB == 1 || e <= c1 + 2)) {
+        const double *w = rtab + ((slot + kASlots - 1) & (kASlots - 1)) * adv_slot(FLOW2D, HB);
         Fp.x = face_ieee(LN0.x, LN1.x, LN2.x, LP0.x, LP1.x, LP2.x, w, 1);
         Fp.y = face_ieee(LN0.y, LN1.y, LN2.y, LP0.y, LP1.y, LP2.y, w, 1);
         if (PH == 2) {
-          FA = face_ieee(LNm, LNt.x, LNt.y, LPt.x, LPt.y, LPp, asm_ + 2 * lane, 64);
-          FB = face_ieee(LNt.x, LNt.y, LNp, LPt.y, LPp, LPq, asm_ + 2 * lane + 1, 64);
+          FA = face_ieee(LNm, LNt.x, LNt.y, LPt.x, LPt.y, LPp, asm_ + 2 * hl, 64);
+          FB = face_ieee(LNt.x, LNt.y, LNp, LPt.y, LPp, LPq, asm_ + 2 * hl + 1, 64);
         }
       }
       if (PH == 2) {
@@ -438,15 +457,16 @@ __global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Fl
                                     : make_double2(a.cb.A * fc.x + a.cb.B * x0.x - C * aopx,
                                                    a.cb.A * fc.y + a.cb.B * x0.y - C * aopy);
         const int k = e - 2;
+        const bool sa = va && (HB == 1 || k <= c1), sb = vb && (HB == 1 || k <= c1);
         char *g = go + ((Off)(k - 1) * ldb + rowb);
-        st_if(va && vb, g, y);
+        st_if(sa && sb, g, y);
         if (edge || k == 2 || k == npm - 1) {
           const int64_t sm = k == 2 ? (int64_t)n2 * m.ldt : k == npm - 1 ? -(int64_t)n2 * m.ldt : 0;
           double *d = reinterpret_cast<double *>(g);
-          if (va) d[sm] = y.x;
-          if (vb) d[sm + 1] = y.y;
-          if (va && !vb) d[0] = y.x;
-          if (vb && !va) d[1] = y.y;
+          if (sa) d[sm] = y.x;
+          if (sb) d[sm + 1] = y.y;
+          if (sa && !sb) d[0] = y.x;
+          if (sb && !sa) d[1] = y.y;
         }
       }
     }
@@ -464,7 +484,7 @@ __global__ void __launch_bounds__(32 * kAWarps, kABlocks) k_adv_march(Mesh m, Fl
   for (int e = c0 - 2; e <= c0; ++e) step(e, IntC<0>{});
   step(c0 + 1, IntC<1>{});
 #pragma unroll 1
-  for (int e = c0 + 2; e <= c1 + 2; ++e) step(e, IntC<2>{});
+  for (int e = c0 + 2; e < c0 + 2 + n0; ++e) step(e, IntC<2>{});
   cp_async_wait<0>();
 }
 

@@ -774,14 +774,15 @@ static int ptl_cells(hipft_gpu *h, const unsigned long long *absmax, unsigned lo
 // to a realization when non-null; rdt scales each realization's step), on
 // stream s.  chained: the launch before it on the stream is the stage before.
 typedef void (*AdvKernel)(Mesh, Flow, Weno, AdvArgs);
-template <typename Off, bool BOTH>
+template <typename Off, bool BOTH, int HB>
 static AdvKernel adv_kernel(bool flow2d, bool mode) {
-  return flow2d ? (mode ? k_adv_march<true, 1, Off, BOTH> : k_adv_march<true, 0, Off, BOTH>)
-                : (mode ? k_adv_march<false, 1, Off, BOTH> : k_adv_march<false, 0, Off, BOTH>);
+  return flow2d ? (mode ? k_adv_march<true, 1, Off, BOTH, HB> : k_adv_march<true, 0, Off, BOTH, HB>)
+                : (mode ? k_adv_march<false, 1, Off, BOTH, HB> : k_adv_march<false, 0, Off, BOTH, HB>);
 }
-static AdvKernel adv_kernel(bool flow2d, bool mode, bool wide, bool both) {
-  if (wide) return adv_kernel<uint64_t, false>(flow2d, mode);
-  return both ? adv_kernel<uint32_t, true>(flow2d, mode) : adv_kernel<uint32_t, false>(flow2d, mode);
+static AdvKernel adv_kernel(bool flow2d, bool mode, bool wide, bool both, int hb) {
+  if (wide) return adv_kernel<uint64_t, false, 1>(flow2d, mode);
+  if (!both) return adv_kernel<uint32_t, false, 1>(flow2d, mode);
+  return hb == 2 ? adv_kernel<uint32_t, true, 2>(flow2d, mode) : adv_kernel<uint32_t, true, 1>(flow2d, mode);
 }
 
 static cudaError_t launch_adv_stage(const hipft_gpu *h, cudaStream_t s, unsigned nz, const double *x, const double *f0,
@@ -808,8 +809,10 @@ static cudaError_t launch_adv_stage(const hipft_gpu *h, cudaStream_t s, unsigned
   const bool wide = std::max(h->plane, h->FL.vplane) >= (int64_t)1 << 29;
   a.pgrid = wide ? 2 * a.poles : adv_pole_grid(n2, (int)nz);  // eight such planes do not fit the GPU
   a.share = (n2 + a.poles - 1) / a.poles;
-  a.strips = (h->ntm - 1 + kAOwn - 1) / kAOwn;  // rows up to ntm-1
-  a.cols = adv_cols(n2, a.strips, (int)nz, kABlocks * kAWarps * h->num_sms);
+  const int slots = kABlocks * kAWarps * h->num_sms;
+  const int hb = a.pgrid == 1 ? adv_halves(h->ntm) : 1;
+  a.strips = adv_strips(h->ntm, hb);
+  a.cols = adv_cols(n2, a.strips, (int)nz, slots, hb);
   const int nch = (n2 + a.cols - 1) / a.cols;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
@@ -818,11 +821,11 @@ static cudaError_t launch_adv_stage(const hipft_gpu *h, cudaStream_t s, unsigned
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cfg.gridDim = dim3((unsigned)(a.pgrid + a.strips * ((nch + kAWarps - 1) / kAWarps)), nz);
+  cfg.gridDim = dim3((unsigned)(a.pgrid + a.strips * ((nch + hb * kAWarps - 1) / (hb * kAWarps))), nz);
   cfg.blockDim = dim3(32 * kAWarps);
-  cfg.dynamicSmemBytes = adv_smem(h->FL.flow2d);
-  const AdvKernel kernel = adv_kernel(h->FL.flow2d, cb.mode != 0, wide, a.pgrid == 1);
-  const cudaError_t e = smem_limit(h, (const void *)kernel, adv_smem(h->FL.flow2d));
+  cfg.dynamicSmemBytes = adv_smem(h->FL.flow2d, hb);
+  const AdvKernel kernel = adv_kernel(h->FL.flow2d, cb.mode != 0, wide, a.pgrid == 1, hb);
+  const cudaError_t e = smem_limit(h, (const void *)kernel, adv_smem(h->FL.flow2d, hb));
   return e == cudaSuccess ? cudaLaunchKernelEx(&cfg, kernel, h->M, h->FL, h->W, a) : e;
 }
 
